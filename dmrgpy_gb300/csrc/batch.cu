@@ -242,6 +242,7 @@ struct LzPlan {
   const void* gtab[4];
   int gn[4];
   long long gtiles[4];
+  int gtile[4];
   int nprob;
   long long nmax;
   double tol;
@@ -255,7 +256,7 @@ int lz_steps(const LzPlan<T>& pl, int j0, int j1, unsigned long long* kernels, c
   unsigned long long before = dmrg_kernel_launches();
   for (int j = j0; j < j1; ++j) {
     for (int k = 0; k < 4; ++k)
-      DMRG_TRY(tgemm_grouped_launch<T>(pl.gtab[k], pl.gn[k], pl.gtiles[k], Sc<T>::one(), Sc<T>::zero(), s));
+      DMRG_TRY(tgemm_grouped_launch<T>(pl.gtab[k], pl.gn[k], pl.gtiles[k], pl.gtile[k], Sc<T>::one(), Sc<T>::zero(), s));
     lz_alpha_axpy_kernel<T><<<pl.nprob, kVecThreads, 0, s>>>(pl.seg, j);
     DMRG_CHECK_LAUNCH();
     if (j > 0) {
@@ -362,11 +363,11 @@ int batch_lanczos(int nprob, const dmrg_heff_t* ops, void* const* x, int kmax, d
       C[p] = st.C;
     }
     DMRG_TRY(tgemm_grouped_build(nprob, g.data(), A.data(), B.data(), C.data(), hdesc.data(), &pl.gn[k],
-                                 &pl.gtiles[k]));
+                                 &pl.gtiles[k], &pl.gtile[k]));
     DMRG_CUDA_TRY(cudaMemcpyAsync(base + L.gemm_tab[k], hdesc.data(), tgemm_grouped_desc_bytes(nprob),
                                   cudaMemcpyHostToDevice, s));
     pl.gtab[k] = base + L.gemm_tab[k];
-    key += ":" + std::to_string(pl.gn[k]) + "/" + std::to_string(pl.gtiles[k]);
+    key += ":" + std::to_string(pl.gn[k]) + "/" + std::to_string(pl.gtiles[k]) + "x" + std::to_string(pl.gtile[k]);
   }
   key += ":" + std::to_string(nmax);
   DMRG_CUDA_TRY(cudaMemcpyAsync(base + L.seg_tab, seg.data(), sizeof(LSeg<T>) * nprob, cudaMemcpyHostToDevice, s));

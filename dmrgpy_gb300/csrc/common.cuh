@@ -156,9 +156,9 @@ size_t tgemm_grouped_desc_bytes(int nprob);
 // the same split in two: the problem table built on the host (desc_host),
 // then -- after the caller has copied it to device memory -- the launch
 int tgemm_grouped_build(int nprob, const TGemm* g, const void* const* A, const void* const* B, void* const* C,
-                        void* desc_host, int* nout, long long* tiles_out);
+                        void* desc_host, int* nout, long long* tiles_out, int* tile_out);
 template <typename T>
-int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, T alpha, T beta, cudaStream_t stream);
+int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, int tile, T alpha, T beta, cudaStream_t stream);
 template <typename T>
 int tgemm_grouped(int nprob, const TGemm* g, const void* const* A, const void* const* B, void* const* C, T alpha,
                   T beta, void* desc_dev, void* desc_host, cudaStream_t stream);

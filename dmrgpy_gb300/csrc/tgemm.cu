@@ -1,9 +1,10 @@
 // Generic strided batched contraction C = alpha*opA(A)*opB(B) + beta*C in
-// FP64 / complex FP64 on the CUDA cores.  This is the FP64 reference path of
-// the sweep: on GB300 the FP64 pipe (about 1 TFLOP/s) is the bound, so the
-// kernel only has to keep that pipe fed: 64x64 output tile per 256-thread
-// CTA, 4x4 register block per thread, K staged through shared memory in
-// slices of 16.  Every logical dimension is an (outer, inner) index pair
+// FP64 / complex FP64 on the CUDA cores.  On GB300 the FP64 pipe (2 FMA per
+// clock per SM, about 1 TFLOP/s) is the bound, so the kernel only has to keep
+// every SM's pipe fed: K staged through shared memory in slices of 16, the
+// next slice held in registers while the current one is multiplied, and an
+// output tile of 64x64, 32x32 or 16x16 by the number of tiles a shape gives
+// (pick_tile).  Every logical dimension is an (outer, inner) index pair
 // with its own element strides, which expresses all the permuted views the
 // H_eff / environment / Gram contractions need without copies.
 #include "common.cuh"
@@ -12,10 +13,14 @@ namespace dmrg {
 
 namespace {
 
-constexpr int BM = 64;
-constexpr int BN = 64;
 constexpr int BK = 16;
-constexpr int NT = 256;
+
+// Output tile edge and its thread block: a thread owns TM x TN outputs.
+// 64x64: 256 threads, 4x4; 32x32: 128 threads, 4x2; 16x16: 128 threads, 2x1.
+template <int BT> struct Tile;
+template <> struct Tile<64> { static constexpr int NT = 256, TM = 4, TN = 4; };
+template <> struct Tile<32> { static constexpr int NT = 128, TM = 4, TN = 2; };
+template <> struct Tile<16> { static constexpr int NT = 128, TM = 2, TN = 1; };
 
 struct Dev {
   int B2, M, M2, N, N2, K, K2;
@@ -32,79 +37,90 @@ __device__ __forceinline__ long long off2(int i, int n2, long long s1, long long
   return (long long)q * s1 + (long long)r * s2;
 }
 
-// one BM x BN output tile (m0, n0) of batch entry bz
+// one BT x BT output tile (m0, n0) of batch entry bz
 // MIRROR: C is square with equal M and N layouts and the product is
 // symmetric (C = X^T X); an off-diagonal tile also writes its transpose.
-template <typename T, bool MIRROR = false>
+// Every output sums its products in ascending k whatever the tile, so the
+// choice of tile does not change a result.
+template <typename T, int BT, bool MIRROR = false>
 __device__ __forceinline__ void tgemm_tile(const Dev& d, T alpha, const T* __restrict__ A, const T* __restrict__ B,
                                            T beta, T* __restrict__ C, int m0, int n0, int bz) {
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Bs[BK][BN + 1];
+  constexpr int NT = Tile<BT>::NT, TM = Tile<BT>::TM, TN = Tile<BT>::TN;
+  constexpr int LD = (BT * BK) / NT;          // elements of one operand slice per thread
+  constexpr int SX = BT / TN, SY = BT / TM;   // thread grid: SX * SY == NT
+  __shared__ T As[BK][BT + 1];
+  __shared__ T Bs[BK][BT + 1];
   const int tid = threadIdx.x;
-  const int tx = tid & 15;
-  const int ty = tid >> 4;
+  const int tx = tid % SX;
+  const int ty = tid / SX;
   const int bq = bz / d.B2, br = bz - bq * d.B2;
   const T* Ab = A + (long long)bq * d.ab1 + (long long)br * d.ab2;
   const T* Bb = B + (long long)bq * d.bb1 + (long long)br * d.bb2;
   T* Cb = C + (long long)bq * d.cb1 + (long long)br * d.cb2;
 
-  T acc[4][4];
+  T acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = Sc<T>::zero();
+    for (int j = 0; j < TN; ++j) acc[i][j] = Sc<T>::zero();
 
+  // this thread's elements of a slice: the row (m or n) is the same in every
+  // slice, the k advances by BK
+  int am[LD], ak[LD], bn[LD], bk[LD];
+  const T* ap[LD];
+  const T* bp[LD];
+#pragma unroll
+  for (int r = 0; r < LD; ++r) {
+    const int e = tid + r * NT;
+    if (d.a_kfast) { ak[r] = e % BK; am[r] = e / BK; } else { am[r] = e % BT; ak[r] = e / BT; }
+    if (d.b_kfast) { bk[r] = e % BK; bn[r] = e / BK; } else { bn[r] = e % BT; bk[r] = e / BT; }
+    const int gm = m0 + am[r], gn = n0 + bn[r];
+    ap[r] = gm < d.M ? Ab + off2(gm, d.M2, d.am1, d.am2) : nullptr;
+    bp[r] = gn < d.N ? Bb + off2(gn, d.N2, d.bn1, d.bn2) : nullptr;
+  }
+  T ra[LD], rb[LD];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int r = 0; r < LD; ++r) {
+      const int ka = k0 + ak[r], kb = k0 + bk[r];
+      ra[r] = Sc<T>::zero();
+      rb[r] = Sc<T>::zero();
+      if (ap[r] && ka < d.K) ra[r] = cond_conj(ap[r][off2(ka, d.K2, d.ak1, d.ak2)], d.conjA);
+      if (bp[r] && kb < d.K) rb[r] = cond_conj(bp[r][off2(kb, d.K2, d.bk1, d.bk2)], d.conjB);
+    }
+  };
+  load(0);
   for (int k0 = 0; k0 < d.K; k0 += BK) {
 #pragma unroll
-    for (int r = 0; r < (BM * BK) / NT; ++r) {
-      int e = tid + r * NT;
-      int mm, kk;
-      if (d.a_kfast) { kk = e % BK; mm = e / BK; } else { mm = e % BM; kk = e / BM; }
-      int gm = m0 + mm, gk = k0 + kk;
-      T v = Sc<T>::zero();
-      if (gm < d.M && gk < d.K) {
-        v = Ab[off2(gm, d.M2, d.am1, d.am2) + off2(gk, d.K2, d.ak1, d.ak2)];
-        v = cond_conj(v, d.conjA);
-      }
-      As[kk][mm] = v;
-    }
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / NT; ++r) {
-      int e = tid + r * NT;
-      int nn, kk;
-      if (d.b_kfast) { kk = e % BK; nn = e / BK; } else { nn = e % BN; kk = e / BN; }
-      int gn = n0 + nn, gk = k0 + kk;
-      T v = Sc<T>::zero();
-      if (gn < d.N && gk < d.K) {
-        v = Bb[off2(gk, d.K2, d.bk1, d.bk2) + off2(gn, d.N2, d.bn1, d.bn2)];
-        v = cond_conj(v, d.conjB);
-      }
-      Bs[kk][nn] = v;
+    for (int r = 0; r < LD; ++r) {
+      As[ak[r]][am[r]] = ra[r];
+      Bs[bk[r]][bn[r]] = rb[r];
     }
     __syncthreads();
+    if (k0 + BK < d.K) load(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      T a[4], b[4];
+      T a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty + SY * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+      for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx + SX * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = Sc<T>::fma(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[i][j] = Sc<T>::fma(a[i], b[j], acc[i][j]);
     }
     __syncthreads();
   }
   const bool use_beta = (Sc<T>::re(beta) != 0.0) || (Sc<T>::im(beta) != 0.0);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int gm = m0 + ty + 16 * i;
+  for (int i = 0; i < TM; ++i) {
+    int gm = m0 + ty + SY * i;
     if (gm >= d.M) continue;
     long long om = off2(gm, d.M2, d.cm1, d.cm2);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int gn = n0 + tx + 16 * j;
+    for (int j = 0; j < TN; ++j) {
+      int gn = n0 + tx + SX * j;
       if (gn >= d.N) continue;
       long long o = om + off2(gn, d.N2, d.cn1, d.cn2);
       T v = Sc<T>::mul(alpha, acc[i][j]);
@@ -117,22 +133,23 @@ __device__ __forceinline__ void tgemm_tile(const Dev& d, T alpha, const T* __res
 
 // Symmetric product: only the tiles with tile row <= tile column, numbered
 // row by row over the upper triangle of a tiles x tiles grid.
-template <typename T>
-__global__ void __launch_bounds__(NT) tgemm_sym_kernel(Dev d, T alpha, const T* __restrict__ A,
-                                                       const T* __restrict__ B, T* __restrict__ C, int tiles) {
+template <typename T, int BT>
+__global__ void __launch_bounds__(Tile<BT>::NT) tgemm_sym_kernel(Dev d, T alpha, const T* __restrict__ A,
+                                                                 const T* __restrict__ B, T* __restrict__ C,
+                                                                 int tiles) {
   int rem = blockIdx.x, tm = 0;
   while (tm < tiles && rem >= tiles - tm) {
     rem -= tiles - tm;
     ++tm;
   }
   if (tm >= tiles) return;
-  tgemm_tile<T, true>(d, alpha, A, B, Sc<T>::zero(), C, tm * BM, (tm + rem) * BN, 0);
+  tgemm_tile<T, BT, true>(d, alpha, A, B, Sc<T>::zero(), C, tm * BT, (tm + rem) * BT, 0);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT) tgemm_kernel(Dev d, T alpha, const T* __restrict__ A,
-                                                   const T* __restrict__ B, T beta, T* __restrict__ C) {
-  tgemm_tile<T>(d, alpha, A, B, beta, C, blockIdx.x * BM, blockIdx.y * BN, blockIdx.z);
+template <typename T, int BT>
+__global__ void __launch_bounds__(Tile<BT>::NT) tgemm_kernel(Dev d, T alpha, const T* __restrict__ A,
+                                                             const T* __restrict__ B, T beta, T* __restrict__ C) {
+  tgemm_tile<T, BT>(d, alpha, A, B, beta, C, blockIdx.x * BT, blockIdx.y * BT, blockIdx.z);
 }
 
 // Grouped launch: problem p owns the flat tile range [start, start + tiles)
@@ -147,9 +164,9 @@ struct GProb {
   long long start;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(NT) tgemm_grouped_kernel(const GProb* __restrict__ probs, int nprob, T alpha,
-                                                           T beta) {
+template <typename T, int BT>
+__global__ void __launch_bounds__(Tile<BT>::NT) tgemm_grouped_kernel(const GProb* __restrict__ probs, int nprob,
+                                                                     T alpha, T beta) {
   const long long t = blockIdx.x;
   int lo = 0, hi = nprob - 1;
   while (lo < hi) {
@@ -162,8 +179,23 @@ __global__ void __launch_bounds__(NT) tgemm_grouped_kernel(const GProb* __restri
   const int bz = (int)(local / per_b);
   const int rem = (int)(local - (long long)bz * per_b);
   const int tm = rem % g.tiles_m, tn = rem / g.tiles_m;
-  tgemm_tile<T>(g.d, alpha, static_cast<const T*>(g.A), static_cast<const T*>(g.B), beta, static_cast<T*>(g.C),
-                tm * BM, tn * BN, bz);
+  tgemm_tile<T, BT>(g.d, alpha, static_cast<const T*>(g.A), static_cast<const T*>(g.B), beta, static_cast<T*>(g.C),
+                    tm * BT, tn * BT, bz);
+}
+
+inline long long tiles_of(long long n, int bt) { return (n + bt - 1) / bt; }
+
+// Tile edge for n64 / n32 / n16 tiles of the three sizes.  An SM's FP64 pipe
+// takes bt^2 * K / 2 clocks per tile however many CTAs share it, so the time
+// goes as (tiles on the fullest SM) * bt^2; the factors are the smaller
+// tiles' extra staging per product (measured per output on large shapes:
+// 32x32 5% and 16x16 20% above 64x64).
+inline int pick_tile(long long n64, long long n32, long long n16) {
+  const double c64 = (double)tiles_of(n64, 152) * 4096.0;
+  const double c32 = (double)tiles_of(n32, 152) * 1024.0 * 1.05;
+  const double c16 = (double)tiles_of(n16, 152) * 256.0 * 1.2;
+  if (c16 < c32 && c16 < c64) return 16;
+  return c32 < c64 ? 32 : 64;
 }
 
 // Dev from a TGemm; returns false when there is nothing to do, *err on bad input
@@ -206,9 +238,14 @@ int tgemm(const TGemm& g, T alpha, const T* A, const T* B, T beta, T* C, cudaStr
   int err = DMRG_OK;
   if (!make_dev(g, &d, &err)) return err;
   const long long nb = (long long)g.B.n1 * g.B.n2;
-  dim3 grid((d.M + BM - 1) / BM, (d.N + BN - 1) / BN, (unsigned)nb);
-  if (grid.y > 65535) return DMRG_ERR_ARG;
-  tgemm_kernel<T><<<grid, NT, 0, stream>>>(d, alpha, A, B, beta, C);
+  auto tiles = [&](int bt) { return nb * tiles_of(d.M, bt) * tiles_of(d.N, bt); };
+  int bt = pick_tile(tiles(64), tiles(32), tiles(16));
+  while (bt < 64 && tiles_of(d.N, bt) > 65535) bt *= 2;   // grid.y limit
+  dim3 grid((unsigned)tiles_of(d.M, bt), (unsigned)tiles_of(d.N, bt), (unsigned)nb);
+  if (tiles_of(d.N, 64) > 65535) return DMRG_ERR_ARG;
+  if (bt == 64) tgemm_kernel<T, 64><<<grid, Tile<64>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
+  else if (bt == 32) tgemm_kernel<T, 32><<<grid, Tile<32>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
+  else tgemm_kernel<T, 16><<<grid, Tile<16>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -223,10 +260,14 @@ int tgemm_gram(const double* X, long long ld, int m, int k, double* G, cudaStrea
   Dev d;
   int err = DMRG_OK;
   if (!make_dev(g, &d, &err)) return err;
-  const int tiles = (k + BM - 1) / BM;
-  const long long ntri = (long long)tiles * (tiles + 1) / 2;
-  if (ntri > 0x7fffffffLL) return DMRG_ERR_ARG;
-  tgemm_sym_kernel<double><<<(unsigned)ntri, NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
+  auto tri = [&](int bt) { const long long t = tiles_of(k, bt); return t * (t + 1) / 2; };
+  if (tri(64) > 0x7fffffffLL) return DMRG_ERR_ARG;
+  const int bt = pick_tile(tri(64), tri(32), tri(16));
+  const unsigned ntri = (unsigned)tri(bt);
+  const int tiles = (int)tiles_of(k, bt);
+  if (bt == 64) tgemm_sym_kernel<double, 64><<<ntri, Tile<64>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
+  else if (bt == 32) tgemm_sym_kernel<double, 32><<<ntri, Tile<32>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
+  else tgemm_sym_kernel<double, 16><<<ntri, Tile<16>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -234,10 +275,11 @@ int tgemm_gram(const double* X, long long ld, int m, int k, double* G, cudaStrea
 size_t tgemm_grouped_desc_bytes(int nprob) { return align_up(sizeof(GProb) * (size_t)(nprob > 0 ? nprob : 1)); }
 
 int tgemm_grouped_build(int nprob, const TGemm* g, const void* const* A, const void* const* B, void* const* C,
-                        void* desc_host, int* nout, long long* tiles_out) {
+                        void* desc_host, int* nout, long long* tiles_out, int* tile_out) {
   GProb* h = static_cast<GProb*>(desc_host);
   int n = 0;
-  long long tiles = 0;
+  long long total[3] = {0, 0, 0};
+  const int edge[3] = {64, 32, 16};
   for (int p = 0; p < nprob; ++p) {
     Dev d;
     int err = DMRG_OK;
@@ -250,21 +292,34 @@ int tgemm_grouped_build(int nprob, const TGemm* g, const void* const* A, const v
     q.A = A[p];
     q.B = B[p];
     q.C = C[p];
-    q.tiles_m = (d.M + BM - 1) / BM;
-    q.tiles_n = (d.N + BN - 1) / BN;
-    q.start = tiles;
-    tiles += (long long)g[p].B.n1 * g[p].B.n2 * q.tiles_m * q.tiles_n;
+    q.start = (long long)g[p].B.n1 * g[p].B.n2;   // batch entries, until the starts are known
+    for (int e = 0; e < 3; ++e) total[e] += q.start * tiles_of(d.M, edge[e]) * tiles_of(d.N, edge[e]);
   }
-  if (tiles > 0x7fffffffLL) return DMRG_ERR_ARG;
+  if (total[0] > 0x7fffffffLL) return DMRG_ERR_ARG;
+  const int bt = pick_tile(total[0], total[1], total[2]);
+  long long tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    GProb& q = h[i];
+    const long long nb = q.start;
+    q.tiles_m = (int)tiles_of(q.d.M, bt);
+    q.tiles_n = (int)tiles_of(q.d.N, bt);
+    q.start = tiles;
+    tiles += nb * q.tiles_m * q.tiles_n;
+  }
   *nout = n;
   *tiles_out = tiles;
+  *tile_out = bt;
   return DMRG_OK;
 }
 
 template <typename T>
-int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, T alpha, T beta, cudaStream_t stream) {
+int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, int tile, T alpha, T beta,
+                         cudaStream_t stream) {
   if (n == 0 || tiles == 0) return DMRG_OK;
-  tgemm_grouped_kernel<T><<<(unsigned)tiles, NT, 0, stream>>>(static_cast<const GProb*>(desc_dev), n, alpha, beta);
+  const GProb* p = static_cast<const GProb*>(desc_dev);
+  if (tile == 64) tgemm_grouped_kernel<T, 64><<<(unsigned)tiles, Tile<64>::NT, 0, stream>>>(p, n, alpha, beta);
+  else if (tile == 32) tgemm_grouped_kernel<T, 32><<<(unsigned)tiles, Tile<32>::NT, 0, stream>>>(p, n, alpha, beta);
+  else tgemm_grouped_kernel<T, 16><<<(unsigned)tiles, Tile<16>::NT, 0, stream>>>(p, n, alpha, beta);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -272,18 +327,18 @@ int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, T alpha, 
 template <typename T>
 int tgemm_grouped(int nprob, const TGemm* g, const void* const* A, const void* const* B, void* const* C, T alpha,
                   T beta, void* desc_dev, void* desc_host, cudaStream_t stream) {
-  int n = 0;
+  int n = 0, tile = 64;
   long long tiles = 0;
-  DMRG_TRY(tgemm_grouped_build(nprob, g, A, B, C, desc_host, &n, &tiles));
+  DMRG_TRY(tgemm_grouped_build(nprob, g, A, B, C, desc_host, &n, &tiles, &tile));
   if (n == 0) return DMRG_OK;
   DMRG_CUDA_TRY(cudaMemcpyAsync(desc_dev, desc_host, sizeof(GProb) * (size_t)n, cudaMemcpyHostToDevice, stream));
-  return tgemm_grouped_launch<T>(desc_dev, n, tiles, alpha, beta, stream);
+  return tgemm_grouped_launch<T>(desc_dev, n, tiles, tile, alpha, beta, stream);
 }
 
 template int tgemm<double>(const TGemm&, double, const double*, const double*, double, double*, cudaStream_t);
 template int tgemm<cplx>(const TGemm&, cplx, const cplx*, const cplx*, cplx, cplx*, cudaStream_t);
-template int tgemm_grouped_launch<double>(const void*, int, long long, double, double, cudaStream_t);
-template int tgemm_grouped_launch<cplx>(const void*, int, long long, cplx, cplx, cudaStream_t);
+template int tgemm_grouped_launch<double>(const void*, int, long long, int, double, double, cudaStream_t);
+template int tgemm_grouped_launch<cplx>(const void*, int, long long, int, cplx, cplx, cudaStream_t);
 template int tgemm_grouped<double>(int, const TGemm*, const void* const*, const void* const*, void* const*, double,
                                    double, void*, void*, cudaStream_t);
 template int tgemm_grouped<cplx>(int, const TGemm*, const void* const*, const void* const*, void* const*, cplx, cplx,
