@@ -7,7 +7,9 @@
 #include <cstring>
 #include <vector>
 
+#include "dgemm.cuh"
 #include "heff.cuh"
+#include "heff64.cuh"
 #include "tf32x3.cuh"
 
 #include <atomic>
@@ -45,17 +47,27 @@ long long heff_n(const dmrg_heff_t* o) {
 // ---- workspace of one H_eff application
 size_t heff_ws(const dmrg_heff_t* o) {
   if (o->precision == DMRG_PREC_TF32X3) return tf32x3_heff_workspace_bytes(*o);
+  return heff64_workspace_bytes(*o);
+}
+
+// The least an FP64 operator runs in: the contraction chain on the FP64 pipe
+// (two intermediates), for callers with a fixed scratch budget.
+size_t heff_lean_ws(const dmrg_heff_t* o) {
+  if (o->precision == DMRG_PREC_TF32X3) return heff_ws(o);
   size_t P, Q;
   if (o->dtype == DMRG_COMPLEX128) heff_fp64_elems<cplx>(*o, &P, &Q);
   else heff_fp64_elems<double>(*o, &P, &Q);
   return align_up(P * esize(o->dtype)) + align_up(Q * esize(o->dtype));
 }
 
+size_t heff_min_ws(const dmrg_heff_t* o) { return std::min(heff_ws(o), heff_lean_ws(o)); }
+
 // One-off preparation of an operator (split-TF32: operand splitting of L, R
-// and the two-site MPO), then heff_run per Krylov iteration.
+// and the two-site MPO; FP64: digits of L and R, the MPO's row lists), then
+// heff_run per Krylov iteration.  bytes: what the workspace holds.
 template <typename T>
-int heff_prepare(const dmrg_heff_t* o, void* work, cudaStream_t s) {
-  if (o->precision != DMRG_PREC_TF32X3) return DMRG_OK;
+int heff_prepare(const dmrg_heff_t* o, void* work, size_t bytes, cudaStream_t s) {
+  if (o->precision != DMRG_PREC_TF32X3) return bytes < heff_ws(o) ? DMRG_OK : heff64_prepare<T>(*o, work, s);
   if (o->dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
   return tf32x3_heff_prepare(*o, work, s);
 }
@@ -67,11 +79,12 @@ int heff_finish(const dmrg_heff_t* o, void* work, cudaStream_t s) {
 }
 
 template <typename T>
-int heff_run(const dmrg_heff_t* o, const T* x, T* y, void* work, cudaStream_t s) {
+int heff_run(const dmrg_heff_t* o, const T* x, T* y, void* work, size_t bytes, cudaStream_t s) {
   if (o->precision == DMRG_PREC_TF32X3) {
     if (o->dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
     return tf32x3_heff_apply_prepared(*o, reinterpret_cast<const double*>(x), reinterpret_cast<double*>(y), work, s);
   }
+  if (bytes >= heff_ws(o)) return heff64_run<T>(*o, x, y, work, s);
   size_t P, Q;
   heff_fp64_elems<T>(*o, &P, &Q);
   T* Pp = static_cast<T*>(work);
@@ -174,9 +187,10 @@ struct KrylovWs {
   double* part;   // multidot partials 2 * MULTIDOT_MAX_GRID * kcap
   double* red;    // reduction scratch: 8 + 2*RB
   void* hw;       // heff workspace
+  size_t hbytes;  // its size
 };
 
-size_t krylov_ws(const dmrg_heff_t* o, int kcap, KrylovWs* out, void* base) {
+size_t krylov_ws(const dmrg_heff_t* o, int kcap, bool lean, KrylovWs* out, void* base) {
   const size_t es = esize(o->dtype);
   const size_t n = (size_t)heff_n(o);
   char* p = static_cast<char*>(base);
@@ -193,7 +207,8 @@ size_t krylov_ws(const dmrg_heff_t* o, int kcap, KrylovWs* out, void* base) {
   w.sc = static_cast<double*>(take(16 * sizeof(double)));
   w.part = static_cast<double*>(take(2 * (size_t)MULTIDOT_MAX_GRID * kcap * sizeof(double)));
   w.red = static_cast<double*>(take((8 + 2 * 2 * 152) * sizeof(double)));
-  w.hw = take(heff_ws(o));
+  w.hbytes = lean ? heff_lean_ws(o) : heff_ws(o);
+  w.hw = take(w.hbytes);
   if (out) *out = w;
   return off;
 }
@@ -211,8 +226,8 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
   const int m = (int)std::min<long long>(niter, n);
   if (m < 1) return DMRG_ERR_ARG;
   KrylovWs ws;
-  size_t need = krylov_ws(o, m, &ws, work);
-  if (need > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (krylov_ws(o, m, false, &ws, work) > work_bytes && krylov_ws(o, m, true, &ws, work) > work_bytes)
+    return DMRG_ERR_WORKSPACE;
   T* Q = static_cast<T*>(ws.Q);
   T* w = static_cast<T*>(ws.w);
   T* h = static_cast<T*>(ws.hdev);
@@ -233,8 +248,8 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
     DMRG_TRY(vnorm<T>(x, n, nrm_d, ws.red, s));
   }
   DMRG_TRY(vscale_dev_inv<T>(Q, x, nrm_d, n, s));  // q0
-  DMRG_TRY(heff_prepare<T>(o, ws.hw, s));
-  DMRG_TRY(heff_run<T>(o, Q, w, ws.hw, s));
+  DMRG_TRY(heff_prepare<T>(o, ws.hw, ws.hbytes, s));
+  DMRG_TRY(heff_run<T>(o, Q, w, ws.hw, ws.hbytes, s));
   DMRG_TRY(vdot<T>(Q, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
   DMRG_TRY(vaxpy2<T>(w, Q, alpha_d, nullptr, nullptr, n, s));
   DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
@@ -252,7 +267,7 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
     T* qjm = Q + (long long)(j - 1) * n;
     DMRG_TRY(vscale_dev_inv<T>(qj, w, beta_d, n, s));
     DMRG_CUDA_TRY(cudaMemcpyAsync(bprev_d, beta_d, sizeof(double), cudaMemcpyDeviceToDevice, s));
-    DMRG_TRY(heff_run<T>(o, qj, w, ws.hw, s));
+    DMRG_TRY(heff_run<T>(o, qj, w, ws.hw, ws.hbytes, s));
     DMRG_TRY(vdot<T>(qj, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
     DMRG_TRY(vaxpy2<T>(w, qj, alpha_d, qjm, bprev_d, n, s));
     // full reorthogonalisation against q_0 .. q_{j-1}
@@ -292,8 +307,8 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
   if (m < 1) return DMRG_ERR_ARG;
   if (sizeof(T) == 8 && coeff.imag() != 0.0) return DMRG_ERR_UNSUPPORTED;
   KrylovWs ws;
-  size_t need = krylov_ws(o, m, &ws, work);
-  if (need > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (krylov_ws(o, m, false, &ws, work) > work_bytes && krylov_ws(o, m, true, &ws, work) > work_bytes)
+    return DMRG_ERR_WORKSPACE;
   T* Q = static_cast<T*>(ws.Q);
   T* w = static_cast<T*>(ws.w);
   T* h = static_cast<T*>(ws.hdev);
@@ -314,11 +329,11 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
     return DMRG_OK;
   }
   DMRG_TRY(vscale_dev_inv<T>(Q, x, nrm_d, n, s));
-  DMRG_TRY(heff_prepare<T>(o, ws.hw, s));
+  DMRG_TRY(heff_prepare<T>(o, ws.hw, ws.hbytes, s));
   std::vector<double> al, be;
   for (int it = 0; it < m; ++it) {
     T* qi = Q + (long long)it * n;
-    DMRG_TRY(heff_run<T>(o, qi, w, ws.hw, s));
+    DMRG_TRY(heff_run<T>(o, qi, w, ws.hw, ws.hbytes, s));
     DMRG_TRY(vdot<T>(qi, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
     DMRG_TRY(vaxpy2<T>(w, qi, alpha_d, it > 0 ? Q + (long long)(it - 1) * n : nullptr, it > 0 ? bprev_d : nullptr,
                        n, s));
@@ -485,43 +500,55 @@ size_t dmrg_heff_workspace_bytes(const dmrg_heff_t* op) {
 
 int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (heff_ws(op) > work_bytes || (!work && heff_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (op->dtype == DMRG_COMPLEX128) return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, s);
-  DMRG_TRY(heff_prepare<double>(op, work, s));
-  DMRG_TRY(heff_run<double>(op, static_cast<const double*>(x), static_cast<double*>(y), work, s));
+  if (op->dtype == DMRG_COMPLEX128) {
+    DMRG_TRY(heff_prepare<cplx>(op, work, work_bytes, s));
+    return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, work_bytes, s);
+  }
+  DMRG_TRY(heff_prepare<double>(op, work, work_bytes, s));
+  DMRG_TRY(heff_run<double>(op, static_cast<const double*>(x), static_cast<double*>(y), work, work_bytes, s));
   return heff_finish<double>(op, work, s);
 }
 
 int dmrg_heff_prepare(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (heff_ws(op) > work_bytes || (!work && heff_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (op->dtype == DMRG_COMPLEX128) return heff_prepare<cplx>(op, work, s);
-  return heff_prepare<double>(op, work, s);
+  if (op->dtype == DMRG_COMPLEX128) return heff_prepare<cplx>(op, work, work_bytes, s);
+  return heff_prepare<double>(op, work, work_bytes, s);
 }
 
 int dmrg_heff_apply_prepared(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes,
                              void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (heff_ws(op) > work_bytes || (!work && heff_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (op->dtype == DMRG_COMPLEX128) return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, s);
-  return heff_run<double>(op, static_cast<const double*>(x), static_cast<double*>(y), work, s);
+  if (op->dtype == DMRG_COMPLEX128)
+    return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, work_bytes, s);
+  return heff_run<double>(op, static_cast<const double*>(x), static_cast<double*>(y), work, work_bytes, s);
 }
 
 int dmrg_heff_status(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (heff_ws(op) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (heff_min_ws(op) > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   return heff_finish<double>(op, work, s);
 }
 
+// whether an operator runs in `bytes` of scratch (dmrg_heff_apply_noalloc)
+}  // extern "C"
+namespace dmrg {
+bool heff_fits(const dmrg_heff_t* op, size_t bytes) { return heff_lean_ws(op) <= bytes; }
+}  // namespace dmrg
+extern "C" {
+
 size_t dmrg_env_workspace_bytes(int dtype, int precision, int chil, int d, int chir, int wl, int wr) {
   if (precision == DMRG_PREC_TF32X3) return tf32x3_env_workspace_bytes(chil, d, chir, wl, wr);
-  size_t a = env_fp64_elems(0, chil, d, chir, wl, wr), b = env_fp64_elems(1, chil, d, chir, wl, wr);
-  return align_up((a > b ? a : b) * esize(dtype));
+  if (chil <= 0 || d <= 0 || chir <= 0 || wl <= 0 || wr <= 0) return 0;
+  return std::max(env64_workspace_bytes(0, dtype, chil, chir, chil, chir, d, wl, wr),
+                  env64_workspace_bytes(1, dtype, chil, chir, chil, chir, d, wl, wr));
 }
 
 static int env_common(int side, int dtype, int precision, int chil, int d, int chir, int wl, int wr, const void* E,
@@ -529,25 +556,18 @@ static int env_common(int side, int dtype, int precision, int chil, int d, int c
   if ((dtype != DMRG_REAL64 && dtype != DMRG_COMPLEX128) || chil <= 0 || chir <= 0 || d <= 0 || wl <= 0 || wr <= 0)
     return DMRG_ERR_ARG;
   if (!E || !W || !A || !Enew) return DMRG_ERR_ARG;
-  if (dmrg_env_workspace_bytes(dtype, precision, chil, d, chir, wl, wr) > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (precision == DMRG_PREC_TF32X3) {
+    if (dmrg_env_workspace_bytes(dtype, precision, chil, d, chir, wl, wr) > work_bytes) return DMRG_ERR_WORKSPACE;
     if (dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
     return tf32x3_env(side, chil, d, chir, wl, wr, static_cast<const double*>(E), static_cast<const double*>(W),
                       static_cast<const double*>(A), static_cast<double*>(Enew), work, s);
   }
-  if (dtype == DMRG_COMPLEX128) {
-    if (side == 0)
-      return env_left_fp64<cplx>(chil, d, chir, wl, wr, (const cplx*)E, (const cplx*)W, (const cplx*)A, (cplx*)Enew,
-                                 (cplx*)work, s);
-    return env_right_fp64<cplx>(chil, d, chir, wl, wr, (const cplx*)E, (const cplx*)W, (const cplx*)A, (cplx*)Enew,
-                                (cplx*)work, s);
-  }
-  if (side == 0)
-    return env_left_fp64<double>(chil, d, chir, wl, wr, (const double*)E, (const double*)W, (const double*)A,
-                                 (double*)Enew, (double*)work, s);
-  return env_right_fp64<double>(chil, d, chir, wl, wr, (const double*)E, (const double*)W, (const double*)A,
-                                (double*)Enew, (double*)work, s);
+  if (dtype == DMRG_COMPLEX128)
+    return env64<cplx>(side, chil, chir, chil, chir, d, wl, wr, (const cplx*)E, (const cplx*)W, (const cplx*)A,
+                       (const cplx*)A, (cplx*)Enew, work, work_bytes, s);
+  return env64<double>(side, chil, chir, chil, chir, d, wl, wr, (const double*)E, (const double*)W, (const double*)A,
+                       (const double*)A, (double*)Enew, work, work_bytes, s);
 }
 
 int dmrg_env_extend_left(int dtype, int precision, int chil, int d, int chir, int wl, int wr, const void* L,
@@ -563,7 +583,7 @@ int dmrg_env_extend_right(int dtype, int precision, int chil, int d, int chir, i
 size_t dmrg_lanczos_workspace_bytes(const dmrg_heff_t* op, int niter) {
   if (!heff_valid(op) || niter < 1) return 0;
   int kcap = (int)std::min<long long>(niter, heff_n(op));
-  return krylov_ws(op, kcap, nullptr, nullptr);
+  return krylov_ws(op, kcap, false, nullptr, nullptr);
 }
 
 int dmrg_lanczos_ground(const dmrg_heff_t* op, void* x, int niter, double tol, double* energy, int* iters, void* work,
@@ -610,14 +630,17 @@ int dmrg_svd_truncate(int dtype, int m, int n, const void* M, double cutoff, int
 
 size_t dmrg_gemm_workspace_bytes(int dtype, int precision, int m, int k, int n) {
   if (precision == DMRG_PREC_TF32X3) return tf32x3_gemm_workspace_bytes(m, k, n);
-  return 0;
+  const bool c = dtype == DMRG_COMPLEX128;
+  if (m <= 0 || k <= 0 || n <= 0 || !dg_pays(c, m, n, k, false)) return 0;
+  return dg_bytes(0, c, m, k) + dg_bytes(1, c, n, k);
 }
 
 int dmrg_gemm(int dtype, int precision, int m, int k, int n, const void* A, const void* B, void* C, void* work,
               size_t work_bytes, void* stream) {
   if (m <= 0 || k <= 0 || n <= 0 || !A || !B || !C) return DMRG_ERR_ARG;
   if (dtype != DMRG_REAL64 && dtype != DMRG_COMPLEX128) return DMRG_ERR_ARG;
-  if (dmrg_gemm_workspace_bytes(dtype, precision, m, k, n) > work_bytes) return DMRG_ERR_WORKSPACE;
+  const size_t need = dmrg_gemm_workspace_bytes(dtype, precision, m, k, n);
+  if (precision == DMRG_PREC_TF32X3 && need > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (precision == DMRG_PREC_TF32X3) {
     if (dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
@@ -629,6 +652,15 @@ int dmrg_gemm(int dtype, int precision, int m, int k, int n, const void* A, cons
   g.a_m = st(k); g.a_k = st(1);
   g.b_k = st(n); g.b_n = st(1);
   g.c_m = st(n); g.c_n = st(1);
+  // digit products where they pay and the caller's workspace holds them; the
+  // FP64 pipe needs no workspace
+  if (need > 0 && work && need <= work_bytes) {
+    if (dtype == DMRG_COMPLEX128)
+      return dg_product<cplx>(g, static_cast<const cplx*>(A), static_cast<const cplx*>(B), 1.0, 0,
+                              static_cast<cplx*>(C), work, s);
+    return dg_product<double>(g, static_cast<const double*>(A), static_cast<const double*>(B), 1.0, 0,
+                              static_cast<double*>(C), work, s);
+  }
   if (dtype == DMRG_COMPLEX128)
     return tgemm<cplx>(g, Sc<cplx>::one(), static_cast<const cplx*>(A), static_cast<const cplx*>(B), Sc<cplx>::zero(),
                        static_cast<cplx*>(C), s);

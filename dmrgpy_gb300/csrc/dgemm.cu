@@ -1,0 +1,813 @@
+// FP64 and complex FP64 matrix products on the tensor cores, by exact digit
+// products (an Ozaki-type splitting).
+//
+// Each row x of an operand (A: rows m, B: rows n, both along k) is scaled by
+// its own power of two, y = x 2^-e with |y| < 1, rounded once to the 64-bit
+// integer Q = rint(y 2^63) and cut into eight signed digits of base 2^8,
+//   Q = sum_{i=0..7} d_i 2^(56 - 8 i),  |d_i| <= 128,
+// each exact in FP16.  The product is summed by orders,
+//   P_o = sum_{i + j = o} sum_k a_i b_j,  o = 0 .. 7  (36 digit pairs),
+//   C = 2^(eA + eB) sum_o P_o 2^(-14 - 8 o).
+// Over 128 consecutive k every |P_o| <= (o + 1) 128 2^14 <= 2^24 (run_steps
+// lengthens this where the digits allow), so the tensor core's FP32
+// accumulator holds the integer exactly whatever its rounding.  The epilogue
+// adds the runs as integers in units of order 6 (P_6 + P_7 / 256 rounded once
+// per run) and rounds the 80-bit total once to FP64.  The errors are the
+// rounding of Q (2^-64 of the row's largest element), the digit pairs left
+// out (i + j > 7: together about 2^-64 of both rows' largest elements per
+// product), the run's last place (2^-63 of both rows' largest elements) and
+// that final rounding.  Rows of a sweep mix magnitudes (Schmidt-weighted
+// tensors; an environment's energy channel beside its small entries), which
+// a fixed point pays for and FP64 does not: with seven digits a chi = 1024
+// matvec erred by 4e-15 (28 pairs: 4e-14) where the FP64 sum errs by 2e-15,
+// with eight by less than the FP64 sum (tests/test_gpu_dgemm.py).
+//
+// Why: GB300's FP64 pipe does 2 FMA per clock per SM (1.06 TFLOP/s measured),
+// the FP16 tensor cores 4096; 36 digit products still leave a factor ~55.
+//
+// Complex operands are the real product of twice the rows and twice the k:
+// rows (re, im) of A against the interleaved k of B, (ar, -ai | ai, ar).
+//
+// Digit layout in device memory = the shared-memory image of a stage: per
+// row tile (R = 128 or 64 rows) and K step of 16, [kc 0..1][digit][row][8
+// FP16], the K-major no-swizzle core matrices (8 rows x 16 bytes) of tcgen05.
+// A stage is thus two contiguous bulk copies, and the B digits 0..7-i stacked
+// along N form one operand: a_i times all of them is one or two MMAs of
+// N <= 256 into the adjacent accumulators of orders i..7.
+//
+// GEMM kernel, persistent, one CTA per SM, output tiles of 128 x 64:
+//   warp 0    producer: cp.async.bulk of the A (32 KB) and B (16 KB) blocks
+//             of a K step into a ring of four stages;
+//   warp 1    TMEM allocation (512 columns: 8 orders x 64) and the single
+//             thread that issues 12 MMAs per K step;
+//   warps 2-9 epilogue: after every run the eight accumulators are read,
+//             converted to integers and added to the running sums (registers),
+//             two warps per TMEM lane quarter, 32 columns each.
+// All mbarrier waits are bounded; a wait that gives up makes the CTA write NaN.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <climits>
+
+#include "dgemm.cuh"
+#include "tcgen05.cuh"
+
+namespace dmrg {
+
+namespace {
+
+constexpr int ND = 8;                       // digits
+constexpr int NO = 8;                       // orders kept
+constexpr int TM = 128, TN = 64;            // output tile
+constexpr int KS = 16;                      // K step (one MMA)
+constexpr int RUN = 8;                      // K steps per accumulation run whatever the digits (128 k)
+constexpr int STAGES = 4;
+constexpr int A_BLK = 2 * ND * TM * 16;     // 32 KB
+constexpr int B_BLK = 2 * ND * TN * 16;     // 16 KB
+constexpr int ST_BYTES = A_BLK + B_BLK;
+constexpr int DG_SMEM = STAGES * ST_BYTES + 1024 + 256;
+constexpr int DG_THREADS = 320;
+// the 64-bit sums grow by up to 3 2^46 per k: at most 20480 k per launch
+constexpr int MAX_STEPS = 1280;
+constexpr int EXP_BAD = INT_MAX;            // row with a non-finite element
+
+// set by a wait that gave up; the kernel then writes NaN to its tiles
+__device__ int g_dg_timeout;
+
+__host__ __device__ constexpr int tile_rows(int side) { return side == 0 ? TM : TN; }
+
+inline long long up(long long x, long long a) { return (x + a - 1) / a; }
+
+struct SplitArgs {
+  const double* p;      // complex: interleaved
+  long long R, K;       // logical (real) rows and k
+  int R2, K2;           // inner extents, in elements
+  long long r1, r2, k1, k2;   // strides, in elements
+  int conj;
+  int kvec;             // 1: 8 consecutive k are 64 contiguous, 16-byte aligned bytes
+  long long steps;      // K steps
+};
+
+// |x| exponent field of a double's high word
+__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// Q = rint(x 2^(63 - e)) for a row whose largest exponent field is E
+// (E >= 1, e = E - 1022), |Q| < 2^63
+__device__ __forceinline__ long long fixed64(double x, int E) {
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
+  int ex = (int)((b >> 52) & 0x7ff);
+  unsigned long long m = b & 0xfffffffffffffull;
+  if (ex) m |= 0x10000000000000ull;
+  else ex = 1;
+  const int sh = E - ex;              // 0 .. 2045
+  unsigned long long q;
+  if (sh <= 10) q = m << (10 - sh);
+  else if (sh < 65) q = (m + (1ull << (sh - 11))) >> (sh - 10);
+  else q = 0ull;
+  const long long v = static_cast<long long>(q);
+  return (b >> 63) ? -v : v;
+}
+
+// CPLX 0: real; 1: complex, M side (two rows per element); 2: complex, N side
+template <int CPLX>
+__device__ __forceinline__ void load8(const SplitArgs& a, long long row, long long k0, double* v) {
+  if (CPLX == 0) {
+    const double* base = a.p + (row / a.R2) * a.r1 + (row % a.R2) * a.r2;
+    if (a.kvec && k0 + 8 <= a.K) {
+      const double2* q = reinterpret_cast<const double2*>(base + k0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double2 t = q[j];
+        v[2 * j] = t.x;
+        v[2 * j + 1] = t.y;
+      }
+      return;
+    }
+    if (a.K2 == 1 || a.k1 == a.k2 * a.K2) {   // single stride
+      const long long ks = a.K2 == 1 ? a.k1 : a.k2;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = k0 + j < a.K ? base[(k0 + j) * ks] : 0.0;
+      return;
+    }
+    long long q = k0 / a.K2;
+    int r = (int)(k0 - q * a.K2);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = k0 + j < a.K ? base[q * a.k1 + r * a.k2] : 0.0;
+      if (++r == a.K2) { r = 0; ++q; }
+    }
+  } else {
+    const long long el = CPLX == 1 ? row >> 1 : row;
+    const int part = CPLX == 1 ? (int)(row & 1) : 0;
+    const double* base = a.p + 2 * ((el / a.R2) * a.r1 + (el % a.R2) * a.r2);
+    const long long kc = k0 >> 1, KC = a.K >> 1;
+    long long q = kc / a.K2;
+    int r = (int)(kc - q * a.K2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double2 t = make_double2(0.0, 0.0);
+      if (kc + j < KC) t = *reinterpret_cast<const double2*>(base + 2 * (q * a.k1 + r * a.k2));
+      if (++r == a.K2) { r = 0; ++q; }
+      if (a.conj) t.y = -t.y;
+      if (CPLX == 2) {            // (re, im)
+        v[2 * j] = t.x;
+        v[2 * j + 1] = t.y;
+      } else if (part == 0) {     // re row: (ar, -ai)
+        v[2 * j] = t.x;
+        v[2 * j + 1] = -t.y;
+      } else {                    // im row: (ai, ar)
+        v[2 * j] = t.y;
+        v[2 * j + 1] = t.x;
+      }
+    }
+  }
+}
+
+// One CTA: 8 rows, all k; thread = (row, 8-wide k column).  First pass: the
+// rows' largest exponents; second: digits.  HBM- and issue-bound (8 bytes
+// in, 14 out per element, ~40 instructions); the second read of the rows
+// comes from L1/L2.
+template <int CPLX, int R>
+__global__ void __launch_bounds__(256) dg_split_kernel(SplitArgs a, int* __restrict__ exps, int* __restrict__ sq,
+                                                       uint4* __restrict__ dig) {
+  __shared__ int sh[8][8];
+  const int tid = threadIdx.x;
+  const int rl = tid & 7, kt = tid >> 3;
+  const long long row = (long long)blockIdx.x * 8 + rl;
+  const long long cols = a.steps * 2;            // 8-wide k columns (padded)
+  const bool live = row < a.R;
+  int E = 0;
+  if (live)
+    for (long long c = kt; c * 8 < a.K; c += 32) {
+      double v[8];
+      load8<CPLX>(a, row, c * 8, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) E = max(E, expo(v[j]));
+    }
+  E = max(E, __shfl_xor_sync(0xffffffffu, E, 8));
+  E = max(E, __shfl_xor_sync(0xffffffffu, E, 16));
+  if ((tid & 31) < 8) sh[tid >> 5][rl] = E;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) E = max(E, sh[w][rl]);
+  const bool bad = E == 0x7ff;
+  if (E < 1) E = 1;
+  if (kt == 0) exps[row] = bad ? EXP_BAD : E - 1022;
+  // block (row tile, K step): [kc][digit][row][16 bytes]
+  const long long tile = row / R;
+  const int rt = (int)(row - tile * R);
+  uint4* base = dig + tile * a.steps * (2 * ND * R) + rt;
+  // a warp takes units of ucols columns in turn: 128 k (the granule of the
+  // run length, below), 32 where K is short and 128 would idle warps
+  const int ucols = cols >= 128 ? 16 : 4;
+  int most = 0;
+  for (long long u0 = (long long)(tid >> 5) * ucols; u0 < cols; u0 += 8 * ucols) {
+    int n2 = 0;
+    for (int j = 0; j < ucols; j += 4) {
+    const long long c = u0 + j + (kt & 3);
+    if (c >= cols) break;
+    double v[8];
+    if (live && !bad) {
+      load8<CPLX>(a, row, c * 8, v);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = 0.0;
+    }
+    uint32_t lo[8], hi[8];   // low 56 bits of Q plus bias: bytes 6..0 are digits 1..7 plus 128
+    int d0[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const long long q = fixed64(v[j], E);
+      const unsigned long long t = (static_cast<unsigned long long>(q) & 0xffffffffffffffull) + 0x80808080808080ull;
+      lo[j] = static_cast<uint32_t>(t);
+      hi[j] = static_cast<uint32_t>(t >> 32);
+      d0[j] = static_cast<int>(q >> 56) + static_cast<int>(hi[j] >> 24);   // with the carry
+      // sum of squares of digits 0 .. 5
+      const int d14 = static_cast<int>(__byte_perm(lo[j], hi[j], 0x6543) ^ 0x80808080u);
+      const int d5 = static_cast<int>((lo[j] >> 16) & 0xffu) - 128;
+      n2 = __dp4a(d14, d14, n2) + d0[j] * d0[j] + d5 * d5;
+    }
+    uint4* o = base + c * (ND * R);
+#pragma unroll
+    for (int i = 1; i < ND; ++i) {
+      const int byte = 7 - i;
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t x = byte < 4 ? lo[2 * j] : hi[2 * j], y = byte < 4 ? lo[2 * j + 1] : hi[2 * j + 1];
+        const int b = byte & 3;
+        // FP16 0x6400 | byte = 1024 + byte; minus 1152 gives byte - 128
+        const uint32_t h2 = (__byte_perm(x, y, b | ((4 + b) << 8)) & 0x00ff00ffu) | 0x64006400u;
+        const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&h2), __half2half2(__ushort_as_half(0x6480)));
+        w[j] = *reinterpret_cast<const uint32_t*>(&d);
+      }
+      o[i * R] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __half2 d = __halves2half2(__int2half_rn(d0[2 * j]), __int2half_rn(d0[2 * j + 1]));
+      w[j] = *reinterpret_cast<const uint32_t*>(&d);
+    }
+    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    n2 += __shfl_xor_sync(0xffffffffu, n2, 8);
+    n2 += __shfl_xor_sync(0xffffffffu, n2, 16);
+    most = max(most, n2 * (16 / ucols));
+  }
+  // largest sum over 128 k of these 8 rows
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 1));
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 2));
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 4));
+  __syncthreads();
+  if ((tid & 31) == 0) sh[tid >> 5][0] = most;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < 8; ++w) most = max(most, sh[w][0]);
+    sq[blockIdx.x] = most;
+  }
+}
+
+// ---------------------------------------------------------------- GEMM
+struct GArgs {
+  const unsigned char* A;
+  const unsigned char* B;
+  const int* eA;
+  const int* eB;
+  const int* sqA;       // per 8 rows: largest sum over 128 k of squared digits
+  const int* sqB;
+  long long steps;      // K steps per row tile (block stride)
+  int ks0, ks1;         // K steps of this launch
+  int tiles_m, tiles_n, group;
+  int M, N;             // logical (real) rows and columns of C
+  double* C;
+  int M2, N2;
+  long long cm1, cm2, cn1, cn2;   // element strides of C
+  int nflat;            // columns at one stride cn1
+  int cplx_;
+  int negate, accumulate;
+};
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// K steps per accumulation run of tile (mt, nt).  With S_A, S_B the largest
+// sums over 128 k of the squares of digits 0 .. 5 in any row of the two
+// operands' tiles, |P_o| <= sum over k of sum_{i+j=o} (a_i^2 + b_j^2) / 2
+// <= (S_A + S_B) / 2 per 128 k (o <= 5): 256 or 512 k stay within 2^24 where
+// that allows, 128 k always (orders 6 and 7 need no exact sum beyond that: a
+// unit of FP32 rounding there is the last place kept).
+// Digits of ordinary data are nearly uniform (mean square 5461 of 16384), so
+// 512 k pass; each run costs ~3400 clocks of reading the accumulators, during
+// which the tensor core waits.
+__device__ __forceinline__ int run_steps(const GArgs& a, int mt, int nt) {
+  const int4* qa = reinterpret_cast<const int4*>(a.sqA + (long long)mt * (TM / 8));
+  const int4* qb = reinterpret_cast<const int4*>(a.sqB + (long long)nt * (TN / 8));
+  int ma = 0, mb = 0;
+#pragma unroll
+  for (int i = 0; i < TM / 32; ++i) {
+    const int4 q = qa[i];
+    ma = max(ma, max(max(q.x, q.y), max(q.z, q.w)));
+  }
+#pragma unroll
+  for (int i = 0; i < TN / 32; ++i) {
+    const int4 q = qb[i];
+    mb = max(mb, max(max(q.x, q.y), max(q.z, q.w)));
+  }
+  const long long half = ((long long)ma + mb) / 2 + 1;
+  return half <= (1 << 22) ? 4 * RUN : half <= (1 << 23) ? 2 * RUN : RUN;
+}
+
+// K-major operand without swizzle: 8-row x 16-byte core matrices, lbo bytes
+// between the two core matrices of a K step, 128 bytes between 8-row groups
+__device__ __forceinline__ uint64_t sdesc_nosw(uint32_t saddr, uint32_t lbo) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(lbo >> 4) << 16) |
+         (static_cast<uint64_t>(128 >> 4) << 32) | (static_cast<uint64_t>(1) << 46);
+}
+
+// FP64 value of +-(h 2^48 + m) 2^(e - 64), rounded once (to nearest, ties to
+// even); |h| < 2^29, |m| < 2^62.3.  Integer instructions only (the FP64 pipe
+// would take 3 x 64 clocks per warp) and no branches; *odd is set where the
+// result is outside the FP64 normal range and not zero, for assemble_edge.
+__device__ __forceinline__ double assemble(int h, long long m, int e, uint32_t neg, bool* odd) {
+  const int mh = static_cast<int>(m >> 32);
+  const uint32_t ml = static_cast<uint32_t>(m);
+  const int t = h + (mh >> 16);                      // the sum's bits from 48 up
+  // 64 bits of the sum shifted by 0, 8 or 16 with a sticky last bit: at least
+  // 54 significant ones where bits are lost
+  const uint32_t w2 = static_cast<uint32_t>(t >> 16);
+  const uint32_t w1 = (static_cast<uint32_t>(t) << 16) | (static_cast<uint32_t>(mh) & 0xffffu);
+  const int sh = static_cast<uint32_t>(t + (1 << 14)) < (1u << 15) ? 0
+                 : static_cast<uint32_t>(t + (1 << 22)) < (1u << 23) ? 8 : 16;
+  const uint32_t vh = __funnelshift_r(w1, w2, sh);
+  const uint32_t vl = __funnelshift_r(ml, w1, sh) | ((ml & ((1u << sh) - 1u)) ? 1u : 0u);
+  const long long v = static_cast<long long>((static_cast<unsigned long long>(vh) << 32) | vl);
+  const uint32_t sg = static_cast<uint32_t>(v >> 63);              // 0 or ~0
+  unsigned long long u = (static_cast<unsigned long long>(v) ^ static_cast<unsigned long long>(v >> 63)) + (sg & 1u);
+  const int lz = __clzll(static_cast<long long>(u)) & 63;
+  u <<= lz;
+  const uint32_t low = static_cast<uint32_t>(u) & 0x7ffu;
+  // ties to even: up where the rest exceeds a half, or equals it below an odd last place
+  const unsigned long long mant = (u >> 11) + ((low + (static_cast<uint32_t>(u >> 11) & 1u)) > 0x400u ? 1ull : 0ull);
+  const int be = 1021 - lz + e + sh;   // exponent field - 1: 63 - lz - 64 + e + 1023 - 1
+  *odd = *odd || (v != 0 && (be < 0 || be > 2044));
+  // the leading one (or a carry out of the fraction) moves into the exponent field
+  const unsigned long long bits = (static_cast<unsigned long long>((sg ^ (neg ? ~0u : 0u)) & 0x80000000u) << 32) +
+                                  (static_cast<unsigned long long>(static_cast<uint32_t>(be)) << 52) + mant;
+  return v == 0 ? 0.0 : __longlong_as_double(static_cast<long long>(bits));
+}
+
+// the same for any result (a subnormal one is rounded twice: within one of
+// its places)
+__device__ __noinline__ double assemble_edge(int h, long long m, int e, uint32_t neg) {
+  const __int128 s = (static_cast<__int128>(h) << 48) + static_cast<__int128>(m);
+  if (s == 0) return 0.0;
+  const int sg = (s < 0) != (neg != 0u);
+  const unsigned __int128 u = static_cast<unsigned __int128>(s < 0 ? -s : s);
+  const unsigned long long top = static_cast<unsigned long long>(u >> 62);
+  const int cut = top ? 64 - __clzll(static_cast<long long>(top)) : 0;   // leaves 62 bits, the last one sticky
+  unsigned long long t = static_cast<unsigned long long>(u >> cut);
+  if (static_cast<unsigned long long>(u) & ((1ull << cut) - 1ull)) t |= 1ull;
+  const double r = scalbn(static_cast<double>(t), cut + e - 64);
+  return sg ? -r : r;
+}
+
+// 16 TMEM columns of this warp's lanes: the read issued, and the wait that
+// makes its registers valid (tied to them, so that no use moves above it)
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait16(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+
+// as bulk_load, into the same offset (data and mbarrier) of both CTAs of a pair
+__device__ __forceinline__ void bulk_load_pair(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;" ::
+          "r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+
+// arrive on the mbarrier of both CTAs of a pair when the MMAs issued so far are done
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// CL = 2: a pair of CTAs takes two N tiles of one M tile; each loads its own B
+// block and half of the A block, multicast to both.
+template <int CL>
+__global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_gemm_kernel(const GArgs a) {
+  int* err = &g_dg_timeout;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * ST_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = CL == 1 ? 0 : (int)(blockIdx.x % CL);
+  const int cols = (a.tiles_n + CL - 1) / CL;   // N tile groups
+  const int ntiles = a.tiles_m * cols;
+  const int t0 = (int)(blockIdx.x / CL), tstep = (int)(gridDim.x / CL);
+  const int nk = a.ks1 - a.ks0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], CL);   // one arrival per CTA that reads the stage's slot
+    }
+    mbar_init(acc_full, 1);
+    mbar_init(acc_empty, 8);   // one arrival per epilogue warp
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (CL > 1) cluster_sync();   // the peer's barriers are initialised
+  const uint32_t tmem = *tmem_slot;
+
+  auto origin = [&](int t, int& mt, int& nt) {
+    const int per_group = a.group * cols;
+    const int gid = t / per_group;
+    const int first = gid * a.group;
+    const int gsz = min(a.tiles_m - first, a.group);
+    const int local = t - gid * per_group;
+    mt = first + local % gsz;
+    nt = (local / gsz) * CL + rank;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      long long g = 0;
+      bool ok = true;
+      for (int t = t0; t < ntiles && ok; t += tstep) {
+        int mt, nt;
+        origin(t, mt, nt);
+        const unsigned char* pa = a.A + ((long long)mt * a.steps + a.ks0) * A_BLK;
+        // a pair's second tile may lie beyond the last: it then loads that one
+        const unsigned char* pb = a.B + ((long long)min(nt, a.tiles_n - 1) * a.steps + a.ks0) * B_BLK;
+        for (int k = 0; k < nk; ++k, ++g) {
+          const int s = (int)(g % STAGES);
+          const long long it = g / STAGES;
+          if (g >= STAGES && !mbar_wait(&empty[s], (uint32_t)((it - 1) & 1), err)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = smem + s * ST_BYTES;
+          mbar_expect_tx(&full[s], ST_BYTES);
+          if (CL == 1) {
+            bulk_load(st, pa + (long long)k * A_BLK, A_BLK, &full[s]);
+          } else {
+            const uint32_t o = rank * (A_BLK / 2);
+            bulk_load_pair(st + o, pa + (long long)k * A_BLK + o, A_BLK / 2, &full[s]);
+          }
+          bulk_load(st + A_BLK, pb + (long long)k * B_BLK, B_BLK, &full[s]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      long long g = 0, runs = 0;
+      bool ok = true;
+      for (int t = t0; t < ntiles && ok; t += tstep) {
+        int mt, nt;
+        origin(t, mt, nt);
+        const int R = run_steps(a, mt, min(nt, a.tiles_n - 1));
+        for (int k = 0; k < nk && ok; ++k, ++g) {
+          const int s = (int)(g % STAGES);
+          const bool first = k % R == 0;
+          if (first && runs > 0 && !mbar_wait(acc_empty, (uint32_t)((runs - 1) & 1), err)) { ok = false; break; }
+          if (!mbar_wait(&full[s], (uint32_t)((g / STAGES) & 1), err)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t base = smem_u32(smem + s * ST_BYTES);
+          const uint64_t da = sdesc_nosw(base, ND * TM * 16);
+          const uint64_t db = sdesc_nosw(base + A_BLK, ND * TN * 16);
+          // a_i times b_0 .. b_{7-i} into the adjacent orders i .. 7; the
+          // first K step of a run overwrites through i = 0, which reaches
+          // every order
+          const uint32_t acc = first ? 0u : 1u;
+          const uint64_t ai = TM * 16 >> 4, bj = TN * 16 >> 4;   // one digit, in descriptor units
+          mma_f16(tmem, da, db, idesc_f16(TM, 4 * TN), acc);
+          mma_f16(tmem + 4 * TN, da, db + 4 * bj, idesc_f16(TM, 4 * TN), acc);
+          mma_f16(tmem + TN, da + ai, db, idesc_f16(TM, 4 * TN), 1u);
+          mma_f16(tmem + 5 * TN, da + ai, db + 4 * bj, idesc_f16(TM, 3 * TN), 1u);
+          mma_f16(tmem + 2 * TN, da + 2 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+          mma_f16(tmem + 5 * TN, da + 2 * ai, db + 3 * bj, idesc_f16(TM, 3 * TN), 1u);
+          mma_f16(tmem + 3 * TN, da + 3 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+          mma_f16(tmem + 6 * TN, da + 3 * ai, db + 3 * bj, idesc_f16(TM, 2 * TN), 1u);
+          mma_f16(tmem + 4 * TN, da + 4 * ai, db, idesc_f16(TM, 4 * TN), 1u);
+          mma_f16(tmem + 5 * TN, da + 5 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+          mma_f16(tmem + 6 * TN, da + 6 * ai, db, idesc_f16(TM, 2 * TN), 1u);
+          mma_f16(tmem + 7 * TN, da + 7 * ai, db, idesc_f16(TM, TN), 1u);
+          if (CL == 1) mma_commit(&empty[s]);
+          else mma_commit_pair(&empty[s]);
+          if (k % R == R - 1 || k == nk - 1) {
+            mma_commit(acc_full);
+            ++runs;
+          }
+        }
+      }
+    }
+  } else {
+    const int q = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const int row = q * 32 + lane;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(q * 32) << 16) + half * 32;
+    long long run = 0;
+    bool ok = true;
+    for (int t = t0; t < ntiles; t += tstep) {
+      int mt, nt;
+      origin(t, mt, nt);
+      int h0[32];
+      long long m[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        h0[c] = 0;
+        m[c] = 0;
+      }
+      const int R = run_steps(a, mt, min(nt, a.tiles_n - 1));
+      for (int k = 0; k < nk && ok; k += R, ++run) {
+        ok = mbar_wait(acc_full, (uint32_t)(run & 1), err);
+        tc_fence_after();
+        if (ok) {
+          // 16 columns at a time (with 32 the kernel spills: 12 warps' worth
+          // of register file leaves 168 a thread), the next read in flight
+          // while one is converted
+          uint32_t v[2][16];
+          float tail[16];
+          tmem_ld16_async(lane_addr + 7 * TN, v[0]);
+#pragma unroll
+          for (int i = 0; i < 2 * NO; ++i) {
+            const int hc = (i / NO) * 16;
+            // order 7 first, so that the tail is folded from its small end
+            const int o = i % NO == 0 ? 7 : i % NO == 1 ? 6 : i % NO - 2;
+            const int i1 = i + 1, o1 = i1 % NO == 0 ? 7 : i1 % NO == 1 ? 6 : i1 % NO - 2;
+            tmem_wait16(v[i & 1]);
+            if (i1 < 2 * NO) tmem_ld16_async(lane_addr + o1 * TN + (i1 / NO) * 16, v[i1 & 1]);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              const float f = __uint_as_float(v[i & 1][c]);
+              if (o == 7) {
+                tail[c] = f;
+              } else {
+                const int n = __float2int_rn(o == 6 ? fmaf(tail[c], 0x1p-8f, f) : f);
+                if (o == 0) {
+                  h0[hc + c] += n;
+                } else if (o == 1) {   // units of order 0, the rest (a byte) to the sum below
+                  const int q = (n + 128) >> 8;
+                  h0[hc + c] += q;
+                  m[hc + c] += static_cast<long long>(n - (q << 8)) * (1ll << 40);
+                } else {
+                  m[hc + c] += static_cast<long long>(n) * (1ll << (8 * (6 - o)));
+                }
+              }
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty)) : "memory");
+      }
+      const int gm = mt * TM + row;
+      const int n0 = nt * TN + half * 32;
+      // column exponents one per lane, read back by shuffles
+      const int ebl = n0 + lane < a.N ? a.eB[n0 + lane] : 0;
+      if (n0 < a.N) {   // warp-uniform
+        const bool live = gm < a.M;
+        const int ea = live ? a.eA[gm] : 0;
+        const int el = a.cplx_ ? gm >> 1 : gm;
+        const int es = a.cplx_ ? 2 : 1;
+        double* pc = a.C;
+        if (live)
+          pc += es * ((long long)(el / a.M2) * a.cm1 + (long long)(el % a.M2) * a.cm2) + (a.cplx_ ? (gm & 1) : 0);
+        const bool vec = a.nflat && a.cn1 == 1 && es == 1 && n0 + 32 <= a.N && !a.accumulate &&
+                         ((reinterpret_cast<uintptr_t>(pc + n0) & 15) == 0);
+        // four columns per pass of a rolled loop, the sums moved down between
+        // passes: unrolled over 32 columns this code is ~40 KB and a short
+        // product spent ~20 us fetching it
+#pragma unroll 1
+        for (int c0 = 0; c0 < 32; c0 += 4) {
+          double r[4];
+          bool odd = !ok;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int eb = __shfl_sync(0xffffffffu, ebl, c0 + c);
+            odd = odd || ea == EXP_BAD || eb == EXP_BAD;
+            r[c] = assemble(h0[c], m[c], ea + eb + 2, a.negate, &odd);
+          }
+          if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int eb = __shfl_sync(0xffffffffu, ebl, c0 + c);
+              if (!ok || ea == EXP_BAD || eb == EXP_BAD) r[c] = __longlong_as_double(0x7ff8000000000000ll);
+              else r[c] = assemble_edge(h0[c], m[c], ea + eb + 2, a.negate);
+            }
+          }
+          if (live) {
+            if (vec) {
+              reinterpret_cast<double2*>(pc + n0 + c0)[0] = make_double2(r[0], r[1]);
+              reinterpret_cast<double2*>(pc + n0 + c0)[1] = make_double2(r[2], r[3]);
+            } else {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const int gn = n0 + c0 + c;
+                if (gn < a.N) {
+                  double* d = pc + es * (a.nflat ? (long long)gn * a.cn1
+                                                 : (long long)(gn / a.N2) * a.cn1 + (long long)(gn % a.N2) * a.cn2);
+                  *d = a.accumulate ? *d + r[c] : r[c];
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 28; ++c) {
+            h0[c] = h0[c + 4];
+            m[c] = m[c + 4];
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (CL > 1) cluster_sync();   // nothing more lands in the peer's shared memory
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+// head of a digit buffer: row exponents, then one sum per 8 rows
+inline size_t exps_bytes(int side, long long rows) {
+  return align_up(sizeof(int) * (size_t)(up(rows, tile_rows(side)) * tile_rows(side)), 1024);
+}
+inline size_t head_bytes(int side, long long rows) {
+  return exps_bytes(side, rows) + align_up(sizeof(int) * (size_t)(up(rows, tile_rows(side)) * tile_rows(side) / 8), 1024);
+}
+
+inline long long real_rows(int side, bool c, long long rows) { return c && side == 0 ? 2 * rows : rows; }
+
+}  // namespace
+
+bool dg_pays(bool cplx_, long long M, long long N, long long K, bool one_split) {
+  // microseconds.  FP64 pipe: the fullest SM's tiles at 2 FMA per clock, the
+  // best of the three tile sizes (as tgemm picks); digit product: launches
+  // plus 0.5 per K step and 5 to finish a tile.
+  const double mul = cplx_ ? 4.0 : 1.0;
+  double pipe = 1e30;
+  for (int bt = 16; bt <= 64; bt *= 2) {
+    const double waves = (double)up(up(M, bt) * up(N, bt), 152);
+    pipe = std::min(pipe, waves * bt * bt * (bt == 16 ? 1.2 : bt == 32 ? 1.05 : 1.0) * (double)K * mul / 3840.0);
+  }
+  const long long Mr = cplx_ ? 2 * M : M, Kr = cplx_ ? 2 * K : K;
+  const double waves = (double)up(up(Mr, TM) * up(N, TN), 152);
+  const double dig = (one_split ? 8.0 : 12.0) + waves * ((double)up(Kr, KS) * 0.5 + 5.0);
+  return dig < pipe + 4.0;
+}
+
+size_t dg_bytes(int side, bool cplx_, long long rows, long long K) {
+  const long long R = real_rows(side, cplx_, rows);
+  const long long steps = up(cplx_ ? 2 * K : K, KS);
+  return head_bytes(side, R) + (size_t)(up(R, tile_rows(side)) * steps) * (side == 0 ? A_BLK : B_BLK);
+}
+
+template <typename T>
+int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
+  constexpr bool C = sizeof(T) == 16;
+  SplitArgs a;
+  const long long rows = (long long)o.rows.n1 * o.rows.n2, K = (long long)o.K.n1 * o.K.n2;
+  if (rows < 1 || K < 1 || !o.p || !buf) return DMRG_ERR_ARG;
+  a.p = static_cast<const double*>(o.p);
+  a.R = real_rows(side, C, rows);
+  a.K = C ? 2 * K : K;
+  a.R2 = o.rows.n2; a.K2 = o.K.n2;
+  a.r1 = o.sr.s1; a.r2 = o.sr.s2; a.k1 = o.sk.s1; a.k2 = o.sk.s2;
+  a.conj = C ? o.conj : 0;
+  a.steps = up(a.K, KS);
+  const long long kin = a.K2 == 1 ? a.k1 : (a.k1 == a.k2 * a.K2 ? a.k2 : 0);
+  a.kvec = !C && kin == 1 && (reinterpret_cast<uintptr_t>(o.p) & 15) == 0 && a.r1 % 2 == 0 &&
+           (a.R2 == 1 || a.r2 % 2 == 0);
+  const int tr = tile_rows(side);
+  const long long Rp = up(a.R, tr) * tr;
+  if (Rp / 8 > 0x7fffffffLL) return DMRG_ERR_ARG;
+  int* exps = static_cast<int*>(buf);
+  int* sq = reinterpret_cast<int*>(static_cast<char*>(buf) + exps_bytes(side, a.R));
+  uint4* dig = reinterpret_cast<uint4*>(static_cast<char*>(buf) + head_bytes(side, a.R));
+  const unsigned grid = (unsigned)(Rp / 8);
+  if (side == 0) {
+    dg_split_kernel<C ? 1 : 0, TM><<<grid, 256, 0, s>>>(a, exps, sq, dig);
+  } else {
+    dg_split_kernel<C ? 2 : 0, TN><<<grid, 256, 0, s>>>(a, exps, sq, dig);
+  }
+  DMRG_CHECK_LAUNCH();
+  return DMRG_OK;
+}
+
+template <typename T>
+int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long long K, const DgOut& out,
+            cudaStream_t s) {
+  constexpr bool C = sizeof(T) == 16;
+  if (M < 1 || N < 1 || K < 1 || !Adig || !Bdig || !out.C) return DMRG_ERR_ARG;
+  const long long Mr = C ? 2 * M : M, Kr = C ? 2 * K : K;
+  const long long tm = up(Mr, TM), tn = up(N, TN);
+  if (Mr > 0x7fffffffLL || N > 0x7fffffffLL || tm * tn > 0x7fffffffLL) return DMRG_ERR_ARG;
+  GArgs a;
+  a.eA = static_cast<const int*>(Adig);
+  a.eB = static_cast<const int*>(Bdig);
+  a.sqA = reinterpret_cast<const int*>(static_cast<const char*>(Adig) + exps_bytes(0, Mr));
+  a.sqB = reinterpret_cast<const int*>(static_cast<const char*>(Bdig) + exps_bytes(1, N));
+  a.A = static_cast<const unsigned char*>(Adig) + head_bytes(0, Mr);
+  a.B = static_cast<const unsigned char*>(Bdig) + head_bytes(1, N);
+  a.steps = up(Kr, KS);
+  a.tiles_m = (int)tm; a.tiles_n = (int)tn;
+  a.group = (int)std::min<long long>(tm, 16);
+  a.M = (int)Mr; a.N = (int)N;
+  a.C = static_cast<double*>(out.C);
+  a.M2 = out.M.n2; a.N2 = out.N.n2;
+  a.cm1 = out.cm.s1; a.cm2 = out.cm.s2; a.cn1 = out.cn.s1; a.cn2 = out.cn.s2;
+  a.nflat = 0;
+  if (a.N2 == 1) a.nflat = 1;
+  else if (out.N.n1 == 1 || a.cn1 == a.cn2 * a.N2) { a.nflat = 1; a.cn1 = a.cn2; }
+  a.cplx_ = C ? 1 : 0;
+  a.negate = out.alpha < 0.0;
+  const bool pair = tn >= 2;
+  static std::atomic<unsigned long long> attr1{0}, attr2{0};
+  if (pair) DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(dg_gemm_kernel<2>), DG_SMEM, attr2));
+  else DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(dg_gemm_kernel<1>), DG_SMEM, attr1));
+  const unsigned grid = pair ? 2u * (unsigned)std::min<long long>(tm * up(tn, 2), 76)
+                             : (unsigned)std::min<long long>(tm * tn, 152);
+  // K in launches of at most MAX_STEPS steps (64-bit sums), the later ones adding
+  for (long long k0 = 0; k0 < a.steps; k0 += MAX_STEPS) {
+    a.ks0 = (int)k0;
+    a.ks1 = (int)std::min<long long>(a.steps, k0 + MAX_STEPS);
+    a.accumulate = out.accumulate || k0 > 0;
+    if (pair) dg_gemm_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    else dg_gemm_kernel<1><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    DMRG_CHECK_LAUNCH();
+  }
+  return DMRG_OK;
+}
+
+template <typename T>
+size_t dg_product_bytes(const TGemm& g) {
+  constexpr bool C = sizeof(T) == 16;
+  const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
+  return dg_bytes(0, C, M, K) + dg_bytes(1, C, N, K);
+}
+
+template <typename T>
+int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumulate, T* C, void* work,
+               cudaStream_t s) {
+  const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
+  void* da = work;
+  void* db = static_cast<char*>(work) + dg_bytes(0, sizeof(T) == 16, M, K);
+  DMRG_TRY(dg_split<T>(0, DgOperand{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, da, s));
+  DMRG_TRY(dg_split<T>(1, DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, s));
+  return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, s);
+}
+
+template size_t dg_product_bytes<double>(const TGemm&);
+template size_t dg_product_bytes<cplx>(const TGemm&);
+template int dg_product<double>(const TGemm&, const double*, const double*, double, int, double*, void*,
+                                cudaStream_t);
+template int dg_product<cplx>(const TGemm&, const cplx*, const cplx*, double, int, cplx*, void*, cudaStream_t);
+template int dg_split<double>(int, const DgOperand&, void*, cudaStream_t);
+template int dg_split<cplx>(int, const DgOperand&, void*, cudaStream_t);
+template int dg_gemm<double>(const void*, const void*, long long, long long, long long, const DgOut&,
+                             cudaStream_t);
+template int dg_gemm<cplx>(const void*, const void*, long long, long long, long long, const DgOut&,
+                           cudaStream_t);
+
+}  // namespace dmrg

@@ -1,0 +1,44 @@
+// FP64 matrix products on the tensor cores by exact digit products (dgemm.cu).
+#pragma once
+#include "common.cuh"
+
+namespace dmrg {
+
+// One operand of C[M][N] = sum_k A[m][k] B[n][k]: element (row, k) of the
+// FP64 / complex FP64 array p at row and k strides (outer, inner), in
+// elements.  rows and K count elements (complex: complex elements).
+struct DgOperand {
+  const void* p;
+  Ax2 rows, K;
+  St2 sr, sk;
+  int conj;
+};
+
+// Digit form of an operand in device memory: row exponents, then the digit
+// blocks.  side 0: the M side (tiles of 128 rows), side 1: the N side (64).
+size_t dg_bytes(int side, bool cplx_, long long rows, long long K);
+template <typename T> int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s);
+
+// C = alpha A B (+ C): alpha +1 or -1; C at (row, column) strides in elements.
+struct DgOut {
+  void* C;
+  Ax2 M, N;
+  St2 cm, cn;
+  double alpha;
+  int accumulate;
+};
+template <typename T>
+int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long long K, const DgOut& out,
+            cudaStream_t s);
+// whether the digit product of this shape is faster than the FP64 pipe
+// (one_split: the other operand's digits are kept from an earlier call)
+bool dg_pays(bool cplx_, long long M, long long N, long long K, bool one_split);
+
+// C = alpha A B (+ C) for one unbatched strided contraction: both operands
+// split into work (dg_product_bytes), then multiplied.
+template <typename T> size_t dg_product_bytes(const TGemm& g);
+template <typename T>
+int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumulate, T* C, void* work,
+               cudaStream_t s);
+
+}  // namespace dmrg

@@ -17,7 +17,7 @@
 //   G[(k,s)][s'][m]       = sum_{(a',b')} Y2[(a',b')][(k,s,m)] conj(A)[a'][s'][b']
 //                           (tall-skinny reduction over chi^2 rows, split into
 //                            row chunks, deterministic two-pass sum)
-#include "common.cuh"
+#include "heff64.cuh"
 
 namespace dmrg {
 namespace {
@@ -156,77 +156,6 @@ int env_gradient_mixed(long long clb, long long crb, long long clk, long long cr
   return DMRG_OK;
 }
 
-template <typename T>
-size_t mixed_env_ws(int side, long long clb, long long crb, long long clk, long long crk, long long d, long long wl,
-                    long long wr) {
-  if (side == 0) return align_up(sizeof(T) * (size_t)(clb * wl * d * crk + clb * d * wr * crk), 1024);
-  return align_up(sizeof(T) * (size_t)(crb * wr * clk * d + crb * wl * d * clk), 1024);
-}
-
-// side 0: Lnew (crb, wr, crk) = L (clb, wl, clk) . conj(B) . W . A
-// side 1: Rnew (clb, wl, clk) = R (crb, wr, crk) . conj(B) . W . A
-template <typename T>
-int env_mixed(int side, long long clb, long long crb, long long clk, long long crk, long long d, long long wl,
-              long long wr, const T* E, const T* W, const T* B, const T* A, T* Enew, void* work, size_t work_bytes,
-              cudaStream_t s) {
-  if (mixed_env_ws<T>(side, clb, crb, clk, crk, d, wl, wr) > work_bytes) return DMRG_ERR_WORKSPACE;
-  const T one = Sc<T>::one(), zero = Sc<T>::zero();
-  T* P1 = static_cast<T*>(work);
-  TGemm g{};
-  if (side == 0) {
-    T* Y2 = P1 + clb * wl * d * crk;
-    // Y1[(a',k)][(s,b)] = L[(a',k)][a] A[a][(s,b)]
-    g.B = ax(1); g.M = ax((int)(clb * wl)); g.K = ax((int)clk); g.N = ax((int)(d * crk));
-    g.a_m = st(clk); g.a_k = st(1);
-    g.b_k = st(d * crk); g.b_n = st(1);
-    g.c_m = st(d * crk); g.c_n = st(1);
-    DMRG_TRY(tgemm<T>(g, one, E, A, zero, P1, s));
-    // Y2[a'][(s',m)][b] = W[(k,s)][(s',m)] Y1[a'][(k,s)][b]
-    g = TGemm{};
-    g.B = ax((int)clb); g.M = ax((int)(d * wr)); g.K = ax((int)(wl * d)); g.N = ax((int)crk);
-    g.a_b = st(0); g.a_m = st(1); g.a_k = st(d * wr);
-    g.b_b = st(wl * d * crk); g.b_k = st(crk); g.b_n = st(1);
-    g.c_b = st(d * wr * crk); g.c_m = st(crk); g.c_n = st(1);
-    DMRG_TRY(tgemm<T>(g, one, W, P1, zero, Y2, s));
-    // Lnew[b'][(m,b)] = conj(B)[(a',s')][b'] Y2[(a',s')][(m,b)]
-    g = TGemm{};
-    g.B = ax(1); g.M = ax((int)crb); g.K = ax((int)(clb * d)); g.N = ax((int)(wr * crk));
-    g.a_m = st(1); g.a_k = st(crb); g.conjA = 1;
-    g.b_k = st(wr * crk); g.b_n = st(1);
-    g.c_m = st(wr * crk); g.c_n = st(1);
-    DMRG_TRY(tgemm<T>(g, one, B, Y2, zero, Enew, s));
-  } else {
-    T* Z2 = P1 + crb * wr * clk * d;
-    // Z1[(b',m)][(a,s)] = R[(b',m)][b] A[(a,s)][b]
-    g.B = ax(1); g.M = ax((int)(crb * wr)); g.K = ax((int)crk); g.N = ax((int)(clk * d));
-    g.a_m = st(crk); g.a_k = st(1);
-    g.b_k = st(1); g.b_n = st(crk);
-    g.c_m = st(clk * d); g.c_n = st(1);
-    DMRG_TRY(tgemm<T>(g, one, E, A, zero, P1, s));
-    // Z2[b'][(k,s')][a] = W[k][s][s'][m] Z1[b'][m][a][s]   (K = (m, s))
-    g = TGemm{};
-    g.B = ax((int)crb);
-    g.M = ax((int)wl, (int)d);
-    g.K = ax((int)wr, (int)d);
-    g.N = ax((int)clk);
-    g.a_b = st(0); g.a_m = st(d * d * wr, wr); g.a_k = st(1, d * wr);
-    g.b_b = st(wr * clk * d); g.b_k = st(clk * d, 1); g.b_n = st(d);
-    g.c_b = st(wl * d * clk); g.c_m = st(d * clk, clk); g.c_n = st(1);
-    DMRG_TRY(tgemm<T>(g, one, W, P1, zero, Z2, s));
-    // Rnew[a'][(k,a)] = conj(B)[a'][(b',s')] Z2[(b',s')][(k,a)]
-    g = TGemm{};
-    g.B = ax(1);
-    g.M = ax((int)clb);
-    g.K = ax((int)crb, (int)d);
-    g.N = ax((int)wl, (int)clk);
-    g.a_m = st(d * crb); g.a_k = st(1, crb); g.conjA = 1;
-    g.b_k = st(wl * d * clk, clk); g.b_n = st(d * clk, 1);
-    g.c_m = st(wl * clk); g.c_n = st(clk, 1);
-    DMRG_TRY(tgemm<T>(g, one, B, Z2, zero, Enew, s));
-  }
-  return DMRG_OK;
-}
-
 bool mixed_dims_ok(int clb, int crb, int clk, int crk, int d, int wl, int wr) {
   if (clb < 1 || crb < 1 || clk < 1 || crk < 1 || d < 1 || wl < 1 || wr < 1) return false;
   const long long y2 = (long long)clb * crb * wl * d * wr;
@@ -265,8 +194,7 @@ extern "C" int dmrg_env_gradient(int dtype, int chil, int d, int chir, int wl, i
 extern "C" size_t dmrg_env_mixed_workspace_bytes(int side, int dtype, int clb, int crb, int clk, int crk, int d, int wl,
                                                  int wr) {
   if ((side != 0 && side != 1) || !mixed_dims_ok(clb, crb, clk, crk, d, wl, wr)) return 0;
-  return dtype == DMRG_COMPLEX128 ? mixed_env_ws<cplx>(side, clb, crb, clk, crk, d, wl, wr)
-                                  : mixed_env_ws<double>(side, clb, crb, clk, crk, d, wl, wr);
+  return env64_workspace_bytes(side, dtype, clb, crb, clk, crk, d, wl, wr);
 }
 
 extern "C" int dmrg_env_extend_mixed(int side, int dtype, int clb, int crb, int clk, int crk, int d, int wl, int wr,
@@ -277,11 +205,11 @@ extern "C" int dmrg_env_extend_mixed(int side, int dtype, int clb, int crb, int 
     return DMRG_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == DMRG_COMPLEX128)
-    return env_mixed<cplx>(side, clb, crb, clk, crk, d, wl, wr, static_cast<const cplx*>(E),
+    return env64<cplx>(side, clb, crb, clk, crk, d, wl, wr, static_cast<const cplx*>(E),
                            static_cast<const cplx*>(W), static_cast<const cplx*>(B), static_cast<const cplx*>(A),
                            static_cast<cplx*>(Enew), work, work_bytes, s);
   if (dtype != DMRG_REAL64) return DMRG_ERR_ARG;
-  return env_mixed<double>(side, clb, crb, clk, crk, d, wl, wr, static_cast<const double*>(E),
+  return env64<double>(side, clb, crb, clk, crk, d, wl, wr, static_cast<const double*>(E),
                            static_cast<const double*>(W), static_cast<const double*>(B), static_cast<const double*>(A),
                            static_cast<double*>(Enew), work, work_bytes, s);
 }

@@ -148,17 +148,6 @@ int env_left_plan(long long cl, long long d, long long cr, long long wl, long lo
 }
 
 template <typename T>
-int env_left_fp64(long long cl, long long d, long long cr, long long wl, long long wr, const T* L, const T* W,
-                  const T* A, T* Lnew, T* P, cudaStream_t s) {
-  GStep steps[3];
-  const int n = env_left_plan<T>(cl, d, cr, wl, wr, L, W, A, Lnew, P, steps);
-  for (int i = 0; i < n; ++i)
-    DMRG_TRY(tgemm<T>(steps[i].g, Sc<T>::one(), static_cast<const T*>(steps[i].A), static_cast<const T*>(steps[i].B),
-                      Sc<T>::zero(), static_cast<T*>(steps[i].C), s));
-  return DMRG_OK;
-}
-
-template <typename T>
 int env_right_plan(long long cl, long long d, long long cr, long long wl, long long wr, const T* R, const T* W,
                    const T* B, T* Rnew, T* P, GStep* steps) {
   int n = 0;
@@ -194,17 +183,6 @@ int env_right_plan(long long cl, long long d, long long cr, long long wl, long l
   return n;
 }
 
-template <typename T>
-int env_right_fp64(long long cl, long long d, long long cr, long long wl, long long wr, const T* R, const T* W,
-                   const T* B, T* Rnew, T* P, cudaStream_t s) {
-  GStep steps[3];
-  const int n = env_right_plan<T>(cl, d, cr, wl, wr, R, W, B, Rnew, P, steps);
-  for (int i = 0; i < n; ++i)
-    DMRG_TRY(tgemm<T>(steps[i].g, Sc<T>::one(), static_cast<const T*>(steps[i].A), static_cast<const T*>(steps[i].B),
-                      Sc<T>::zero(), static_cast<T*>(steps[i].C), s));
-  return DMRG_OK;
-}
-
 template size_t heff_fp64_elems<double>(const dmrg_heff_t&, size_t*, size_t*);
 template size_t heff_fp64_elems<cplx>(const dmrg_heff_t&, size_t*, size_t*);
 template int heff_apply_fp64<double>(const dmrg_heff_t&, const double*, double*, double*, double*, cudaStream_t);
@@ -219,13 +197,5 @@ template int env_right_plan<double>(long long, long long, long long, long long, 
                                     const double*, const double*, double*, double*, GStep*);
 template int env_right_plan<cplx>(long long, long long, long long, long long, long long, const cplx*, const cplx*,
                                   const cplx*, cplx*, cplx*, GStep*);
-template int env_left_fp64<double>(long long, long long, long long, long long, long long, const double*, const double*,
-                                   const double*, double*, double*, cudaStream_t);
-template int env_left_fp64<cplx>(long long, long long, long long, long long, long long, const cplx*, const cplx*,
-                                 const cplx*, cplx*, cplx*, cudaStream_t);
-template int env_right_fp64<double>(long long, long long, long long, long long, long long, const double*, const double*,
-                                    const double*, double*, double*, cudaStream_t);
-template int env_right_fp64<cplx>(long long, long long, long long, long long, long long, const cplx*, const cplx*,
-                                  const cplx*, cplx*, cplx*, cudaStream_t);
 
 }  // namespace dmrg

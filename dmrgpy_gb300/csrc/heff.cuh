@@ -6,7 +6,9 @@
 
 namespace dmrg {
 
-// FP64 / complex FP64 path (strided CUDA-core contractions)
+// FP64 / complex FP64 contraction plans (strided CUDA-core contractions):
+// the batched sweeps, and single operators whose workspace is too small for
+// heff64.cu
 // one strided contraction of a plan (alpha 1, beta 0)
 struct GStep {
   TGemm g;
@@ -24,12 +26,6 @@ int env_right_plan(long long cl, long long d, long long cr, long long wl, long l
 template <typename T> size_t heff_fp64_elems(const dmrg_heff_t& o, size_t* p_elems, size_t* q_elems);
 template <typename T> int heff_apply_fp64(const dmrg_heff_t& o, const T* x, T* y, T* P, T* Q, cudaStream_t s);
 size_t env_fp64_elems(int side, long long cl, long long d, long long cr, long long wl, long long wr);
-template <typename T>
-int env_left_fp64(long long cl, long long d, long long cr, long long wl, long long wr, const T* L, const T* W,
-                  const T* A, T* Lnew, T* P, cudaStream_t s);
-template <typename T>
-int env_right_fp64(long long cl, long long d, long long cr, long long wl, long long wr, const T* R, const T* W,
-                   const T* B, T* Rnew, T* P, cudaStream_t s);
 
 // truncated SVD (one-sided Jacobi)
 size_t svd_work_bytes(int dtype, int m, int n);

@@ -30,6 +30,9 @@
 #include "common.cuh"
 
 namespace dmrg {
+
+bool heff_fits(const dmrg_heff_t* op, size_t bytes);   // capi.cu
+
 namespace {
 
 static __device__ __align__(256) unsigned char g_heff_scratch[DMRG_NOALLOC_SCRATCH_BYTES];
@@ -60,9 +63,9 @@ int scratch_address(void** out) {
 extern "C" int dmrg_heff_apply_noalloc(const dmrg_heff_t* op, const void* x, void* y, void* stream) {
   if (!op || !x || !y || x == y) return DMRG_ERR_ARG;
   if (op->precision != DMRG_PREC_FP64) return DMRG_ERR_UNSUPPORTED;
-  const size_t need = dmrg_heff_workspace_bytes(op);
-  if (need == 0) return DMRG_ERR_ARG;
-  if (need > (size_t)DMRG_NOALLOC_SCRATCH_BYTES) return DMRG_ERR_WORKSPACE;
+  if (dmrg_heff_workspace_bytes(op) == 0) return DMRG_ERR_ARG;
+  // the digit path where its operands fit too, else the FP64 pipe
+  if (!dmrg::heff_fits(op, (size_t)DMRG_NOALLOC_SCRATCH_BYTES)) return DMRG_ERR_WORKSPACE;
   void* scratch = nullptr;
   DMRG_TRY(dmrg::scratch_address(&scratch));
   return dmrg_heff_apply(op, x, y, scratch, (size_t)DMRG_NOALLOC_SCRATCH_BYTES, stream);

@@ -80,7 +80,10 @@ const char* dmrg_status_string(int status);
 unsigned long long dmrg_kernel_launches(void);
 
 /* ---- effective-Hamiltonian matvec ------------------------------------- */
-/* Workspace for dmrg_heff_apply (also covers the operand preparation). */
+/* Workspace for dmrg_heff_apply (also covers the operand preparation).  An
+ * FP64 operator also runs in the two intermediates of its contraction chain
+ * alone, without the operands of the tensor-core digit products: slower,
+ * same accuracy class; below that DMRG_ERR_WORKSPACE. */
 size_t dmrg_heff_workspace_bytes(const dmrg_heff_t* op);
 /* y = H_eff x.  Replaces the matvec closure of pyitensor/kernels.py:353-410
  * (_make_matvec_planned) built by pyitensor/dmrg.py:224-299.  x and y must
@@ -90,7 +93,8 @@ int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y,
 
 /* The same matvec split in two, for callers that drive their own Krylov
  * loop: dmrg_heff_prepare() does the per-operator work once (split-TF32:
- * splitting L, R and the two-site MPO into the workspace; FP64: nothing),
+ * splitting L, R and the two-site MPO into the workspace; FP64: the digits
+ * of L and R and the MPO's row lists),
  * dmrg_heff_apply_prepared() applies H_eff for each new vector with the same
  * op and workspace (the plan-once / replay-per-iteration structure of
  * pyitensor/kernels.py:353-410).  dmrg_heff_status() synchronises the stream
@@ -109,7 +113,8 @@ int dmrg_heff_status(const dmrg_heff_t* op, void* work, size_t work_bytes, void*
  * allocator of their own, or a memory budget fixed at start-up).
  * precision must be DMRG_PREC_FP64 (else DMRG_ERR_UNSUPPORTED); an operator
  * whose dmrg_heff_workspace_bytes() exceeds DMRG_NOALLOC_SCRATCH_BYTES is
- * rejected with DMRG_ERR_WORKSPACE.  The first call on a device sets up the
+ * rejected with DMRG_ERR_WORKSPACE (counting the two intermediates; the
+ * digit products run where their operands fit too).  The first call on a device sets up the
  * array's address and should come before any stream capture; the address is
  * cached per device number, so the library assumes the device's primary
  * context (the CUDA runtime's) and no cudaDeviceReset between calls.  All
@@ -381,6 +386,8 @@ int dmrg_wait_timeout_probe(void* work, size_t work_bytes, void* stream);
 
 /* ---- dense contraction ---------------------------------------------------- */
 size_t dmrg_gemm_workspace_bytes(int dtype, int precision, int m, int k, int n);
+/* (FP64 products need none: with the workspace they run as digit products on
+ * the tensor cores where that is faster, without it on the FP64 pipe.) */
 /* C (m x n) = A (m x k) . B (k x n), all row-major.  Used for the two-site
  * merge theta = A_i . A_{i+1} (pyitensor/dmrg.py:233, Ti * Tj) and for the
  * bond-matrix absorption of one-site TDVP (pyitensor/tdvp.py:300-313). */
