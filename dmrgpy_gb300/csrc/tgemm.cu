@@ -3,8 +3,8 @@
 // clock per SM, about 1 TFLOP/s) is the bound, so the kernel only has to keep
 // every SM's pipe fed: K staged through shared memory in slices of 16, the
 // next slice held in registers while the current one is multiplied, and an
-// output tile of 64x64, 32x32 or 16x16 by the number of tiles a shape gives
-// (pick_tile).  Every logical dimension is an (outer, inner) index pair
+// output tile of 64x64, 32x32, 16x16 or 8x8 by the number of tiles a shape
+// gives (pick_tile).  Every logical dimension is an (outer, inner) index pair
 // with its own element strides, which expresses all the permuted views the
 // H_eff / environment / Gram contractions need without copies.
 #include "common.cuh"
@@ -17,10 +17,12 @@ constexpr int BK = 16;
 
 // Output tile edge and its thread block: a thread owns TM x TN outputs.
 // 64x64: 256 threads, 4x4; 32x32: 128 threads, 4x2; 16x16: 128 threads, 2x1.
+// (8x8: 256 threads, one output each over a quarter of K; tgemm_tile8.)
 template <int BT> struct Tile;
 template <> struct Tile<64> { static constexpr int NT = 256, TM = 4, TN = 4; };
 template <> struct Tile<32> { static constexpr int NT = 128, TM = 4, TN = 2; };
 template <> struct Tile<16> { static constexpr int NT = 128, TM = 2, TN = 1; };
+template <> struct Tile<8> { static constexpr int NT = 256, TM = 1, TN = 1; };
 
 struct Dev {
   int B2, M, M2, N, N2, K, K2;
@@ -40,8 +42,9 @@ __device__ __forceinline__ long long off2(int i, int n2, long long s1, long long
 // one BT x BT output tile (m0, n0) of batch entry bz
 // MIRROR: C is square with equal M and N layouts and the product is
 // symmetric (C = X^T X); an off-diagonal tile also writes its transpose.
-// Every output sums its products in ascending k whatever the tile, so the
-// choice of tile does not change a result.
+// Every output sums its products in ascending k whatever the tile (8x8: four
+// such sums added), so the choice of tile changes a result by rounding at
+// most.
 template <typename T, int BT, bool MIRROR = false>
 __device__ __forceinline__ void tgemm_tile(const Dev& d, T alpha, const T* __restrict__ A, const T* __restrict__ B,
                                            T beta, T* __restrict__ C, int m0, int n0, int bz) {
@@ -131,6 +134,68 @@ __device__ __forceinline__ void tgemm_tile(const Dev& d, T alpha, const T* __res
   }
 }
 
+// One 8x8 tile, for products of few outputs: with 16x16 tiles a 60 x 60
+// product keeps 16 of 152 SMs busy.  K in slices of 32; thread group g (64
+// threads, one output each) multiplies k = 8 g .. 8 g + 7 of every slice, and
+// the four partial sums are added in order at the end.
+template <typename T, bool MIRROR>
+__device__ __forceinline__ void tgemm_tile8(const Dev& d, T alpha, const T* __restrict__ A, const T* __restrict__ B,
+                                            T beta, T* __restrict__ C, int m0, int n0, int bz) {
+  constexpr int BT = 8, BK8 = 32;
+  __shared__ T As[BK8][BT + 1];
+  __shared__ T Bs[BK8][BT + 1];
+  __shared__ T part[3][BT * BT];
+  const int tid = threadIdx.x;
+  const int bq = bz / d.B2, br = bz - bq * d.B2;
+  const int ka = d.a_kfast ? tid % BK8 : tid / BT, ma = d.a_kfast ? tid / BK8 : tid % BT;
+  const int kb = d.b_kfast ? tid % BK8 : tid / BT, nb = d.b_kfast ? tid / BK8 : tid % BT;
+  const T* ap = m0 + ma < d.M ? A + (long long)bq * d.ab1 + (long long)br * d.ab2 + off2(m0 + ma, d.M2, d.am1, d.am2)
+                              : nullptr;
+  const T* bp = n0 + nb < d.N ? B + (long long)bq * d.bb1 + (long long)br * d.bb2 + off2(n0 + nb, d.N2, d.bn1, d.bn2)
+                              : nullptr;
+  T* Cb = C + (long long)bq * d.cb1 + (long long)br * d.cb2;
+  const int g = tid >> 6, o = tid & 63, tm = o >> 3, tn = o & 7;
+  T ra, rb;
+  auto load = [&](int k0) {
+    ra = Sc<T>::zero();
+    rb = Sc<T>::zero();
+    if (ap && k0 + ka < d.K) ra = cond_conj(ap[off2(k0 + ka, d.K2, d.ak1, d.ak2)], d.conjA);
+    if (bp && k0 + kb < d.K) rb = cond_conj(bp[off2(k0 + kb, d.K2, d.bk1, d.bk2)], d.conjB);
+  };
+  T acc = Sc<T>::zero();
+  load(0);
+  for (int k0 = 0; k0 < d.K; k0 += BK8) {
+    As[ka][ma] = ra;
+    Bs[kb][nb] = rb;
+    __syncthreads();
+    if (k0 + BK8 < d.K) load(k0 + BK8);
+    // a group past the end of K holds zeros only: skipped
+    if (k0 + 8 * g < d.K) {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) acc = Sc<T>::fma(As[8 * g + kk][tm], Bs[8 * g + kk][tn], acc);
+    }
+    __syncthreads();
+  }
+  if (g > 0) part[g - 1][o] = acc;
+  __syncthreads();
+  const int gm = m0 + tm, gn = n0 + tn;
+  if (g > 0 || gm >= d.M || gn >= d.N) return;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) acc = Sc<T>::add(acc, part[j][o]);
+  const long long oc = off2(gm, d.M2, d.cm1, d.cm2) + off2(gn, d.N2, d.cn1, d.cn2);
+  T v = Sc<T>::mul(alpha, acc);
+  if (Sc<T>::re(beta) != 0.0 || Sc<T>::im(beta) != 0.0) v = Sc<T>::fma(beta, Cb[oc], v);
+  Cb[oc] = v;
+  if (MIRROR && m0 != n0) Cb[off2(gn, d.M2, d.cm1, d.cm2) + off2(gm, d.N2, d.cn1, d.cn2)] = v;
+}
+
+template <typename T, int BT, bool MIRROR = false>
+__device__ __forceinline__ void any_tile(const Dev& d, T alpha, const T* __restrict__ A, const T* __restrict__ B,
+                                         T beta, T* __restrict__ C, int m0, int n0, int bz) {
+  if constexpr (BT == 8) tgemm_tile8<T, MIRROR>(d, alpha, A, B, beta, C, m0, n0, bz);
+  else tgemm_tile<T, BT, MIRROR>(d, alpha, A, B, beta, C, m0, n0, bz);
+}
+
 // Symmetric product: only the tiles with tile row <= tile column, numbered
 // row by row over the upper triangle of a tiles x tiles grid.
 template <typename T, int BT>
@@ -143,13 +208,13 @@ __global__ void __launch_bounds__(Tile<BT>::NT) tgemm_sym_kernel(Dev d, T alpha,
     ++tm;
   }
   if (tm >= tiles) return;
-  tgemm_tile<T, BT, true>(d, alpha, A, B, Sc<T>::zero(), C, tm * BT, (tm + rem) * BT, 0);
+  any_tile<T, BT, true>(d, alpha, A, B, Sc<T>::zero(), C, tm * BT, (tm + rem) * BT, 0);
 }
 
 template <typename T, int BT>
 __global__ void __launch_bounds__(Tile<BT>::NT) tgemm_kernel(Dev d, T alpha, const T* __restrict__ A,
                                                              const T* __restrict__ B, T beta, T* __restrict__ C) {
-  tgemm_tile<T, BT>(d, alpha, A, B, beta, C, blockIdx.x * BT, blockIdx.y * BT, blockIdx.z);
+  any_tile<T, BT>(d, alpha, A, B, beta, C, blockIdx.x * BT, blockIdx.y * BT, blockIdx.z);
 }
 
 // Grouped launch: problem p owns the flat tile range [start, start + tiles)
@@ -179,23 +244,31 @@ __global__ void __launch_bounds__(Tile<BT>::NT) tgemm_grouped_kernel(const GProb
   const int bz = (int)(local / per_b);
   const int rem = (int)(local - (long long)bz * per_b);
   const int tm = rem % g.tiles_m, tn = rem / g.tiles_m;
-  tgemm_tile<T, BT>(g.d, alpha, static_cast<const T*>(g.A), static_cast<const T*>(g.B), beta, static_cast<T*>(g.C),
+  any_tile<T, BT>(g.d, alpha, static_cast<const T*>(g.A), static_cast<const T*>(g.B), beta, static_cast<T*>(g.C),
                     tm * BT, tn * BT, bz);
 }
 
 inline long long tiles_of(long long n, int bt) { return (n + bt - 1) / bt; }
 
-// Tile edge for n64 / n32 / n16 tiles of the three sizes.  An SM's FP64 pipe
-// takes bt^2 * K / 2 clocks per tile however many CTAs share it, so the time
-// goes as (tiles on the fullest SM) * bt^2; the factors are the smaller
-// tiles' extra staging per product (measured per output on large shapes:
-// 32x32 5% and 16x16 20% above 64x64).
-inline int pick_tile(long long n64, long long n32, long long n16) {
-  const double c64 = (double)tiles_of(n64, 152) * 4096.0;
-  const double c32 = (double)tiles_of(n32, 152) * 1024.0 * 1.05;
-  const double c16 = (double)tiles_of(n16, 152) * 256.0 * 1.2;
-  if (c16 < c32 && c16 < c64) return 16;
-  return c32 < c64 ? 32 : 64;
+// Tile edge for n[0..3] tiles of 64, 32, 16 and 8.  An SM's FP64 pipe takes
+// bt^2 * K / 2 clocks per tile however many CTAs share it, so the time goes
+// as (tiles on the fullest SM) * bt^2; the factors are the smaller tiles'
+// extra staging per product (measured per output on large shapes: 32x32 5%,
+// 16x16 20%, 8x8 60% above 64x64).
+constexpr int EDGES = 4;
+constexpr int EDGE[EDGES] = {64, 32, 16, 8};
+constexpr double EDGE_COST[EDGES] = {1.0, 1.05, 1.2, 1.6};
+inline int pick_tile(const long long* n) {
+  int best = 0;
+  double least = 0.0;
+  for (int e = 0; e < EDGES; ++e) {
+    const double c = (double)tiles_of(n[e], 152) * EDGE[e] * EDGE[e] * EDGE_COST[e];
+    if (e == 0 || c < least) {
+      best = e;
+      least = c;
+    }
+  }
+  return EDGE[best];
 }
 
 // Dev from a TGemm; returns false when there is nothing to do, *err on bad input
@@ -238,14 +311,16 @@ int tgemm(const TGemm& g, T alpha, const T* A, const T* B, T beta, T* C, cudaStr
   int err = DMRG_OK;
   if (!make_dev(g, &d, &err)) return err;
   const long long nb = (long long)g.B.n1 * g.B.n2;
-  auto tiles = [&](int bt) { return nb * tiles_of(d.M, bt) * tiles_of(d.N, bt); };
-  int bt = pick_tile(tiles(64), tiles(32), tiles(16));
+  long long tiles[EDGES];
+  for (int e = 0; e < EDGES; ++e) tiles[e] = nb * tiles_of(d.M, EDGE[e]) * tiles_of(d.N, EDGE[e]);
+  int bt = pick_tile(tiles);
   while (bt < 64 && tiles_of(d.N, bt) > 65535) bt *= 2;   // grid.y limit
   dim3 grid((unsigned)tiles_of(d.M, bt), (unsigned)tiles_of(d.N, bt), (unsigned)nb);
   if (tiles_of(d.N, 64) > 65535) return DMRG_ERR_ARG;
   if (bt == 64) tgemm_kernel<T, 64><<<grid, Tile<64>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
   else if (bt == 32) tgemm_kernel<T, 32><<<grid, Tile<32>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
-  else tgemm_kernel<T, 16><<<grid, Tile<16>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
+  else if (bt == 16) tgemm_kernel<T, 16><<<grid, Tile<16>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
+  else tgemm_kernel<T, 8><<<grid, Tile<8>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -262,12 +337,14 @@ int tgemm_gram(const double* X, long long ld, int m, int k, double* G, cudaStrea
   if (!make_dev(g, &d, &err)) return err;
   auto tri = [&](int bt) { const long long t = tiles_of(k, bt); return t * (t + 1) / 2; };
   if (tri(64) > 0x7fffffffLL) return DMRG_ERR_ARG;
-  const int bt = pick_tile(tri(64), tri(32), tri(16));
+  const long long ntris[EDGES] = {tri(64), tri(32), tri(16), tri(8)};
+  const int bt = pick_tile(ntris);
   const unsigned ntri = (unsigned)tri(bt);
   const int tiles = (int)tiles_of(k, bt);
   if (bt == 64) tgemm_sym_kernel<double, 64><<<ntri, Tile<64>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
   else if (bt == 32) tgemm_sym_kernel<double, 32><<<ntri, Tile<32>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
-  else tgemm_sym_kernel<double, 16><<<ntri, Tile<16>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
+  else if (bt == 16) tgemm_sym_kernel<double, 16><<<ntri, Tile<16>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
+  else tgemm_sym_kernel<double, 8><<<ntri, Tile<8>::NT, 0, stream>>>(d, 1.0, X, X, G, tiles);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -278,8 +355,7 @@ int tgemm_grouped_build(int nprob, const TGemm* g, const void* const* A, const v
                         void* desc_host, int* nout, long long* tiles_out, int* tile_out) {
   GProb* h = static_cast<GProb*>(desc_host);
   int n = 0;
-  long long total[3] = {0, 0, 0};
-  const int edge[3] = {64, 32, 16};
+  long long total[EDGES] = {0, 0, 0, 0};
   for (int p = 0; p < nprob; ++p) {
     Dev d;
     int err = DMRG_OK;
@@ -293,10 +369,10 @@ int tgemm_grouped_build(int nprob, const TGemm* g, const void* const* A, const v
     q.B = B[p];
     q.C = C[p];
     q.start = (long long)g[p].B.n1 * g[p].B.n2;   // batch entries, until the starts are known
-    for (int e = 0; e < 3; ++e) total[e] += q.start * tiles_of(d.M, edge[e]) * tiles_of(d.N, edge[e]);
+    for (int e = 0; e < EDGES; ++e) total[e] += q.start * tiles_of(d.M, EDGE[e]) * tiles_of(d.N, EDGE[e]);
   }
   if (total[0] > 0x7fffffffLL) return DMRG_ERR_ARG;
-  const int bt = pick_tile(total[0], total[1], total[2]);
+  const int bt = pick_tile(total);
   long long tiles = 0;
   for (int i = 0; i < n; ++i) {
     GProb& q = h[i];
@@ -319,7 +395,8 @@ int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, int tile,
   const GProb* p = static_cast<const GProb*>(desc_dev);
   if (tile == 64) tgemm_grouped_kernel<T, 64><<<(unsigned)tiles, Tile<64>::NT, 0, stream>>>(p, n, alpha, beta);
   else if (tile == 32) tgemm_grouped_kernel<T, 32><<<(unsigned)tiles, Tile<32>::NT, 0, stream>>>(p, n, alpha, beta);
-  else tgemm_grouped_kernel<T, 16><<<(unsigned)tiles, Tile<16>::NT, 0, stream>>>(p, n, alpha, beta);
+  else if (tile == 16) tgemm_grouped_kernel<T, 16><<<(unsigned)tiles, Tile<16>::NT, 0, stream>>>(p, n, alpha, beta);
+  else tgemm_grouped_kernel<T, 8><<<(unsigned)tiles, Tile<8>::NT, 0, stream>>>(p, n, alpha, beta);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }

@@ -1,5 +1,5 @@
-"""The CUDA-core FP64 contraction at the edges of its three output tiles
-(16, 32, 64), against NumPy.
+"""The CUDA-core FP64 contraction at the edges of its output tiles
+(8, 16, 32, 64), against NumPy.
 
 Bound: both sums run over K products in FP64 in some order, so each errs by
 at most K 2^-53 sum |a| |b| (complex: 2 K products per part)."""
@@ -11,10 +11,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# 16: few outputs; 32: just under 152 tiles of 32 x 32; 64: many tiles of 64 x 64
+# 8 and 16: few outputs; 32: just under 152 tiles of 32 x 32; 64: many tiles of 64 x 64
 @pytest.mark.parametrize("cplx", [False, True])
-@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (17, 33, 15), (16, 16, 32), (150, 30, 120), (380, 17, 383),
-                                   (1500, 20, 1601)])
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (17, 33, 15), (8, 32, 16), (60, 60, 60), (9, 150, 31), (150, 30, 120),
+                                   (380, 17, 383), (1500, 20, 1601)])
 def test_cuda_core_product_tiles(m, k, n, cplx):
     import torch
     from dmrgpy_gb300 import _lib
