@@ -101,15 +101,88 @@ __device__ __forceinline__ void gram2<cplx>(const cplx* xp, const cplx* xq, int 
   }
 }
 
-// apply X <- X J on columns (p, q): J = [[c, s e], [-s conj(e), c]]
+// Sums of four values over the warp, every lane with all of them: the first
+// two steps also halve what a lane carries, 6 FP64 adds instead of 20 (an FP64
+// warp instruction occupies its sub-partition for 64 clocks on GB300, and
+// these sums and the rotation's scalars, not the columns, were most of a
+// round).
+__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
+  const int lane = threadIdx.x & 31;
+  const bool h4 = lane & 16, h3 = lane & 8;
+  const double k0 = h4 ? c : a, s0 = h4 ? a : c, k1 = h4 ? d : b, s1 = h4 ? b : d;
+  const double r0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 16), r1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
+  double r = (h3 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, h3 ? r0 : r1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  a = __shfl_sync(0xffffffffu, r, 0);
+  b = __shfl_sync(0xffffffffu, r, 8);
+  c = __shfl_sync(0xffffffffu, r, 16);
+  d = __shfl_sync(0xffffffffu, r, 24);
+}
+
+// Rotation of a column pair from its Gram block (al = |x_p|^2, be = |x_q|^2,
+// g = x_p^H x_q): cs and se = sn g/|g|; false where the coupling is below tol
+// relative to the pair, below the absolute floor, or nothing.  The scalars
+// come from FP32 seeds refined in FP64 (t to ~1e-14: what it misses is left
+// to the next sweep; cs to rounding: the rotations stay orthonormal), about
+// 20 FP64 instructions where square roots and divisions take 100.
 template <typename T>
-__device__ __forceinline__ void rot_cols(T* xp, T* xq, int r, int lane, double c, double s, T e) {
-  const T se = Sc<T>::scale(e, s);
-  const T sce = Sc<T>::scale(Sc<T>::conj(e), s);
+__device__ __forceinline__ bool pair_rotation(double al, double be, double gre, double gim, double tol, double floor_,
+                                              double& cs, T& se) {
+  // the pair scaled by a power of two so that the larger norm is in [1, 2)
+  const int ex = max(__double2hiint(al), __double2hiint(be)) >> 20;
+  if (ex <= 0 || ex >= 2046) return false;   // nothing there, or not finite (the norms report that)
+  const double sc = __hiloint2double((2046 - ex) << 20, 0);
+  al *= sc;
+  be *= sc;
+  gre *= sc;
+  double ag, inv = 0.0;
+  if (sizeof(T) == 8) {
+    ag = fabs(gre);
+  } else {
+    gim *= sc;
+    const double g2 = fma(gre, gre, gim * gim);
+    if (!(g2 > 1e-290)) return false;
+    inv = rsqrt(g2);
+    ag = g2 * inv;
+  }
+  if (!(ag > floor_ * sc) || !(ag * ag > tol * tol * (al * be)) || !(ag > 1e-290)) return false;
+  const double d = be - al;
+  // t = tan of the angle, the smaller root of ag t^2 + d t - ag = 0
+  const float df = narrow(d), gf = narrow(ag);
+  double t;
+  if (gf > 1e-30f) {
+    const float tf = copysignf(__fdividef(2.f * gf, fabsf(df) + sqrtf(fmaf(df, df, 4.f * gf * gf))), df);
+    t = widen(tf);
+    const double f = fma(t, fma(ag, t, d), -ag);
+    t = fma(-f, widen(__fdividef(1.f, fmaf(2.f * gf, tf, df))), t);
+  } else {
+    t = ag / d;
+  }
+  const double w = fma(t, t, 1.0), hw = 0.5 * w;
+  double y = widen(rsqrtf(narrow(w)));
+  y = y * fma(-hw * y, y, 1.5);
+  y = y * fma(-hw * y, y, 1.5);
+  cs = y;
+  const double sn = t * y;
+  se = sizeof(T) == 8 ? Sc<T>::make(gre < 0.0 ? -sn : sn, 0.0) : Sc<T>::make(sn * (gre * inv), sn * (gim * inv));
+  return true;
+}
+
+// apply X <- X J on columns (p, q): J = [[c, se], [-conj(se), c]]
+__device__ __forceinline__ void rot_cols(double* xp, double* xq, int r, int lane, double c, double se) {
   for (int i = lane; i < r; i += 32) {
-    T a = xp[i], b = xq[i];
-    xp[i] = Sc<T>::sub(Sc<T>::scale(a, c), Sc<T>::mul(sce, b));
-    xq[i] = Sc<T>::add(Sc<T>::mul(se, a), Sc<T>::scale(b, c));
+    const double a = xp[i], b = xq[i];
+    xp[i] = fma(a, c, -se * b);
+    xq[i] = fma(b, c, se * a);
+  }
+}
+__device__ __forceinline__ void rot_cols(cplx* xp, cplx* xq, int r, int lane, double c, cplx se) {
+  for (int i = lane; i < r; i += 32) {
+    const cplx a = xp[i], b = xq[i];
+    // c a - conj(se) b and se a + c b
+    xp[i] = make_cuDoubleComplex(fma(c, a.x, fma(-se.x, b.x, -se.y * b.y)), fma(c, a.y, fma(-se.x, b.y, se.y * b.x)));
+    xq[i] = make_cuDoubleComplex(fma(c, b.x, fma(se.x, a.x, -se.y * a.y)), fma(c, b.y, fma(se.x, a.y, se.y * a.x)));
   }
 }
 
@@ -160,25 +233,17 @@ __global__ void __launch_bounds__(1024) hestenes_kernel(HArgs<T> a) {
         T* xq = a.X + (long long)q * a.r;
         double al, be, gre, gim;
         gram2<T>(xp, xq, a.r, lane, al, be, gre, gim);
-        al = warp_sum(al);
-        be = warp_sum(be);
-        gre = warp_sum(gre);
-        gim = warp_sum(gim);
-        double ag = sqrt(gre * gre + gim * gim);
-        double scale = sqrt(al) * sqrt(be);  // no overflow of the product
+        warp_sum4(al, be, gre, gim);
         // rotate only couplings above tol relative to the pair and above an
         // absolute floor (1e-16 |M|_F^2): singular values come out to the
         // absolute accuracy of a standard SVD without chasing the relative
         // accuracy of negligible ones, which costs many extra sweeps on the
         // steeply graded spectra of DMRG bonds
-        if (!(ag > a.tol * scale) || !(ag > abs_floor) || !(ag > 1e-300)) continue;
-        double tau = (be - al) / (2.0 * ag);
-        double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-        double cs = 1.0 / sqrt(1.0 + t * t);
-        double sn = t * cs;
-        T e = Sc<T>::make(gre / ag, gim / ag);
-        rot_cols<T>(xp, xq, a.r, lane, cs, sn, e);
-        rot_cols<T>(a.V + (long long)p * a.c, a.V + (long long)q * a.c, a.c, lane, cs, sn, e);
+        double cs;
+        T se;
+        if (!pair_rotation<T>(al, be, gre, gim, a.tol, abs_floor, cs, se)) continue;
+        rot_cols(xp, xq, a.r, lane, cs, se);
+        rot_cols(a.V + (long long)p * a.c, a.V + (long long)q * a.c, a.c, lane, cs, se);
         if (lane == 0) atomicAdd(&a.rotcnt[sweep % 3], 1u);
       }
       if (COOP) { if (!grid_barrier(a.bar)) return; } else { __syncthreads(); }
@@ -346,20 +411,12 @@ __global__ void __launch_bounds__(1024) hestenes_batch_kernel(const BSvd<T>* __r
         T* xq = X + (long long)q * r;
         double al, be, gre, gim;
         gram2<T>(xp, xq, r, lane, al, be, gre, gim);
-        al = warp_sum(al);
-        be = warp_sum(be);
-        gre = warp_sum(gre);
-        gim = warp_sum(gim);
-        const double ag = sqrt(gre * gre + gim * gim);
-        const double scale = sqrt(al) * sqrt(be);
-        if (!(ag > tol * scale) || !(ag > abs_floor) || !(ag > 1e-300)) continue;
-        const double tau = (be - al) / (2.0 * ag);
-        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-        const double cs = 1.0 / sqrt(1.0 + t * t);
-        const double sn = t * cs;
-        const T e = Sc<T>::make(gre / ag, gim / ag);
-        rot_cols<T>(xp, xq, r, lane, cs, sn, e);
-        rot_cols<T>(V + (long long)p * c, V + (long long)q * c, c, lane, cs, sn, e);
+        warp_sum4(al, be, gre, gim);
+        double cs;
+        T se;
+        if (!pair_rotation<T>(al, be, gre, gim, tol, abs_floor, cs, se)) continue;
+        rot_cols(xp, xq, r, lane, cs, se);
+        rot_cols(V + (long long)p * c, V + (long long)q * c, c, lane, cs, se);
         if (lane == 0) atomicAdd(&rot, 1u);
       }
       __syncthreads();
