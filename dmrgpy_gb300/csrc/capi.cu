@@ -433,9 +433,10 @@ bool gram_route(int dtype, int m, int n, int absorb) {
   return ck <= 2 * c && ck <= 4096;
 }
 
-size_t svd_total_bytes(int dtype, int m, int n, int absorb) {
+// lean: without the operands of digit products
+size_t svd_total_bytes(int dtype, int m, int n, int absorb, bool lean) {
   size_t b = svd_work_bytes(dtype, m, n);
-  if (gram_route(dtype, m, n, absorb)) b = std::max(b, gram_truncate_workspace_bytes(m, n, absorb));
+  if (gram_route(dtype, m, n, absorb)) b = std::max(b, gram_truncate_workspace_bytes(m, n, absorb, lean));
   return b;
 }
 
@@ -443,7 +444,7 @@ template <typename T>
 int svd_impl(int m, int n, const T* M, double cutoff, int maxdim, int mindim, int absorb, T* lo, T* ro, double* svals,
              int* keep, double* disc, void* work, size_t work_bytes, cudaStream_t s) {
   const int dtype = sizeof(T) == 16 ? DMRG_COMPLEX128 : DMRG_REAL64;
-  if (svd_total_bytes(dtype, m, n, absorb) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (svd_total_bytes(dtype, m, n, absorb, true) > work_bytes) return DMRG_ERR_WORKSPACE;
   if (gram_route(dtype, m, n, absorb)) {
     const int st = gram_truncate(m, n, reinterpret_cast<const double*>(M), cutoff, maxdim, mindim, absorb,
                                  reinterpret_cast<double*>(lo), reinterpret_cast<double*>(ro), svals, keep, disc,
@@ -610,7 +611,7 @@ int dmrg_krylov_expm(const dmrg_heff_t* op, void* x, double coeff_re, double coe
 size_t dmrg_svd_workspace_bytes(int dtype, int m, int n) {
   if (m <= 0 || n <= 0) return 0;
   size_t b = 0;
-  for (int absorb = 0; absorb < 3; ++absorb) b = std::max(b, svd_total_bytes(dtype, m, n, absorb));
+  for (int absorb = 0; absorb < 3; ++absorb) b = std::max(b, svd_total_bytes(dtype, m, n, absorb, false));
   return b;
 }
 
@@ -742,7 +743,9 @@ int dmrg_subspace_truncate_ex(int precision, int m, int n, int k, const void* th
       (kstart > 0 && !start) || (absorb != 0 && absorb != 1) || (precision == DMRG_PREC_FP64 && !svals))
     return DMRG_ERR_ARG;
   if (precision != DMRG_PREC_FP64 && precision != DMRG_PREC_TF32X3) return DMRG_ERR_ARG;
-  if (!work || dmrg_subspace_truncate_ex_workspace_bytes(precision, m, n, k) > work_bytes) return DMRG_ERR_WORKSPACE;
+  const size_t least = precision == DMRG_PREC_FP64 ? rr_truncate_lean_bytes(m, n, k)
+                                                   : dmrg_subspace_truncate_ex_workspace_bytes(precision, m, n, k);
+  if (!work || least > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const double* th = static_cast<const double*>(theta);
   double* lo = static_cast<double*>(left_out);

@@ -798,6 +798,15 @@ int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumul
   return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, s);
 }
 
+int fgemm(const TGemm& g, double alpha, const double* A, const double* B, int accumulate, double* C, void* ws,
+          size_t ws_bytes, cudaStream_t s) {
+  const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
+  if (ws_bytes > 0 && ws && (long long)g.B.n1 * g.B.n2 == 1 && M > 0 && N > 0 && K > 0 &&
+      dg_pays(false, M, N, K, false) && dg_product_bytes<double>(g) <= ws_bytes)
+    return dg_product<double>(g, A, B, alpha, accumulate, C, ws, s);
+  return tgemm<double>(g, alpha, A, B, accumulate ? 1.0 : 0.0, C, s);
+}
+
 template size_t dg_product_bytes<double>(const TGemm&);
 template size_t dg_product_bytes<cplx>(const TGemm&);
 template int dg_product<double>(const TGemm&, const double*, const double*, double, int, double*, void*,

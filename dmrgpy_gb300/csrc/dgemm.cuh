@@ -41,4 +41,9 @@ template <typename T>
 int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumulate, T* C, void* work,
                cudaStream_t s);
 
+// C = alpha A B (+ C), alpha 1 or -1: a digit product where that is faster
+// and ws holds its operands, else on the FP64 pipe
+int fgemm(const TGemm& g, double alpha, const double* A, const double* B, int accumulate, double* C, void* ws,
+          size_t ws_bytes, cudaStream_t s);
+
 }  // namespace dmrg

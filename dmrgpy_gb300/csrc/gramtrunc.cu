@@ -27,6 +27,7 @@
 #include <cstring>
 #include <vector>
 
+#include "dgemm.cuh"
 #include "heff.cuh"
 #include "tf32x3.cuh"
 
@@ -161,30 +162,55 @@ __global__ void gt_half_dev_kernel(const double* __restrict__ G, int k, double* 
     memcpy(&b, &a, sizeof(b));
     if (b > mx) mx = b;
   }
-  if (mx) atomicMax(dev, mx);
+  // one atomic per warp: one per thread kept a 256 x 256 launch busy for 43 us
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx ? v : mx;
+  }
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(dev, mx);
 }
+
+// Operands of digit products (bytes may be 0: products on the FP64 pipe).
+struct Scratch {
+  void* p;
+  size_t bytes;
+};
 
 // C (m x n) = op(A) op(B) in FP64 (tgemm with strides); A is m x k (ld lda)
 // or, transposed, k x m; B is k x n (ldb) or, transposed, n x k
 int gemm64(int tA, int tB, int m, int n, int k, const double* A, long long lda, const double* B, long long ldb,
-           double* C, long long ldc, cudaStream_t s) {
+           double* C, long long ldc, const Scratch& x, cudaStream_t s) {
   TGemm g{};
   g.B = ax(1); g.M = ax(m); g.K = ax(k); g.N = ax(n);
   if (!tA) { g.a_m = st(lda); g.a_k = st(1); } else { g.a_m = st(1); g.a_k = st(lda); }
   if (!tB) { g.b_k = st(ldb); g.b_n = st(1); } else { g.b_k = st(1); g.b_n = st(ldb); }
   g.c_m = st(ldc); g.c_n = st(1);
-  return tgemm<double>(g, 1.0, A, B, 0.0, C, s);
+  return fgemm(g, 1.0, A, B, 0, C, x.p, x.bytes, s);
+}
+
+// scratch that lets gemm64 of this shape run as a digit product (0 where the
+// FP64 pipe is as fast)
+size_t dig_need(long long m, long long n, long long k) {
+  return dg_pays(false, m, n, k, false) ? dg_bytes(0, false, m, k) + dg_bytes(1, false, n, k) : 0;
+}
+
+// G (k x k) = X^T X, X m x k (ld)
+int gram64(const double* X, long long ld, int m, int k, double* G, const Scratch& x, cudaStream_t s) {
+  const size_t need = dig_need(k, k, m);
+  if (need > 0 && x.p && need <= x.bytes) return gemm64(1, 0, k, k, m, X, ld, X, ld, G, k, x, s);
+  return tgemm_gram(X, ld, m, k, G, s);
 }
 
 // C <- C - A B (FP64; A rows x k (ld lda), B k x cols (ld ldb))
 int gemm64_sub(int rows, int cols, int k, const double* A, long long lda, const double* B, long long ldb, double* C,
-               long long ldc, cudaStream_t s) {
+               long long ldc, const Scratch& x, cudaStream_t s) {
   TGemm g{};
   g.B = ax(1); g.M = ax(rows); g.K = ax(k); g.N = ax(cols);
   g.a_m = st(lda); g.a_k = st(1);
   g.b_k = st(ldb); g.b_n = st(1);
   g.c_m = st(ldc); g.c_n = st(1);
-  return tgemm<double>(g, -1.0, A, B, 1.0, C, s);
+  return fgemm(g, -1.0, A, B, 1, C, x.p, x.bytes, s);
 }
 
 }  // namespace
@@ -198,13 +224,18 @@ int sumsq_dev(const double* x, long long n, double* out, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------- full route
-// Workspace: transposed copy (rows route), Gram, Jacobi state, scale vector.
-size_t gram_truncate_workspace_bytes(int m, int n, int absorb) {
+// Workspace: transposed copy (rows route), Gram, scale vector, Jacobi state,
+// operands of digit products (not counted with lean: the products then run
+// on the FP64 pipe).
+size_t gram_truncate_workspace_bytes(int m, int n, int absorb, bool lean) {
   const int rows = absorb == 0 || (absorb == 2 && m <= n);
-  const size_t c = rows ? m : n;
+  const long long c = rows ? m : n, r = rows ? n : m, cmin = std::min(m, n);
   const size_t d = sizeof(double);
-  return align_up(d * (size_t)m * n) + align_up(d * c * c) + syev_jacobi_workspace_bytes((int)c) +
-         align_up(d * c) + 256;
+  const size_t base = align_up(d * (size_t)m * n) + align_up(d * (size_t)(c * c)) + align_up(d * (size_t)c);
+  if (lean) return base + syev_lean_bytes((int)c) + 256;
+  const size_t dig = std::max(std::max(syev_jacobi_workspace_bytes((int)c) - syev_lean_bytes((int)c), dig_need(c, c, r)),
+                              std::max(dig_need(cmin, n, m), dig_need(m, cmin, n)));
+  return base + syev_lean_bytes((int)c) + dig + 256;
 }
 
 // The Gram route of pyitensor/svd.py:108-151 with the keep rule of
@@ -215,7 +246,7 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
                   double* ro, double* svals, int* keep, double* disc, int* sweeps, void* work, size_t work_bytes,
                   cudaStream_t s) {
   if (m <= 0 || n <= 0 || !M || !lo || !ro || absorb < 0 || absorb > 2) return DMRG_ERR_ARG;
-  if (!work || gram_truncate_workspace_bytes(m, n, absorb) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (!work || gram_truncate_workspace_bytes(m, n, absorb, true) > work_bytes) return DMRG_ERR_WORKSPACE;
   const int rows = absorb == 0 || (absorb == 2 && m <= n);
   const int c = rows ? m : n;        // Gram size (kept side)
   const int r = rows ? n : m;        // contracted dimension
@@ -224,15 +255,18 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
   char* p = static_cast<char*>(work);
   double* T = reinterpret_cast<double*>(p); p += align_up(d * (size_t)m * n);
   double* G = reinterpret_cast<double*>(p); p += align_up(d * (size_t)c * c);
-  void* sw = p; p += syev_jacobi_workspace_bytes(c);
-  double* fdev = reinterpret_cast<double*>(p);
-  const size_t sw_bytes = syev_jacobi_workspace_bytes(c);
+  double* fdev = reinterpret_cast<double*>(p); p += align_up(d * (size_t)c);
+  void* sw = p;
+  const size_t sw_bytes = work_bytes - (size_t)(p - static_cast<char*>(work));
+  const Scratch x{static_cast<char*>(sw) + syev_lean_bytes(c), sw_bytes - syev_lean_bytes(c)};
   // G = X^T X with X = M^T (rows route) or M
-  if (rows) {
+  if (rows && dig_need(c, c, r) > 0 && dig_need(c, c, r) <= x.bytes) {
+    DMRG_TRY(gemm64(0, 1, c, c, r, M, n, M, n, G, c, x, s));
+  } else if (rows) {
     DMRG_TRY(gt_transpose(M, n, m, n, T, m, s));   // T = M^T (n x m)
-    DMRG_TRY(tgemm_gram(T, m, r, c, G, s));
+    DMRG_TRY(gram64(T, m, r, c, G, x, s));
   } else {
-    DMRG_TRY(tgemm_gram(M, n, r, c, G, s));
+    DMRG_TRY(gram64(M, n, r, c, G, x, s));
   }
   std::vector<double> w(c);
   DMRG_TRY(syev_jacobi(c, G, c, w.data(), 40, sweeps, sw, sw_bytes, s));
@@ -248,7 +282,7 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
   if (rows) {
     // U = E[:, :keep] (m x keep), right = U^T M (keep x n)
     DMRG_TRY(syev_vectors(c, kp, lo, kp, 0, sw, s));
-    DMRG_TRY(gemm64(1, 0, kp, n, m, lo, kp, M, n, ro, n, s));
+    DMRG_TRY(gemm64(1, 0, kp, n, m, lo, kp, M, n, ro, n, x, s));
     if (absorb == 2) {
       DMRG_CUDA_TRY(cudaMemcpyAsync(fdev, f.data(), d * kp, cudaMemcpyHostToDevice, s));
       DMRG_TRY(gt_scale(ro, n, kp, n, fdev, 1, s));
@@ -256,7 +290,7 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
   } else {
     // V^T = E[:, :keep]^T (keep x n), left = M V (m x keep)
     DMRG_TRY(syev_vectors(c, kp, ro, n, 1, sw, s));
-    DMRG_TRY(gemm64(0, 1, m, kp, n, M, n, ro, n, lo, kp, s));
+    DMRG_TRY(gemm64(0, 1, m, kp, n, M, n, ro, n, lo, kp, x, s));
     if (absorb == 2) {
       DMRG_CUDA_TRY(cudaMemcpyAsync(fdev, f.data(), d * kp, cudaMemcpyHostToDevice, s));
       DMRG_TRY(gt_scale(lo, kp, m, kp, fdev, 0, s));
@@ -312,9 +346,12 @@ struct RRWs {
   unsigned long long* dev;
   void* sw;
   size_t sw_bytes;
+  Scratch x;           // behind the Jacobi state
 };
 
-size_t rr_layout(int m, int n, int k, RRWs* w, void* base) {
+// bytes: what the workspace holds (0 when sizing); lean: without the operands
+// of digit products
+size_t rr_layout(int m, int n, int k, bool lean, size_t bytes, RRWs* w, void* base) {
   const size_t big = (size_t)std::max(m, n);
   const size_t d = sizeof(double);
   char* p = static_cast<char*>(base);
@@ -335,8 +372,17 @@ size_t rr_layout(int m, int n, int k, RRWs* w, void* base) {
   r.f = static_cast<double*>(take(d * k));
   r.acc = static_cast<double*>(take(64));
   r.dev = reinterpret_cast<unsigned long long*>(r.acc + 4);
-  r.sw_bytes = syev_jacobi_workspace_bytes(k);
-  r.sw = take(r.sw_bytes);
+  r.sw = take(syev_lean_bytes(k));
+  const size_t head = off;
+  if (!lean) {
+    const size_t small = std::max(dig_need(k, k, (long long)big), dig_need((long long)big, k, k));
+    size_t dig = std::max(syev_jacobi_workspace_bytes(k) - syev_lean_bytes(k), small);
+    dig = std::max(dig, std::max(dig_need(m, k, n), dig_need(n, k, m)));
+    dig = std::max(dig, std::max(dig_need(k, n, m), dig_need(k, m, n)));
+    take(dig);
+  }
+  r.x = Scratch{p ? p + head : nullptr, bytes > head ? bytes - head : 0};
+  r.sw_bytes = syev_lean_bytes(k) + r.x.bytes;
   if (w) *w = r;
   return off;
 }
@@ -364,7 +410,7 @@ int count_nonnull(const std::vector<double>& lam, int k, double null = 1e-13) {
 // Gram of Z (rows x kz, ld) and its eigenpairs (host lam, descending; the
 // vectors stay in the Jacobi workspace)
 int rr_ritz(const double* Z, long long ld, int rows, int kz, RRWs& w, std::vector<double>& lam, cudaStream_t s) {
-  DMRG_TRY(tgemm_gram(Z, ld, rows, kz, w.G, s));
+  DMRG_TRY(gram64(Z, ld, rows, kz, w.G, w.x, s));
   lam.assign(kz, 0.0);
   return syev_jacobi(kz, w.G, kz, lam.data(), 40, nullptr, w.sw, w.sw_bytes, s);
 }
@@ -377,7 +423,7 @@ int rr_ritz(const double* Z, long long ld, int rows, int kz, RRWs& w, std::vecto
 int rr_basis(const double* Z, long long ld, int rows, int kz, int nc, const std::vector<double>& lam, double* out,
              double* tmp, RRWs& w, double** result, cudaStream_t s) {
   DMRG_TRY(syev_vectors(kz, nc, w.E, nc, 0, w.sw, s));
-  DMRG_TRY(gemm64(0, 0, rows, nc, kz, Z, ld, w.E, nc, out, ld, s));
+  DMRG_TRY(gemm64(0, 0, rows, nc, kz, Z, ld, w.E, nc, out, ld, w.x, s));
   std::vector<double> f(nc);
   for (int j = 0; j < nc; ++j) f[j] = 1.0 / std::sqrt(lam[j]);
   DMRG_CUDA_TRY(cudaMemcpyAsync(w.f, f.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, s));
@@ -388,7 +434,7 @@ int rr_basis(const double* Z, long long ld, int rows, int kz, int nc, const std:
   double dev = 1.0;
   bool second = false;
   for (int it = 0; it < 6; ++it) {
-    DMRG_TRY(tgemm_gram(X, ld, rows, nc, w.G, s));
+    DMRG_TRY(gram64(X, ld, rows, nc, w.G, w.x, s));
     DMRG_CUDA_TRY(cudaMemsetAsync(w.dev, 0, sizeof(unsigned long long), s));
     gt_half_dev_kernel<<<grid1((long long)nc * nc), 256, 0, s>>>(w.G, nc, w.B, w.dev);
     DMRG_CHECK_LAUNCH();
@@ -403,7 +449,7 @@ int rr_basis(const double* Z, long long ld, int rows, int kz, int nc, const std:
       DMRG_TRY(syev_jacobi(nc, w.G, nc, l2.data(), 40, nullptr, w.sw, w.sw_bytes, s));
       if (!(l2[nc - 1] > 1e-8)) return DMRG_ERR_NOCONV;
       DMRG_TRY(syev_vectors(nc, nc, w.E, nc, 0, w.sw, s));
-      DMRG_TRY(gemm64(0, 0, rows, nc, nc, X, ld, w.E, nc, Y, ld, s));
+      DMRG_TRY(gemm64(0, 0, rows, nc, nc, X, ld, w.E, nc, Y, ld, w.x, s));
       for (int j = 0; j < nc; ++j) f[j] = 1.0 / std::sqrt(l2[j]);
       DMRG_CUDA_TRY(cudaMemcpyAsync(w.f, f.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, s));
       DMRG_TRY(gt_scale(Y, ld, rows, nc, w.f, 0, s));
@@ -411,7 +457,7 @@ int rr_basis(const double* Z, long long ld, int rows, int kz, int nc, const std:
       std::swap(X, Y);
       continue;
     }
-    DMRG_TRY(gemm64(0, 0, rows, nc, nc, X, ld, w.B, nc, Y, ld, s));
+    DMRG_TRY(gemm64(0, 0, rows, nc, nc, X, ld, w.B, nc, Y, ld, w.x, s));
     std::swap(X, Y);
   }
   *result = X;
@@ -430,8 +476,8 @@ int rr_complete(double* U, long long ld, int rows, int nz, int nc, double* spare
   gt_random_kernel<<<grid1((long long)rows * r), 256, 0, s>>>(U, ld, rows, nz, nc, 0xc0ffee5eedULL + rows);
   DMRG_CHECK_LAUNCH();
   for (int pass = 0; pass < 2 && nz > 0; ++pass) {
-    DMRG_TRY(gemm64(1, 0, nz, r, rows, U, ld, R, ld, w.B, r, s));         // T = U^T R  (nz x r)
-    DMRG_TRY(gemm64_sub(rows, r, nz, U, ld, w.B, r, R, ld, s));          // R -= U T
+    DMRG_TRY(gemm64(1, 0, nz, r, rows, U, ld, R, ld, w.B, r, w.x, s));         // T = U^T R  (nz x r)
+    DMRG_TRY(gemm64_sub(rows, r, nz, U, ld, w.B, r, R, ld, w.x, s));          // R -= U T
   }
   std::vector<double> lam;
   DMRG_TRY(rr_ritz(R, ld, rows, r, w, lam, s));
@@ -445,8 +491,10 @@ int rr_complete(double* U, long long ld, int rows, int nz, int nc, double* spare
 
 size_t rr_truncate_workspace_bytes(int m, int n, int k) {
   if (m <= 0 || n <= 0 || k <= 0) return 0;
-  return rr_layout(m, n, k, nullptr, nullptr);
+  return rr_layout(m, n, k, false, 0, nullptr, nullptr);
 }
+
+size_t rr_truncate_lean_bytes(int m, int n, int k) { return rr_layout(m, n, k, true, 0, nullptr, nullptr); }
 
 // theta (m x n).  absorb 0 keeps an orthonormal LEFT basis, X = the right
 // tensor across the bond (kx x n, orthonormal rows); absorb 1 keeps a RIGHT
@@ -460,9 +508,9 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
   if (m <= 0 || n <= 0 || k <= 0 || k > std::min(m, n) || kx < 0 || kx > k || (kx > 0 && !X) || iters < 1 ||
       iters > 8 || !theta || !lo || !ro || (absorb != 0 && absorb != 1))
     return DMRG_ERR_ARG;
-  if (!work || rr_truncate_workspace_bytes(m, n, k) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (!work || rr_truncate_lean_bytes(m, n, k) > work_bytes) return DMRG_ERR_WORKSPACE;
   RRWs w;
-  rr_layout(m, n, k, &w, work);
+  rr_layout(m, n, k, true, work_bytes, &w, work);
   const double nul = null_fraction(cutoff);
   const double* Th = theta;
   int M = m, N = n;
@@ -503,14 +551,14 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
   int kp = 0;
   for (int round = 0;; ++round) {
     for (int it = 0;; ++it) {
-      DMRG_TRY(gemm64(0, 0, M, kw, N, Th, N, w.W, k, w.Z, k, s));   // Z = Th W
+      DMRG_TRY(gemm64(0, 0, M, kw, N, Th, N, w.W, k, w.Z, k, w.x, s));   // Z = Th W
       DMRG_TRY(rr_ritz(w.Z, k, M, kw, w, lam, s));
       const int nz = count_nonnull(lam, kw, nul);
       if (nz < 1) return DMRG_ERR_NOCONV;
       if (it + 1 >= (round == 0 ? iters : 1)) break;
       // W = orth(Th^T orth(Z))
       DMRG_TRY(rr_basis(w.Z, k, M, kw, nz, lam, w.Z2, w.W, w, &res, s));
-      DMRG_TRY(gemm64(1, 0, N, nz, M, Th, N, res, k, w.Z, k, s));
+      DMRG_TRY(gemm64(1, 0, N, nz, M, Th, N, res, k, w.Z, k, w.x, s));
       DMRG_TRY(rr_ritz(w.Z, k, N, nz, w, lam, s));
       kw = count_nonnull(lam, nz, nul);
       if (kw < 1) return DMRG_ERR_NOCONV;
@@ -524,7 +572,7 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
     double* other = res == w.Z2 ? w.W : w.Z2;
     if (kw > nz) DMRG_TRY(rr_complete(res, k, M, nz, kw, w.Z, other, w, s));
     C = other;
-    DMRG_TRY(gemm64(1, 0, kw, N, M, res, k, Th, N, C, N, s));              // C = U^T Th (kw x N)
+    DMRG_TRY(gemm64(1, 0, kw, N, M, res, k, Th, N, C, N, w.x, s));              // C = U^T Th (kw x N)
     // the weight of theta along each kept direction, |C_j|^2 = u_j^T theta
     // theta^T u_j (one power beyond the Ritz value, and exactly what the
     // truncation keeps); the rule of pyitensor/svd.py:32-68 runs on these,
@@ -545,7 +593,7 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
     const bool near = rem < 10.0 * cutoff + 1e-11;
     if (!(cutoff > 0.0 && (kp < kw || near) && round < 2)) break;
     // W = orth(Th^T U), then the next round from it
-    DMRG_TRY(gemm64(1, 0, N, kw, M, Th, N, res, k, w.Z, k, s));
+    DMRG_TRY(gemm64(1, 0, N, kw, M, Th, N, res, k, w.Z, k, w.x, s));
     const int kz = kw;
     DMRG_TRY(rr_ritz(w.Z, k, N, kz, w, lam, s));
     kw = count_nonnull(lam, kz, nul);
@@ -558,14 +606,14 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
     // the cutoff binds: the rule needs the singular values of theta within
     // the kept space, not the weights of a basis only approximately aligned
     // with them -- Ritz pairs of theta theta^T on span(U) from C C^T (FP64)
-    DMRG_TRY(gemm64(0, 1, kw, kw, N, C, N, C, N, w.G, kw, s));
+    DMRG_TRY(gemm64(0, 1, kw, kw, N, C, N, C, N, w.G, kw, w.x, s));
     std::vector<double> l2(kw);
     DMRG_TRY(syev_jacobi(kw, w.G, kw, l2.data(), 40, nullptr, w.sw, w.sw_bytes, s));
     double dc;
     keep_rule_partial(l2.data(), kw, std::min(m, n), hacc, cutoff, k, std::max(1, mindim), -1.0, &kp, &dc);
     DMRG_TRY(syev_vectors(kw, kp, w.E, kp, 0, w.sw, s));
-    DMRG_TRY(gemm64(0, 0, M, kp, kw, U, k, w.E, kp, w.Z, k, s));       // U E   (M x kp)
-    DMRG_TRY(gemm64(1, 0, kp, N, kw, w.E, kp, C, N, U, N, s));         // E^T C (kp x N)
+    DMRG_TRY(gemm64(0, 0, M, kp, kw, U, k, w.E, kp, w.Z, k, w.x, s));       // U E   (M x kp)
+    DMRG_TRY(gemm64(1, 0, kp, N, kw, w.E, kp, C, N, U, N, w.x, s));         // E^T C (kp x N)
     C = U;
     U = w.Z;
     wt.assign(l2.begin(), l2.end());
@@ -591,7 +639,7 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
 size_t subspace_ritz_workspace_bytes(int m, int n, int k) {
   const size_t d = sizeof(double);
   const size_t big = (size_t)std::max(m, n);
-  return align_up(64) + align_up(d * big * k) + align_up(d * (size_t)k * k) + syev_jacobi_workspace_bytes(k) +
+  return align_up(64) + align_up(d * big * k) + align_up(d * (size_t)k * k) + syev_lean_bytes(k) +
          gram_digits_workspace_bytes((int)big, k) + align_up(64);
 }
 
@@ -610,8 +658,8 @@ int subspace_ritz(int m, int n, int k, int absorb, double* lo, double* ro, doubl
   int* err = reinterpret_cast<int*>(p); p += align_up(64);
   double* T1 = reinterpret_cast<double*>(p); p += align_up(d * big * k);
   double* G = reinterpret_cast<double*>(p); p += align_up(d * (size_t)k * k);
-  void* sw = p; p += syev_jacobi_workspace_bytes(k);
-  void* gw = p;
+  void* gw = p; p += gram_digits_workspace_bytes((int)big, k);
+  void* sw = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
   const size_t gw_bytes = gram_digits_workspace_bytes((int)big, k);
   DMRG_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), s));
   if (absorb == 0) {
@@ -621,7 +669,7 @@ int subspace_ritz(int m, int n, int k, int absorb, double* lo, double* ro, doubl
     DMRG_TRY(gram_digits(lo, k, m, k, G, gw, gw_bytes, err, s));
   }
   std::vector<double> lam(k);
-  DMRG_TRY(syev_jacobi(k, G, k, lam.data(), 40, nullptr, sw, syev_jacobi_workspace_bytes(k), s, 1));
+  DMRG_TRY(syev_jacobi(k, G, k, lam.data(), 40, nullptr, sw, syev_lean_bytes(k), s, 1));
   int e = 0;
   DMRG_CUDA_TRY(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));

@@ -56,6 +56,7 @@ void keep_rule_partial(const double* lam, int k, int c, double total, double cut
 // symmetric eigendecomposition by blocked Jacobi (syev.cu): eigenvalues to
 // the host (descending), eigenvectors gathered afterwards from the workspace
 size_t syev_jacobi_workspace_bytes(int n);
+size_t syev_lean_bytes(int n);   // without the operands of digit products
 int syev_jacobi(int n, const double* A, long long lda, double* w, int max_sweeps, int* sweeps, void* work,
                 size_t work_bytes, cudaStream_t s, int fp32 = 0);
 int syev_vectors(int n, int ncols, double* out, long long ldo, int transposed, void* work, cudaStream_t s,
@@ -64,11 +65,12 @@ int syev_vectors(int n, int ncols, double* out, long long ldo, int transposed, v
 // Gram-matrix truncation (gramtrunc.cu)
 constexpr int GRAM_FALLBACK = 100;   // internal: use the exact SVD instead
 int sumsq_dev(const double* x, long long n, double* out, cudaStream_t s);
-size_t gram_truncate_workspace_bytes(int m, int n, int absorb);
+size_t gram_truncate_workspace_bytes(int m, int n, int absorb, bool lean);
 int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int mindim, int absorb, double* lo,
                   double* ro, double* svals, int* keep, double* disc, int* sweeps, void* work, size_t work_bytes,
                   cudaStream_t s);
 size_t rr_truncate_workspace_bytes(int m, int n, int k);
+size_t rr_truncate_lean_bytes(int m, int n, int k);   // without the operands of digit products
 int rr_truncate(int m, int n, int k, const double* theta, const double* X, int kx, int absorb, int iters,
                 double cutoff, int mindim, double* lo, double* ro, double* svals, int* nvals, int* keep, double* disc,
                 void* work, size_t work_bytes, cudaStream_t s);

@@ -25,17 +25,22 @@
 // its blocks are skipped by the apply.  The sweep loop stops when a full
 // sweep rotated nothing.
 //
-// Two element types: FP64 (the Gram route and the FP64 subspace route) and
-// FP32 (the Ritz values of the split-TF32 truncation, whose inputs are
-// FP32-accurate anyway; FP32 runs at 64x the FP64 rate on GB300, where FP64
-// is ~2 FMA per clock per SM and bounds the FP64 apply at 8 n^3 FLOP per
-// sweep).
+// Two element types.  FP32 runs at 64x the FP64 rate on GB300 (FP64 is ~2 FMA
+// per clock per SM), so the FP64 eigenproblem is solved by FP32 sweeps
+// between FP64 products (syev_passes): the sweeps diagonalise
+// G = V^T A V rounded to FP32, whose off-diagonals after the first pass are
+// small and elementwise accurate, so each pass gains about six digits; the
+// products (V Q, the Newton-Schulz steps that keep V orthonormal, V^T A V) are
+// FP64, on the tensor cores where that pays.  FP64 sweeps finish what the
+// passes leave (nothing, normally).  FP32 alone serves the Ritz values of the
+// split-TF32 truncation.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <numeric>
 #include <vector>
 
+#include "dgemm.cuh"
 #include "heff.cuh"
 
 namespace dmrg {
@@ -68,13 +73,16 @@ struct SyevWs {
   double* R;                 // npair x 32 x 32: D = R - I of each pair
   int* ident;                // npair
   int* pairs;                // (nb-1) x npair x 2
-  int* flag;                 // [0] rotating subproblems in the sweep
-  unsigned long long* scale; // max |a_ii| as ordered bits
+  int* flag;                 // [0] rotating subproblems in the sweep, [1] those with a large rotation
+  unsigned long long* scale; // max |a_ii| as ordered bits; then two words of the passes
   double* diag;              // np
+  float2* dd;                // np: diagonal of an FP32 run as hi + lo
   int* perm;                 // np
+  void* dig;                 // operands of a digit product (np x np by np x np)
+  size_t dig_bytes;          // 0: not held, products on the FP64 pipe
 };
 
-size_t syev_layout(int n, SyevWs* w, void* base) {
+size_t syev_layout(int n, SyevWs* w, void* base, bool lean) {
   const int np = (n + JP - 1) / JP * JP;
   const int nb = np / JB, npair = nb / 2;
   char* p = static_cast<char*>(base);
@@ -93,23 +101,39 @@ size_t syev_layout(int n, SyevWs* w, void* base) {
   s.ident = static_cast<int*>(take(sizeof(int) * npair));
   s.pairs = static_cast<int*>(take(sizeof(int) * 2 * (size_t)(nb - 1 > 0 ? nb - 1 : 1) * npair));
   s.flag = static_cast<int*>(take(sizeof(int) * 4));
-  s.scale = static_cast<unsigned long long*>(take(sizeof(unsigned long long)));
+  s.scale = static_cast<unsigned long long*>(take(3 * sizeof(unsigned long long)));
   s.diag = static_cast<double*>(take(sizeof(double) * np));
+  s.dd = static_cast<float2*>(take(sizeof(float2) * np));
   s.perm = static_cast<int*>(take(sizeof(int) * np));
+  s.dig_bytes = lean || !dg_pays(false, np, np, np, false) ? 0 : dg_bytes(0, false, np, np) + dg_bytes(1, false, np, np);
+  s.dig = take(s.dig_bytes);
   if (w) *w = s;
   return off;
 }
 
+__device__ __forceinline__ float2 hi_lo(double v) {
+  const float h = (float)v;
+  return make_float2(h, (float)(v - (double)h));
+}
+
+// G = A 2^-e (padded), V = I, *scale = max |g_ii| as ordered bits; with
+// `norm` (max |a_ii| as bits) e is its exponent, so that FP32 holds any A
 template <typename T>
 __global__ void syev_init_kernel(const double* __restrict__ A, long long lda, int n, int np, T* __restrict__ G,
-                                 T* __restrict__ V, unsigned long long* __restrict__ scale) {
+                                 T* __restrict__ V, unsigned long long* __restrict__ scale,
+                                 const unsigned long long* __restrict__ norm, float2* __restrict__ dd) {
   const long long total = (long long)np * np;
   unsigned long long mx = 0;
+  double f = 1.0;
+  if (norm) {
+    const int e = (int)(*norm >> 52);   // 0 for zero, 2047 for inf and nan
+    if (e > 0 && e < 2046) f = __longlong_as_double((long long)(2046 - e) << 52);
+  }
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(e / np), j = (int)(e - (long long)i * np);
     double v = 0.0;
-    if (i < n && j < n) v = A[(long long)i * lda + j];
+    if (i < n && j < n) v = A[(long long)i * lda + j] * f;
     G[e] = (T)v;
     V[e] = i == j ? (T)1 : (T)0;
     if (i == j) {
@@ -118,6 +142,7 @@ __global__ void syev_init_kernel(const double* __restrict__ A, long long lda, in
       unsigned long long b;
       memcpy(&b, &a, sizeof(b));
       if (a == a && b > mx) mx = b;
+      if (sizeof(T) == 4) dd[i] = hi_lo(v);
     }
   }
   if (mx) atomicMax(scale, mx);
@@ -233,6 +258,231 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
   }
 }
 
+// The FP32 form of the solve.  Its rounds are latency-bound (in the FP64 form
+// two barriers and the divide, square root and broadcast of a rotation in a
+// chain, 0.6 us), so every thread computes the rotation of its column pair
+// itself, from approximate reciprocals with a Newton step on c (the FP64
+// products between passes restore what FP32 loses), takes that of its row
+// pair from the lane that holds it, and the matrix is double-buffered: one
+// barrier per round.  rel and abs as JacTol on a matrix scaled to O(1);
+// flag[0] counts pairs that rotated, flag[1] pairs with a rotation above
+// BIG_SIN.
+constexpr float BIG_SIN = 1e-2f;
+
+__device__ __forceinline__ float rsq32(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp32(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Rotation of [app apq; apq aqq] with the diagonal as hi + lo pairs: t = tan
+// of the smaller angle, 0 below the thresholds; c, s and cm = c - 1 from it.
+// No branches.  The difference of the diagonals needs the low parts: spectra
+// have multiplets, and where two eigenvalues agree to more than FP32's eight
+// digits their difference in FP32 is one of its places or nothing, so that
+// each pass shrank the pair's off-diagonal by a factor of two or three only.
+__device__ __forceinline__ void rot32(float2 app, float2 aqq, float apq, float rel, float floor_, float& t, float& c,
+                                      float& s, float& cm) {
+  const bool act = fabsf(apq) > floor_ && apq * apq > fabsf(rel * app.x) * fabsf(rel * aqq.x);
+  // t = 2 apq / (d + sign(d) sqrt(d^2 + 4 apq^2)), d = aqq - app
+  const float d = (aqq.x - app.x) + (aqq.y - app.y), g = 2.f * apq;
+  const float u = fmaf(d, d, g * g);
+  const float q = (d < 0.f ? -g : g) * rcp32(fmaf(u, rsq32(u), fabsf(d)));
+  t = act ? q : 0.f;
+  const float w = fmaf(t, t, 1.f);
+  const float e = rsq32(w);
+  c = e * fmaf(-0.5f * w * e, e, 1.5f);
+  s = t * c;
+  cm = -s * s * rcp32(1.f + c);
+}
+
+// (hi, lo) + x
+__device__ __forceinline__ float2 add_hl(float2 a, float x) {
+  const float h = a.x + x, b = h - a.x;
+  const float l = a.y + ((a.x - (h - b)) + (x - b));
+  const float r = h + l;
+  return make_float2(r, l - (r - h));
+}
+
+__global__ void __launch_bounds__(256) syev_solve32_kernel(const float* __restrict__ G, int np,
+                                                           const int* __restrict__ pr, float* __restrict__ R,
+                                                           int* __restrict__ ident, int* __restrict__ flag,
+                                                           const unsigned long long* __restrict__ scale,
+                                                           float2* __restrict__ dd, float rel, float abs_) {
+  __shared__ float a[2][JP][JLD];
+  __shared__ float2 dg[2][JP];
+  __shared__ float r[JP][JLD];
+  const int pair = blockIdx.x;
+  const int bi = pr[2 * pair], bj = pr[2 * pair + 1];
+  const int tid = threadIdx.x;
+  const float floor_ = abs_ * (float)__longlong_as_double((long long)*scale);
+  for (int e = tid; e < JP * JP; e += blockDim.x) {
+    const int i = e / JP, j = e - (e / JP) * JP;
+    const int gi = i < JB ? bi * JB + i : bj * JB + i - JB;
+    const int gj = j < JB ? bi * JB + j : bj * JB + j - JB;
+    a[0][i][j] = G[(long long)gi * np + gj];
+    r[i][j] = 0.f;
+  }
+  // the diagonal lives in dd (the apply's copy in G is not used)
+  if (tid < JP) dg[0][tid] = dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB];
+  const int ti = tid >> 4, tj = tid & 15;
+  // tournament positions ti, 31 - ti (rows) and tj, 31 - tj (columns)
+  int pi = tour(ti, 0), qi = tour(JP - 1 - ti, 0), pj = tour(tj, 0), qj = tour(JP - 1 - tj, 0);
+  bool rotated = false, big = false;
+  __syncthreads();
+  for (int ir = 0; ir < JP - 1; ++ir) {
+    const float(*x)[JLD] = a[ir & 1];
+    float(*z)[JLD] = a[(ir & 1) ^ 1];
+    const float2 app = dg[ir & 1][pj], aqq = dg[ir & 1][qj];
+    const float apq = x[pj][qj];
+    const float x00 = x[pi][pj], x01 = x[pi][qj], x10 = x[qi][pj], x11 = x[qi][qj];
+    const float u0 = r[ti][pj], v0 = r[ti][qj], u1 = r[ti + 16][pj], v1 = r[ti + 16][qj];
+    float tj_, cj, sj, cmj;
+    rot32(app, aqq, apq, rel, floor_, tj_, cj, sj, cmj);
+    // lane l of a warp holds column pair l % 16, so row pair ti's rotation
+    const float si = __shfl_sync(0xffffffffu, sj, ti), cmi = __shfl_sync(0xffffffffu, cmj, ti);
+    rotated = rotated || si != 0.f;
+    big = big || fabsf(si) > BIG_SIN;
+    // x + (J^T x J - x) through c - 1, so that a small rotation rounds at its own size
+    const float y00 = x00 + (cmi * x00 - si * x10), y01 = x01 + (cmi * x01 - si * x11);
+    const float y10 = x10 + (si * x00 + cmi * x10), y11 = x11 + (si * x01 + cmi * x11);
+    float z00 = y00 + (cmj * y00 - sj * y01), z01 = y01 + (sj * y00 + cmj * y01);
+    float z10 = y10 + (cmj * y10 - sj * y11), z11 = y11 + (sj * y10 + cmj * y11);
+    if (ti == tj) {   // the rotated pair itself
+      dg[(ir & 1) ^ 1][pj] = add_hl(app, -tj_ * apq);
+      dg[(ir & 1) ^ 1][qj] = add_hl(aqq, tj_ * apq);
+      z01 = z10 = sj != 0.f ? 0.f : x01;
+    }
+    z[pi][pj] = z00;
+    z[pi][qj] = z01;
+    z[qi][pj] = z10;
+    z[qi][qj] = z11;
+    // D <- D J + (J - I) on columns pj, qj, rows ti and ti + 16
+    float a0 = fmaf(cmj, u0, u0) - sj * v0, b0 = fmaf(sj, u0, fmaf(cmj, v0, v0));
+    float a1 = fmaf(cmj, u1, u1) - sj * v1, b1 = fmaf(sj, u1, fmaf(cmj, v1, v1));
+    if (ti == pj) { a0 += cmj; b0 += sj; }
+    if (ti == qj) { a0 -= sj; b0 += cmj; }
+    if (ti + 16 == pj) { a1 += cmj; b1 += sj; }
+    if (ti + 16 == qj) { a1 -= sj; b1 += cmj; }
+    r[ti][pj] = a0;
+    r[ti][qj] = b0;
+    r[ti + 16][pj] = a1;
+    r[ti + 16][qj] = b1;
+    // next round: every position but 0 moves on by one
+    pi = ti == 0 ? 0 : (pi == JP - 1 ? 1 : pi + 1);
+    pj = tj == 0 ? 0 : (pj == JP - 1 ? 1 : pj + 1);
+    qi = qi == JP - 1 ? 1 : qi + 1;
+    qj = qj == JP - 1 ? 1 : qj + 1;
+    __syncthreads();
+  }
+  const int any = __syncthreads_or(rotated);
+  const int anybig = __syncthreads_or(big);
+  float* Rp = R + (size_t)pair * JP * JP;
+  for (int e = tid; e < JP * JP; e += blockDim.x) Rp[e] = r[e / JP][e % JP];
+  if (tid < JP) dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB] = dg[(JP - 1) & 1][tid];
+  if (tid == 0) {
+    ident[pair] = any ? 0 : 1;
+    if (any) atomicAdd(flag, 1);
+    if (anybig) atomicAdd(flag + 1, 1);
+  }
+}
+
+// Matrices of one block pair or two (np = 32 or 64): all FP32 sweeps of a pass
+// in one CTA, the matrix and D = Q - I in shared memory; out = Q (FP64,
+// np x np).  Same rounds as syev_solve32_kernel on NP indices.  The blocked
+// form takes three rounds of two launches per sweep at np = 64 (measured, n = 60,
+// all passes: 0.70 ms in its kernels and as much between them).
+template <int NP>
+__global__ void __launch_bounds__(NP * NP / 4) syev_small32_kernel(const double* __restrict__ A, long long lda, int n,
+                                                                   const unsigned long long* __restrict__ norm,
+                                                                   int max_sweeps, float rel, float abs_,
+                                                                   double* __restrict__ out, int* __restrict__ sweeps) {
+  constexpr int LD = NP + 1, H = NP / 2, NT = H * H;
+  extern __shared__ float sm[];
+  float* buf0 = sm;
+  float* buf1 = sm + NP * LD;
+  float* r = sm + 2 * NP * LD;
+  __shared__ float2 dg[2][NP];
+  const int tid = threadIdx.x;
+  double f = 1.0;
+  {
+    const int e = (int)(*norm >> 52);
+    if (e > 0 && e < 2046) f = __longlong_as_double((long long)(2046 - e) << 52);
+  }
+  for (int e = tid; e < NP * NP; e += NT) {
+    const int i = e / NP, j = e % NP;
+    const double v = i < n && j < n ? A[(long long)i * lda + j] * f : 0.0;
+    buf0[i * LD + j] = (float)v;
+    if (i == j) dg[0][i] = hi_lo(v);
+    r[i * LD + j] = 0.f;
+  }
+  __syncthreads();
+  // diagonals scaled by the largest diagonal of the first pass's matrix lie
+  // in [-2, 2]; the floor is relative to 1
+  const float floor_ = abs_;
+  const int ti = tid / H, tj = tid % H;
+  int pi = ti, qi = NP - 1 - ti, pj = tj, qj = NP - 1 - tj;
+  int cur = 0, sw = 0;
+  for (; sw < max_sweeps; ++sw) {
+    bool big = false;
+    for (int ir = 0; ir < NP - 1; ++ir, cur ^= 1) {
+      const float* x = cur ? buf1 : buf0;
+      float* z = cur ? buf0 : buf1;
+      const float x00 = x[pi * LD + pj], x01 = x[pi * LD + qj], x10 = x[qi * LD + pj], x11 = x[qi * LD + qj];
+      const float u0 = r[ti * LD + pj], v0 = r[ti * LD + qj], u1 = r[(ti + H) * LD + pj], v1 = r[(ti + H) * LD + qj];
+      float tj_, cj, sj, cmj;
+      const float2 app = dg[cur][pj], aqq = dg[cur][qj];
+      const float apq = x[pj * LD + qj];
+      rot32(app, aqq, apq, rel, floor_, tj_, cj, sj, cmj);
+      // lane ti of the warp holds row pair ti's rotation (as column pair)
+      const float si = __shfl_sync(0xffffffffu, sj, ti), cmi = __shfl_sync(0xffffffffu, cmj, ti);
+      big = big || fabsf(si) > BIG_SIN;
+      const float y00 = x00 + (cmi * x00 - si * x10), y01 = x01 + (cmi * x01 - si * x11);
+      const float y10 = x10 + (si * x00 + cmi * x10), y11 = x11 + (si * x01 + cmi * x11);
+      float z00 = y00 + (cmj * y00 - sj * y01), z01 = y01 + (sj * y00 + cmj * y01);
+      float z10 = y10 + (cmj * y10 - sj * y11), z11 = y11 + (sj * y10 + cmj * y11);
+      if (ti == tj) {
+        dg[cur ^ 1][pj] = add_hl(app, -tj_ * apq);
+        dg[cur ^ 1][qj] = add_hl(aqq, tj_ * apq);
+        z01 = z10 = sj != 0.f ? 0.f : x01;
+      }
+      z[pi * LD + pj] = z00;
+      z[pi * LD + qj] = z01;
+      z[qi * LD + pj] = z10;
+      z[qi * LD + qj] = z11;
+      float a0 = fmaf(cmj, u0, u0) - sj * v0, b0 = fmaf(sj, u0, fmaf(cmj, v0, v0));
+      float a1 = fmaf(cmj, u1, u1) - sj * v1, b1 = fmaf(sj, u1, fmaf(cmj, v1, v1));
+      if (ti == pj) { a0 += cmj; b0 += sj; }
+      if (ti == qj) { a0 -= sj; b0 += cmj; }
+      if (ti + H == pj) { a1 += cmj; b1 += sj; }
+      if (ti + H == qj) { a1 -= sj; b1 += cmj; }
+      r[ti * LD + pj] = a0;
+      r[ti * LD + qj] = b0;
+      r[(ti + H) * LD + pj] = a1;
+      r[(ti + H) * LD + qj] = b1;
+      pi = ti == 0 ? 0 : (pi == NP - 1 ? 1 : pi + 1);
+      pj = tj == 0 ? 0 : (pj == NP - 1 ? 1 : pj + 1);
+      qi = qi == NP - 1 ? 1 : qi + 1;
+      qj = qj == NP - 1 ? 1 : qj + 1;
+      __syncthreads();
+    }
+    if (!__syncthreads_or(big)) {
+      ++sw;
+      break;
+    }
+  }
+  for (int e = tid; e < NP * NP; e += NT) {
+    const int i = e / NP, j = e % NP;
+    out[e] = (i == j ? 1.0 : 0.0) + (double)r[i * LD + j];
+  }
+  if (tid == 0) *sweeps = sw;
+}
+
 __device__ __forceinline__ int pair_index(int b0, int b1, int l) { return l < JB ? b0 * JB + l : b1 * JB + l - JB; }
 
 // G <- P^T G P on blocks (X, Y), X <= Y (grid part 1, npair^2 CTAs, the
@@ -341,11 +591,36 @@ __global__ void syev_ns_kernel(double* __restrict__ B, int np) {
   }
 }
 
+// out[0] = max over i != j of |g_ij| / max(rel sqrt|g_ii g_jj|, abs max|g_ii|)
+// as ordered bits (out zeroed before; *scale = max |g_ii| as bits; nan counts
+// as infinite)
+__global__ void syev_off_kernel(const double* __restrict__ G, int np, const unsigned long long* __restrict__ scale,
+                                unsigned long long* __restrict__ out) {
+  const long long total = (long long)np * np;
+  const double fl = JacTol<double>::abs * __longlong_as_double((long long)*scale);
+  float mx = 0.f;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(e / np), j = (int)(e - (long long)i * np);
+    if (i >= j) continue;
+    const double g = fabs(G[e]);
+    // the FP64 threshold matters only above the floor
+    if (g <= fl) continue;
+    const double d = sqrt(fabs(G[(long long)i * np + i])) * sqrt(fabs(G[(long long)j * np + j]));
+    const float q = (float)(g / fmax(JacTol<double>::rel * d, fl));
+    mx = q > mx || !(q == q) ? (q == q ? q : INFINITY) : mx;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0 && mx > 0.f) atomicMax(out, (unsigned long long)__float_as_uint(mx));
+}
+
 // *scale = max_i |G_ii| as ordered bits
-__global__ void syev_scale_kernel(const double* __restrict__ G, int np, unsigned long long* __restrict__ scale) {
+__global__ void syev_scale_kernel(const double* __restrict__ G, int np, long long ld,
+                                  unsigned long long* __restrict__ scale) {
   unsigned long long mx = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const double a = fabs(G[(long long)i * np + i]);
+    const double a = fabs(G[(long long)i * ld + i]);
     unsigned long long b;
     memcpy(&b, &a, sizeof(b));
     if (a == a && b > mx) mx = b;
@@ -395,40 +670,52 @@ void tournament(int nb, std::vector<int>& out) {
     }
 }
 
-// sweeps over (G, V) until one rotates nothing (at most max_sweeps)
+inline void solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, double, double, cudaStream_t s) {
+  syev_solve_kernel<double><<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
+}
+inline void solve_launch(SyevWs& ws, const float* G, const int* pr, float* R, double rel, double abs_,
+                         cudaStream_t s) {
+  syev_solve32_kernel<<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd, (float)rel,
+                                                (float)abs_);
+}
+
+// sweeps over (G, V) until one rotates nothing (at most max_sweeps); with
+// small_end, until one rotates by nothing above BIG_SIN
 template <typename T>
-int syev_sweeps(SyevWs& ws, T* G, T* V, int max_sweeps, int* done, int* converged, cudaStream_t s) {
+int syev_sweeps(SyevWs& ws, T* G, T* V, int max_sweeps, double rel, double abs_, bool small_end, int* done,
+                int* converged, cudaStream_t s) {
   const int np = ws.np, npair = ws.npair, rounds = ws.nb - 1;
   T* R = reinterpret_cast<T*>(ws.R);
   const int apply_grid = npair * npair + (np / JP) * npair;
   int sw = 0, conv = 0;
   for (; sw < max_sweeps && !conv; ++sw) {
-    DMRG_CUDA_TRY(cudaMemsetAsync(ws.flag, 0, sizeof(int), s));
+    DMRG_CUDA_TRY(cudaMemsetAsync(ws.flag, 0, 2 * sizeof(int), s));
     for (int r = 0; r < rounds; ++r) {
       const int* pr = ws.pairs + (size_t)2 * r * npair;
-      syev_solve_kernel<T><<<npair, 256, 0, s>>>(G, np, pr, R, ws.ident, ws.flag, ws.scale);
+      solve_launch(ws, G, pr, R, rel, abs_, s);
       DMRG_CHECK_LAUNCH();
       syev_apply_kernel<T><<<apply_grid, 256, 0, s>>>(G, V, np, pr, R, ws.ident, npair);
       DMRG_CHECK_LAUNCH();
     }
-    int h = 0;
-    DMRG_CUDA_TRY(cudaMemcpyAsync(&h, ws.flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int h[2] = {0, 0};
+    DMRG_CUDA_TRY(cudaMemcpyAsync(h, ws.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
-    conv = h == 0;
+    conv = h[small_end ? 1 : 0] == 0;
   }
   *done += sw;
   *converged = conv;
   return DMRG_OK;
 }
 
-// C (np x np) = A B, all np x np row-major FP64
-int syev_gemm(int np, const double* A, const double* B, double* C, cudaStream_t s) {
+// C (m x n, ld n) = op(A) B, A m x k (ld lda) or, transposed, k x m; B k x n (ld n)
+int syev_gemm(SyevWs& ws, int tA, int m, int n, int k, const double* A, long long lda, const double* B, double* C,
+              cudaStream_t s) {
   TGemm g{};
-  g.B = ax(1); g.M = ax(np); g.K = ax(np); g.N = ax(np);
-  g.a_m = st(np); g.a_k = st(1);
-  g.b_k = st(np); g.b_n = st(1);
-  g.c_m = st(np); g.c_n = st(1);
-  return tgemm<double>(g, 1.0, A, B, 0.0, C, s);
+  g.B = ax(1); g.M = ax(m); g.K = ax(k); g.N = ax(n);
+  if (!tA) { g.a_m = st(lda); g.a_k = st(1); } else { g.a_m = st(1); g.a_k = st(lda); }
+  g.b_k = st(n); g.b_n = st(1);
+  g.c_m = st(n); g.c_n = st(1);
+  return fgemm(g, 1.0, A, B, 0, C, ws.dig, ws.dig_bytes, s);
 }
 
 // Sorted eigenvalues to the host and the permutation to the workspace.
@@ -452,85 +739,155 @@ int syev_finish(int n, SyevWs& ws, const T* G, double* w, cudaStream_t s) {
   return DMRG_OK;
 }
 
-// Eigenvectors of an FP64 matrix from n = 256 on come from an FP32 presolve
-// and an FP64 polish: the FP32 sweeps (64x the FP64 rate on GB300) take the
-// matrix from cold to off-diagonals ~1e-6 of the diagonal; their rotation Q
-// is made orthonormal in FP64 by two Newton-Schulz steps
-// (Q <- Q (3 I - Q^T Q) / 2), the matrix transformed as Q^T A Q in FP64, and
-// the FP64 sweeps, starting from V = Q, converge quadratically from there
-// (two or three sweeps instead of the ten to fifteen of a cold start).
-constexpr int PRESOLVE_MIN_N = 256;
+// FP32 passes.  Pass p: G (FP64) scaled and rounded to FP32, FP32 sweeps
+// until no rotation above BIG_SIN is left, V <- V Q made orthonormal by two
+// Newton-Schulz steps, G = V^T A V in FP64.  The first pass leaves what FP32
+// cannot see, about 1e-7 of the largest eigenvalue, so it stops there
+// (PASS0_ABS); the later ones work on that remainder, which FP32 holds
+// elementwise (1e-15 floor, one sweep where all rotations are small).  Up to
+// np = 64 a pass's sweeps are one launch.  Done
+// when every off-diagonal is within PASS_DONE of the FP64 sweeps' threshold:
+// three or four passes, about twenty FP32 sweeps, against ten to twenty FP64
+// sweeps of a cold start (n = 200: 41 ms).  *done_: sweeps run.
+constexpr int MAX_PASSES = 8;
+constexpr int small_smem(int np) { return 3 * np * (np + 1) * (int)sizeof(float); }
+constexpr double PASS0_ABS = 1e-6;
+constexpr float PASS_DONE = 3.f;
+
+int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, int* converged, cudaStream_t s) {
+  const int np = ws.np;
+  const long long nn = (long long)np * np;
+  // ws.R holds the rotations of the sweeps; G32 and Q32 share ws.T
+  float* G32 = reinterpret_cast<float*>(ws.T);
+  float* Q32 = G32 + nn;
+  *converged = 0;
+  static std::atomic<unsigned long long> attr{0};
+  if (np == 64) DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(syev_small32_kernel<64>), small_smem(64), attr));
+  unsigned long long* off = ws.scale + 1;
+  unsigned long long* norm = ws.scale + 2;
+  DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, sizeof(unsigned long long), s));
+  syev_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, norm);
+  DMRG_CHECK_LAUNCH();
+  bool polish = false;   // V diagonalises A but is orthonormal to 1e-12 only
+  for (int p = 0; p < MAX_PASSES; ++p) {
+    // the pass's rotation Q (FP64) into ws.G
+    double* Q = ws.G;
+    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : JacTol<double>::abs;
+    const int most = p == 0 ? 12 : 8;
+    const double* src0 = p == 0 ? A : ws.G;
+    const long long ld0 = p == 0 ? lda : np;
+    const int n0 = p == 0 ? n : np;
+    if (polish) {
+      // nothing left to rotate
+    } else if (np <= 64) {
+      // reads ws.G before it writes it (one CTA)
+      if (np == 32)
+        syev_small32_kernel<32><<<1, 256, small_smem(32), s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
+                                                               ws.flag);
+      else
+        syev_small32_kernel<64><<<1, 1024, small_smem(64), s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
+                                                                ws.flag);
+      DMRG_CHECK_LAUNCH();
+    } else {
+      DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 2 * sizeof(unsigned long long), s));
+      syev_init_kernel<float><<<grid_for(nn), 256, 0, s>>>(src0, ld0, n0, np, G32, Q32, ws.scale, norm, ws.dd);
+      DMRG_CHECK_LAUNCH();
+      int conv = 0;
+      DMRG_TRY(syev_sweeps<float>(ws, G32, Q32, most, rel, abs_, true, done_, &conv, s));
+      syev_widen_kernel<<<grid_for(nn), 256, 0, s>>>(Q32, Q, nn);
+      DMRG_CHECK_LAUNCH();
+    }
+    // V <- V Q (first pass: Q)
+    double* src = Q;
+    double* dst = ws.V;
+    if (polish) {
+      src = ws.V;
+      dst = ws.T;
+    } else if (p > 0) {
+      DMRG_TRY(syev_gemm(ws, 0, np, np, np, ws.V, np, Q, ws.T, s));
+      src = ws.T;
+    }
+    // Newton-Schulz steps, ending in ws.V: one brings the 1e-6 of an FP32
+    // rotation to 1e-12, enough for the first two passes; then two (or one
+    // more, where those already left nothing to rotate)
+    const int steps = p < 2 ? 1 : 2;
+    for (int it = 0; it < steps; ++it) {
+      // three of G, V, T: the factor in the one that is neither src nor dst
+      double* fac = src != ws.G && dst != ws.G ? ws.G : src != ws.V && dst != ws.V ? ws.V : ws.T;
+      DMRG_TRY(syev_gemm(ws, 1, np, np, np, src, np, src, fac, s));
+      syev_ns_kernel<<<grid_for(nn), 256, 0, s>>>(fac, np);
+      DMRG_CHECK_LAUNCH();
+      DMRG_TRY(syev_gemm(ws, 0, np, np, np, src, np, fac, dst, s));
+      std::swap(src, dst);
+    }
+    if (src != ws.V) DMRG_CUDA_TRY(cudaMemcpyAsync(ws.V, src, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
+    // G = V^T A V (the padded rows of A are zero): P = A V[:n] in ws.T
+    DMRG_TRY(syev_gemm(ws, 0, n, np, n, A, lda, ws.V, ws.T, s));
+    DMRG_TRY(syev_gemm(ws, 1, np, np, n, ws.V, np, ws.T, ws.G, s));
+    DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 2 * sizeof(unsigned long long), s));
+    syev_scale_kernel<<<(np + 255) / 256, 256, 0, s>>>(ws.G, np, np, ws.scale);
+    DMRG_CHECK_LAUNCH();
+    syev_off_kernel<<<grid_for(nn), 256, 0, s>>>(ws.G, np, ws.scale, off);
+    DMRG_CHECK_LAUNCH();
+    unsigned long long h = 0;
+    int small_sweeps = 0;
+    DMRG_CUDA_TRY(cudaMemcpyAsync(&h, off, sizeof(h), cudaMemcpyDeviceToHost, s));
+    if (np <= 64) DMRG_CUDA_TRY(cudaMemcpyAsync(&small_sweeps, ws.flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (!polish) *done_ += small_sweeps;
+    const uint32_t bits = (uint32_t)h;
+    float mx;
+    std::memcpy(&mx, &bits, sizeof(mx));
+    if (mx <= PASS_DONE && (p >= 2 || polish)) {
+      *converged = 1;
+      return DMRG_OK;
+    }
+    polish = mx <= PASS_DONE;
+    if (!(mx < 3e38f)) return DMRG_OK;   // not finite: left to the FP64 sweeps' checks
+  }
+  return DMRG_OK;
+}
 
 template <typename T>
 int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, int* sweeps, void* work,
-              cudaStream_t s) {
+              size_t work_bytes, cudaStream_t s) {
   SyevWs ws;
-  syev_layout(n, &ws, work);
+  const bool lean = syev_layout(n, nullptr, nullptr, false) > work_bytes;
+  syev_layout(n, &ws, work, lean);
   const int np = ws.np, nb = ws.nb;
   std::vector<int> tab;
   tournament(nb, tab);
   DMRG_CUDA_TRY(cudaMemcpyAsync(ws.pairs, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, s));
-  DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, sizeof(unsigned long long), s));
   int done = 0, conv = 0;
-  const bool presolve = sizeof(T) == 8 && n >= PRESOLVE_MIN_N;
-  if (!presolve) {
-    T* G = reinterpret_cast<T*>(ws.G);
-    T* V = reinterpret_cast<T*>(ws.V);
-    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale);
+  T* G = reinterpret_cast<T*>(ws.G);
+  T* V = reinterpret_cast<T*>(ws.V);
+  bool started = false;
+  if (sizeof(T) == 8 && n > 1) {
+    DMRG_TRY(syev_passes(n, A, lda, ws, &done, &conv, s));
+    started = true;
+  }
+  if (!conv && !started) {
+    DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, sizeof(unsigned long long), s));
+    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale, nullptr, ws.dd);
     DMRG_CHECK_LAUNCH();
-    DMRG_TRY(syev_sweeps<T>(ws, G, V, max_sweeps, &done, &conv, s));
-    if (sweeps) *sweeps = done;
-    DMRG_TRY(syev_finish<T>(n, ws, G, w, s));
-    return conv ? DMRG_OK : DMRG_ERR_NOCONV;
   }
-  // FP32 presolve: G32 in ws.G, V32 in ws.T
-  float* G32 = reinterpret_cast<float*>(ws.G);
-  float* V32 = reinterpret_cast<float*>(ws.T);
-  syev_init_kernel<float><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G32, V32, ws.scale);
-  DMRG_CHECK_LAUNCH();
-  int done32 = 0;
-  DMRG_TRY(syev_sweeps<float>(ws, G32, V32, 15, &done32, &conv, s));
-  const long long nn = (long long)np * np;
-  syev_widen_kernel<<<grid_for(nn), 256, 0, s>>>(V32, ws.V, nn);    // Q0 (ws.V)
-  DMRG_CHECK_LAUNCH();
-  // two Newton-Schulz steps: ws.V -> ws.T -> ws.V
-  double* src = ws.V;
-  double* dst = ws.T;
-  for (int it = 0; it < 2; ++it) {
-    DMRG_TRY(tgemm_gram(src, np, np, np, ws.G, s));                  // B = Q^T Q
-    syev_ns_kernel<<<grid_for(nn), 256, 0, s>>>(ws.G, np);            // B = 1.5 I - 0.5 B
-    DMRG_CHECK_LAUNCH();
-    DMRG_TRY(syev_gemm(np, src, ws.G, dst, s));                      // Q B
-    std::swap(src, dst);
+  if (!conv) {
+    // FP32 runs stop once a sweep rotates by nothing above BIG_SIN, plus one
+    // sweep: what is left is of second order, below FP32's own rounding
+    const bool f32 = sizeof(T) == 4;
+    DMRG_TRY(syev_sweeps<T>(ws, G, V, max_sweeps, JacTol<T>::rel, JacTol<T>::abs, f32, &done, &conv, s));
+    int last = 0;
+    if (f32 && conv) DMRG_TRY(syev_sweeps<T>(ws, G, V, 1, JacTol<T>::rel, JacTol<T>::abs, true, &done, &last, s));
   }
-  // G = Q^T A Q (the padded rows and columns of A are zero): P = A Q[:n] in
-  // ws.T, then Q^T P in ws.G
-  {
-    TGemm g{};
-    g.B = ax(1); g.M = ax(n); g.K = ax(n); g.N = ax(np);
-    g.a_m = st(lda); g.a_k = st(1);
-    g.b_k = st(np); g.b_n = st(1);
-    g.c_m = st(np); g.c_n = st(1);
-    DMRG_TRY(tgemm<double>(g, 1.0, A, ws.V, 0.0, ws.T, s));
-    TGemm h{};
-    h.B = ax(1); h.M = ax(np); h.K = ax(n); h.N = ax(np);
-    h.a_m = st(1); h.a_k = st(np);
-    h.b_k = st(np); h.b_n = st(1);
-    h.c_m = st(np); h.c_n = st(1);
-    DMRG_TRY(tgemm<double>(h, 1.0, ws.V, ws.T, 0.0, ws.G, s));
-  }
-  DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, sizeof(unsigned long long), s));
-  syev_scale_kernel<<<(np + 255) / 256, 256, 0, s>>>(ws.G, np, ws.scale);
-  DMRG_CHECK_LAUNCH();
-  DMRG_TRY(syev_sweeps<double>(ws, ws.G, ws.V, max_sweeps, &done, &conv, s));
   if (sweeps) *sweeps = done;
-  DMRG_TRY(syev_finish<double>(n, ws, ws.G, w, s));
+  DMRG_TRY(syev_finish<T>(n, ws, G, w, s));
   return conv ? DMRG_OK : DMRG_ERR_NOCONV;
 }
 
 }  // namespace
 
-size_t syev_jacobi_workspace_bytes(int n) { return n > 0 ? syev_layout(n, nullptr, nullptr) : 0; }
+size_t syev_jacobi_workspace_bytes(int n) { return n > 0 ? syev_layout(n, nullptr, nullptr, false) : 0; }
+size_t syev_lean_bytes(int n) { return n > 0 ? syev_layout(n, nullptr, nullptr, true) : 0; }
 
 // Eigenvalues (host w, descending) of the symmetric n x n matrix A (ld lda);
 // the eigenvectors stay in the workspace for syev_vectors.  fp32 != 0 runs
@@ -539,9 +896,9 @@ size_t syev_jacobi_workspace_bytes(int n) { return n > 0 ? syev_layout(n, nullpt
 int syev_jacobi(int n, const double* A, long long lda, double* w, int max_sweeps, int* sweeps, void* work,
                 size_t work_bytes, cudaStream_t s, int fp32) {
   if (n <= 0 || !A || lda < n || !w || max_sweeps < 1) return DMRG_ERR_ARG;
-  if (!work || syev_jacobi_workspace_bytes(n) > work_bytes) return DMRG_ERR_WORKSPACE;
-  return fp32 ? syev_impl<float>(n, A, lda, w, max_sweeps, sweeps, work, s)
-              : syev_impl<double>(n, A, lda, w, max_sweeps, sweeps, work, s);
+  if (!work || syev_lean_bytes(n) > work_bytes) return DMRG_ERR_WORKSPACE;
+  return fp32 ? syev_impl<float>(n, A, lda, w, max_sweeps, sweeps, work, work_bytes, s)
+              : syev_impl<double>(n, A, lda, w, max_sweeps, sweeps, work, work_bytes, s);
 }
 
 // The eigenvectors of the ncols largest eigenvalues of the last syev_jacobi
@@ -552,7 +909,7 @@ int syev_vectors(int n, int ncols, double* out, long long ldo, int transposed, v
   if (ncols == 0) return DMRG_OK;
   if (ldo < (transposed ? n : ncols)) return DMRG_ERR_ARG;
   SyevWs ws;
-  syev_layout(n, &ws, work);
+  syev_layout(n, &ws, work, true);
   if (fp32)
     syev_gather_kernel<float><<<grid_for((long long)n * ncols), 256, 0, s>>>(
         reinterpret_cast<const float*>(ws.V), ws.np, ws.perm, n, ncols, out, ldo, transposed);
