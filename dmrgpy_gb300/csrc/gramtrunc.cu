@@ -415,8 +415,9 @@ int rr_ritz(const double* Z, long long ld, int rows, int kz, RRWs& w, std::vecto
   return syev_jacobi(kz, w.G, kz, lam.data(), 40, nullptr, w.sw, w.sw_bytes, s);
 }
 
-// out = Z E[:, :nc] Lambda^(-1/2), then X <- X (I - (X^T X - I)/2) until
-// max|X^T X - I| < 1e-13; a basis still far from orthonormal after the
+// out = Z E[:, :nc] Lambda^(-1/2), then X <- X (I - (X^T X - I)/2) once and
+// until max|X^T X - I| < 1e-13 (the scaling's own roundings, 2e-15 at 512 x
+// 256, become 3e-16); a basis still far from orthonormal after the
 // scaling (weak directions) first gets a second Gram-eigen scaling, whose
 // Gram matrix is then well conditioned (as Cholesky-QR run twice).  out and
 // tmp: rows x ld buffers; *result is the buffer that holds the basis.
@@ -442,7 +443,7 @@ int rr_basis(const double* Z, long long ld, int rows, int kz, int nc, const std:
     DMRG_CUDA_TRY(cudaMemcpyAsync(&h, w.dev, sizeof(h), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
     std::memcpy(&dev, &h, sizeof(dev));
-    if (dev < 1e-13 || it == 5) break;
+    if ((dev < 1e-13 && it > 0) || it == 5) break;
     if (dev > 0.1 && !second) {
       second = true;
       std::vector<double> l2(nc);
