@@ -146,6 +146,9 @@ inline St2 st(long long s1, long long s2 = 0) { St2 s; s.s1 = s1; s.s2 = s2; ret
 
 template <typename T>
 int tgemm(const TGemm& g, T alpha, const T* A, const T* B, T beta, T* C, cudaStream_t stream);
+// Outputs (weighted by the tile's staging cost) that the fullest SM computes
+// for nb products of M x N in tgemm's best tile: K / 2 clocks each.
+double tgemm_cost(long long M, long long N, long long nb);
 // Many strided contractions of different shapes in one launch.  desc_host
 // (pageable, tgemm_grouped_desc_bytes(nprob)) stages the problem table that
 // is copied to desc_dev (device, same size) on the stream.

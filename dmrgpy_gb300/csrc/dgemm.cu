@@ -304,7 +304,9 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // Digits of ordinary data are nearly uniform (mean square 5461 of 16384), so
 // 512 k pass; each run costs ~3400 clocks of reading the accumulators, during
 // which the tensor core waits.
-__device__ __forceinline__ int run_steps(const GArgs& a, int mt, int nt) {
+// slack: windows a run may touch beyond those it covers (1 where its start is
+// not a multiple of 128 k).
+__device__ __forceinline__ int run_steps(const GArgs& a, int mt, int nt, int slack) {
   const int4* qa = reinterpret_cast<const int4*>(a.sqA + (long long)mt * (TM / 8));
   const int4* qb = reinterpret_cast<const int4*>(a.sqB + (long long)nt * (TN / 8));
   int ma = 0, mb = 0;
@@ -319,7 +321,7 @@ __device__ __forceinline__ int run_steps(const GArgs& a, int mt, int nt) {
     mb = max(mb, max(max(q.x, q.y), max(q.z, q.w)));
   }
   const long long half = ((long long)ma + mb) / 2 + 1;
-  return half <= (1 << 22) ? 4 * RUN : half <= (1 << 23) ? 2 * RUN : RUN;
+  return half * (4 + slack) <= (1 << 24) ? 4 * RUN : half * (2 + slack) <= (1 << 24) ? 2 * RUN : RUN;
 }
 
 // K-major operand without swizzle: 8-row x 16-byte core matrices, lbo bytes
@@ -416,6 +418,124 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
+// the MMAs of one K step: a_i times b_0 .. b_{7-i} into orders i .. 7
+__device__ __forceinline__ void mma_stage(uint32_t base, uint32_t tmem, bool first) {
+  const uint64_t da = sdesc_nosw(base, ND * TM * 16);
+  const uint64_t db = sdesc_nosw(base + A_BLK, ND * TN * 16);
+  // a_i times b_0 .. b_{7-i} into the adjacent orders i .. 7; the
+  // first K step of a run overwrites through i = 0, which reaches
+  // every order
+  const uint32_t acc = first ? 0u : 1u;
+  const uint64_t ai = TM * 16 >> 4, bj = TN * 16 >> 4;   // one digit, in descriptor units
+  mma_f16(tmem, da, db, idesc_f16(TM, 4 * TN), acc);
+  mma_f16(tmem + 4 * TN, da, db + 4 * bj, idesc_f16(TM, 4 * TN), acc);
+  mma_f16(tmem + TN, da + ai, db, idesc_f16(TM, 4 * TN), 1u);
+  mma_f16(tmem + 5 * TN, da + ai, db + 4 * bj, idesc_f16(TM, 3 * TN), 1u);
+  mma_f16(tmem + 2 * TN, da + 2 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+  mma_f16(tmem + 5 * TN, da + 2 * ai, db + 3 * bj, idesc_f16(TM, 3 * TN), 1u);
+  mma_f16(tmem + 3 * TN, da + 3 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+  mma_f16(tmem + 6 * TN, da + 3 * ai, db + 3 * bj, idesc_f16(TM, 2 * TN), 1u);
+  mma_f16(tmem + 4 * TN, da + 4 * ai, db, idesc_f16(TM, 4 * TN), 1u);
+  mma_f16(tmem + 5 * TN, da + 5 * ai, db, idesc_f16(TM, 3 * TN), 1u);
+  mma_f16(tmem + 6 * TN, da + 6 * ai, db, idesc_f16(TM, 2 * TN), 1u);
+  mma_f16(tmem + 7 * TN, da + 7 * ai, db, idesc_f16(TM, TN), 1u);
+}
+
+// adds a run's eight accumulators (this warp's 32 lanes, 32 columns) to the
+// running sums
+__device__ __forceinline__ void drain_run(uint32_t lane_addr, int* h0, long long* m) {
+  // 16 columns at a time (with 32 the kernel spills: 12 warps' worth
+  // of register file leaves 168 a thread), the next read in flight
+  // while one is converted
+  uint32_t v[2][16];
+  float tail[16];
+  tmem_ld16_async(lane_addr + 7 * TN, v[0]);
+#pragma unroll
+  for (int i = 0; i < 2 * NO; ++i) {
+    const int hc = (i / NO) * 16;
+    // order 7 first, so that the tail is folded from its small end
+    const int o = i % NO == 0 ? 7 : i % NO == 1 ? 6 : i % NO - 2;
+    const int i1 = i + 1, o1 = i1 % NO == 0 ? 7 : i1 % NO == 1 ? 6 : i1 % NO - 2;
+    tmem_wait16(v[i & 1]);
+    if (i1 < 2 * NO) tmem_ld16_async(lane_addr + o1 * TN + (i1 / NO) * 16, v[i1 & 1]);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      const float f = __uint_as_float(v[i & 1][c]);
+      if (o == 7) {
+        tail[c] = f;
+      } else {
+        const int n = __float2int_rn(o == 6 ? fmaf(tail[c], 0x1p-8f, f) : f);
+        if (o == 0) {
+          h0[hc + c] += n;
+        } else if (o == 1) {   // units of order 0, the rest (a byte) to the sum below
+          const int q = (n + 128) >> 8;
+          h0[hc + c] += q;
+          m[hc + c] += static_cast<long long>(n - (q << 8)) * (1ll << 40);
+        } else {
+          m[hc + c] += static_cast<long long>(n) * (1ll << (8 * (6 - o)));
+        }
+      }
+    }
+  }
+}
+
+// where a row of C goes
+struct RowOut {
+  bool live, vec;
+  int ea, es;
+  double* pc;
+};
+
+__device__ __forceinline__ RowOut row_out(const GArgs& a, int gm, int n0, int width) {
+  RowOut o;
+  o.live = gm < a.M;
+  o.ea = o.live ? a.eA[gm] : 0;
+  const int el = a.cplx_ ? gm >> 1 : gm;
+  o.es = a.cplx_ ? 2 : 1;
+  o.pc = a.C;
+  if (o.live)
+    o.pc += o.es * ((long long)(el / a.M2) * a.cm1 + (long long)(el % a.M2) * a.cm2) + (a.cplx_ ? (gm & 1) : 0);
+  o.vec = a.nflat && a.cn1 == 1 && o.es == 1 && n0 + width <= a.N && !a.accumulate &&
+          ((reinterpret_cast<uintptr_t>(o.pc + n0) & 15) == 0);
+  return o;
+}
+
+// columns gn .. gn + 3 of a row from the sums h[0..3], m[0..3]; lane c + j of
+// the warp holds column j's exponent in ebl
+__device__ __forceinline__ void store4(const GArgs& a, const RowOut& o, int gn, int ebl, int c, const int* h,
+                                       const long long* m, bool ok) {
+  double r[4];
+  bool odd = !ok;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int eb = __shfl_sync(0xffffffffu, ebl, c + j);
+    odd = odd || o.ea == EXP_BAD || eb == EXP_BAD;
+    r[j] = assemble(h[j], m[j], o.ea + eb + 2, a.negate, &odd);
+  }
+  if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int eb = __shfl_sync(0xffffffffu, ebl, c + j);
+      if (!ok || o.ea == EXP_BAD || eb == EXP_BAD) r[j] = __longlong_as_double(0x7ff8000000000000ll);
+      else r[j] = assemble_edge(h[j], m[j], o.ea + eb + 2, a.negate);
+    }
+  }
+  if (!o.live) return;
+  if (o.vec) {
+    reinterpret_cast<double2*>(o.pc + gn)[0] = make_double2(r[0], r[1]);
+    reinterpret_cast<double2*>(o.pc + gn)[1] = make_double2(r[2], r[3]);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (gn + j < a.N) {
+      double* d = o.pc + o.es * (a.nflat ? (long long)(gn + j) * a.cn1
+                                         : (long long)((gn + j) / a.N2) * a.cn1 + (long long)((gn + j) % a.N2) * a.cn2);
+      *d = a.accumulate ? *d + r[j] : r[j];
+    }
+  }
+}
+
 // CL = 2: a pair of CTAs takes two N tiles of one M tile; each loads its own B
 // block and half of the A block, multicast to both.
 template <int CL>
@@ -504,33 +624,14 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
       for (int t = t0; t < ntiles && ok; t += tstep) {
         int mt, nt;
         origin(t, mt, nt);
-        const int R = run_steps(a, mt, min(nt, a.tiles_n - 1));
+        const int R = nk <= RUN ? RUN : run_steps(a, mt, min(nt, a.tiles_n - 1), 0);
         for (int k = 0; k < nk && ok; ++k, ++g) {
           const int s = (int)(g % STAGES);
           const bool first = k % R == 0;
           if (first && runs > 0 && !mbar_wait(acc_empty, (uint32_t)((runs - 1) & 1), err)) { ok = false; break; }
           if (!mbar_wait(&full[s], (uint32_t)((g / STAGES) & 1), err)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t base = smem_u32(smem + s * ST_BYTES);
-          const uint64_t da = sdesc_nosw(base, ND * TM * 16);
-          const uint64_t db = sdesc_nosw(base + A_BLK, ND * TN * 16);
-          // a_i times b_0 .. b_{7-i} into the adjacent orders i .. 7; the
-          // first K step of a run overwrites through i = 0, which reaches
-          // every order
-          const uint32_t acc = first ? 0u : 1u;
-          const uint64_t ai = TM * 16 >> 4, bj = TN * 16 >> 4;   // one digit, in descriptor units
-          mma_f16(tmem, da, db, idesc_f16(TM, 4 * TN), acc);
-          mma_f16(tmem + 4 * TN, da, db + 4 * bj, idesc_f16(TM, 4 * TN), acc);
-          mma_f16(tmem + TN, da + ai, db, idesc_f16(TM, 4 * TN), 1u);
-          mma_f16(tmem + 5 * TN, da + ai, db + 4 * bj, idesc_f16(TM, 3 * TN), 1u);
-          mma_f16(tmem + 2 * TN, da + 2 * ai, db, idesc_f16(TM, 3 * TN), 1u);
-          mma_f16(tmem + 5 * TN, da + 2 * ai, db + 3 * bj, idesc_f16(TM, 3 * TN), 1u);
-          mma_f16(tmem + 3 * TN, da + 3 * ai, db, idesc_f16(TM, 3 * TN), 1u);
-          mma_f16(tmem + 6 * TN, da + 3 * ai, db + 3 * bj, idesc_f16(TM, 2 * TN), 1u);
-          mma_f16(tmem + 4 * TN, da + 4 * ai, db, idesc_f16(TM, 4 * TN), 1u);
-          mma_f16(tmem + 5 * TN, da + 5 * ai, db, idesc_f16(TM, 3 * TN), 1u);
-          mma_f16(tmem + 6 * TN, da + 6 * ai, db, idesc_f16(TM, 2 * TN), 1u);
-          mma_f16(tmem + 7 * TN, da + 7 * ai, db, idesc_f16(TM, TN), 1u);
+          mma_stage(smem_u32(smem + s * ST_BYTES), tmem, first);
           if (CL == 1) mma_commit(&empty[s]);
           else mma_commit_pair(&empty[s]);
           if (k % R == R - 1 || k == nk - 1) {
@@ -557,44 +658,12 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
         h0[c] = 0;
         m[c] = 0;
       }
-      const int R = run_steps(a, mt, min(nt, a.tiles_n - 1));
+      const int R = nk <= RUN ? RUN : run_steps(a, mt, min(nt, a.tiles_n - 1), 0);
       for (int k = 0; k < nk && ok; k += R, ++run) {
         ok = mbar_wait(acc_full, (uint32_t)(run & 1), err);
         tc_fence_after();
         if (ok) {
-          // 16 columns at a time (with 32 the kernel spills: 12 warps' worth
-          // of register file leaves 168 a thread), the next read in flight
-          // while one is converted
-          uint32_t v[2][16];
-          float tail[16];
-          tmem_ld16_async(lane_addr + 7 * TN, v[0]);
-#pragma unroll
-          for (int i = 0; i < 2 * NO; ++i) {
-            const int hc = (i / NO) * 16;
-            // order 7 first, so that the tail is folded from its small end
-            const int o = i % NO == 0 ? 7 : i % NO == 1 ? 6 : i % NO - 2;
-            const int i1 = i + 1, o1 = i1 % NO == 0 ? 7 : i1 % NO == 1 ? 6 : i1 % NO - 2;
-            tmem_wait16(v[i & 1]);
-            if (i1 < 2 * NO) tmem_ld16_async(lane_addr + o1 * TN + (i1 / NO) * 16, v[i1 & 1]);
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              const float f = __uint_as_float(v[i & 1][c]);
-              if (o == 7) {
-                tail[c] = f;
-              } else {
-                const int n = __float2int_rn(o == 6 ? fmaf(tail[c], 0x1p-8f, f) : f);
-                if (o == 0) {
-                  h0[hc + c] += n;
-                } else if (o == 1) {   // units of order 0, the rest (a byte) to the sum below
-                  const int q = (n + 128) >> 8;
-                  h0[hc + c] += q;
-                  m[hc + c] += static_cast<long long>(n - (q << 8)) * (1ll << 40);
-                } else {
-                  m[hc + c] += static_cast<long long>(n) * (1ll << (8 * (6 - o)));
-                }
-              }
-            }
-          }
+          drain_run(lane_addr, h0, m);
         }
         tc_fence_before();
         __syncwarp();
@@ -605,52 +674,13 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
       // column exponents one per lane, read back by shuffles
       const int ebl = n0 + lane < a.N ? a.eB[n0 + lane] : 0;
       if (n0 < a.N) {   // warp-uniform
-        const bool live = gm < a.M;
-        const int ea = live ? a.eA[gm] : 0;
-        const int el = a.cplx_ ? gm >> 1 : gm;
-        const int es = a.cplx_ ? 2 : 1;
-        double* pc = a.C;
-        if (live)
-          pc += es * ((long long)(el / a.M2) * a.cm1 + (long long)(el % a.M2) * a.cm2) + (a.cplx_ ? (gm & 1) : 0);
-        const bool vec = a.nflat && a.cn1 == 1 && es == 1 && n0 + 32 <= a.N && !a.accumulate &&
-                         ((reinterpret_cast<uintptr_t>(pc + n0) & 15) == 0);
+        const RowOut o = row_out(a, gm, n0, 32);
         // four columns per pass of a rolled loop, the sums moved down between
         // passes: unrolled over 32 columns this code is ~40 KB and a short
         // product spent ~20 us fetching it
 #pragma unroll 1
         for (int c0 = 0; c0 < 32; c0 += 4) {
-          double r[4];
-          bool odd = !ok;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int eb = __shfl_sync(0xffffffffu, ebl, c0 + c);
-            odd = odd || ea == EXP_BAD || eb == EXP_BAD;
-            r[c] = assemble(h0[c], m[c], ea + eb + 2, a.negate, &odd);
-          }
-          if (__any_sync(0xffffffffu, odd)) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int eb = __shfl_sync(0xffffffffu, ebl, c0 + c);
-              if (!ok || ea == EXP_BAD || eb == EXP_BAD) r[c] = __longlong_as_double(0x7ff8000000000000ll);
-              else r[c] = assemble_edge(h0[c], m[c], ea + eb + 2, a.negate);
-            }
-          }
-          if (live) {
-            if (vec) {
-              reinterpret_cast<double2*>(pc + n0 + c0)[0] = make_double2(r[0], r[1]);
-              reinterpret_cast<double2*>(pc + n0 + c0)[1] = make_double2(r[2], r[3]);
-            } else {
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                const int gn = n0 + c0 + c;
-                if (gn < a.N) {
-                  double* d = pc + es * (a.nflat ? (long long)gn * a.cn1
-                                                 : (long long)(gn / a.N2) * a.cn1 + (long long)(gn % a.N2) * a.cn2);
-                  *d = a.accumulate ? *d + r[c] : r[c];
-                }
-              }
-            }
-          }
+          store4(a, o, n0 + c0, ebl, c0, h0, m, ok);
 #pragma unroll
           for (int c = 0; c < 28; ++c) {
             h0[c] = h0[c + 4];
@@ -669,6 +699,178 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
   }
 }
 
+// Few output tiles: a cluster of SK CTAs shares one, each with a part of K.
+// Partial sums are integers, so their order does not matter: the result is
+// bitwise that of one CTA.  When all are done with their stages, every CTA
+// sends the others their 64 / SK columns' sums through distributed shared
+// memory (in the stages' place), adds up its own columns and stores them.
+// One tile per cluster.  Latency bound (fill, drain, exchange and finish,
+// 12 us together).  Measured, with the two splits: 640 x 64 x 640 58 -> 28 us,
+// 512 x 512 x 512 51 -> 29 us, 256 x 256 x 256 35 -> 20 us.
+__device__ __forceinline__ void cluster_arrive_wait() {   // any subset of a warp's lanes may be here
+  asm volatile("barrier.cluster.arrive;" ::: "memory");
+  asm volatile("barrier.cluster.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+template <int SK>
+__global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(SK, 1, 1) dg_splitk_kernel(const GArgs a) {
+  constexpr int CN = TN / SK;            // columns a CTA finishes
+  // exchange area: sums of [source][column][row], 8 then 4 bytes each, then a flag per source
+  constexpr int XM = SK * CN * TM * 8, XH = SK * CN * TM * 4;
+  static_assert(XM + XH + 64 <= STAGES * ST_BYTES, "exchange area");
+  int* err = &g_dg_timeout;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * ST_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = (int)(blockIdx.x % SK);
+  const int t = (int)(blockIdx.x / SK);
+  const int mt = t % a.tiles_m, nt = t / a.tiles_m;
+  const int all = a.ks1 - a.ks0;
+  const int k0 = a.ks0 + (int)((long long)all * rank / SK), k1 = a.ks0 + (int)((long long)all * (rank + 1) / SK);
+  const int nk = k1 - k0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    mbar_init(acc_empty, 8);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  // (one run where there are no more steps than the shortest holds)
+  const int R = nk <= RUN ? RUN : run_steps(a, mt, nt, 1);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const unsigned char* pa = a.A + ((long long)mt * a.steps + k0) * A_BLK;
+      const unsigned char* pb = a.B + ((long long)nt * a.steps + k0) * B_BLK;
+      for (int k = 0; k < nk; ++k) {
+        const int s = k % STAGES;
+        if (k >= STAGES && !mbar_wait(&empty[s], (uint32_t)((k / STAGES - 1) & 1), err)) break;
+        unsigned char* st = smem + s * ST_BYTES;
+        mbar_expect_tx(&full[s], ST_BYTES);
+        bulk_load(st, pa + (long long)k * A_BLK, A_BLK, &full[s]);
+        bulk_load(st + A_BLK, pb + (long long)k * B_BLK, B_BLK, &full[s]);
+      }
+    }
+    cluster_arrive_wait();
+    cluster_arrive_wait();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int runs = 0;
+      for (int k = 0; k < nk; ++k) {
+        const int s = k % STAGES;
+        const bool first = k % R == 0;
+        if (first && runs > 0 && !mbar_wait(acc_empty, (uint32_t)((runs - 1) & 1), err)) break;
+        if (!mbar_wait(&full[s], (uint32_t)((k / STAGES) & 1), err)) break;
+        tc_fence_after();
+        mma_stage(smem_u32(smem + s * ST_BYTES), tmem, first);
+        mma_commit(&empty[s]);
+        if (k % R == R - 1 || k == nk - 1) {
+          mma_commit(acc_full);
+          ++runs;
+        }
+      }
+    }
+    cluster_arrive_wait();
+    cluster_arrive_wait();
+  } else {
+    const int q = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const int row = q * 32 + lane;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(q * 32) << 16) + half * 32;
+    int h0[32];
+    long long m[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      h0[c] = 0;
+      m[c] = 0;
+    }
+    bool ok = true;
+    int run = 0;
+    for (int k = 0; k < nk && ok; k += R, ++run) {
+      ok = mbar_wait(acc_full, (uint32_t)(run & 1), err);
+      tc_fence_after();
+      if (ok) drain_run(lane_addr, h0, m);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty)) : "memory");
+    }
+    // the stages of every CTA are idle: its last accumulators were complete,
+    // so all its loads had landed and all its MMAs had read them
+    cluster_arrive_wait();
+    const uint32_t xm = smem_u32(smem), xh = xm + XM, xf = xh + XH;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      const int col = half * 32 + c;             // destination: CTA col / CN
+      const int off = (rank * CN + col % CN) * TM + row;
+      asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(peer_addr(xm + off * 8, col / CN)), "l"(m[c]) : "memory");
+      asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(peer_addr(xh + off * 4, col / CN)), "r"(h0[c]) : "memory");
+    }
+    // one flag per source and epilogue warp
+    if (lane < SK)
+      asm volatile("st.shared::cluster.b8 [%0], %1;" ::"r"(peer_addr(xf + rank * 8 + (warp - 2), lane)),
+                   "r"(static_cast<uint32_t>(ok ? 0 : 1))
+                   : "memory");
+    cluster_arrive_wait();
+    const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(smem + XM + XH);
+#pragma unroll
+    for (int j = 0; j < SK; ++j) ok = ok && flags[j] == 0ull;
+    // this CTA's CN columns: CN / 2 per thread half, four at a time
+    const int gm = mt * TM + row;
+    const int n0 = nt * TN + rank * CN;
+    const int ebl = lane < CN && n0 + lane < a.N ? a.eB[n0 + lane] : 0;
+    constexpr int PW = CN / 2;
+    const RowOut o = row_out(a, gm, n0 + half * PW, PW);
+    if (n0 + half * PW < a.N) {   // warp-uniform
+#pragma unroll 1
+      for (int c0 = half * PW; c0 < half * PW + PW; c0 += 4) {
+        int hs[4] = {0, 0, 0, 0};
+        long long ms[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < SK; ++j)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int off = (j * CN + c0 + c) * TM + row;
+            ms[c] += reinterpret_cast<const long long*>(smem)[off];
+            hs[c] += reinterpret_cast<const int*>(smem + XM)[off];
+          }
+        store4(a, o, n0 + c0, ebl, c0, hs, ms, ok);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
 // head of a digit buffer: row exponents, then one sum per 8 rows
 inline size_t exps_bytes(int side, long long rows) {
   return align_up(sizeof(int) * (size_t)(up(rows, tile_rows(side)) * tile_rows(side)), 1024);
@@ -677,24 +879,35 @@ inline size_t head_bytes(int side, long long rows) {
   return exps_bytes(side, rows) + align_up(sizeof(int) * (size_t)(up(rows, tile_rows(side)) * tile_rows(side) / 8), 1024);
 }
 
+// CTAs per output tile: as many of 8, 4, 2 as run at once (15, 36 and 76
+// clusters of that size, one CTA per SM, by the occupancy query; a 16th
+// cluster of 8 doubles the time), with two K steps or more each.
+inline int split_of(long long tiles, long long steps) {
+  if (steps > MAX_STEPS) return 1;
+  if (tiles <= 15 && steps >= 16) return 8;
+  if (tiles <= 36 && steps >= 8) return 4;
+  if (tiles <= 76 && steps >= 4) return 2;
+  return 1;
+}
+
 inline long long real_rows(int side, bool c, long long rows) { return c && side == 0 ? 2 * rows : rows; }
 
 }  // namespace
 
 bool dg_pays(bool cplx_, long long M, long long N, long long K, bool one_split) {
-  // microseconds.  FP64 pipe: the fullest SM's tiles at 2 FMA per clock, the
-  // best of the three tile sizes (as tgemm picks); digit product: launches
-  // plus 0.5 per K step and 5 to finish a tile.
-  const double mul = cplx_ ? 4.0 : 1.0;
-  double pipe = 1e30;
-  for (int bt = 16; bt <= 64; bt *= 2) {
-    const double waves = (double)up(up(M, bt) * up(N, bt), 152);
-    pipe = std::min(pipe, waves * bt * bt * (bt == 16 ? 1.2 : bt == 32 ? 1.05 : 1.0) * (double)K * mul / 3840.0);
-  }
-  const long long Mr = cplx_ ? 2 * M : M, Kr = cplx_ ? 2 * K : K;
-  const double waves = (double)up(up(Mr, TM) * up(N, TN), 152);
-  const double dig = (one_split ? 8.0 : 12.0) + waves * ((double)up(Kr, KS) * 0.5 + 5.0);
-  return dig < pipe + 4.0;
+  // Microseconds, fitted to measured products of 32 to 640 (real and
+  // complex).  FP64 pipe: the fullest SM's tiles at 2 FMA per clock.  Digit
+  // product: the splits (one where the other operand's digits are kept),
+  // launch, fill and finish of the kernel, and 0.62 per K step of a CTA.  The
+  // line lies above 200 x 200 x 200 (pipe 23, digits 20 and two launch gaps) and
+  // below 256 (45 and 20).
+  const double pipe = 4.0 + tgemm_cost(M, N, 1) * (double)K * (cplx_ ? 4.0 : 1.0) / 3840.0;
+  const long long Mr = cplx_ ? 2 * M : M, steps = up(cplx_ ? 2 * K : K, KS);
+  const long long tiles = up(Mr, TM) * up(N, TN);
+  const int sk = split_of(tiles, steps);
+  const double waves = (double)up(tiles * sk, 152);
+  const double dig = (one_split ? 5.0 : 10.0) + 13.0 + waves * (double)up(steps, sk) * 0.62 + (waves - 1.0) * 4.0;
+  return dig < pipe;
 }
 
 size_t dg_bytes(int side, bool cplx_, long long rows, long long K) {
@@ -762,18 +975,27 @@ int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long l
   else if (out.N.n1 == 1 || a.cn1 == a.cn2 * a.N2) { a.nflat = 1; a.cn1 = a.cn2; }
   a.cplx_ = C ? 1 : 0;
   a.negate = out.alpha < 0.0;
-  const bool pair = tn >= 2;
-  static std::atomic<unsigned long long> attr1{0}, attr2{0};
-  if (pair) DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(dg_gemm_kernel<2>), DG_SMEM, attr2));
-  else DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(dg_gemm_kernel<1>), DG_SMEM, attr1));
-  const unsigned grid = pair ? 2u * (unsigned)std::min<long long>(tm * up(tn, 2), 76)
-                             : (unsigned)std::min<long long>(tm * tn, 152);
+  const int sk = split_of(tm * tn, a.steps);
+  const bool pair = sk == 1 && tn >= 2;
+  static std::atomic<unsigned long long> attr[5];
+  const void* fn = sk == 8   ? reinterpret_cast<const void*>(dg_splitk_kernel<8>)
+                   : sk == 4 ? reinterpret_cast<const void*>(dg_splitk_kernel<4>)
+                   : sk == 2 ? reinterpret_cast<const void*>(dg_splitk_kernel<2>)
+                   : pair    ? reinterpret_cast<const void*>(dg_gemm_kernel<2>)
+                             : reinterpret_cast<const void*>(dg_gemm_kernel<1>);
+  DMRG_TRY(smem_attr_once(fn, DG_SMEM, attr[sk == 8 ? 4 : sk == 4 ? 3 : sk == 2 ? 2 : pair ? 1 : 0]));
+  const unsigned grid = sk > 1 ? (unsigned)(tm * tn) * (unsigned)sk
+                        : pair ? 2u * (unsigned)std::min<long long>(tm * up(tn, 2), 76)
+                               : (unsigned)std::min<long long>(tm * tn, 152);
   // K in launches of at most MAX_STEPS steps (64-bit sums), the later ones adding
   for (long long k0 = 0; k0 < a.steps; k0 += MAX_STEPS) {
     a.ks0 = (int)k0;
     a.ks1 = (int)std::min<long long>(a.steps, k0 + MAX_STEPS);
     a.accumulate = out.accumulate || k0 > 0;
-    if (pair) dg_gemm_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    if (sk == 8) dg_splitk_kernel<8><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    else if (sk == 4) dg_splitk_kernel<4><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    else if (sk == 2) dg_splitk_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
+    else if (pair) dg_gemm_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
     else dg_gemm_kernel<1><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
     DMRG_CHECK_LAUNCH();
   }

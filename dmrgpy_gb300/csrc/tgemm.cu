@@ -254,10 +254,10 @@ inline long long tiles_of(long long n, int bt) { return (n + bt - 1) / bt; }
 // bt^2 * K / 2 clocks per tile however many CTAs share it, so the time goes
 // as (tiles on the fullest SM) * bt^2; the factors are the smaller tiles'
 // extra staging per product (measured per output on large shapes: 32x32 5%,
-// 16x16 20%, 8x8 60% above 64x64).
+// 16x16 20%, 8x8 25% above 64x64).
 constexpr int EDGES = 4;
 constexpr int EDGE[EDGES] = {64, 32, 16, 8};
-constexpr double EDGE_COST[EDGES] = {1.0, 1.05, 1.2, 1.6};
+constexpr double EDGE_COST[EDGES] = {1.0, 1.05, 1.2, 1.25};
 inline int pick_tile(const long long* n) {
   int best = 0;
   double least = 0.0;
@@ -270,6 +270,20 @@ inline int pick_tile(const long long* n) {
   }
   return EDGE[best];
 }
+
+}  // namespace
+
+double tgemm_cost(long long M, long long N, long long nb) {
+  double least = 0.0;
+  for (int e = 0; e < EDGES; ++e) {
+    const double c = (double)tiles_of(nb * tiles_of(M, EDGE[e]) * tiles_of(N, EDGE[e]), 152) * EDGE[e] * EDGE[e] *
+                     EDGE_COST[e];
+    if (e == 0 || c < least) least = c;
+  }
+  return least;
+}
+
+namespace {
 
 // Dev from a TGemm; returns false when there is nothing to do, *err on bad input
 bool make_dev(const TGemm& g, Dev* out, int* err) {

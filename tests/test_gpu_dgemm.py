@@ -119,3 +119,14 @@ def test_digit_product_special_values():
     scale = np.abs(np.where(np.isfinite(a), a, 0)).max(1)[:, None] * np.abs(np.where(np.isfinite(b), b, 0)).max(0)
     assert np.all(np.abs(c - ref)[fin] <= (150 * 2.0 ** -52 * scale + 1e-323)[fin])
     assert np.all(c[3][fin[3]] == 0.0)
+
+
+# few output tiles: clusters of 2, 4 and 8 CTAs share a tile's K steps, at the
+# first and last tile counts of each (76, 36, 15 tiles) and with steps that do
+# not divide evenly
+@pytest.mark.parametrize("cplx,m,k,n", [(0, 640, 300, 960), (0, 600, 79, 960), (0, 1152, 129, 256), (0, 520, 500, 400),
+                                        (0, 300, 300, 300), (0, 640, 643, 192), (0, 383, 1100, 63), (1, 200, 131, 250),
+                                        (1, 129, 300, 65)])
+def test_digit_product_with_split_k(cplx, m, k, n):
+    rng = np.random.default_rng(m * 1000 + k)
+    _check(_graded(rng, m, k, cplx), _graded(rng, k, n, cplx))
