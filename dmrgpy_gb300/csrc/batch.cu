@@ -399,9 +399,7 @@ int batch_lanczos(int nprob, const dmrg_heff_t* ops, void* const* x, int kmax, d
         } else if (b[jj - 1] < tol) {
           done[p] = 1;
         } else {
-          std::vector<double> av(a, a + jj + 1), bv(b, b + jj);
-          double cur = 0.0;
-          DMRG_TRY(lowest_ritz(av, bv, &cur, nullptr));
+          const double cur = lowest_ritz_next(a, b, jj + 1, prev[p]);
           kfin[p] = jj + 1;
           if (std::fabs(cur - prev[p]) < tol * std::max(1.0, std::fabs(cur))) done[p] = 1;
           prev[p] = cur;

@@ -48,6 +48,7 @@ int hestenes_batch_output(int nprob, const int* m, const int* n, const int* keep
 
 // host-side pieces of the Krylov drivers and of the truncation rule
 bool tridiag_eig(int n, std::vector<double>& d, std::vector<double> e, std::vector<double>* z);
+double lowest_ritz_next(const double* al, const double* be, int k, double prev);
 int lowest_ritz(const std::vector<double>& al, const std::vector<double>& be, double* ev, std::vector<double>* vec);
 void keep_rule(const double* s, int n, double cutoff, int maxdim, int mindim, int* keep, double* disc);
 void keep_rule_partial(const double* lam, int k, int c, double total, double cutoff, int maxdim, int mindim,

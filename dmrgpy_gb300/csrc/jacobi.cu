@@ -13,6 +13,7 @@
 // are the column norms of X; the singular vectors are X/sigma and V.  Unlike
 // the Gram-matrix route this keeps small singular values to high relative
 // accuracy, so no exact-SVD fallback is needed.
+#include <cstring>
 #include <vector>
 
 #include "common.cuh"
@@ -649,7 +650,7 @@ namespace {
 struct BLayout {
   size_t total;
   std::vector<size_t> X, V, sig, sorted, perm, info;
-  size_t tab, otab;
+  size_t tab, otab, host, host_bytes;
 };
 
 BLayout batch_layout(size_t es, int nprob, const int* m, const int* n, size_t tab_es, size_t otab_es) {
@@ -665,10 +666,20 @@ BLayout batch_layout(size_t es, int nprob, const int* m, const int* n, size_t ta
     L.X[p] = off; off += align_up(r * c * es);
     L.V[p] = off; off += align_up(c * c * es);
     L.sig[p] = off; off += align_up(c * 8);
-    L.sorted[p] = off; off += align_up(c * 8);
     L.perm[p] = off; off += align_up(c * 4);
-    L.info[p] = off; off += align_up(8);
   }
+  // what the host reads, in one piece: sorted values, then the status words
+  L.host = off;
+  for (int p = 0; p < nprob; ++p) {
+    L.sorted[p] = off;
+    off += 8 * (size_t)(m[p] < n[p] ? m[p] : n[p]);
+  }
+  for (int p = 0; p < nprob; ++p) {
+    L.info[p] = off;
+    off += 8;
+  }
+  L.host_bytes = off - L.host;
+  off = align_up(off);
   L.total = off;
   return L;
 }
@@ -706,14 +717,14 @@ int hestenes_batch_factor(int nprob, const int* m, const int* n, const T* const*
   DMRG_CUDA_TRY(cudaMemcpyAsync(base + L.tab, tab.data(), sizeof(BSvd<T>) * nprob, cudaMemcpyHostToDevice, s));
   hestenes_batch_kernel<T><<<nprob, 1024, 0, s>>>(reinterpret_cast<const BSvd<T>*>(base + L.tab), 60);
   DMRG_CHECK_LAUNCH();
+  std::vector<char> back(L.host_bytes);
+  DMRG_CUDA_TRY(cudaMemcpyAsync(back.data(), base + L.host, L.host_bytes, cudaMemcpyDeviceToHost, s));
+  DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   std::vector<int> info(nprob);
   for (int p = 0; p < nprob; ++p) {
-    const int c = tab[p].c;
-    DMRG_CUDA_TRY(cudaMemcpyAsync(host_s + (size_t)p * ld_s, tab[p].sorted, sizeof(double) * c,
-                                  cudaMemcpyDeviceToHost, s));
-    DMRG_CUDA_TRY(cudaMemcpyAsync(&info[p], tab[p].info, sizeof(int), cudaMemcpyDeviceToHost, s));
+    std::memcpy(host_s + (size_t)p * ld_s, back.data() + (L.sorted[p] - L.host), sizeof(double) * tab[p].c);
+    std::memcpy(&info[p], back.data() + (L.info[p] - L.host), sizeof(int));
   }
-  DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   int st = DMRG_OK;
   for (int p = 0; p < nprob; ++p) {
     for (int k = 0; k < tab[p].c; ++k) {
