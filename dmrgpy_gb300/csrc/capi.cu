@@ -313,13 +313,21 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
   DMRG_TRY(vscale_dev_inv<T>(Q, x, nrm_d, n, s));  // q0
   DMRG_TRY(heff_prepare<T>(o, ws.hw, ws.hbytes, s));
   DMRG_TRY(heff_run<T>(o, Q, w, ws.hw, ws.hbytes, s));
-  DMRG_TRY(vdot<T>(Q, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
-  DMRG_TRY(vaxpy2<T>(w, Q, alpha_d, nullptr, nullptr, n, s));
-  DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+  const bool one = krylov_step_fits<T>(n, m);
+  unsigned epoch = 0;
+  if (one) {
+    DMRG_TRY(krylov_step<T>(Q, w, n, 0, 0, m > 1, ws.sc, ws.red, ws.part, epoch, s));
+    epoch += 2;
+  } else {
+    DMRG_TRY(vdot<T>(Q, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
+    DMRG_TRY(vaxpy2<T>(w, Q, alpha_d, nullptr, nullptr, n, s));
+    DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+  }
   DMRG_CUDA_TRY(cudaMemcpyAsync(hbuf, ws.sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   std::vector<double> al{hbuf[0]}, be;
   double beta = hbuf[2];
+  if (hbuf[3] != 0.0) return (int)hbuf[3];
   if (!(hbuf[0] == hbuf[0]) || !(beta == beta)) return DMRG_ERR_NAN;
   double prev = al[0];
   int k = 1;
@@ -328,17 +336,24 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
     be.push_back(beta);
     T* qj = Q + (long long)j * n;
     T* qjm = Q + (long long)(j - 1) * n;
-    DMRG_TRY(vscale_dev_inv<T>(qj, w, beta_d, n, s));
-    DMRG_CUDA_TRY(cudaMemcpyAsync(bprev_d, beta_d, sizeof(double), cudaMemcpyDeviceToDevice, s));
-    DMRG_TRY(heff_run<T>(o, qj, w, ws.hw, ws.hbytes, s));
-    DMRG_TRY(vdot<T>(qj, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
-    DMRG_TRY(vaxpy2<T>(w, qj, alpha_d, qjm, bprev_d, n, s));
-    // full reorthogonalisation against q_0 .. q_{j-1}
-    DMRG_TRY(multidot_ws<T>(Q, n, j, w, n, h, ws.part, s));
-    DMRG_TRY(gemv_sub<T>(Q, n, j, h, w, n, 0, s));
-    DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+    if (one) {
+      DMRG_TRY(heff_run<T>(o, qj, w, ws.hw, ws.hbytes, s));
+      DMRG_TRY(krylov_step<T>(Q, w, n, j, j, j + 1 < m, ws.sc, ws.red, ws.part, epoch, s));
+      epoch += 3;
+    } else {
+      DMRG_TRY(vscale_dev_inv<T>(qj, w, beta_d, n, s));
+      DMRG_CUDA_TRY(cudaMemcpyAsync(bprev_d, beta_d, sizeof(double), cudaMemcpyDeviceToDevice, s));
+      DMRG_TRY(heff_run<T>(o, qj, w, ws.hw, ws.hbytes, s));
+      DMRG_TRY(vdot<T>(qj, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
+      DMRG_TRY(vaxpy2<T>(w, qj, alpha_d, qjm, bprev_d, n, s));
+      // full reorthogonalisation against q_0 .. q_{j-1}
+      DMRG_TRY(multidot_ws<T>(Q, n, j, w, n, h, ws.part, s));
+      DMRG_TRY(gemv_sub<T>(Q, n, j, h, w, n, 0, s));
+      DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+    }
     DMRG_CUDA_TRY(cudaMemcpyAsync(hbuf, ws.sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (hbuf[3] != 0.0) return (int)hbuf[3];
     if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return DMRG_ERR_NAN;
     al.push_back(hbuf[0]);
     beta = hbuf[2];
@@ -392,18 +407,26 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
   }
   DMRG_TRY(vscale_dev_inv<T>(Q, x, nrm_d, n, s));
   DMRG_TRY(heff_prepare<T>(o, ws.hw, ws.hbytes, s));
+  const bool one = krylov_step_fits<T>(n, m);
+  unsigned epoch = 0;
   std::vector<double> al, be;
   for (int it = 0; it < m; ++it) {
     T* qi = Q + (long long)it * n;
     DMRG_TRY(heff_run<T>(o, qi, w, ws.hw, ws.hbytes, s));
-    DMRG_TRY(vdot<T>(qi, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
-    DMRG_TRY(vaxpy2<T>(w, qi, alpha_d, it > 0 ? Q + (long long)(it - 1) * n : nullptr, it > 0 ? bprev_d : nullptr,
-                       n, s));
-    DMRG_TRY(multidot_ws<T>(Q, n, it + 1, w, n, h, ws.part, s));
-    DMRG_TRY(gemv_sub<T>(Q, n, it + 1, h, w, n, 0, s));
-    DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+    if (one) {
+      DMRG_TRY(krylov_step<T>(Q, w, n, it, it + 1, it + 1 < m, ws.sc, ws.red, ws.part, epoch, s));
+      epoch += 3;
+    } else {
+      DMRG_TRY(vdot<T>(qi, w, n, reinterpret_cast<T*>(alpha_d), ws.red, s));
+      DMRG_TRY(vaxpy2<T>(w, qi, alpha_d, it > 0 ? Q + (long long)(it - 1) * n : nullptr, it > 0 ? bprev_d : nullptr,
+                         n, s));
+      DMRG_TRY(multidot_ws<T>(Q, n, it + 1, w, n, h, ws.part, s));
+      DMRG_TRY(gemv_sub<T>(Q, n, it + 1, h, w, n, 0, s));
+      DMRG_TRY(vnorm<T>(w, n, beta_d, ws.red, s));
+    }
     DMRG_CUDA_TRY(cudaMemcpyAsync(hbuf, ws.sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (hbuf[3] != 0.0) return (int)hbuf[3];
     if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return DMRG_ERR_NAN;
     al.push_back(hbuf[0]);
     const double beta = hbuf[2];
@@ -433,6 +456,7 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
       return DMRG_OK;
     }
     be.push_back(beta);
+    if (one) continue;
     DMRG_CUDA_TRY(cudaMemcpyAsync(bprev_d, beta_d, sizeof(double), cudaMemcpyDeviceToDevice, s));
     DMRG_TRY(vscale_dev_inv<T>(Q + (long long)(it + 1) * n, w, beta_d, n, s));
   }

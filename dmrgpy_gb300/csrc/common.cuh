@@ -174,6 +174,16 @@ template <typename T> int vscale(T* x, T a, long long n, cudaStream_t s);
 // CTAs per vector of the block dot products h = Q^H w (two per SM); the
 // caller's partial scratch holds 2 * MULTIDOT_MAX_GRID doubles per vector
 constexpr int MULTIDOT_MAX_GRID = 2 * 152;
+// A Krylov step after its matvec w = H q_j: alpha, the three-term update, the
+// reorthogonalisation against q_0 .. q_(nq-1), beta and (next) q_(j+1), in one
+// cooperative launch.  sc: [0..1] alpha, [2] beta (in: the previous one),
+// [3] status; red, zeroed at the loop's start: 8 + 2 MULTIDOT_MAX_GRID
+// doubles; part: as multidot_ws; epoch: 3 per earlier call with nq > 0, 2
+// with nq = 0.
+template <typename T> bool krylov_step_fits(long long n, int nq);
+template <typename T>
+int krylov_step(T* Q, const T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
+                unsigned epoch, cudaStream_t s);
 template <typename T> int vcopy(T* y, const T* x, long long n, cudaStream_t s);
 template <typename T> int vfill_random(T* x, long long n, unsigned long long seed, cudaStream_t s);
 // w = w - Q h (or w = Q h when overwrite); Q column-major n x k, leading dim ldq

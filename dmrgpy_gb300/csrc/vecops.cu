@@ -12,6 +12,7 @@ namespace {
 
 constexpr int RT = 256;          // threads per reduction CTA
 constexpr int RB = 2 * 152;      // reduction CTAs (two per SM)
+static_assert(RB == MULTIDOT_MAX_GRID, "reduction scratch");
 
 template <typename T>
 __device__ __forceinline__ void acc_dot(const T& a, const T& b, double& re, double& im);
@@ -191,6 +192,171 @@ __global__ void gemv_kernel(const T* __restrict__ Q, long long ldq, int k, const
   }
 }
 
+// ---- one Krylov step after its matvec, in one cooperative launch: bound by
+// latency (three barriers of 1 to 2 us and the FP64 pipe's 2 n nq / 152 / 2
+// clocks); the eight short kernels and the copy it replaces took 25 us at
+// n = 3600, nq = 8, and as long again to launch.
+constexpr int KT = 512;                   // threads
+constexpr int KW = KT / 32;
+constexpr int KRYLOV_STEP_SMEM = 64 * 1024;
+constexpr int KRYLOV_SLICE = 1536;        // elements of a CTA's slice at most
+constexpr int KC = 128;                   // elements of a CTA's slice handled at a time by the update
+constexpr unsigned kStepSpinLimit = 1u << 22;   // polls, seconds: far beyond any real wait
+
+// All CTAs are co-resident (cooperative launch).  *count only grows: barrier
+// number b of the loop is passed when it reaches (b + 1) gridDim.x.  Gives up
+// after the limit, sets *err and lets every CTA fall through.
+__device__ __forceinline__ void step_barrier(unsigned* count, int* err, unsigned b) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    const unsigned want = (b + 1) * gridDim.x;
+    unsigned it = 0;
+    while (*(volatile unsigned*)count < want && *(volatile int*)err == 0) {
+      if (++it > kStepSpinLimit) {
+        atomicExch(err, DMRG_ERR_TIMEOUT);
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+}
+
+// sum of the CTAs' pairs part[2 b], part[2 b + 1], in every thread
+__device__ __forceinline__ void grid_sum2(const double* part, double& re, double& im, double* sh) {
+  re = 0.0;
+  im = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += KT) {
+    re += __ldcg(part + 2 * b);
+    im += __ldcg(part + 2 * b + 1);
+  }
+  block_sum2(re, im, sh);
+  if (threadIdx.x == 0) {
+    sh[0] = re;
+    sh[1] = im;
+  }
+  __syncthreads();
+  re = sh[0];
+  im = sh[1];
+  __syncthreads();
+}
+
+// alpha = q_j^H w, w -= alpha q_j + beta_(j-1) q_(j-1), w -= Q_nq Q_nq^H w,
+// beta = |w|, q_(j+1) = w / beta (next != 0): sc[0..1] = alpha, sc[2] = beta
+// (on entry beta_(j-1)), sc[3] = error.  CTA b keeps elements b slice ... of
+// w in shared memory throughout.  The sums over CTAs pass through global
+// memory, added in CTA order by everyone, so all agree bit for bit.
+template <typename T>
+__global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, const T* __restrict__ w, long long n, int j,
+                                                         int nq, int next, long long slice, double* sc, double* red,
+                                                         double* part, unsigned epoch) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double sh[64];
+  T* ws = reinterpret_cast<T*>(smem_raw);   // slice
+  T* comb = ws + slice;                     // KT
+  T* hs = comb + KT;                        // nq
+  unsigned* count = reinterpret_cast<unsigned*>(red) + 4;
+  int* err = reinterpret_cast<int*>(red) + 8;
+  double* ra = red + 8;                     // alpha's partials, then the norm's
+  double* rn = ra + MULTIDOT_MAX_GRID;
+  const int G = gridDim.x, b = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long lo = (long long)b * slice;
+  const int cnt = (int)(n - lo < slice ? n - lo : slice);   // >= 1
+  const T* qj = Q + (long long)j * n + lo;
+  const double bprev = j > 0 ? sc[2] : 0.0;
+  double re = 0.0, im = 0.0;
+  for (int e = threadIdx.x; e < cnt; e += KT) {
+    const T v = w[lo + e];
+    ws[e] = v;
+    acc_dot<T>(qj[e], v, re, im);
+  }
+  block_sum2(re, im, sh);
+  if (threadIdx.x == 0) {
+    ra[2 * b] = re;
+    ra[2 * b + 1] = im;
+  }
+  step_barrier(count, err, epoch);
+  double are, aim;
+  grid_sum2(ra, are, aim, sh);
+  for (int e = threadIdx.x; e < cnt; e += KT) {
+    T v = Sc<T>::sub(ws[e], Sc<T>::scale(qj[e], are));
+    if (j > 0) v = Sc<T>::sub(v, Sc<T>::scale(qj[e - n], bprev));
+    ws[e] = v;
+  }
+  __syncthreads();
+  if (nq > 0) {
+    // a warp per vector
+    for (int i = wid; i < nq; i += KW) {
+      const T* q = Q + (long long)i * n + lo;
+      re = im = 0.0;
+#pragma unroll 4
+      for (int e = lane; e < cnt; e += 32) acc_dot<T>(q[e], ws[e], re, im);
+      re = warp_sum(re);
+      if (sizeof(T) == 16) im = warp_sum(im);
+      if (lane == 0) {
+        part[2 * ((long long)i * G + b)] = re;
+        part[2 * ((long long)i * G + b) + 1] = im;
+      }
+    }
+    step_barrier(count, err, epoch + 1);
+    for (int i = wid; i < nq; i += KW) {
+      const double* pi = part + 2 * (long long)i * G;
+      re = im = 0.0;
+      for (int g = lane; g < G; g += 32) {
+        re += __ldcg(pi + 2 * g);
+        if (sizeof(T) == 16) im += __ldcg(pi + 2 * g + 1);
+      }
+      re = warp_sum(re);
+      if (sizeof(T) == 16) im = warp_sum(im);
+      if (lane == 0) hs[i] = Sc<T>::make(re, im);
+    }
+    __syncthreads();
+  }
+  // four threads per element, each with every fourth vector
+  re = im = 0.0;
+  const int ce = threadIdx.x & (KC - 1), cp = threadIdx.x / KC;
+  for (int e0 = 0; e0 < cnt; e0 += KC) {
+    const int e = e0 + ce;
+    if (nq > 0) {
+      T acc = Sc<T>::zero();
+      if (e < cnt) {
+        const T* q = Q + lo + e;
+#pragma unroll 4
+        for (int i = cp; i < nq; i += KT / KC) acc = Sc<T>::fma(q[(long long)i * n], hs[i], acc);
+      }
+      comb[threadIdx.x] = acc;
+      __syncthreads();
+      if (cp == 0 && e < cnt) {
+        for (int c = 1; c < KT / KC; ++c) acc = Sc<T>::add(acc, comb[c * KC + ce]);
+        ws[e] = Sc<T>::sub(ws[e], acc);
+      }
+    }
+    if (cp == 0 && e < cnt) acc_dot<T>(ws[e], ws[e], re, im);
+    __syncthreads();
+  }
+  block_sum2(re, im, sh);
+  if (threadIdx.x == 0) {
+    rn[2 * b] = re;
+    rn[2 * b + 1] = 0.0;
+  }
+  step_barrier(count, err, epoch + (nq > 0 ? 2 : 1));
+  grid_sum2(rn, re, im, sh);
+  const double beta = sqrt(re);
+  if (next) {
+    const double inv = 1.0 / beta;
+    T* qn = Q + (long long)(j + 1) * n + lo;
+    for (int e = threadIdx.x; e < cnt; e += KT) qn[e] = Sc<T>::scale(ws[e], inv);
+  }
+  if (b == 0 && threadIdx.x == 0) {
+    sc[0] = are;
+    sc[1] = aim;
+    sc[2] = beta;
+    sc[3] = *(volatile int*)err;
+  }
+}
+
 __global__ void nan_kernel(const double* __restrict__ x, long long n, int* __restrict__ flag) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   int bad = 0;
@@ -285,6 +451,46 @@ int gemv_sub(const T* Q, long long ldq, int k, const T* h, T* w, long long n, in
   return DMRG_OK;
 }
 
+// Elements per CTA of krylov_step, or 0 where the separate kernels are the
+// better choice (long vectors: one CTA per SM no longer draws the bandwidth)
+// or the only one.  A bond's ground state, separate -> one kernel: n = 1024
+// 2.84 -> 2.31 ms, 16 k 7.49 -> 6.07, 102 k 14.8 -> 10.9, 230 k 17.1 -> 15.9,
+// 590 k 41.3 -> 55.2 (left apart); a complex step of exp(-i tau H): n = 16 k
+// 0.94 -> 0.82, 160 k 2.10 -> 1.95.
+static long long step_slice(size_t es, long long n, int nq, int* grid) {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (nsm > 152) nsm = 152;
+  long long g = (n + KC - 1) / KC;
+  if (g > nsm) g = nsm;
+  const long long slice = (n + g - 1) / g;
+  if (slice > KRYLOV_SLICE || (size_t)(slice + KT + nq) * es > (size_t)KRYLOV_STEP_SMEM) return 0;
+  *grid = (int)((n + slice - 1) / slice);
+  return slice;
+}
+
+template <typename T>
+bool krylov_step_fits(long long n, int nq) {
+  int g;
+  return step_slice(sizeof(T), n, nq, &g) > 0;
+}
+
+template <typename T>
+int krylov_step(T* Q, const T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
+                unsigned epoch, cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0};
+  const void* fn = reinterpret_cast<const void*>(krylov_step_kernel<T>);
+  DMRG_TRY(smem_attr_once(fn, KRYLOV_STEP_SMEM, attr));
+  int g = 0, nx = next ? 1 : 0;
+  long long slice = step_slice(sizeof(T), n, nq, &g);
+  if (slice <= 0) return DMRG_ERR_ARG;
+  void* args[] = {&Q, &w, &n, &j, &nq, &nx, &slice, &sc, &red, &part, &epoch};
+  DMRG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, g, KT, args, (size_t)(slice + KT + nq) * sizeof(T), s));
+  count_launch();
+  return DMRG_OK;
+}
+
 int nan_check(const void* x, long long n_doubles, int* flag, cudaStream_t s) {
   nan_kernel<<<egrid(n_doubles), 256, 0, s>>>(static_cast<const double*>(x), n_doubles, flag);
   DMRG_CHECK_LAUNCH();
@@ -300,7 +506,10 @@ int nan_check(const void* x, long long n_doubles, int* flag, cudaStream_t s) {
   template int vcopy<T>(T*, const T*, long long, cudaStream_t);                                 \
   template int vfill_random<T>(T*, long long, unsigned long long, cudaStream_t);                \
   template int multidot_ws<T>(const T*, long long, int, const T*, long long, T*, double*, cudaStream_t); \
-  template int gemv_sub<T>(const T*, long long, int, const T*, T*, long long, int, cudaStream_t);
+  template int gemv_sub<T>(const T*, long long, int, const T*, T*, long long, int, cudaStream_t); \
+  template bool krylov_step_fits<T>(long long, int);                                            \
+  template int krylov_step<T>(T*, const T*, long long, int, int, bool, double*, double*, double*, unsigned, \
+                              cudaStream_t);
 INST(double)
 INST(cplx)
 #undef INST
