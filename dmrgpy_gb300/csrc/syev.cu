@@ -393,22 +393,26 @@ __global__ void __launch_bounds__(256) syev_solve32_kernel(const float* __restri
 }
 
 // Matrices of one block pair or two (np = 32 or 64): all FP32 sweeps of a pass
-// in one CTA, the matrix and D = Q - I in shared memory; out = Q (FP64,
-// np x np).  Same rounds as syev_solve32_kernel on NP indices.  The blocked
-// form takes three rounds of two launches per sweep at np = 64 (measured, n = 60,
-// all passes: 0.70 ms in its kernels and as much between them).
+// in one launch, the matrix and D = Q - I in shared memory; out = Q (FP64,
+// np x np; not A).  Same rounds as syev_solve32_kernel on NP indices.  Bound by
+// the latency of a round (the rotation's chain of four approximations) and
+// its issue slots, so: a lane takes column pair t and the blocks of row pair t
+// with column pairs t + k, k = 0 .. H / 2, written twice (the matrix is
+// symmetric); every CTA rotates the whole matrix, to the same bits, but only
+// NP / gridDim.x rows of D.  One CTA of a thread per 2 x 2 block, with all of
+// D: 384 us a pass at n = 60.
 template <int NP>
-__global__ void __launch_bounds__(NP * NP / 4) syev_small32_kernel(const double* __restrict__ A, long long lda, int n,
-                                                                   const unsigned long long* __restrict__ norm,
-                                                                   int max_sweeps, float rel, float abs_,
-                                                                   double* __restrict__ out, int* __restrict__ sweeps) {
-  constexpr int LD = NP + 1, H = NP / 2, NT = H * H;
-  extern __shared__ float sm[];
-  float* buf0 = sm;
-  float* buf1 = sm + NP * LD;
-  float* r = sm + 2 * NP * LD;
+__global__ void __launch_bounds__(256) syev_small32_kernel(const double* __restrict__ A, long long lda, int n,
+                                                           const unsigned long long* __restrict__ norm,
+                                                           int max_sweeps, float rel, float abs_,
+                                                           double* __restrict__ out, int* __restrict__ sweeps) {
+  // LD even: blocks of lanes at strides LD + 1 (p, p and q, q) and LD - 1 (p, q)
+  constexpr int LD = NP + 2, H = NP / 2, NT = 256, SL = NT / H, IT = H / 2 / SL + 1;
+  __shared__ float buf[2][NP * LD];
+  __shared__ float r[SL][NP];
   __shared__ float2 dg[2][NP];
   const int tid = threadIdx.x;
+  const int t = tid % H, slot = tid / H, row = blockIdx.x * SL + slot;
   double f = 1.0;
   {
     const int e = (int)(*norm >> 52);
@@ -417,58 +421,70 @@ __global__ void __launch_bounds__(NP * NP / 4) syev_small32_kernel(const double*
   for (int e = tid; e < NP * NP; e += NT) {
     const int i = e / NP, j = e % NP;
     const double v = i < n && j < n ? A[(long long)i * lda + j] * f : 0.0;
-    buf0[i * LD + j] = (float)v;
+    buf[0][i * LD + j] = (float)v;
     if (i == j) dg[0][i] = hi_lo(v);
-    r[i * LD + j] = 0.f;
   }
+  for (int e = tid; e < SL * NP; e += NT) r[e / NP][e % NP] = 0.f;
   __syncthreads();
   // diagonals scaled by the largest diagonal of the first pass's matrix lie
   // in [-2, 2]; the floor is relative to 1
   const float floor_ = abs_;
-  const int ti = tid / H, tj = tid % H;
-  int pi = ti, qi = NP - 1 - ti, pj = tj, qj = NP - 1 - tj;
+  int p = t, q = NP - 1 - t;
+  int pk[IT], qk[IT], src[IT];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    src[it] = (t + slot + SL * it) & (H - 1);
+    pk[it] = src[it];
+    qk[it] = NP - 1 - src[it];
+  }
   int cur = 0, sw = 0;
   for (; sw < max_sweeps; ++sw) {
     bool big = false;
     for (int ir = 0; ir < NP - 1; ++ir, cur ^= 1) {
-      const float* x = cur ? buf1 : buf0;
-      float* z = cur ? buf0 : buf1;
-      const float x00 = x[pi * LD + pj], x01 = x[pi * LD + qj], x10 = x[qi * LD + pj], x11 = x[qi * LD + qj];
-      const float u0 = r[ti * LD + pj], v0 = r[ti * LD + qj], u1 = r[(ti + H) * LD + pj], v1 = r[(ti + H) * LD + qj];
-      float tj_, cj, sj, cmj;
-      const float2 app = dg[cur][pj], aqq = dg[cur][qj];
-      const float apq = x[pj * LD + qj];
-      rot32(app, aqq, apq, rel, floor_, tj_, cj, sj, cmj);
-      // lane ti of the warp holds row pair ti's rotation (as column pair)
-      const float si = __shfl_sync(0xffffffffu, sj, ti), cmi = __shfl_sync(0xffffffffu, cmj, ti);
-      big = big || fabsf(si) > BIG_SIN;
-      const float y00 = x00 + (cmi * x00 - si * x10), y01 = x01 + (cmi * x01 - si * x11);
-      const float y10 = x10 + (si * x00 + cmi * x10), y11 = x11 + (si * x01 + cmi * x11);
-      float z00 = y00 + (cmj * y00 - sj * y01), z01 = y01 + (sj * y00 + cmj * y01);
-      float z10 = y10 + (cmj * y10 - sj * y11), z11 = y11 + (sj * y10 + cmj * y11);
-      if (ti == tj) {
-        dg[cur ^ 1][pj] = add_hl(app, -tj_ * apq);
-        dg[cur ^ 1][qj] = add_hl(aqq, tj_ * apq);
-        z01 = z10 = sj != 0.f ? 0.f : x01;
+      const float* x = buf[cur];
+      float* z = buf[cur ^ 1];
+      const float2 app = dg[cur][p], aqq = dg[cur][q];
+      const float apq = x[p * LD + q];
+      const float u = r[slot][p], v = r[slot][q];
+      float t_, c_, sn, cm;
+      rot32(app, aqq, apq, rel, floor_, t_, c_, sn, cm);
+      big = big || fabsf(sn) > BIG_SIN;
+      float d0 = fmaf(cm, u, u) - sn * v, d1 = fmaf(sn, u, fmaf(cm, v, v));
+      if (row == p) { d0 += cm; d1 += sn; }
+      if (row == q) { d0 -= sn; d1 += cm; }
+      r[slot][p] = d0;
+      r[slot][q] = d1;
+#pragma unroll
+      for (int it = 0; it < IT; ++it) {
+        const int k = slot + SL * it;
+        const float sk = __shfl_sync(0xffffffffu, sn, src[it]), ck = __shfl_sync(0xffffffffu, cm, src[it]);
+        if (k == 0) {
+          dg[cur ^ 1][p] = add_hl(app, -t_ * apq);
+          dg[cur ^ 1][q] = add_hl(aqq, t_ * apq);
+          const float w = sn != 0.f ? 0.f : apq;
+          z[p * LD + q] = w;
+          z[q * LD + p] = w;
+        } else if (k < H / 2 || (k == H / 2 && t < H / 2)) {
+          const int p1 = pk[it], q1 = qk[it];
+          const float x00 = x[p * LD + p1], x01 = x[p * LD + q1], x10 = x[q * LD + p1], x11 = x[q * LD + q1];
+          const float y00 = x00 + (cm * x00 - sn * x10), y01 = x01 + (cm * x01 - sn * x11);
+          const float y10 = x10 + (sn * x00 + cm * x10), y11 = x11 + (sn * x01 + cm * x11);
+          const float z00 = y00 + (ck * y00 - sk * y01), z01 = y01 + (sk * y00 + ck * y01);
+          const float z10 = y10 + (ck * y10 - sk * y11), z11 = y11 + (sk * y10 + ck * y11);
+          z[p * LD + p1] = z00;
+          z[p * LD + q1] = z01;
+          z[q * LD + p1] = z10;
+          z[q * LD + q1] = z11;
+          z[p1 * LD + p] = z00;
+          z[q1 * LD + p] = z01;
+          z[p1 * LD + q] = z10;
+          z[q1 * LD + q] = z11;
+        }
+        pk[it] = src[it] == 0 ? 0 : (pk[it] == NP - 1 ? 1 : pk[it] + 1);
+        qk[it] = qk[it] == NP - 1 ? 1 : qk[it] + 1;
       }
-      z[pi * LD + pj] = z00;
-      z[pi * LD + qj] = z01;
-      z[qi * LD + pj] = z10;
-      z[qi * LD + qj] = z11;
-      float a0 = fmaf(cmj, u0, u0) - sj * v0, b0 = fmaf(sj, u0, fmaf(cmj, v0, v0));
-      float a1 = fmaf(cmj, u1, u1) - sj * v1, b1 = fmaf(sj, u1, fmaf(cmj, v1, v1));
-      if (ti == pj) { a0 += cmj; b0 += sj; }
-      if (ti == qj) { a0 -= sj; b0 += cmj; }
-      if (ti + H == pj) { a1 += cmj; b1 += sj; }
-      if (ti + H == qj) { a1 -= sj; b1 += cmj; }
-      r[ti * LD + pj] = a0;
-      r[ti * LD + qj] = b0;
-      r[(ti + H) * LD + pj] = a1;
-      r[(ti + H) * LD + qj] = b1;
-      pi = ti == 0 ? 0 : (pi == NP - 1 ? 1 : pi + 1);
-      pj = tj == 0 ? 0 : (pj == NP - 1 ? 1 : pj + 1);
-      qi = qi == NP - 1 ? 1 : qi + 1;
-      qj = qj == NP - 1 ? 1 : qj + 1;
+      p = t == 0 ? 0 : (p == NP - 1 ? 1 : p + 1);
+      q = q == NP - 1 ? 1 : q + 1;
       __syncthreads();
     }
     if (!__syncthreads_or(big)) {
@@ -476,11 +492,11 @@ __global__ void __launch_bounds__(NP * NP / 4) syev_small32_kernel(const double*
       break;
     }
   }
-  for (int e = tid; e < NP * NP; e += NT) {
-    const int i = e / NP, j = e % NP;
-    out[e] = (i == j ? 1.0 : 0.0) + (double)r[i * LD + j];
+  for (int e = tid; e < SL * NP; e += NT) {
+    const int i = blockIdx.x * SL + e / NP, j = e % NP;
+    out[i * NP + j] = (i == j ? 1.0 : 0.0) + (double)r[e / NP][j];
   }
-  if (tid == 0) *sweeps = sw;
+  if (blockIdx.x == 0 && tid == 0) *sweeps = sw;
 }
 
 __device__ __forceinline__ int pair_index(int b0, int b1, int l) { return l < JB ? b0 * JB + l : b1 * JB + l - JB; }
@@ -781,7 +797,6 @@ int syev_finish(int n, SyevWs& ws, const T* G, double* w, cudaStream_t s) {
 // three or four passes, about twenty FP32 sweeps, against ten to twenty FP64
 // sweeps of a cold start (n = 200: 41 ms).  *done_: sweeps run.
 constexpr int MAX_PASSES = 8;
-constexpr int small_smem(int np) { return 3 * np * (np + 1) * (int)sizeof(float); }
 constexpr double PASS0_ABS = 1e-6;
 constexpr float PASS_DONE = 3.f;
 
@@ -792,8 +807,6 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
   float* G32 = reinterpret_cast<float*>(ws.T);
   float* Q32 = G32 + nn;
   *converged = 0;
-  static std::atomic<unsigned long long> attr{0};
-  if (np == 64) DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(syev_small32_kernel<64>), small_smem(64), attr));
   unsigned long long* off = ws.scale + 1;
   unsigned long long* norm = ws.scale + 2;
   DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, sizeof(unsigned long long), s));
@@ -801,8 +814,9 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
   DMRG_CHECK_LAUNCH();
   bool polish = false;   // V diagonalises A but is orthonormal to 1e-12 only
   for (int p = 0; p < MAX_PASSES; ++p) {
-    // the pass's rotation Q (FP64) into ws.G
-    double* Q = ws.G;
+    // the pass's rotation Q (FP64) into ws.G; into ws.T where the kernel's
+    // CTAs read ws.G as they please
+    double* Q = np <= 64 && p > 0 ? ws.T : ws.G;
     const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : JacTol<double>::abs;
     const int most = p == 0 ? 12 : 8;
     const double* src0 = p == 0 ? A : ws.G;
@@ -811,13 +825,10 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     if (polish) {
       // nothing left to rotate
     } else if (np <= 64) {
-      // reads ws.G before it writes it (one CTA)
       if (np == 32)
-        syev_small32_kernel<32><<<1, 256, small_smem(32), s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
-                                                               ws.flag);
+        syev_small32_kernel<32><<<2, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q, ws.flag);
       else
-        syev_small32_kernel<64><<<1, 1024, small_smem(64), s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
-                                                                ws.flag);
+        syev_small32_kernel<64><<<8, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q, ws.flag);
       DMRG_CHECK_LAUNCH();
     } else {
       DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 2 * sizeof(unsigned long long), s));
@@ -835,8 +846,8 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
       src = ws.V;
       dst = ws.T;
     } else if (p > 0) {
-      DMRG_TRY(syev_gemm(ws, 0, np, np, np, ws.V, np, Q, ws.T, s));
-      src = ws.T;
+      src = Q == ws.T ? ws.G : ws.T;
+      DMRG_TRY(syev_gemm(ws, 0, np, np, np, ws.V, np, Q, src, s));
     }
     // Newton-Schulz steps, ending in ws.V: one brings the 1e-6 of an FP32
     // rotation to 1e-12, enough for the first two passes; then two (or one
