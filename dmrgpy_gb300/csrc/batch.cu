@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "heff.cuh"
+#include "krylov.cuh"
 
 namespace dmrg {
 namespace {
@@ -40,7 +41,7 @@ struct LSeg {
   T* v;          // n: input of the matvec (= current q_j)
   double* alpha; // kmax
   double* beta;  // kmax
-  T* h;          // kmax + 1: reorthogonalisation coefficients
+  T* h;          // 2 LZ_CTAS x (kmax + 1): reorthogonalisation coefficients
   const T* y;    // kmax: Ritz coefficients (uploaded by the host)
   long long n;
   int* dead;     // 1 after a breakdown (beta < tol)
@@ -57,13 +58,6 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
   return s;
 }
-
-template <typename T>
-__device__ __forceinline__ double re_dot(T a, T b);
-template <>
-__device__ __forceinline__ double re_dot<double>(double a, double b) { return a * b; }
-template <>
-__device__ __forceinline__ double re_dot<cplx>(cplx a, cplx b) { return a.x * b.x + a.y * b.y; }
 
 // q0 = x / |x| (a zero start becomes a fixed pseudo-random vector), into Q[0] and v
 template <typename T>
@@ -96,74 +90,23 @@ __global__ void __launch_bounds__(kVecThreads) lz_init_kernel(const LSeg<T>* __r
   if (threadIdx.x == 0) *a.dead = 0;
 }
 
-// alpha_j = Re <q_j, w>;  w -= alpha_j q_j + beta_{j-1} q_{j-1}
+// Step j of every problem: alpha_j, the three-term update, the
+// reorthogonalisation against q_0 .. q_(j-1), beta_j, and q_(j+1) into Q[j+1]
+// and v (zero after a breakdown); a cluster of eight CTAs per problem.  As
+// four kernels, of one CTA per problem or per vector, this was 29 us a step
+// for 24 problems of up to 4096 elements; 10 us now, bound by the FP64 pipes of
+// eight SMs.
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) lz_alpha_axpy_kernel(const LSeg<T>* __restrict__ tab, int j) {
-  __shared__ double red[32];
-  const LSeg<T> a = tab[blockIdx.x];
-  const T* qj = a.Q + (long long)j * a.n;
-  double s = 0.0;
-  for (long long i = threadIdx.x; i < a.n; i += blockDim.x) s += re_dot<T>(qj[i], a.w[i]);
-  const double al = block_sum<T>(s, red);
-  const double bp = j > 0 ? a.beta[j - 1] : 0.0;
-  const T* qm = j > 0 ? a.Q + (long long)(j - 1) * a.n : qj;
-  for (long long i = threadIdx.x; i < a.n; i += blockDim.x) {
-    T w = a.w[i];
-    w = Sc<T>::sub(w, Sc<T>::scale(qj[i], al));
-    if (j > 0) w = Sc<T>::sub(w, Sc<T>::scale(qm[i], bp));
-    a.w[i] = w;
-  }
-  if (threadIdx.x == 0) a.alpha[j] = al;
-}
-
-// h_i = <q_i, w> for i < j; grid (j, nprob)
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) lz_multidot_kernel(const LSeg<T>* __restrict__ tab) {
-  __shared__ double red[32];
-  const LSeg<T> a = tab[blockIdx.y];
-  const int i = blockIdx.x;
-  const T* q = a.Q + (long long)i * a.n;
-  double sr = 0.0, si = 0.0;
-  for (long long e = threadIdx.x; e < a.n; e += blockDim.x) {
-    const T c = Sc<T>::mul(Sc<T>::conj(q[e]), a.w[e]);
-    sr += Sc<T>::re(c);
-    si += Sc<T>::im(c);
-  }
-  sr = block_sum<T>(sr, red);
-  si = block_sum<T>(si, red);
-  if (threadIdx.x == 0) a.h[i] = Sc<T>::make(sr, si);
-}
-
-// w -= sum_{i<j} h_i q_i; grid (blocks, nprob)
-template <typename T>
-__global__ void lz_gemv_kernel(const LSeg<T>* __restrict__ tab, int j) {
-  const LSeg<T> a = tab[blockIdx.y];
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < a.n; e += (long long)gridDim.x * blockDim.x) {
-    T w = a.w[e];
-    for (int i = 0; i < j; ++i) w = Sc<T>::sub(w, Sc<T>::mul(a.h[i], a.Q[(long long)i * a.n + e]));
-    a.w[e] = w;
-  }
-}
-
-// beta_j = |w|; q_{j+1} = w / beta_j into Q[j+1] and v (zero after a breakdown)
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) lz_beta_kernel(const LSeg<T>* __restrict__ tab, int j, double tol) {
-  __shared__ double red[32];
-  const LSeg<T> a = tab[blockIdx.x];
-  double s = 0.0;
-  for (long long i = threadIdx.x; i < a.n; i += blockDim.x) s += Sc<T>::abs2(a.w[i]);
-  const double be = sqrt(block_sum<T>(s, red));
-  const bool dead = *((volatile int*)a.dead) != 0 || !(be >= tol);
-  const double inv = dead ? 0.0 : 1.0 / be;
-  T* qn = a.Q + (long long)(j + 1) * a.n;
-  for (long long i = threadIdx.x; i < a.n; i += blockDim.x) {
-    const T q = Sc<T>::scale(a.w[i], inv);
-    qn[i] = q;
-    a.v[i] = q;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    a.beta[j] = be;
+__global__ void __launch_bounds__(LZ_THREADS) __cluster_dims__(LZ_CTAS, 1, 1)
+lz_step_kernel(const LSeg<T>* __restrict__ tab, int j, int ldh, double tol) {
+  const LSeg<T> a = tab[blockIdx.x / LZ_CTAS];
+  bool dead = *((volatile int*)a.dead) != 0;
+  const double bp = j > 0 ? *((volatile double*)a.beta + j - 1) : 0.0;
+  double are, aim, beta;
+  lz_cluster_step<T>(a.Q, a.w, a.v, a.n, j, j, true, bp, a.h, ldh, tol, dead, are, aim, beta);
+  if (blockIdx.x % LZ_CTAS == 0 && threadIdx.x == 0) {
+    a.alpha[j] = are;
+    a.beta[j] = beta;
     if (dead) *a.dead = 1;
   }
 }
@@ -211,7 +154,7 @@ bool lz_layout(int nprob, const dmrg_heff_t* ops, int kmax, LzLayout* L) {
     L->Q[p] = off; off += align_up(sizeof(T) * n * (size_t)(kmax + 1));
     L->w[p] = off; off += align_up(sizeof(T) * n);
     L->v[p] = off; off += align_up(sizeof(T) * n);
-    L->h[p] = off; off += align_up(sizeof(T) * (size_t)(kmax + 1));
+    L->h[p] = off; off += align_up(sizeof(T) * 2 * LZ_CTAS * (size_t)(kmax + 1));
     L->P[p] = off; off += align_up(sizeof(T) * P);
     L->Pq[p] = off; off += align_up(sizeof(T) * (Q > 0 ? Q : 1));
   }
@@ -244,28 +187,18 @@ struct LzPlan {
   long long gtiles[4];
   int gtile[4];
   int nprob;
-  long long nmax;
+  int kmax;
   double tol;
 };
 
 // steps j0 .. j1-1 of the recurrence for every problem
 template <typename T>
 int lz_steps(const LzPlan<T>& pl, int j0, int j1, unsigned long long* kernels, cudaStream_t s) {
-  long long gx = (pl.nmax + 255) / 256;
-  if (gx > 64) gx = 64;
   unsigned long long before = dmrg_kernel_launches();
   for (int j = j0; j < j1; ++j) {
     for (int k = 0; k < 4; ++k)
       DMRG_TRY(tgemm_grouped_launch<T>(pl.gtab[k], pl.gn[k], pl.gtiles[k], pl.gtile[k], Sc<T>::one(), Sc<T>::zero(), s));
-    lz_alpha_axpy_kernel<T><<<pl.nprob, kVecThreads, 0, s>>>(pl.seg, j);
-    DMRG_CHECK_LAUNCH();
-    if (j > 0) {
-      lz_multidot_kernel<T><<<dim3((unsigned)j, (unsigned)pl.nprob), kVecThreads, 0, s>>>(pl.seg);
-      DMRG_CHECK_LAUNCH();
-      lz_gemv_kernel<T><<<dim3((unsigned)gx, (unsigned)pl.nprob), 256, 0, s>>>(pl.seg, j);
-      DMRG_CHECK_LAUNCH();
-    }
-    lz_beta_kernel<T><<<pl.nprob, kVecThreads, 0, s>>>(pl.seg, j, pl.tol);
+    lz_step_kernel<T><<<pl.nprob * LZ_CTAS, LZ_THREADS, 0, s>>>(pl.seg, j, pl.kmax + 1, pl.tol);
     DMRG_CHECK_LAUNCH();
   }
   if (kernels) *kernels = dmrg_kernel_launches() - before;
@@ -346,7 +279,7 @@ int batch_lanczos(int nprob, const dmrg_heff_t* ops, void* const* x, int kmax, d
   LzPlan<T> pl;
   pl.seg = reinterpret_cast<const LSeg<T>*>(base + L.seg_tab);
   pl.nprob = nprob;
-  pl.nmax = nmax;
+  pl.kmax = kmax;
   pl.tol = tol;
   std::vector<char> hdesc(tgemm_grouped_desc_bytes(nprob));
   std::vector<TGemm> g(nprob);

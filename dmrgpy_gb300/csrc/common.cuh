@@ -182,7 +182,7 @@ constexpr int MULTIDOT_MAX_GRID = 2 * 152;
 // with nq = 0.
 template <typename T> bool krylov_step_fits(long long n, int nq);
 template <typename T>
-int krylov_step(T* Q, const T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
+int krylov_step(T* Q, T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
                 unsigned epoch, cudaStream_t s);
 template <typename T> int vcopy(T* y, const T* x, long long n, cudaStream_t s);
 template <typename T> int vfill_random(T* x, long long n, unsigned long long seed, cudaStream_t s);

@@ -4,7 +4,7 @@
 // scaling with scalars that stay in device memory, and the block
 // reorthogonalisation h = Q^H w, w -= Q h.  All HBM-bound; grids are sized in
 // multiples of the 152 SMs.
-#include "common.cuh"
+#include "krylov.cuh"
 
 namespace dmrg {
 
@@ -199,6 +199,7 @@ __global__ void gemv_kernel(const T* __restrict__ Q, long long ldq, int k, const
 constexpr int KT = 512;                   // threads
 constexpr int KW = KT / 32;
 constexpr int KRYLOV_STEP_SMEM = 64 * 1024;
+constexpr long long KRYLOV_CLUSTER = 2048;   // elements of a vector that one cluster handles at most
 constexpr int KRYLOV_SLICE = 1536;        // elements of a CTA's slice at most
 constexpr int KC = 128;                   // elements of a CTA's slice handled at a time by the update
 constexpr unsigned kStepSpinLimit = 1u << 22;   // polls, seconds: far beyond any real wait
@@ -224,23 +225,30 @@ __device__ __forceinline__ void step_barrier(unsigned* count, int* err, unsigned
   __syncthreads();
 }
 
-// sum of the CTAs' pairs part[2 b], part[2 b + 1], in every thread
-__device__ __forceinline__ void grid_sum2(const double* part, double& re, double& im, double* sh) {
-  re = 0.0;
-  im = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += KT) {
-    re += __ldcg(part + 2 * b);
-    im += __ldcg(part + 2 * b + 1);
-  }
-  block_sum2(re, im, sh);
-  if (threadIdx.x == 0) {
-    sh[0] = re;
-    sh[1] = im;
+// sum of the CTAs' pairs part[2 b], part[2 b + 1], in every thread (NORM: the
+// norm and its reciprocal from the sum of squares)
+template <bool IM, bool NORM>
+__device__ __forceinline__ void grid_sum2(const double* part, double& re, double& im, double* all) {
+  if (threadIdx.x < 32) {
+    re = im = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) {
+      re += __ldcg(part + 2 * b);
+      if (IM) im += __ldcg(part + 2 * b + 1);
+    }
+    re = warp_sum(re);
+    if (IM) im = warp_sum(im);
+    if (threadIdx.x == 0) {
+      if (NORM) {
+        lz_norm(re, all);
+      } else {
+        all[0] = re;
+        all[1] = im;
+      }
+    }
   }
   __syncthreads();
-  re = sh[0];
-  im = sh[1];
-  __syncthreads();
+  re = all[0];
+  im = all[1];
 }
 
 // alpha = q_j^H w, w -= alpha q_j + beta_(j-1) q_(j-1), w -= Q_nq Q_nq^H w,
@@ -253,7 +261,9 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
                                                          int nq, int next, long long slice, double* sc, double* red,
                                                          double* part, unsigned epoch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double sh[64];
+  __shared__ double red2[KW][2];
+  __shared__ double sums[2][2];
+  constexpr bool C = sizeof(T) == 16;
   T* ws = reinterpret_cast<T*>(smem_raw);   // slice
   T* comb = ws + slice;                     // KT
   T* hs = comb + KT;                        // nq
@@ -272,14 +282,15 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
     ws[e] = v;
     acc_dot<T>(qj[e], v, re, im);
   }
-  block_sum2(re, im, sh);
+  const int act = cnt >= KT ? KW : (cnt + 31) / 32;
+  lz_block_sum<C>(re, im, act, red2);
   if (threadIdx.x == 0) {
     ra[2 * b] = re;
     ra[2 * b + 1] = im;
   }
   step_barrier(count, err, epoch);
   double are, aim;
-  grid_sum2(ra, are, aim, sh);
+  grid_sum2<C, false>(ra, are, aim, sums[0]);
   for (int e = threadIdx.x; e < cnt; e += KT) {
     T v = Sc<T>::sub(ws[e], Sc<T>::scale(qj[e], are));
     if (j > 0) v = Sc<T>::sub(v, Sc<T>::scale(qj[e - n], bprev));
@@ -294,7 +305,7 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
 #pragma unroll 4
       for (int e = lane; e < cnt; e += 32) acc_dot<T>(q[e], ws[e], re, im);
       re = warp_sum(re);
-      if (sizeof(T) == 16) im = warp_sum(im);
+      if (C) im = warp_sum(im);
       if (lane == 0) {
         part[2 * ((long long)i * G + b)] = re;
         part[2 * ((long long)i * G + b) + 1] = im;
@@ -306,10 +317,10 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
       re = im = 0.0;
       for (int g = lane; g < G; g += 32) {
         re += __ldcg(pi + 2 * g);
-        if (sizeof(T) == 16) im += __ldcg(pi + 2 * g + 1);
+        if (C) im += __ldcg(pi + 2 * g + 1);
       }
       re = warp_sum(re);
-      if (sizeof(T) == 16) im = warp_sum(im);
+      if (C) im = warp_sum(im);
       if (lane == 0) hs[i] = Sc<T>::make(re, im);
     }
     __syncthreads();
@@ -336,16 +347,16 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
     if (cp == 0 && e < cnt) acc_dot<T>(ws[e], ws[e], re, im);
     __syncthreads();
   }
-  block_sum2(re, im, sh);
+  // (only the first KC threads hold sums)
+  lz_block_sum<false>(re, im, cnt >= KC ? KC / 32 : (cnt + 31) / 32, red2);
   if (threadIdx.x == 0) {
     rn[2 * b] = re;
     rn[2 * b + 1] = 0.0;
   }
   step_barrier(count, err, epoch + (nq > 0 ? 2 : 1));
-  grid_sum2(rn, re, im, sh);
-  const double beta = sqrt(re);
+  double beta, inv;
+  grid_sum2<false, true>(rn, beta, inv, sums[1]);
   if (next) {
-    const double inv = 1.0 / beta;
     T* qn = Q + (long long)(j + 1) * n + lo;
     for (int e = threadIdx.x; e < cnt; e += KT) qn[e] = Sc<T>::scale(ws[e], inv);
   }
@@ -354,6 +365,24 @@ __global__ void __launch_bounds__(KT) krylov_step_kernel(T* __restrict__ Q, cons
     sc[1] = aim;
     sc[2] = beta;
     sc[3] = *(volatile int*)err;
+  }
+}
+
+// The same for short vectors: one cluster, whose barriers take a fraction of a
+// microsecond (a bond's ground state at n = 1024: 2.06 -> 1.92 ms; at 4096 its
+// eight SMs' FP64 pipes cost as much as they save, at 8100 2.46 -> 2.74).
+template <typename T>
+__global__ void __launch_bounds__(LZ_THREADS) __cluster_dims__(LZ_CTAS, 1, 1)
+krylov_cluster_kernel(T* Q, T* w, long long n, int j, int nq, int next, double* sc, T* h) {
+  const double bprev = j > 0 ? *((volatile double*)sc + 2) : 0.0;
+  double are, aim, beta;
+  bool dead = false;
+  lz_cluster_step<T>(Q, w, nullptr, n, j, nq, next != 0, bprev, h, nq, 0.0, dead, are, aim, beta);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc[0] = are;
+    sc[1] = aim;
+    sc[2] = beta;
+    sc[3] = 0.0;
   }
 }
 
@@ -454,9 +483,9 @@ int gemv_sub(const T* Q, long long ldq, int k, const T* h, T* w, long long n, in
 // Elements per CTA of krylov_step, or 0 where the separate kernels are the
 // better choice (long vectors: one CTA per SM no longer draws the bandwidth)
 // or the only one.  A bond's ground state, separate -> one kernel: n = 1024
-// 2.84 -> 2.31 ms, 16 k 7.49 -> 6.07, 102 k 14.8 -> 10.9, 230 k 17.1 -> 15.9,
+// 2.84 -> 1.92 ms, 16 k 7.49 -> 5.70, 102 k 14.8 -> 10.9, 230 k 17.1 -> 15.9,
 // 590 k 41.3 -> 55.2 (left apart); a complex step of exp(-i tau H): n = 16 k
-// 0.94 -> 0.82, 160 k 2.10 -> 1.95.
+// 0.94 -> 0.75, 160 k 2.10 -> 1.95.
 static long long step_slice(size_t es, long long n, int nq, int* grid) {
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -477,8 +506,14 @@ bool krylov_step_fits(long long n, int nq) {
 }
 
 template <typename T>
-int krylov_step(T* Q, const T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
+int krylov_step(T* Q, T* w, long long n, int j, int nq, bool next, double* sc, double* red, double* part,
                 unsigned epoch, cudaStream_t s) {
+  if (n <= KRYLOV_CLUSTER) {
+    krylov_cluster_kernel<T><<<LZ_CTAS, LZ_THREADS, 0, s>>>(Q, w, n, j, nq, next ? 1 : 0, sc,
+                                                           reinterpret_cast<T*>(part));
+    DMRG_CHECK_LAUNCH();
+    return DMRG_OK;
+  }
   static std::atomic<unsigned long long> attr{0};
   const void* fn = reinterpret_cast<const void*>(krylov_step_kernel<T>);
   DMRG_TRY(smem_attr_once(fn, KRYLOV_STEP_SMEM, attr));
@@ -508,7 +543,7 @@ int nan_check(const void* x, long long n_doubles, int* flag, cudaStream_t s) {
   template int multidot_ws<T>(const T*, long long, int, const T*, long long, T*, double*, cudaStream_t); \
   template int gemv_sub<T>(const T*, long long, int, const T*, T*, long long, int, cudaStream_t); \
   template bool krylov_step_fits<T>(long long, int);                                            \
-  template int krylov_step<T>(T*, const T*, long long, int, int, bool, double*, double*, double*, unsigned, \
+  template int krylov_step<T>(T*, T*, long long, int, int, bool, double*, double*, double*, unsigned, \
                               cudaStream_t);
 INST(double)
 INST(cplx)
