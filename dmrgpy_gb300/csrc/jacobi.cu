@@ -24,6 +24,9 @@ namespace {
 
 constexpr long long kBarrierSpinLimit = 1ll << 26;  // ~seconds: far beyond any real wait
 
+constexpr int HESTENES_ONE = 7;          // pairs of a round that one CTA handles at most
+constexpr int HESTENES_CTA_COLS = 64;   // columns of the cluster variant at most
+
 struct GridBar {
   unsigned* count;
   unsigned* gen;
@@ -67,6 +70,7 @@ struct HArgs {
   int r, c, cp;  // cp = c rounded up to even
   int max_sweeps;
   double tol;
+  double* nrm;   // c (cooperative variant): squared column norms
   const double* frob;  // |M|_F (device): absolute floor of the rotation test
   GridBar bar;
   unsigned* rotcnt;  // [3], used cyclically: sweep k counts into slot k%3
@@ -74,101 +78,6 @@ struct HArgs {
   int X_in_smem;
   int abs_floor;  // 1: skip couplings below 1e-16 |M|_F^2 (the divided factor is not returned)
 };
-
-template <typename T>
-__device__ __forceinline__ void gram2(const T* xp, const T* xq, int r, int lane, double& al, double& be, double& gre,
-                                      double& gim);
-template <>
-__device__ __forceinline__ void gram2<double>(const double* xp, const double* xq, int r, int lane, double& al,
-                                              double& be, double& gre, double& gim) {
-  al = be = gre = gim = 0.0;
-  for (int i = lane; i < r; i += 32) {
-    double a = xp[i], b = xq[i];
-    al = ::fma(a, a, al);
-    be = ::fma(b, b, be);
-    gre = ::fma(a, b, gre);
-  }
-}
-template <>
-__device__ __forceinline__ void gram2<cplx>(const cplx* xp, const cplx* xq, int r, int lane, double& al, double& be,
-                                            double& gre, double& gim) {
-  al = be = gre = gim = 0.0;
-  for (int i = lane; i < r; i += 32) {
-    cplx a = xp[i], b = xq[i];
-    al = ::fma(a.x, a.x, ::fma(a.y, a.y, al));
-    be = ::fma(b.x, b.x, ::fma(b.y, b.y, be));
-    gre = ::fma(a.x, b.x, ::fma(a.y, b.y, gre));   // Re conj(a) b
-    gim = ::fma(a.x, b.y, ::fma(-a.y, b.x, gim));  // Im conj(a) b
-  }
-}
-
-// Sums of four values over the warp, every lane with all of them: the first
-// two steps also halve what a lane carries, 6 FP64 adds instead of 20 (an FP64
-// warp instruction occupies its sub-partition for 64 clocks on GB300, and
-// these sums and the rotation's scalars, not the columns, were most of a
-// round).
-__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
-  const int lane = threadIdx.x & 31;
-  const bool h4 = lane & 16, h3 = lane & 8;
-  const double k0 = h4 ? c : a, s0 = h4 ? a : c, k1 = h4 ? d : b, s1 = h4 ? b : d;
-  const double r0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 16), r1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-  double r = (h3 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, h3 ? r0 : r1, 8);
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-  a = __shfl_sync(0xffffffffu, r, 0);
-  b = __shfl_sync(0xffffffffu, r, 8);
-  c = __shfl_sync(0xffffffffu, r, 16);
-  d = __shfl_sync(0xffffffffu, r, 24);
-}
-
-// Rotation of a column pair from its Gram block (al = |x_p|^2, be = |x_q|^2,
-// g = x_p^H x_q): cs and se = sn g/|g|; false where the coupling is below tol
-// relative to the pair, below the absolute floor, or nothing.  The scalars
-// come from FP32 seeds refined in FP64 (t to ~1e-14: what it misses is left
-// to the next sweep; cs to rounding: the rotations stay orthonormal), about
-// 20 FP64 instructions where square roots and divisions take 100.
-template <typename T>
-__device__ __forceinline__ bool pair_rotation(double al, double be, double gre, double gim, double tol, double floor_,
-                                              double& cs, T& se) {
-  // the pair scaled by a power of two so that the larger norm is in [1, 2)
-  const int ex = max(__double2hiint(al), __double2hiint(be)) >> 20;
-  if (ex <= 0 || ex >= 2046) return false;   // nothing there, or not finite (the norms report that)
-  const double sc = __hiloint2double((2046 - ex) << 20, 0);
-  al *= sc;
-  be *= sc;
-  gre *= sc;
-  double ag, inv = 0.0;
-  if (sizeof(T) == 8) {
-    ag = fabs(gre);
-  } else {
-    gim *= sc;
-    const double g2 = fma(gre, gre, gim * gim);
-    if (!(g2 > 1e-290)) return false;
-    inv = rsqrt(g2);
-    ag = g2 * inv;
-  }
-  if (!(ag > floor_ * sc) || !(ag * ag > tol * tol * (al * be)) || !(ag > 1e-290)) return false;
-  const double d = be - al;
-  // t = tan of the angle, the smaller root of ag t^2 + d t - ag = 0
-  const float df = narrow(d), gf = narrow(ag);
-  double t;
-  if (gf > 1e-30f) {
-    const float tf = copysignf(__fdividef(2.f * gf, fabsf(df) + sqrtf(fmaf(df, df, 4.f * gf * gf))), df);
-    t = widen(tf);
-    const double f = fma(t, fma(ag, t, d), -ag);
-    t = fma(-f, widen(__fdividef(1.f, fmaf(2.f * gf, tf, df))), t);
-  } else {
-    t = ag / d;
-  }
-  const double w = fma(t, t, 1.0), hw = 0.5 * w;
-  double y = widen(rsqrtf(narrow(w)));
-  y = y * fma(-hw * y, y, 1.5);
-  y = y * fma(-hw * y, y, 1.5);
-  cs = y;
-  const double sn = t * y;
-  se = sizeof(T) == 8 ? Sc<T>::make(gre < 0.0 ? -sn : sn, 0.0) : Sc<T>::make(sn * (gre * inv), sn * (gim * inv));
-  return true;
-}
 
 // apply X <- X J on columns (p, q): J = [[c, se], [-conj(se), c]]
 __device__ __forceinline__ void rot_cols(double* xp, double* xq, int r, int lane, double c, double se) {
@@ -187,16 +96,161 @@ __device__ __forceinline__ void rot_cols(cplx* xp, cplx* xq, int r, int lane, do
   }
 }
 
-__device__ __forceinline__ int player(int pos, int round, int cp) {
-  return pos == 0 ? 0 : 1 + (pos - 1 + round) % (cp - 1);
+// g = x_p^H x_q, summed over the warp
+__device__ __forceinline__ void coupling(const double* xp, const double* xq, int r, int lane, double& gre,
+                                         double& gim) {
+  gre = gim = 0.0;
+  for (int i = lane; i < r; i += 32) gre = ::fma(xp[i], xq[i], gre);
+  gre = warp_sum(gre);
+}
+__device__ __forceinline__ void coupling(const cplx* xp, const cplx* xq, int r, int lane, double& gre, double& gim) {
+  double re = 0.0, im = 0.0;
+  for (int i = lane; i < r; i += 32) {
+    const cplx a = xp[i], b = xq[i];
+    re = ::fma(a.x, b.x, ::fma(a.y, b.y, re));   // Re conj(a) b
+    im = ::fma(a.x, b.y, ::fma(-a.y, b.x, im));  // Im conj(a) b
+  }
+  // half a warp takes each sum: 5 adds instead of 10
+  const bool h = lane & 16;
+  double s = (h ? im : re) + __shfl_xor_sync(0xffffffffu, h ? re : im, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  gre = __shfl_sync(0xffffffffu, s, 0);
+  gim = __shfl_sync(0xffffffffu, s, 16);
 }
 
-template <typename T, bool COOP>
+// |x|^2 in every lane
+template <typename T>
+__device__ __forceinline__ double col_norm2(const T* x, int r, int lane) {
+  double s = 0.0;
+  for (int i = lane; i < r; i += 32) s += Sc<T>::abs2(x[i]);
+  return warp_sum(s);
+}
+
+__device__ __forceinline__ int exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// x 2^k from the bit pattern (zero below the normal range; no overflow here)
+__device__ __forceinline__ double shift2(double x, int k) {
+  const int e = exponent(x);
+  return e == 0 || e + k <= 0 ? 0.0 : __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+}
+
+// 1 / sqrt(w) from an FP32 seed, one third-order step: 2^-21 becomes rounding
+__device__ __forceinline__ double rsqrt_from(double w, float seed) {
+  const double y = widen(seed);
+  const double e = fma(-w * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Rotation of a column pair from al = |x_p|^2, be = |x_q|^2 and g = x_p^H x_q:
+// cs and se = sn g/|g|, and dn, what |x_p|^2 loses and |x_q|^2 gains; false
+// where the coupling is below tol relative to the pair, below the absolute
+// floor, or nothing.  An FP64 warp instruction occupies its sub-partition for
+// 64 clocks on GB300, so the angle is found in FP32 (what it misses, 1e-7 of
+// the coupling, is left to the next sweep) and scaling and comparisons work on
+// bit patterns; cs and the phase are to rounding, so that the rotations stay
+// unitary.  9 FP64 instructions (20 complex).
+template <typename T>
+__device__ __forceinline__ bool pair_rotation(double al, double be, double gre, double gim, double tol, double floor_,
+                                              double& cs, T& se, double& dn) {
+  // the pair scaled by a power of two so that the larger norm is in [1, 2)
+  const int ex = max(exponent(al), exponent(be));
+  if (ex == 0 || ex >= 2046) return false;   // nothing there, or not finite (the norms report that)
+  double ag, px = 0.0, py = 0.0;
+  if (sizeof(T) == 8) {
+    ag = fabs(gre);
+  } else {
+    const int eg = max(exponent(gre), exponent(gim));
+    if (eg == 0 || eg >= 2047) return false;
+    const double gx = shift2(gre, 1023 - eg), gy = shift2(gim, 1023 - eg);
+    const double g2 = fma(gx, gx, gy * gy);   // in [1, 8)
+    const double inv = rsqrt_from(g2, rsqrtf(narrow(g2)));
+    px = gx * inv;
+    py = gy * inv;
+    ag = shift2(g2 * inv, eg - 1023);
+  }
+  if (!(__double_as_longlong(ag) > __double_as_longlong(floor_)) || exponent(ag) == 0) return false;
+  const double d = be - al;
+  const float gf = narrow(shift2(ag, 1023 - ex)), df = narrow(shift2(d, 1023 - ex));
+  const float af = narrow(shift2(al, 1023 - ex)), bf = narrow(shift2(be, 1023 - ex));
+  double t;
+  float tf;
+  if (gf > 1e-30f && af > 1e-30f && bf > 1e-30f) {
+    if (!(gf > (float)tol * (sqrtf(af) * sqrtf(bf)))) return false;
+    // t = tan of the angle, the smaller root of g t^2 + d t - g = 0
+    tf = copysignf(__fdividef(2.f * gf, fabsf(df) + sqrtf(fmaf(df, df, 4.f * gf * gf))), df);
+    t = widen(tf);
+  } else {
+    if (!(ag * ag > tol * tol * (al * be)) || !(ag > 1e-290)) return false;
+    t = ag / (d == 0.0 ? ag : d);
+    if (fabs(t) > 1.0) t = copysign(1.0, t);
+    tf = narrow(t);
+  }
+  const double y = rsqrt_from(fma(t, t, 1.0), rsqrtf(fmaf(tf, tf, 1.f)));
+  cs = y;
+  const double sn = t * y;
+  dn = t * ag;
+  se = sizeof(T) == 8 ? Sc<T>::make(gre < 0.0 ? -sn : sn, 0.0) : Sc<T>::make(sn * px, sn * py);
+  return true;
+}
+
+// One pair of a round: nrm holds the columns' squared norms, kept up by the
+// rotations and, where one shrinks by 2^6 or more (the update cancels), summed
+// again.  True where it rotated.
+template <typename T>
+__device__ __forceinline__ bool rotate_pair(T* X, T* V, int r, int c, int p, int q, volatile double* nrm, int lane,
+                                            double tol, double abs_floor) {
+  T* xp = X + (long long)p * r;
+  T* xq = X + (long long)q * r;
+  double al = nrm[p], be = nrm[q], gre, gim, cs, dn;
+  T se;
+  coupling(xp, xq, r, lane, gre, gim);
+  if (!pair_rotation<T>(al, be, gre, gim, tol, abs_floor, cs, se, dn)) return false;
+  rot_cols(xp, xq, r, lane, cs, se);
+  rot_cols(V + (long long)p * c, V + (long long)q * c, c, lane, cs, se);
+  const double an = al - dn, bn = be + dn;
+  __syncwarp();
+  double av = an, bv = bn;
+  if (__double2hiint(an) < 0 || exponent(an) + 6 <= exponent(al)) av = col_norm2(xp, r, lane);
+  if (__double2hiint(bn) < 0 || exponent(bn) + 6 <= exponent(be)) bv = col_norm2(xq, r, lane);
+  if (lane == 0) {
+    nrm[p] = av;
+    nrm[q] = bv;
+  }
+  return true;
+}
+
+__device__ __forceinline__ int player(int pos, int round, int cp) {
+  const int v = pos - 1 + round;   // below 2 (cp - 1)
+  return pos == 0 ? 0 : 1 + (v >= cp - 1 ? v - (cp - 1) : v);
+}
+
+// One CTA; a cluster of HESTENES_CLUSTER, which shares the pairs of a round out
+// to as many SMs' FP64 pipes and meets at the hardware's barrier; a
+// cooperative grid.
+enum { ONE_CTA = 0, GRID = 1, CLUSTER = 2 };
+constexpr int HESTENES_CLUSTER = 8;
+
+template <int MODE>
+__device__ __forceinline__ bool round_barrier(const GridBar& b) {
+  if (MODE == GRID) return grid_barrier(b);
+  if (MODE == CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+  return true;
+}
+
+template <typename T, int MODE>
 __global__ void __launch_bounds__(1024) hestenes_kernel(HArgs<T> a) {
   extern __shared__ unsigned char hsm[];
+  __shared__ double nrm_s[HESTENES_CTA_COLS];
+  volatile double* const nrm = MODE == ONE_CTA ? nrm_s : a.nrm;
   // single-CTA variant: work on a shared-memory copy of X when it fits
   T* const Xg = a.X;
-  if (!COOP && a.X_in_smem) {
+  if (MODE == ONE_CTA && a.X_in_smem) {
     T* xs = reinterpret_cast<T*>(hsm);
     for (long long i = threadIdx.x; i < (long long)a.r * a.c; i += blockDim.x) xs[i] = Xg[i];
     a.X = xs;
@@ -217,7 +271,7 @@ __global__ void __launch_bounds__(1024) hestenes_kernel(HArgs<T> a) {
     a.V[idx] = row == col ? Sc<T>::one() : Sc<T>::zero();
   }
   if (gtid == 0) { a.rotcnt[0] = 0u; a.rotcnt[1] = 0u; a.rotcnt[2] = 0u; }
-  if (COOP) { if (!grid_barrier(a.bar)) return; } else { __syncthreads(); }
+  if (!round_barrier<MODE>(a.bar)) return;
 
   int sweep = 0;
   bool converged = a.cp < 2;
@@ -225,34 +279,30 @@ __global__ void __launch_bounds__(1024) hestenes_kernel(HArgs<T> a) {
     // slot (sweep+1)%3 was last read at the end of sweep-2, before at least
     // one barrier of sweep-1, so no CTA can still be reading it
     if (gtid == 0) a.rotcnt[(sweep + 1) % 3] = 0u;
+    for (int col = gw; col < a.c; col += nw) {
+      const double v = col_norm2(a.X + (long long)col * a.r, a.r, lane);
+      if (lane == 0) nrm[col] = v;
+    }
+    if (!round_barrier<MODE>(a.bar)) return;
     for (int round = 0; round < a.cp - 1; ++round) {
       for (int i = gw; i < half; i += nw) {
         int p = player(i, round, a.cp), q = player(a.cp - 1 - i, round, a.cp);
         if (p > q) { int t = p; p = q; q = t; }
         if (q >= a.c) continue;  // dummy column of an odd count
-        T* xp = a.X + (long long)p * a.r;
-        T* xq = a.X + (long long)q * a.r;
-        double al, be, gre, gim;
-        gram2<T>(xp, xq, a.r, lane, al, be, gre, gim);
-        warp_sum4(al, be, gre, gim);
         // rotate only couplings above tol relative to the pair and above an
         // absolute floor (1e-16 |M|_F^2): singular values come out to the
         // absolute accuracy of a standard SVD without chasing the relative
         // accuracy of negligible ones, which costs many extra sweeps on the
         // steeply graded spectra of DMRG bonds
-        double cs;
-        T se;
-        if (!pair_rotation<T>(al, be, gre, gim, a.tol, abs_floor, cs, se)) continue;
-        rot_cols(xp, xq, a.r, lane, cs, se);
-        rot_cols(a.V + (long long)p * a.c, a.V + (long long)q * a.c, a.c, lane, cs, se);
-        if (lane == 0) atomicAdd(&a.rotcnt[sweep % 3], 1u);
+        if (rotate_pair<T>(a.X, a.V, a.r, a.c, p, q, nrm, lane, a.tol, abs_floor) && lane == 0)
+          atomicAdd(&a.rotcnt[sweep % 3], 1u);
       }
-      if (COOP) { if (!grid_barrier(a.bar)) return; } else { __syncthreads(); }
+      if (!round_barrier<MODE>(a.bar)) return;
     }
     converged = (((volatile unsigned*)a.rotcnt)[sweep % 3] == 0u);
   }
   if (gtid == 0) *a.sweeps_out = converged ? sweep : -sweep;
-  if (!COOP && a.X_in_smem) {
+  if (MODE == ONE_CTA && a.X_in_smem) {
     __syncthreads();
     for (long long i = threadIdx.x; i < (long long)a.r * a.c; i += blockDim.x) Xg[i] = a.X[i];
   }
@@ -369,10 +419,12 @@ __global__ void __launch_bounds__(1024) hestenes_batch_kernel(const BSvd<T>* __r
   const BSvd<T> a = tab[blockIdx.x];
   __shared__ double red[32];
   __shared__ unsigned rot;
+  __shared__ double nrm_s[HESTENES_CTA_COLS];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int r = a.r, c = a.c, cp = c + (c & 1), half = cp / 2;
   T* X = a.X;
   T* V = a.V;
+  volatile double* const nrm = c <= HESTENES_CTA_COLS ? nrm_s : a.sig;
   const long long mn = (long long)a.m * a.n;
   double part = 0.0;
   for (long long idx = threadIdx.x; idx < mn; idx += blockDim.x) {
@@ -403,22 +455,17 @@ __global__ void __launch_bounds__(1024) hestenes_batch_kernel(const BSvd<T>* __r
   for (; sweep < max_sweeps && !converged; ++sweep) {
     if (threadIdx.x == 0) rot = 0u;
     __syncthreads();
+    for (int col = wid; col < c; col += nw) {
+      const double v = col_norm2(X + (long long)col * r, r, lane);
+      if (lane == 0) nrm[col] = v;
+    }
+    __syncthreads();
     for (int round = 0; round < cp - 1; ++round) {
       for (int i = wid; i < half; i += nw) {
         int p = player(i, round, cp), q = player(cp - 1 - i, round, cp);
         if (p > q) { const int t = p; p = q; q = t; }
         if (q >= c) continue;
-        T* xp = X + (long long)p * r;
-        T* xq = X + (long long)q * r;
-        double al, be, gre, gim;
-        gram2<T>(xp, xq, r, lane, al, be, gre, gim);
-        warp_sum4(al, be, gre, gim);
-        double cs;
-        T se;
-        if (!pair_rotation<T>(al, be, gre, gim, tol, abs_floor, cs, se)) continue;
-        rot_cols(xp, xq, r, lane, cs, se);
-        rot_cols(V + (long long)p * c, V + (long long)q * c, c, lane, cs, se);
-        if (lane == 0) atomicAdd(&rot, 1u);
+        if (rotate_pair<T>(X, V, r, c, p, q, nrm, lane, tol, abs_floor) && lane == 0) atomicAdd(&rot, 1u);
       }
       __syncthreads();
     }
@@ -575,12 +622,29 @@ int hestenes_factor(const T* M, int m, int n, int left, void* work, double* host
   a.bar.err = reinterpret_cast<int*>(w.ctrl + 5);
   a.sweeps_out = reinterpret_cast<int*>(w.ctrl + 6);
   a.frob = frob;
+  a.nrm = w.sig;
   a.X_in_smem = 0;
   a.abs_floor = abs_floor;
   const int half = a.cp / 2;
-  // one CTA while the pairs of a round fit in 32 warps of one CTA and the
-  // columns are short; otherwise a cooperative grid with one warp per pair
-  if ((half <= 64 && (long long)r * c <= (1ll << 20)) || half <= 8) {
+  // One CTA up to 7 pairs a round (two warps per sub-partition, each FP64
+  // instruction 64 clocks there), a cluster up to HESTENES_CTA_COLS columns,
+  // beyond that a cooperative grid, four warps a CTA.  One CTA -> cluster,
+  // complex: 60 x 16 0.93 -> 0.75 ms, 60 x 60 18.0 -> 4.6; real 60 x 16 equal;
+  // grid: 100 x 90 104 -> 19.4 (cluster of eight warps a CTA: 22.4).
+  if (half > HESTENES_ONE && 2 * half <= HESTENES_CTA_COLS) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(HESTENES_CLUSTER);
+    cfg.blockDim = dim3(128);
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = HESTENES_CLUSTER;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, hestenes_kernel<T, CLUSTER>, a));
+    count_launch();
+  } else if (half <= HESTENES_ONE) {
     int threads = 32 * (half < 32 ? (half > 0 ? half : 1) : 32);
     const size_t xbytes = sizeof(T) * (size_t)r * c;
     size_t smem = 0;
@@ -588,10 +652,10 @@ int hestenes_factor(const T* M, int m, int n, int left, void* work, double* host
       a.X_in_smem = 1;
       smem = xbytes;
       static std::atomic<unsigned long long> attr_d{0}, attr_z{0};
-      DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(hestenes_kernel<double, false>), 160 * 1024, attr_d));
-      DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(hestenes_kernel<cplx, false>), 160 * 1024, attr_z));
+      DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(hestenes_kernel<double, ONE_CTA>), 160 * 1024, attr_d));
+      DMRG_TRY(smem_attr_once(reinterpret_cast<const void*>(hestenes_kernel<cplx, ONE_CTA>), 160 * 1024, attr_z));
     }
-    hestenes_kernel<T, false><<<1, threads, smem, s>>>(a);
+    hestenes_kernel<T, ONE_CTA><<<1, threads, smem, s>>>(a);
     DMRG_CHECK_LAUNCH();
   } else {
     int dev = 0;
@@ -599,15 +663,15 @@ int hestenes_factor(const T* M, int m, int n, int left, void* work, double* host
     int nsm = 0;
     DMRG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     int per_sm = 0;
-    const int threads = 256;
-    DMRG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hestenes_kernel<T, true>, threads, 0));
+    const int threads = 128;
+    DMRG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hestenes_kernel<T, GRID>, threads, 0));
     if (per_sm < 1) return DMRG_ERR_CUDA;
     int want = (half + (threads / 32) - 1) / (threads / 32);
     int maxb = per_sm * nsm;
     int blocks = want < maxb ? want : maxb;
     if (blocks < 1) blocks = 1;
     void* args[] = {&a};
-    DMRG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)hestenes_kernel<T, true>, blocks, threads, args, 0, s));
+    DMRG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)hestenes_kernel<T, GRID>, blocks, threads, args, 0, s));
     count_launch();
   }
   colnorm_kernel<T><<<(c * 32 + 255) / 256, 256, 0, s>>>(a.X, r, c, w.sig);
