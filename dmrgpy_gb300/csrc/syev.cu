@@ -309,86 +309,109 @@ __device__ __forceinline__ float2 add_hl(float2 a, float x) {
   return make_float2(r, l - (r - h));
 }
 
-__global__ void __launch_bounds__(256) syev_solve32_kernel(const float* __restrict__ G, int np,
-                                                           const int* __restrict__ pr, float* __restrict__ R,
-                                                           int* __restrict__ ident, int* __restrict__ flag,
-                                                           const unsigned long long* __restrict__ scale,
-                                                           float2* __restrict__ dd, float rel, float abs_) {
-  __shared__ float a[2][JP][JLD];
+// Kernels of the sweep chain come up while the one before them drains
+// (launch_chain): nothing of it is touched before this.  Their pointers are
+// not __restrict__, which would let the compiler move loads up past it.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The FP32 subproblem of a block pair: one sweep over its 32 indices.  Bound by
+// the latency of a round (loads, the rotation's chain of four approximations,
+// a shuffle, the update, a barrier) and its issue slots: lane t of a half warp
+// takes pair t and the 2 x 2 blocks of pair t with pair t + k, k = 0 .. 8,
+// written twice (the matrix is symmetric); the two CTAs of a cluster rotate it
+// to the same bits and keep half of D = Q - I each.  A launch takes 12.4 us;
+// with a thread for each of the 256 blocks and all of D in one CTA 13.2, with
+// four CTAs of 128 threads 16.6 (a warp then has two blocks in turn).
+__global__ void __launch_bounds__(256) __cluster_dims__(2, 1, 1)
+syev_solve32_kernel(const float* G, int np, const int* pr, float* R,
+                    int* ident, int* flag, const unsigned long long* scale,
+                    float2* dd, float rel, float abs_) {
+  constexpr int LD = JP + 2, H = JP / 2;   // LD even: strides LD + 1 and LD - 1 across lanes
+  __shared__ float a[2][JP * LD];
   __shared__ float2 dg[2][JP];
-  __shared__ float r[JP][JLD];
-  const int pair = blockIdx.x;
+  __shared__ float r[H][JP];
+  const int pair = blockIdx.x >> 1, sub = blockIdx.x & 1;
+  chain_wait();
+  chain_next();   // the apply's CTAs fit beside the few of this kernel
   const int bi = pr[2 * pair], bj = pr[2 * pair + 1];
   const int tid = threadIdx.x;
   const float floor_ = abs_ * (float)__longlong_as_double((long long)*scale);
-  for (int e = tid; e < JP * JP; e += blockDim.x) {
-    const int i = e / JP, j = e - (e / JP) * JP;
+  for (int e = tid; e < JP * JP; e += 256) {
+    const int i = e / JP, j = e % JP;
     const int gi = i < JB ? bi * JB + i : bj * JB + i - JB;
     const int gj = j < JB ? bi * JB + j : bj * JB + j - JB;
-    a[0][i][j] = G[(long long)gi * np + gj];
-    r[i][j] = 0.f;
+    a[0][i * LD + j] = G[(long long)gi * np + gj];
   }
+  for (int e = tid; e < H * JP; e += 256) r[e / JP][e % JP] = 0.f;
   // the diagonal lives in dd (the apply's copy in G is not used)
   if (tid < JP) dg[0][tid] = dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB];
-  const int ti = tid >> 4, tj = tid & 15;
-  // tournament positions ti, 31 - ti (rows) and tj, 31 - tj (columns)
-  int pi = tour(ti, 0), qi = tour(JP - 1 - ti, 0), pj = tour(tj, 0), qj = tour(JP - 1 - tj, 0);
-  bool rotated = false, big = false;
   __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // has read dd
+  const int t = tid % H, k = tid / H, row = sub * H + k;
+  const int src = (t + k) & (H - 1);
+  const bool block = k > 0 && (k < H / 2 || (k == H / 2 && t < H / 2));
+  int p = t, q = JP - 1 - t, p1 = src, q1 = JP - 1 - src;
+  bool rotated = false, big = false;
   for (int ir = 0; ir < JP - 1; ++ir) {
-    const float(*x)[JLD] = a[ir & 1];
-    float(*z)[JLD] = a[(ir & 1) ^ 1];
-    const float2 app = dg[ir & 1][pj], aqq = dg[ir & 1][qj];
-    const float apq = x[pj][qj];
-    const float x00 = x[pi][pj], x01 = x[pi][qj], x10 = x[qi][pj], x11 = x[qi][qj];
-    const float u0 = r[ti][pj], v0 = r[ti][qj], u1 = r[ti + 16][pj], v1 = r[ti + 16][qj];
-    float tj_, cj, sj, cmj;
-    rot32(app, aqq, apq, rel, floor_, tj_, cj, sj, cmj);
-    // lane l of a warp holds column pair l % 16, so row pair ti's rotation
-    const float si = __shfl_sync(0xffffffffu, sj, ti), cmi = __shfl_sync(0xffffffffu, cmj, ti);
-    rotated = rotated || si != 0.f;
-    big = big || fabsf(si) > BIG_SIN;
-    // x + (J^T x J - x) through c - 1, so that a small rotation rounds at its own size
-    const float y00 = x00 + (cmi * x00 - si * x10), y01 = x01 + (cmi * x01 - si * x11);
-    const float y10 = x10 + (si * x00 + cmi * x10), y11 = x11 + (si * x01 + cmi * x11);
-    float z00 = y00 + (cmj * y00 - sj * y01), z01 = y01 + (sj * y00 + cmj * y01);
-    float z10 = y10 + (cmj * y10 - sj * y11), z11 = y11 + (sj * y10 + cmj * y11);
-    if (ti == tj) {   // the rotated pair itself
-      dg[(ir & 1) ^ 1][pj] = add_hl(app, -tj_ * apq);
-      dg[(ir & 1) ^ 1][qj] = add_hl(aqq, tj_ * apq);
-      z01 = z10 = sj != 0.f ? 0.f : x01;
+    const float* x = a[ir & 1];
+    float* z = a[(ir & 1) ^ 1];
+    const float2 app = dg[ir & 1][p], aqq = dg[ir & 1][q];
+    const float apq = x[p * LD + q];
+    const float u = r[k][p], v = r[k][q];
+    float t_, c_, sn, cm;
+    rot32(app, aqq, apq, rel, floor_, t_, c_, sn, cm);
+    // lane l of a warp holds the rotation of pair l % 16
+    const float sk = __shfl_sync(0xffffffffu, sn, src), ck = __shfl_sync(0xffffffffu, cm, src);
+    rotated = rotated || sn != 0.f;
+    big = big || fabsf(sn) > BIG_SIN;
+    // D <- D J + (J - I) on columns p, q, row `row`
+    float d0 = fmaf(cm, u, u) - sn * v, d1 = fmaf(sn, u, fmaf(cm, v, v));
+    if (row == p) { d0 += cm; d1 += sn; }
+    if (row == q) { d0 -= sn; d1 += cm; }
+    r[k][p] = d0;
+    r[k][q] = d1;
+    if (k == 0) {   // the rotated pair itself
+      dg[(ir & 1) ^ 1][p] = add_hl(app, -t_ * apq);
+      dg[(ir & 1) ^ 1][q] = add_hl(aqq, t_ * apq);
+      const float w = sn != 0.f ? 0.f : apq;
+      z[p * LD + q] = w;
+      z[q * LD + p] = w;
+    } else if (block) {
+      const float x00 = x[p * LD + p1], x01 = x[p * LD + q1], x10 = x[q * LD + p1], x11 = x[q * LD + q1];
+      // x + (J^T x J - x) through c - 1, so that a small rotation rounds at its own size
+      const float y00 = x00 + (cm * x00 - sn * x10), y01 = x01 + (cm * x01 - sn * x11);
+      const float y10 = x10 + (sn * x00 + cm * x10), y11 = x11 + (sn * x01 + cm * x11);
+      const float z00 = y00 + (ck * y00 - sk * y01), z01 = y01 + (sk * y00 + ck * y01);
+      const float z10 = y10 + (ck * y10 - sk * y11), z11 = y11 + (sk * y10 + ck * y11);
+      z[p * LD + p1] = z00;
+      z[p * LD + q1] = z01;
+      z[q * LD + p1] = z10;
+      z[q * LD + q1] = z11;
+      z[p1 * LD + p] = z00;
+      z[q1 * LD + p] = z01;
+      z[p1 * LD + q] = z10;
+      z[q1 * LD + q] = z11;
     }
-    z[pi][pj] = z00;
-    z[pi][qj] = z01;
-    z[qi][pj] = z10;
-    z[qi][qj] = z11;
-    // D <- D J + (J - I) on columns pj, qj, rows ti and ti + 16
-    float a0 = fmaf(cmj, u0, u0) - sj * v0, b0 = fmaf(sj, u0, fmaf(cmj, v0, v0));
-    float a1 = fmaf(cmj, u1, u1) - sj * v1, b1 = fmaf(sj, u1, fmaf(cmj, v1, v1));
-    if (ti == pj) { a0 += cmj; b0 += sj; }
-    if (ti == qj) { a0 -= sj; b0 += cmj; }
-    if (ti + 16 == pj) { a1 += cmj; b1 += sj; }
-    if (ti + 16 == qj) { a1 -= sj; b1 += cmj; }
-    r[ti][pj] = a0;
-    r[ti][qj] = b0;
-    r[ti + 16][pj] = a1;
-    r[ti + 16][qj] = b1;
     // next round: every position but 0 moves on by one
-    pi = ti == 0 ? 0 : (pi == JP - 1 ? 1 : pi + 1);
-    pj = tj == 0 ? 0 : (pj == JP - 1 ? 1 : pj + 1);
-    qi = qi == JP - 1 ? 1 : qi + 1;
-    qj = qj == JP - 1 ? 1 : qj + 1;
+    p = t == 0 ? 0 : (p == JP - 1 ? 1 : p + 1);
+    q = q == JP - 1 ? 1 : q + 1;
+    p1 = src == 0 ? 0 : (p1 == JP - 1 ? 1 : p1 + 1);
+    q1 = q1 == JP - 1 ? 1 : q1 + 1;
     __syncthreads();
   }
   const int any = __syncthreads_or(rotated);
   const int anybig = __syncthreads_or(big);
-  float* Rp = R + (size_t)pair * JP * JP;
-  for (int e = tid; e < JP * JP; e += blockDim.x) Rp[e] = r[e / JP][e % JP];
-  if (tid < JP) dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB] = dg[(JP - 1) & 1][tid];
-  if (tid == 0) {
-    ident[pair] = any ? 0 : 1;
-    if (any) atomicAdd(flag, 1);
-    if (anybig) atomicAdd(flag + 1, 1);
+  float* Rp = R + (size_t)pair * JP * JP + sub * H * JP;
+  for (int e = tid; e < H * JP; e += 256) Rp[e] = r[e / JP][e % JP];
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (sub == 0) {
+    if (tid < JP) dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB] = dg[(JP - 1) & 1][tid];
+    if (tid == 0) {
+      ident[pair] = any ? 0 : 1;
+      if (any) atomicAdd(flag, 1);
+      if (anybig) atomicAdd(flag + 1, 1);
+    }
   }
 }
 
@@ -504,9 +527,9 @@ __device__ __forceinline__ int pair_index(int b0, int b1, int l) { return l < JB
 // G <- P^T G P on blocks (X, Y), X <= Y (grid part 1, npair^2 CTAs, the
 // lower triangle exits) and V <- V P on 32-row panels (grid part 2)
 template <typename T>
-__global__ void __launch_bounds__(256) syev_apply_kernel(T* __restrict__ G, T* __restrict__ V, int np,
-                                                         const int* __restrict__ pr, const T* __restrict__ R,
-                                                         const int* __restrict__ ident, int npair) {
+__global__ void __launch_bounds__(256) syev_apply_kernel(T* G, T* V, int np,
+                                                         const int* pr, const T* R,
+                                                         const int* ident, int npair) {
   __shared__ T x[JP][JLD];
   __shared__ T rx[JP][JLD];
   __shared__ T ry[JP][JLD];
@@ -514,6 +537,7 @@ __global__ void __launch_bounds__(256) syev_apply_kernel(T* __restrict__ G, T* _
   const int tid = threadIdx.x;
   const int i = tid >> 3, j0 = (tid & 7) * 4;
   int b = blockIdx.x;
+  chain_wait();
   const int nG = npair * npair;
   if (b < nG) {
     const int X = b / npair, Y = b - (b / npair) * npair;
@@ -714,13 +738,35 @@ void tournament(int nb, std::vector<int>& out) {
     }
 }
 
-inline void solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, double, double, cudaStream_t s) {
-  syev_solve_kernel<double><<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
+// A kernel of the sweep chain: may be brought up before the one ahead of it in
+// the stream has finished (its chain_wait waits for that).  A sweep is a chain
+// of two short kernels a round: n = 200 6.46 -> 5.53 ms, 512 17.0 -> 14.2,
+// 1024 45.9 -> 40.2 (with the apply also letting its successor in at its own
+// start: 6.6, 21.4, 54.5 -- the early CTAs then hold the apply's places).
+template <typename... P, typename... A>
+int launch_chain(void (*fn)(P...), int grid, int threads, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
+  count_launch();
+  return DMRG_OK;
 }
-inline void solve_launch(SyevWs& ws, const float* G, const int* pr, float* R, double rel, double abs_,
-                         cudaStream_t s) {
-  syev_solve32_kernel<<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd, (float)rel,
-                                                (float)abs_);
+
+inline int solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, double, double, cudaStream_t s) {
+  syev_solve_kernel<double><<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
+  DMRG_CHECK_LAUNCH();
+  return DMRG_OK;
+}
+inline int solve_launch(SyevWs& ws, const float* G, const int* pr, float* R, double rel, double abs_, cudaStream_t s) {
+  return launch_chain(syev_solve32_kernel, 2 * ws.npair, 256, s, G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd,
+                      (float)rel, (float)abs_);
 }
 
 // sweeps over (G, V) until one rotates nothing (at most max_sweeps); with
@@ -736,10 +782,8 @@ int syev_sweeps(SyevWs& ws, T* G, T* V, int max_sweeps, double rel, double abs_,
     DMRG_CUDA_TRY(cudaMemsetAsync(ws.flag, 0, 2 * sizeof(int), s));
     for (int r = 0; r < rounds; ++r) {
       const int* pr = ws.pairs + (size_t)2 * r * npair;
-      solve_launch(ws, G, pr, R, rel, abs_, s);
-      DMRG_CHECK_LAUNCH();
-      syev_apply_kernel<T><<<apply_grid, 256, 0, s>>>(G, V, np, pr, R, ws.ident, npair);
-      DMRG_CHECK_LAUNCH();
+      DMRG_TRY(solve_launch(ws, G, pr, R, rel, abs_, s));
+      DMRG_TRY(launch_chain(syev_apply_kernel<T>, apply_grid, 256, s, G, V, np, pr, R, ws.ident, npair));
     }
     int h[2] = {0, 0};
     DMRG_CUDA_TRY(cudaMemcpyAsync(h, ws.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
