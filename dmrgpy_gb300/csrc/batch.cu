@@ -7,8 +7,8 @@
 //     (tgemm_grouped: each CTA finds its problem by binary search over a
 //     tile table), built from the same step plans as the single-chain path;
 //   * Lanczos: the recurrence runs for all chains in lock step; the vector
-//     kernels (dot, fused axpy, reorthogonalisation, norm + normalise) run one
-//     CTA per chain; blocks of kBlock steps are captured once as a CUDA graph
+//     work of a step (dot, axpy, reorthogonalisation, norm, next vector) is
+//     one launch, a cluster of eight CTAs per chain; blocks of kBlock steps are captured once as a CUDA graph
 //     and replayed (the graph is cached per shape signature, so the same bond
 //     of the next sweep replays it); only alpha/beta of all chains cross to
 //     the host after each block, where each chain's tridiagonal problem and

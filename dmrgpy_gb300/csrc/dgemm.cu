@@ -168,12 +168,12 @@ __device__ __forceinline__ void load8(const SplitArgs& a, long long row, long lo
 // in, 14 out per element, ~40 instructions); the second read of the rows
 // comes from L1/L2.
 template <int CPLX, int R>
-__global__ void __launch_bounds__(256) dg_split_kernel(SplitArgs a, int* __restrict__ exps, int* __restrict__ sq,
-                                                       uint4* __restrict__ dig) {
+__device__ __forceinline__ void split8(const SplitArgs& a, int* __restrict__ exps, int* __restrict__ sq,
+                                       uint4* __restrict__ dig, unsigned block) {
   __shared__ int sh[8][8];
   const int tid = threadIdx.x;
   const int rl = tid & 7, kt = tid >> 3;
-  const long long row = (long long)blockIdx.x * 8 + rl;
+  const long long row = (long long)block * 8 + rl;
   const long long cols = a.steps * 2;            // 8-wide k columns (padded)
   const bool live = row < a.R;
   int E = 0;
@@ -264,8 +264,29 @@ __global__ void __launch_bounds__(256) dg_split_kernel(SplitArgs a, int* __restr
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < 8; ++w) most = max(most, sh[w][0]);
-    sq[blockIdx.x] = most;
+    sq[block] = most;
   }
+}
+
+struct SplitJob {
+  SplitArgs a;
+  int* exps;
+  int* sq;
+  uint4* dig;
+  unsigned grid;
+};
+
+template <int CPLX, int R>
+__global__ void __launch_bounds__(256) dg_split_kernel(const SplitJob j) {
+  split8<CPLX, R>(j.a, j.exps, j.sq, j.dig, blockIdx.x);
+}
+
+// both operands of a product in one launch: a small split is mostly launch,
+// fill and tail (3.6 us each at 256 x 256)
+template <bool C>
+__global__ void __launch_bounds__(256) dg_split2_kernel(const SplitJob A, const SplitJob B) {
+  if (blockIdx.x < A.grid) split8<C ? 1 : 0, TM>(A.a, A.exps, A.sq, A.dig, blockIdx.x);
+  else split8<C ? 2 : 0, TN>(B.a, B.exps, B.sq, B.dig, blockIdx.x - A.grid);
 }
 
 // ---------------------------------------------------------------- GEMM
@@ -917,9 +938,9 @@ size_t dg_bytes(int side, bool cplx_, long long rows, long long K) {
 }
 
 template <typename T>
-int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
+static int split_job(int side, const DgOperand& o, void* buf, SplitJob* job) {
   constexpr bool C = sizeof(T) == 16;
-  SplitArgs a;
+  SplitArgs& a = job->a;
   const long long rows = (long long)o.rows.n1 * o.rows.n2, K = (long long)o.K.n1 * o.K.n2;
   if (rows < 1 || K < 1 || !o.p || !buf) return DMRG_ERR_ARG;
   a.p = static_cast<const double*>(o.p);
@@ -935,15 +956,34 @@ int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
   const int tr = tile_rows(side);
   const long long Rp = up(a.R, tr) * tr;
   if (Rp / 8 > 0x7fffffffLL) return DMRG_ERR_ARG;
-  int* exps = static_cast<int*>(buf);
-  int* sq = reinterpret_cast<int*>(static_cast<char*>(buf) + exps_bytes(side, a.R));
-  uint4* dig = reinterpret_cast<uint4*>(static_cast<char*>(buf) + head_bytes(side, a.R));
-  const unsigned grid = (unsigned)(Rp / 8);
-  if (side == 0) {
-    dg_split_kernel<C ? 1 : 0, TM><<<grid, 256, 0, s>>>(a, exps, sq, dig);
-  } else {
-    dg_split_kernel<C ? 2 : 0, TN><<<grid, 256, 0, s>>>(a, exps, sq, dig);
+  job->exps = static_cast<int*>(buf);
+  job->sq = reinterpret_cast<int*>(static_cast<char*>(buf) + exps_bytes(side, a.R));
+  job->dig = reinterpret_cast<uint4*>(static_cast<char*>(buf) + head_bytes(side, a.R));
+  job->grid = (unsigned)(Rp / 8);
+  return DMRG_OK;
+}
+
+template <typename T>
+int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
+  constexpr bool C = sizeof(T) == 16;
+  SplitJob j;
+  DMRG_TRY(split_job<T>(side, o, buf, &j));
+  if (side == 0) dg_split_kernel<C ? 1 : 0, TM><<<j.grid, 256, 0, s>>>(j);
+  else dg_split_kernel<C ? 2 : 0, TN><<<j.grid, 256, 0, s>>>(j);
+  DMRG_CHECK_LAUNCH();
+  return DMRG_OK;
+}
+
+template <typename T>
+int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, cudaStream_t s) {
+  SplitJob a, b;
+  DMRG_TRY(split_job<T>(0, A, bufa, &a));
+  DMRG_TRY(split_job<T>(1, B, bufb, &b));
+  if ((unsigned long long)a.grid + b.grid > 0x7fffffffull) {
+    DMRG_TRY(dg_split<T>(0, A, bufa, s));
+    return dg_split<T>(1, B, bufb, s);
   }
+  dg_split2_kernel<sizeof(T) == 16><<<a.grid + b.grid, 256, 0, s>>>(a, b);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
@@ -1015,8 +1055,8 @@ int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumul
   const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
   void* da = work;
   void* db = static_cast<char*>(work) + dg_bytes(0, sizeof(T) == 16, M, K);
-  DMRG_TRY(dg_split<T>(0, DgOperand{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, da, s));
-  DMRG_TRY(dg_split<T>(1, DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, s));
+  DMRG_TRY(dg_split2<T>(DgOperand{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, da,
+                        DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, s));
   return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, s);
 }
 
@@ -1036,6 +1076,8 @@ template int dg_product<double>(const TGemm&, const double*, const double*, doub
 template int dg_product<cplx>(const TGemm&, const cplx*, const cplx*, double, int, cplx*, void*, cudaStream_t);
 template int dg_split<double>(int, const DgOperand&, void*, cudaStream_t);
 template int dg_split<cplx>(int, const DgOperand&, void*, cudaStream_t);
+template int dg_split2<double>(const DgOperand&, void*, const DgOperand&, void*, cudaStream_t);
+template int dg_split2<cplx>(const DgOperand&, void*, const DgOperand&, void*, cudaStream_t);
 template int dg_gemm<double>(const void*, const void*, long long, long long, long long, const DgOut&,
                              cudaStream_t);
 template int dg_gemm<cplx>(const void*, const void*, long long, long long, long long, const DgOut&,

@@ -18,6 +18,9 @@ struct DgOperand {
 // blocks.  side 0: the M side (tiles of 128 rows), side 1: the N side (64).
 size_t dg_bytes(int side, bool cplx_, long long rows, long long K);
 template <typename T> int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s);
+// both operands in one launch: A on side 0, B on side 1
+template <typename T>
+int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, cudaStream_t s);
 
 // C = alpha A B (+ C): alpha +1 or -1; C at (row, column) strides in elements.
 struct DgOut {

@@ -107,8 +107,10 @@ int heff64_prepare(const dmrg_heff_t& o, void* work, cudaStream_t s) {
   if (o.kind != 0)
     DMRG_TRY(mpo_list_build<T>(h.mpo, static_cast<const T*>(o.W1), static_cast<const T*>(o.W2), h.list, s));
   const TGemm gl = gemm_l<T>(o, h), gr = gemm_r<T>(h);
-  if (h.dig1) DMRG_TRY(dg_split<T>(0, DgOperand{o.L, gl.M, gl.K, gl.a_m, gl.a_k, 0}, h.ldig, s));
-  if (h.dig2) DMRG_TRY(dg_split<T>(1, DgOperand{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0}, h.rdig, s));
+  const DgOperand l{o.L, gl.M, gl.K, gl.a_m, gl.a_k, 0}, r{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0};
+  if (h.dig1 && h.dig2) return dg_split2<T>(l, h.ldig, r, h.rdig, s);
+  if (h.dig1) return dg_split<T>(0, l, h.ldig, s);
+  if (h.dig2) return dg_split<T>(1, r, h.rdig, s);
   return DMRG_OK;
 }
 

@@ -3,12 +3,12 @@
 // The columns of a working copy X (r x c, column-major, c = min(m, n)) are
 // orthogonalised pairwise with the round-robin (tournament) ordering, so the
 // c/2 pairs of a round touch disjoint columns and run concurrently, one warp
-// per pair: the warp reduces the 2x2 Gram block (|x_p|^2, |x_q|^2,
-// x_p^H x_q) with shuffles, builds the Hermitian Jacobi rotation and applies
-// it to the two columns of X and of the accumulated V.  Rounds are separated
-// by a barrier: __syncthreads() for the single-CTA variant (small matrices,
-// the common case at the chain edges and at small chi) or a bounded grid
-// barrier for the cooperative multi-CTA variant.  A sweep with no rotation
+// per pair: the warp reduces x_p^H x_q with shuffles (the columns' norms are
+// kept up by the rotations and summed anew each sweep), builds the Hermitian
+// Jacobi rotation and applies it to the two columns of X and of the
+// accumulated V.  Rounds are separated by a barrier: __syncthreads() for one
+// CTA (the chain edges), the hardware's for a cluster of eight, a bounded grid
+// barrier for the cooperative grid of wide matrices.  A sweep with no rotation
 // above tol*sqrt(|x_p|^2 |x_q|^2) ends the iteration.  The singular values
 // are the column norms of X; the singular vectors are X/sigma and V.  Unlike
 // the Gram-matrix route this keeps small singular values to high relative

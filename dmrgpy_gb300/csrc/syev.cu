@@ -7,11 +7,11 @@
 // which no rotation ever touches) and cut into nb = np/16 blocks of 16
 // indices.  One sweep visits every pair of blocks once, in nb-1 rounds of
 // nb/2 disjoint pairs (round-robin tournament).  A round is two launches:
-//   solve  one CTA per pair: one cyclic scalar Jacobi sweep over the 32 x 32
-//          subproblem [G_II G_IJ; G_JI G_JJ] in shared memory (16 disjoint
-//          rotations at a time, one 2 x 2 block of the matrix per thread,
-//          Golub & Van Loan's symmetric Schur rotation), writing the
-//          accumulated rotation out;
+//   solve  one CTA per pair (FP32: two, which share the rotation's rows): one
+//          cyclic scalar Jacobi sweep over the 32 x 32 subproblem
+//          [G_II G_IJ; G_JI G_JJ] in shared memory (16 disjoint rotations at a
+//          time, one 2 x 2 block of the matrix per thread, Golub & Van Loan's
+//          symmetric Schur rotation), writing the accumulated rotation out;
 //   apply  G <- P^T G P and V <- V P with P = the pairs' rotations: one CTA
 //          per 32 x 32 block (X, Y) of pair rows/columns (upper triangle,
 //          mirrored) and one per 32-row panel of V and pair X.

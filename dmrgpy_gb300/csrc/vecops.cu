@@ -2,8 +2,9 @@
 // deterministic single-launch two-level reduction (warp shuffles, then the
 // last CTA folds the per-CTA partials in a fixed order), fused axpy /
 // scaling with scalars that stay in device memory, and the block
-// reorthogonalisation h = Q^H w, w -= Q h.  All HBM-bound; grids are sized in
-// multiples of the 152 SMs.
+// reorthogonalisation h = Q^H w, w -= Q h: HBM-bound, grids sized in multiples
+// of the 152 SMs, for long vectors.  For shorter ones a whole step after its
+// matvec is one launch (krylov_step).
 #include "krylov.cuh"
 
 namespace dmrg {

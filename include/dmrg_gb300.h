@@ -290,10 +290,11 @@ int dmrg_subspace_truncate_ex(int precision, int m, int n, int k, const void* th
 
 /* ---- symmetric eigendecomposition ----------------------------------------
  * A (n x n, row-major, ld lda, symmetric) = V diag(w) V^T in FP64 by the
- * parallel cyclic block-Jacobi method: 16-wide blocks, one CTA per block
- * pair running a Jacobi sweep over the 32 x 32 subproblem in shared memory,
- * the rotations applied to A and V as corrections by a second kernel per
- * round; at most 40 sweeps.  w (host, n) receives the eigenvalues in
+ * parallel cyclic block-Jacobi method: 16-wide blocks, a Jacobi sweep over
+ * the 32 x 32 subproblem of each block pair in shared memory, the rotations
+ * applied to A and V as corrections by a second kernel per round; sweeps in
+ * FP32 between FP64 products, FP64 sweeps (at most 40) for what those
+ * leave.  w (host, n) receives the eigenvalues in
  * descending order; V (device, n x n, ld ldv; may be NULL) the matching
  * eigenvectors as columns.  Stands in for np.linalg.eigh in
  * pyitensor/svd.py:131-133 and eigh_truncate (pyitensor/svd.py:71-88).
