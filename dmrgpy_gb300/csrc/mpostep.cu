@@ -110,9 +110,14 @@ __device__ __forceinline__ cplx madd(cplx w, cplx x, cplx acc) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) mpo_apply_kernel(int rows, int cols, const int* __restrict__ cnt,
-                                                        const Entry<T>* __restrict__ ent, const T* __restrict__ in,
-                                                        T* __restrict__ out, long long outer, long long inner) {
+__global__ void __launch_bounds__(256) mpo_apply_kernel(int rows, int cols, const int* cnt_, const Entry<T>* ent_,
+                                                        const T* in_, T* out_, long long outer, long long inner) {
+  let_next_in();
+  wait_for_last();
+  const int* __restrict__ cnt = after_wait(cnt_);
+  const Entry<T>* __restrict__ ent = after_wait(ent_);
+  const T* __restrict__ in = after_wait(in_);
+  T* __restrict__ out = after_wait(out_);
   const long long i = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
   const int w = threadIdx.x >> 5;
   for (long long o = blockIdx.y; o < outer; o += gridDim.y) {
@@ -157,9 +162,7 @@ int mpo_apply(const MpoShape& sh, const void* list, const T* in, T* out, long lo
   const Entry<T>* ent = reinterpret_cast<const Entry<T>*>(static_cast<const char*>(list) + cnt_bytes(sh));
   if ((inner + 31) / 32 > 0x7fffffffLL) return DMRG_ERR_ARG;
   const dim3 grid((unsigned)((inner + 31) / 32), (unsigned)(outer < 65535 ? outer : 65535));
-  mpo_apply_kernel<T><<<grid, 256, 0, s>>>(d.rows, d.cols, cnt, ent, in, out, outer, inner);
-  DMRG_CHECK_LAUNCH();
-  return DMRG_OK;
+  return launch_after(mpo_apply_kernel<T>, grid, 256, s, d.rows, d.cols, cnt, ent, in, out, outer, inner);
 }
 
 template int mpo_list_build<double>(const MpoShape&, const double*, const double*, void*, cudaStream_t);

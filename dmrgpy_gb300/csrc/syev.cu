@@ -309,12 +309,6 @@ __device__ __forceinline__ float2 add_hl(float2 a, float x) {
   return make_float2(r, l - (r - h));
 }
 
-// Kernels of the sweep chain come up while the one before them drains
-// (launch_chain): nothing of it is touched before this.  Their pointers are
-// not __restrict__, which would let the compiler move loads up past it.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // The FP32 subproblem of a block pair: one sweep over its 32 indices.  Bound by
 // the latency of a round (loads, the rotation's chain of four approximations,
 // a shuffle, the update, a barrier) and its issue slots: lane t of a half warp
@@ -332,8 +326,8 @@ syev_solve32_kernel(const float* G, int np, const int* pr, float* R,
   __shared__ float2 dg[2][JP];
   __shared__ float r[H][JP];
   const int pair = blockIdx.x >> 1, sub = blockIdx.x & 1;
-  chain_wait();
-  chain_next();   // the apply's CTAs fit beside the few of this kernel
+  wait_for_last();
+  let_next_in();   // the apply's CTAs fit beside the few of this kernel
   const int bi = pr[2 * pair], bj = pr[2 * pair + 1];
   const int tid = threadIdx.x;
   const float floor_ = abs_ * (float)__longlong_as_double((long long)*scale);
@@ -537,7 +531,7 @@ __global__ void __launch_bounds__(256) syev_apply_kernel(T* G, T* V, int np,
   const int tid = threadIdx.x;
   const int i = tid >> 3, j0 = (tid & 7) * 4;
   int b = blockIdx.x;
-  chain_wait();
+  wait_for_last();
   const int nG = npair * npair;
   if (b < nG) {
     const int X = b / npair, Y = b - (b / npair) * npair;
@@ -738,34 +732,18 @@ void tournament(int nb, std::vector<int>& out) {
     }
 }
 
-// A kernel of the sweep chain: may be brought up before the one ahead of it in
-// the stream has finished (its chain_wait waits for that).  A sweep is a chain
-// of two short kernels a round: n = 200 6.46 -> 5.53 ms, 512 17.0 -> 14.2,
-// 1024 45.9 -> 40.2 (with the apply also letting its successor in at its own
-// start: 6.6, 21.4, 54.5 -- the early CTAs then hold the apply's places).
-template <typename... P, typename... A>
-int launch_chain(void (*fn)(P...), int grid, int threads, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
-  count_launch();
-  return DMRG_OK;
-}
-
+// The sweep is a chain of two short kernels a round, launched overlapped:
+// n = 200 6.46 -> 5.53 ms, 512 17.0 -> 14.2, 1024 45.9 -> 40.2.  The apply does
+// not let its successor in early (6.6, 21.4, 54.5: the early CTAs then hold the
+// apply's places).  Pointers of both kernels are not __restrict__, which would
+// let the compiler move loads up past the wait.
 inline int solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, double, double, cudaStream_t s) {
   syev_solve_kernel<double><<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
 inline int solve_launch(SyevWs& ws, const float* G, const int* pr, float* R, double rel, double abs_, cudaStream_t s) {
-  return launch_chain(syev_solve32_kernel, 2 * ws.npair, 256, s, G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd,
+  return launch_after(syev_solve32_kernel, dim3(2u * (unsigned)ws.npair), 256, s, G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd,
                       (float)rel, (float)abs_);
 }
 
@@ -783,7 +761,7 @@ int syev_sweeps(SyevWs& ws, T* G, T* V, int max_sweeps, double rel, double abs_,
     for (int r = 0; r < rounds; ++r) {
       const int* pr = ws.pairs + (size_t)2 * r * npair;
       DMRG_TRY(solve_launch(ws, G, pr, R, rel, abs_, s));
-      DMRG_TRY(launch_chain(syev_apply_kernel<T>, apply_grid, 256, s, G, V, np, pr, R, ws.ident, npair));
+      DMRG_TRY(launch_after(syev_apply_kernel<T>, dim3((unsigned)apply_grid), 256, s, G, V, np, pr, R, ws.ident, npair));
     }
     int h[2] = {0, 0};
     DMRG_CUDA_TRY(cudaMemcpyAsync(h, ws.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));

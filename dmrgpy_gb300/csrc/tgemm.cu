@@ -214,7 +214,10 @@ __global__ void __launch_bounds__(Tile<BT>::NT) tgemm_sym_kernel(Dev d, T alpha,
 template <typename T, int BT>
 __global__ void __launch_bounds__(Tile<BT>::NT) tgemm_kernel(Dev d, T alpha, const T* __restrict__ A,
                                                              const T* __restrict__ B, T beta, T* __restrict__ C) {
-  any_tile<T, BT>(d, alpha, A, B, beta, C, blockIdx.x * BT, blockIdx.y * BT, blockIdx.z);
+  let_next_in();
+  wait_for_last();
+  any_tile<T, BT>(d, alpha, after_wait(A), after_wait(B), beta, after_wait(C), blockIdx.x * BT, blockIdx.y * BT,
+                  blockIdx.z);
 }
 
 // Grouped launch: problem p owns the flat tile range [start, start + tiles)
@@ -230,8 +233,11 @@ struct GProb {
 };
 
 template <typename T, int BT>
-__global__ void __launch_bounds__(Tile<BT>::NT) tgemm_grouped_kernel(const GProb* __restrict__ probs, int nprob,
-                                                                     T alpha, T beta) {
+__global__ void __launch_bounds__(Tile<BT>::NT) tgemm_grouped_kernel(const GProb* tab, int nprob, T alpha,
+                                                                     T beta) {
+  let_next_in();
+  wait_for_last();
+  const GProb* probs = after_wait(tab);
   const long long t = blockIdx.x;
   int lo = 0, hi = nprob - 1;
   while (lo < hi) {
@@ -331,12 +337,10 @@ int tgemm(const TGemm& g, T alpha, const T* A, const T* B, T beta, T* C, cudaStr
   while (bt < 64 && tiles_of(d.N, bt) > 65535) bt *= 2;   // grid.y limit
   dim3 grid((unsigned)tiles_of(d.M, bt), (unsigned)tiles_of(d.N, bt), (unsigned)nb);
   if (tiles_of(d.N, 64) > 65535) return DMRG_ERR_ARG;
-  if (bt == 64) tgemm_kernel<T, 64><<<grid, Tile<64>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
-  else if (bt == 32) tgemm_kernel<T, 32><<<grid, Tile<32>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
-  else if (bt == 16) tgemm_kernel<T, 16><<<grid, Tile<16>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
-  else tgemm_kernel<T, 8><<<grid, Tile<8>::NT, 0, stream>>>(d, alpha, A, B, beta, C);
-  DMRG_CHECK_LAUNCH();
-  return DMRG_OK;
+  if (bt == 64) return launch_after(tgemm_kernel<T, 64>, grid, Tile<64>::NT, stream, d, alpha, A, B, beta, C);
+  if (bt == 32) return launch_after(tgemm_kernel<T, 32>, grid, Tile<32>::NT, stream, d, alpha, A, B, beta, C);
+  if (bt == 16) return launch_after(tgemm_kernel<T, 16>, grid, Tile<16>::NT, stream, d, alpha, A, B, beta, C);
+  return launch_after(tgemm_kernel<T, 8>, grid, Tile<8>::NT, stream, d, alpha, A, B, beta, C);
 }
 
 int tgemm_gram(const double* X, long long ld, int m, int k, double* G, cudaStream_t stream) {
@@ -407,12 +411,11 @@ int tgemm_grouped_launch(const void* desc_dev, int n, long long tiles, int tile,
                          cudaStream_t stream) {
   if (n == 0 || tiles == 0) return DMRG_OK;
   const GProb* p = static_cast<const GProb*>(desc_dev);
-  if (tile == 64) tgemm_grouped_kernel<T, 64><<<(unsigned)tiles, Tile<64>::NT, 0, stream>>>(p, n, alpha, beta);
-  else if (tile == 32) tgemm_grouped_kernel<T, 32><<<(unsigned)tiles, Tile<32>::NT, 0, stream>>>(p, n, alpha, beta);
-  else if (tile == 16) tgemm_grouped_kernel<T, 16><<<(unsigned)tiles, Tile<16>::NT, 0, stream>>>(p, n, alpha, beta);
-  else tgemm_grouped_kernel<T, 8><<<(unsigned)tiles, Tile<8>::NT, 0, stream>>>(p, n, alpha, beta);
-  DMRG_CHECK_LAUNCH();
-  return DMRG_OK;
+  const dim3 grid((unsigned)tiles);
+  if (tile == 64) return launch_after(tgemm_grouped_kernel<T, 64>, grid, Tile<64>::NT, stream, p, n, alpha, beta);
+  if (tile == 32) return launch_after(tgemm_grouped_kernel<T, 32>, grid, Tile<32>::NT, stream, p, n, alpha, beta);
+  if (tile == 16) return launch_after(tgemm_grouped_kernel<T, 16>, grid, Tile<16>::NT, stream, p, n, alpha, beta);
+  return launch_after(tgemm_grouped_kernel<T, 8>, grid, Tile<8>::NT, stream, p, n, alpha, beta);
 }
 
 template <typename T>
