@@ -101,7 +101,7 @@ size_t syev_layout(int n, SyevWs* w, void* base, bool lean) {
   s.ident = static_cast<int*>(take(sizeof(int) * npair));
   s.pairs = static_cast<int*>(take(sizeof(int) * 2 * (size_t)(nb - 1 > 0 ? nb - 1 : 1) * npair));
   s.flag = static_cast<int*>(take(sizeof(int) * 4));
-  s.scale = static_cast<unsigned long long*>(take(3 * sizeof(unsigned long long)));
+  s.scale = static_cast<unsigned long long*>(take(16 * sizeof(unsigned long long)));
   s.diag = static_cast<double*>(take(sizeof(double) * np));
   s.dd = static_cast<float2*>(take(sizeof(float2) * np));
   s.perm = static_cast<int*>(take(sizeof(int) * np));
@@ -829,13 +829,20 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
   float* G32 = reinterpret_cast<float*>(ws.T);
   float* Q32 = G32 + nn;
   *converged = 0;
-  unsigned long long* off = ws.scale + 1;
   unsigned long long* norm = ws.scale + 2;
+  // per pass (the fourth and later share a slot): largest off-diagonal, and
+  // up to np = 64 the sweeps run
+  unsigned long long* offs = ws.scale + 4;
+  int* counts = reinterpret_cast<int*>(ws.scale + 8);
+  DMRG_CUDA_TRY(cudaMemsetAsync(offs, 0, 4 * sizeof(unsigned long long), s));
   DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, sizeof(unsigned long long), s));
   syev_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, norm);
   DMRG_CHECK_LAUNCH();
   bool polish = false;   // V diagonalises A but is orthonormal to 1e-12 only
   for (int p = 0; p < MAX_PASSES; ++p) {
+    const int slot = p < 3 ? p : 3;
+    unsigned long long* off = offs + slot;
+    if (p > 3) DMRG_CUDA_TRY(cudaMemsetAsync(off, 0, sizeof(unsigned long long), s));
     // the pass's rotation Q (FP64) into ws.G; into ws.T where the kernel's
     // CTAs read ws.G as they please
     double* Q = np <= 64 && p > 0 ? ws.T : ws.G;
@@ -848,9 +855,11 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
       // nothing left to rotate
     } else if (np <= 64) {
       if (np == 32)
-        syev_small32_kernel<32><<<2, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q, ws.flag);
+        syev_small32_kernel<32><<<2, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
+                                                  counts + slot);
       else
-        syev_small32_kernel<64><<<8, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q, ws.flag);
+        syev_small32_kernel<64><<<8, 256, 0, s>>>(src0, ld0, n0, norm, most, (float)rel, (float)abs_, Q,
+                                                  counts + slot);
       DMRG_CHECK_LAUNCH();
     } else {
       DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 2 * sizeof(unsigned long long), s));
@@ -893,15 +902,25 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     DMRG_CHECK_LAUNCH();
     syev_off_kernel<<<grid_for(nn), 256, 0, s>>>(ws.G, np, ws.scale, off);
     DMRG_CHECK_LAUNCH();
-    unsigned long long h = 0;
-    int small_sweeps = 0;
-    DMRG_CUDA_TRY(cudaMemcpyAsync(&h, off, sizeof(h), cudaMemcpyDeviceToHost, s));
-    if (np <= 64) DMRG_CUDA_TRY(cudaMemcpyAsync(&small_sweeps, ws.flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    // up to np = 64 the first three passes run without the host in between
+    if (np <= 64 && p < 2) continue;
+    struct { unsigned long long off[4]; int count[4]; } h;
+    DMRG_CUDA_TRY(cudaMemcpyAsync(&h, offs, sizeof(h), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
-    if (!polish) *done_ += small_sweeps;
-    const uint32_t bits = (uint32_t)h;
-    float mx;
-    std::memcpy(&mx, &bits, sizeof(mx));
+    auto value = [](unsigned long long v) {
+      const uint32_t bits = (uint32_t)v;
+      float x;
+      std::memcpy(&x, &bits, sizeof(x));
+      return x;
+    };
+    const float mx = value(h.off[slot]);
+    if (np <= 64 && !polish) {
+      // sweeps up to the pass that left nothing (a diagonal matrix: the first)
+      for (int q = p == 2 ? 0 : slot; q <= slot; ++q) {
+        *done_ += h.count[q];
+        if (value(h.off[q]) <= PASS_DONE) break;
+      }
+    }
     if (mx <= PASS_DONE && (p >= 2 || polish)) {
       // eigenvalues; then what is left of the off-diagonals (up to PASS_DONE
       // of the threshold, where a converged sweep leaves their square) out of V
