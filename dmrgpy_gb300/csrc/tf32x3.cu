@@ -1117,13 +1117,25 @@ int launch_mpo_step_t(const Heff2Plan& p, cudaStream_t s) {
   return DMRG_OK;
 }
 
-// Zeroes columns K .. Kp - 1 of rows x Kp (the MPO step writes the others):
-// nothing where K is a multiple of 32.  Clearing the whole operand took 59 of
-// 1130 us of a chi = 1024 matvec.
-int zero_pad(float* X, long long rows, long long K, long long Kp, cudaStream_t s) {
-  if (Kp > K)
-    DMRG_CUDA_TRY(cudaMemset2DAsync(X + K, sizeof(float) * (size_t)Kp, 0, sizeof(float) * (size_t)(Kp - K),
-                                    (size_t)rows, s));
+// Zeroes columns K .. Kp - 1 of the rows x Kp pair (the MPO step writes the
+// others): nothing where K is a multiple of 32.  Clearing the whole pair took 59
+// of 1130 us of a chi = 1024 matvec.
+__global__ void zero_pad_kernel(float* __restrict__ hi, float* __restrict__ lo, long long total, int K, int Kp) {
+  const int w = Kp - K;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (long long)gridDim.x * blockDim.x) {
+    const long long r = e / w, o = r * Kp + K + (e - r * w);
+    hi[o] = 0.f;
+    lo[o] = 0.f;
+  }
+}
+
+int zero_pad(float* hi, float* lo, long long rows, int K, int Kp, cudaStream_t s) {
+  const long long total = rows * (Kp - K);
+  if (total <= 0) return DMRG_OK;
+  const long long g = (total + 255) / 256;
+  zero_pad_kernel<<<(unsigned)(g < 152 * 8 ? g : 152 * 8), 256, 0, s>>>(hi, lo, total, K, Kp);
+  DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
 
@@ -1189,8 +1201,7 @@ int tf32x3_heff_prepare(const dmrg_heff_t& o, void* work, cudaStream_t s) {
   DMRG_TRY(split_rows(static_cast<const double*>(o.R), (long long)p.wr * p.cr, 1, p.cr, p.wr * p.cr, p.Kp4, p.R_hi,
                       p.R_lo, s));
   // padding columns of X3 stay zero for every later matvec
-  DMRG_TRY(zero_pad(p.X3_hi, p.M4, (long long)o.wr * o.chir, p.Kp4, s));
-  DMRG_TRY(zero_pad(p.X3_lo, p.M4, (long long)o.wr * o.chir, p.Kp4, s));
+  DMRG_TRY(zero_pad(p.X3_hi, p.X3_lo, p.M4, o.wr * o.chir, p.Kp4, s));
   return DMRG_OK;
 }
 
@@ -1474,8 +1485,7 @@ int tf32x3_env(int side, int cl, int d, int cr, int wl, int wr, const double* E,
     GemmOut g1{p.Y1, (long long)cl * wl, 1, d * cr, cl * wl, 0, 0, 1.f};
     DMRG_TRY(gemm_split(p.A1hi, p.A1lo, p.E1hi, p.E1lo, d * cr, cl * wl, p.Kp1, g1, p.err, s));
     // MPO step -> Y2 rows (m,b), K = (a',s')
-    DMRG_TRY(zero_pad(p.Y2hi, (long long)wr * cr, (long long)cl * d, p.Kp2, s));
-    DMRG_TRY(zero_pad(p.Y2lo, (long long)wr * cr, (long long)cl * d, p.Kp2, s));
+    DMRG_TRY(zero_pad(p.Y2hi, p.Y2lo, (long long)wr * cr, cl * d, p.Kp2, s));
     const size_t smem = sizeof(float) * ((size_t)d * wr * d * wl + (size_t)EB * d * wl * 32);
     if (smem > 200 * 1024) return DMRG_ERR_UNSUPPORTED;
     dim3 grid((cl + 31) / 32, (cr + EB - 1) / EB);
@@ -1492,8 +1502,7 @@ int tf32x3_env(int side, int cl, int d, int cr, int wl, int wr, const double* E,
     DMRG_TRY(split_rows(E, cr, 1, cr * wr, cr, p.Kp1, p.E1hi, p.E1lo, s));
     GemmOut g1{p.Y1, (long long)cr * wr, 1, cl * d, cr * wr, 0, 0, 1.f};
     DMRG_TRY(gemm_split(p.A1hi, p.A1lo, p.E1hi, p.E1lo, cl * d, cr * wr, p.Kp1, g1, p.err, s));
-    DMRG_TRY(zero_pad(p.Y2hi, (long long)wl * cl, (long long)cr * d, p.Kp2, s));
-    DMRG_TRY(zero_pad(p.Y2lo, (long long)wl * cl, (long long)cr * d, p.Kp2, s));
+    DMRG_TRY(zero_pad(p.Y2hi, p.Y2lo, (long long)wl * cl, cr * d, p.Kp2, s));
     const size_t smem = sizeof(float) * ((size_t)wl * d * d * wr + (size_t)EB * d * wr * 32);
     if (smem > 200 * 1024) return DMRG_ERR_UNSUPPORTED;
     dim3 grid((cr + 31) / 32, (cl + EB - 1) / EB);
