@@ -208,7 +208,7 @@ template <typename T> int vscale(T* x, T a, long long n, cudaStream_t s);
 constexpr int MULTIDOT_MAX_GRID = 2 * 152;
 // A Krylov step after its matvec w = H q_j: alpha, the three-term update, the
 // reorthogonalisation against q_0 .. q_(nq-1), beta and (next) q_(j+1), in one
-// cooperative launch.  sc: [0..1] alpha, [2] beta (in: the previous one),
+// launch (a cluster for short vectors, else a cooperative grid).  sc: [0..1] alpha, [2] beta (in: the previous one),
 // [3] status; red, zeroed at the loop's start: 8 + 2 MULTIDOT_MAX_GRID
 // doubles; part: as multidot_ws; epoch: 3 per earlier call with nq > 0, 2
 // with nq = 0.

@@ -196,7 +196,7 @@ __global__ void gemv_kernel(const T* __restrict__ Q, long long ldq, int k, const
 // ---- one Krylov step after its matvec, in one cooperative launch: bound by
 // latency (three barriers of 1 to 2 us and the FP64 pipe's 2 n nq / 152 / 2
 // clocks); the eight short kernels and the copy it replaces took 25 us at
-// n = 3600, nq = 8, and as long again to launch.
+// n = 3600, nq = 8, and as long again to launch; this one takes 11.
 constexpr int KT = 512;                   // threads
 constexpr int KW = KT / 32;
 constexpr int KRYLOV_STEP_SMEM = 64 * 1024;
