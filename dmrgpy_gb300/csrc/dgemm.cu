@@ -37,7 +37,10 @@
 //
 // GEMM kernel, persistent, one CTA per SM, output tiles of 128 x 64:
 //   warp 0    producer: cp.async.bulk of the A (32 KB) and B (16 KB) blocks
-//             of a K step into a ring of four stages;
+//             of a K step into a ring of four stages (every CTA its own
+//             blocks: with the A block shared by the two CTAs of a cluster,
+//             32 KB a step from L2 instead of 48, a chi = 1024 matvec took
+//             the same 4.66 ms, the tensor pipe being the bound);
 //   warp 1    TMEM allocation (512 columns: 8 orders x 64) and the single
 //             thread that issues 12 MMAs per K step;
 //   warps 2-9 epilogue: after every run the eight accumulators are read,
@@ -422,29 +425,6 @@ __device__ __forceinline__ void tmem_wait16(uint32_t* r) {
                : "memory");
 }
 
-// as bulk_load, into the same offset (data and mbarrier) of both CTAs of a pair
-__device__ __forceinline__ void bulk_load_pair(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-
-// arrive on the mbarrier of both CTAs of a pair when the MMAs issued so far are done
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-}
-
 // the MMAs of one K step: a_i times b_0 .. b_{7-i} into orders i .. 7
 __device__ __forceinline__ void mma_stage(uint32_t base, uint32_t tmem, bool first) {
   const uint64_t da = sdesc_nosw(base, ND * TM * 16);
@@ -563,10 +543,7 @@ __device__ __forceinline__ void store4(const GArgs& a, const RowOut& o, int gn, 
   }
 }
 
-// CL = 2: a pair of CTAs takes two N tiles of one M tile; each loads its own B
-// block and half of the A block, multicast to both.
-template <int CL>
-__global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_gemm_kernel(const GArgs a) {
+__global__ void __launch_bounds__(DG_THREADS, 1) dg_gemm_kernel(const GArgs a) {
   int* err = &g_dg_timeout;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
@@ -579,16 +556,14 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int rank = CL == 1 ? 0 : (int)(blockIdx.x % CL);
-  const int cols = (a.tiles_n + CL - 1) / CL;   // N tile groups
-  const int ntiles = a.tiles_m * cols;
-  const int t0 = (int)(blockIdx.x / CL), tstep = (int)(gridDim.x / CL);
+  const int ntiles = a.tiles_m * a.tiles_n;
+  const int t0 = (int)blockIdx.x, tstep = (int)gridDim.x;
   const int nk = a.ks1 - a.ks0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CL);   // one arrival per CTA that reads the stage's slot
+      mbar_init(&empty[s], 1);
     }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, 8);   // one arrival per epilogue warp
@@ -602,18 +577,17 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (CL > 1) cluster_sync();   // the peer's barriers are initialised
   const uint32_t tmem = *tmem_slot;
   operands_ready();
 
   auto origin = [&](int t, int& mt, int& nt) {
-    const int per_group = a.group * cols;
+    const int per_group = a.group * a.tiles_n;
     const int gid = t / per_group;
     const int first = gid * a.group;
     const int gsz = min(a.tiles_m - first, a.group);
     const int local = t - gid * per_group;
     mt = first + local % gsz;
-    nt = (local / gsz) * CL + rank;
+    nt = local / gsz;
   };
 
   if (warp == 0) {
@@ -624,8 +598,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
         int mt, nt;
         origin(t, mt, nt);
         const unsigned char* pa = a.A + ((long long)mt * a.steps + a.ks0) * A_BLK;
-        // a pair's second tile may lie beyond the last: it then loads that one
-        const unsigned char* pb = a.B + ((long long)min(nt, a.tiles_n - 1) * a.steps + a.ks0) * B_BLK;
+        const unsigned char* pb = a.B + ((long long)nt * a.steps + a.ks0) * B_BLK;
         for (int k = 0; k < nk; ++k, ++g) {
           const int s = (int)(g % STAGES);
           const long long it = g / STAGES;
@@ -635,12 +608,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
           }
           unsigned char* st = smem + s * ST_BYTES;
           mbar_expect_tx(&full[s], ST_BYTES);
-          if (CL == 1) {
-            bulk_load(st, pa + (long long)k * A_BLK, A_BLK, &full[s]);
-          } else {
-            const uint32_t o = rank * (A_BLK / 2);
-            bulk_load_pair(st + o, pa + (long long)k * A_BLK + o, A_BLK / 2, &full[s]);
-          }
+          bulk_load(st, pa + (long long)k * A_BLK, A_BLK, &full[s]);
           bulk_load(st + A_BLK, pb + (long long)k * B_BLK, B_BLK, &full[s]);
         }
       }
@@ -652,7 +620,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
       for (int t = t0; t < ntiles && ok; t += tstep) {
         int mt, nt;
         origin(t, mt, nt);
-        const int R = nk <= RUN ? RUN : run_steps(a, mt, min(nt, a.tiles_n - 1), 0);
+        const int R = nk <= RUN ? RUN : run_steps(a, mt, nt, 0);
         for (int k = 0; k < nk && ok; ++k, ++g) {
           const int s = (int)(g % STAGES);
           const bool first = k % R == 0;
@@ -660,8 +628,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
           if (!mbar_wait(&full[s], (uint32_t)((g / STAGES) & 1), err)) { ok = false; break; }
           tc_fence_after();
           mma_stage(smem_u32(smem + s * ST_BYTES), tmem, first);
-          if (CL == 1) mma_commit(&empty[s]);
-          else mma_commit_pair(&empty[s]);
+          mma_commit(&empty[s]);
           if (k % R == R - 1 || k == nk - 1) {
             mma_commit(acc_full);
             ++runs;
@@ -686,7 +653,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
         h0[c] = 0;
         m[c] = 0;
       }
-      const int R = nk <= RUN ? RUN : run_steps(a, mt, min(nt, a.tiles_n - 1), 0);
+      const int R = nk <= RUN ? RUN : run_steps(a, mt, nt, 0);
       for (int k = 0; k < nk && ok; k += R, ++run) {
         ok = mbar_wait(acc_full, (uint32_t)(run & 1), err);
         tc_fence_after();
@@ -720,7 +687,6 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(CL, 1, 1) dg_g
   }
   tc_fence_before();
   __syncthreads();
-  if (CL > 1) cluster_sync();   // nothing more lands in the peer's shared memory
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -1024,16 +990,13 @@ int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long l
   a.cplx_ = C ? 1 : 0;
   a.negate = out.alpha < 0.0;
   const int sk = split_of(tm * tn, a.steps);
-  const bool pair = sk == 1 && tn >= 2;
-  static std::atomic<unsigned long long> attr[5];
+  static std::atomic<unsigned long long> attr[4];
   const void* fn = sk == 8   ? reinterpret_cast<const void*>(dg_splitk_kernel<8>)
                    : sk == 4 ? reinterpret_cast<const void*>(dg_splitk_kernel<4>)
                    : sk == 2 ? reinterpret_cast<const void*>(dg_splitk_kernel<2>)
-                   : pair    ? reinterpret_cast<const void*>(dg_gemm_kernel<2>)
-                             : reinterpret_cast<const void*>(dg_gemm_kernel<1>);
-  DMRG_TRY(smem_attr_once(fn, DG_SMEM, attr[sk == 8 ? 4 : sk == 4 ? 3 : sk == 2 ? 2 : pair ? 1 : 0]));
+                             : reinterpret_cast<const void*>(dg_gemm_kernel);
+  DMRG_TRY(smem_attr_once(fn, DG_SMEM, attr[sk == 8 ? 3 : sk == 4 ? 2 : sk == 2 ? 1 : 0]));
   const unsigned grid = sk > 1 ? (unsigned)(tm * tn) * (unsigned)sk
-                        : pair ? 2u * (unsigned)std::min<long long>(tm * up(tn, 2), 76)
                                : (unsigned)std::min<long long>(tm * tn, 152);
   // K in launches of at most MAX_STEPS steps (64-bit sums), the later ones adding
   for (long long k0 = 0; k0 < a.steps; k0 += MAX_STEPS) {
