@@ -155,7 +155,7 @@ __device__ __forceinline__ bool pair_rotation(double al, double be, double gre, 
                                               double& cs, T& se, double& dn) {
   // the pair scaled by a power of two so that the larger norm is in [1, 2)
   const int ex = max(exponent(al), exponent(be));
-  if (ex == 0 || ex >= 2046) return false;   // nothing there, or not finite (the norms report that)
+  if (ex == 0 || ex == 2047) return false;   // nothing there, or not finite (the norms report that)
   double ag, px = 0.0, py = 0.0;
   if (sizeof(T) == 8) {
     ag = fabs(gre);
@@ -181,7 +181,9 @@ __device__ __forceinline__ bool pair_rotation(double al, double be, double gre, 
     tf = copysignf(__fdividef(2.f * gf, fabsf(df) + sqrtf(fmaf(df, df, 4.f * gf * gf))), df);
     t = widen(tf);
   } else {
-    if (!(ag * ag > tol * tol * (al * be)) || !(ag > 1e-290)) return false;
+    // norms apart by 1e30 or more: no product of two of them, which leaves
+    // FP64's range where |M| is above 1e84 or below 1e-73
+    if (!(ag > tol * (sqrt(al) * sqrt(be))) || !(ag > 1e-300)) return false;
     t = ag / (d == 0.0 ? ag : d);
     if (fabs(t) > 1.0) t = copysign(1.0, t);
     tf = narrow(t);
