@@ -116,19 +116,23 @@ __device__ __forceinline__ float2 hi_lo(double v) {
   return make_float2(h, (float)(v - (double)h));
 }
 
+// 2^-e for a matrix whose largest |a_ij| has exponent e (its bits in *norm),
+// so that FP32 holds any finite one, and its squares; 1 where it is infinite
+__device__ __forceinline__ double unit_scale(unsigned long long norm) {
+  const int e = (int)(norm >> 52);   // 0: subnormal or zero
+  return e == 2047 ? 1.0 : __longlong_as_double((long long)(e < 2046 ? 2046 - e : 1) << 52);
+}
+
 // G = A 2^-e (padded), V = I, *scale = max |g_ii| as ordered bits; with
-// `norm` (max |a_ii| as bits) e is its exponent, so that FP32 holds any A
+// `norm` (max |a_ij| as bits) e is its exponent.  FP32: max |g_ij|, which a
+// matrix without diagonal has as well.
 template <typename T>
 __global__ void syev_init_kernel(const double* __restrict__ A, long long lda, int n, int np, T* __restrict__ G,
                                  T* __restrict__ V, unsigned long long* __restrict__ scale,
                                  const unsigned long long* __restrict__ norm, float2* __restrict__ dd) {
   const long long total = (long long)np * np;
   unsigned long long mx = 0;
-  double f = 1.0;
-  if (norm) {
-    const int e = (int)(*norm >> 52);   // 0 for zero, 2047 for inf and nan
-    if (e > 0 && e < 2046) f = __longlong_as_double((long long)(2046 - e) << 52);
-  }
+  const double f = norm ? unit_scale(*norm) : 1.0;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(e / np), j = (int)(e - (long long)i * np);
@@ -136,16 +140,21 @@ __global__ void syev_init_kernel(const double* __restrict__ A, long long lda, in
     if (i < n && j < n) v = A[(long long)i * lda + j] * f;
     G[e] = (T)v;
     V[e] = i == j ? (T)1 : (T)0;
-    if (i == j) {
+    if (sizeof(T) == 4 || i == j) {
       // |v| as bits: the order of non-negative doubles is that of their bits
       const double a = fabs(v);
       unsigned long long b;
       memcpy(&b, &a, sizeof(b));
       if (a == a && b > mx) mx = b;
-      if (sizeof(T) == 4) dd[i] = hi_lo(v);
     }
+    if (sizeof(T) == 4 && i == j) dd[i] = hi_lo(v);
   }
-  if (mx) atomicMax(scale, mx);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx ? v : mx;
+  }
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(scale, mx);
 }
 
 // index at tournament position pos (0..31) in inner round ir
@@ -430,11 +439,7 @@ __global__ void __launch_bounds__(256) syev_small32_kernel(const double* __restr
   __shared__ float2 dg[2][NP];
   const int tid = threadIdx.x;
   const int t = tid % H, slot = tid / H, row = blockIdx.x * SL + slot;
-  double f = 1.0;
-  {
-    const int e = (int)(*norm >> 52);
-    if (e > 0 && e < 2046) f = __longlong_as_double((long long)(2046 - e) << 52);
-  }
+  const double f = unit_scale(*norm);
   for (int e = tid; e < NP * NP; e += NT) {
     const int i = e / NP, j = e % NP;
     const double v = i < n && j < n ? A[(long long)i * lda + j] * f : 0.0;
@@ -443,8 +448,8 @@ __global__ void __launch_bounds__(256) syev_small32_kernel(const double* __restr
   }
   for (int e = tid; e < SL * NP; e += NT) r[e / NP][e % NP] = 0.f;
   __syncthreads();
-  // diagonals scaled by the largest diagonal of the first pass's matrix lie
-  // in [-2, 2]; the floor is relative to 1
+  // the matrix scaled by its largest element is of order 1; the floor is
+  // relative to that
   const float floor_ = abs_;
   int p = t, q = NP - 1 - t;
   int pk[IT], qk[IT], src[IT];
@@ -677,6 +682,25 @@ __global__ void syev_off_kernel(const double* __restrict__ G, int np, const unsi
   if ((threadIdx.x & 31) == 0 && mx > 0.f) atomicMax(out, (unsigned long long)__float_as_uint(mx));
 }
 
+// *norm = max_ij |a_ij| as ordered bits
+__global__ void syev_norm_kernel(const double* __restrict__ A, long long lda, int n,
+                                 unsigned long long* __restrict__ norm) {
+  const long long total = (long long)n * n;
+  unsigned long long mx = 0;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(e / n), j = (int)(e - (long long)i * n);
+    const double a = fabs(A[(long long)i * lda + j]);
+    if (a == a && (unsigned long long)__double_as_longlong(a) > mx) mx = (unsigned long long)__double_as_longlong(a);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx ? v : mx;
+  }
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(norm, mx);
+}
+
 // *scale = max_i |G_ii| as ordered bits
 __global__ void syev_scale_kernel(const double* __restrict__ G, int np, long long ld,
                                   unsigned long long* __restrict__ scale) {
@@ -836,7 +860,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
   int* counts = reinterpret_cast<int*>(ws.scale + 8);
   DMRG_CUDA_TRY(cudaMemsetAsync(offs, 0, 4 * sizeof(unsigned long long), s));
   DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, sizeof(unsigned long long), s));
-  syev_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, norm);
+  syev_norm_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(A, lda, n, norm);
   DMRG_CHECK_LAUNCH();
   bool polish = false;   // V diagonalises A but is orthonormal to 1e-12 only
   for (int p = 0; p < MAX_PASSES; ++p) {
