@@ -682,7 +682,7 @@ __global__ void syev_off_kernel(const double* __restrict__ G, int np, const unsi
   if ((threadIdx.x & 31) == 0 && mx > 0.f) atomicMax(out, (unsigned long long)__float_as_uint(mx));
 }
 
-// *norm = max_ij |a_ij| as ordered bits
+// *norm = max_ij |a_ij| as ordered bits (nan is above infinity)
 __global__ void syev_norm_kernel(const double* __restrict__ A, long long lda, int n,
                                  unsigned long long* __restrict__ norm) {
   const long long total = (long long)n * n;
@@ -691,7 +691,8 @@ __global__ void syev_norm_kernel(const double* __restrict__ A, long long lda, in
        e += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(e / n), j = (int)(e - (long long)i * n);
     const double a = fabs(A[(long long)i * lda + j]);
-    if (a == a && (unsigned long long)__double_as_longlong(a) > mx) mx = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+    mx = b > mx ? b : mx;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -846,13 +847,17 @@ constexpr int MAX_PASSES = 8;
 constexpr double PASS0_ABS = 1e-6;
 constexpr float PASS_DONE = 3.f;
 
-int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, int* converged, cudaStream_t s) {
+// *overflow: a pass was not finite, where A holds an infinity or elements so
+// large that sums of products leave FP64's range; a nan in A is an error.
+int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, int* converged, int* overflow,
+                cudaStream_t s) {
   const int np = ws.np;
   const long long nn = (long long)np * np;
   // ws.R holds the rotations of the sweeps; G32 and Q32 share ws.T
   float* G32 = reinterpret_cast<float*>(ws.T);
   float* Q32 = G32 + nn;
   *converged = 0;
+  *overflow = 0;
   unsigned long long* norm = ws.scale + 2;
   // per pass (the fourth and later share a slot): largest off-diagonal, and
   // up to np = 64 the sweeps run
@@ -962,7 +967,14 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
       return DMRG_OK;
     }
     polish = mx <= PASS_DONE;
-    if (!(mx < 3e38f)) return DMRG_OK;   // not finite: left to the FP64 sweeps' checks
+    if (!(mx < 3e38f)) {
+      unsigned long long b = 0;
+      DMRG_CUDA_TRY(cudaMemcpyAsync(&b, norm, sizeof(b), cudaMemcpyDeviceToHost, s));
+      DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+      if (b > 0x7ff0000000000000ull) return DMRG_ERR_NAN;
+      *overflow = 1;
+      return DMRG_OK;
+    }
   }
   return DMRG_OK;
 }
@@ -982,8 +994,9 @@ int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, 
   T* V = reinterpret_cast<T*>(ws.V);
   bool started = false, passed = false;
   if (sizeof(T) == 8 && n > 1) {
-    DMRG_TRY(syev_passes(n, A, lda, ws, &done, &conv, s));
-    started = true;
+    int overflow = 0;
+    DMRG_TRY(syev_passes(n, A, lda, ws, &done, &conv, &overflow, s));
+    started = !overflow;   // else the FP64 sweeps begin with A itself
     passed = conv != 0;
   }
   if (!conv && !started) {

@@ -46,3 +46,24 @@ def test_largest_element_off_the_diagonal(n, diag, scale):
     assert np.max(np.abs(unit @ v - v * got)) <= lim
     assert np.max(np.abs(v.T @ v - np.eye(n))) <= 8 * n * 2.0 ** -53
     assert np.max(np.abs(got - w)) <= lim
+
+
+@pytest.mark.parametrize("n", [2, 20, 100])
+def test_infinite_diagonal_element_stands_alone(n):
+    """No rotation touches it: the sweeps on the matrix itself leave it, the
+    others and the unit vectors exactly."""
+    A = np.eye(n)
+    A[1, 1] = np.inf
+    st, got, v = _syev(A)
+    assert st == 0
+    assert got[0] == np.inf and np.all(got[1:] == 1.0)
+    assert np.array_equal(np.sort(np.abs(v), axis=None)[::-1][:n], np.ones(n)) and np.sum(np.abs(v)) == n
+
+
+@pytest.mark.parametrize("n", [2, 50, 100])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_input_is_reported(n, bad):
+    from dmrgpy_gb300 import _lib
+    A = np.eye(n)
+    A[0, 1] = A[1, 0] = bad
+    assert _syev(A)[0] == _lib.DMRG_ERR_NAN
