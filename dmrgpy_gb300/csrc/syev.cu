@@ -715,10 +715,14 @@ __global__ void syev_scale_kernel(const double* __restrict__ G, int np, long lon
   if (mx) atomicMax(scale, mx);
 }
 
+// d = diagonal of G, over the scale that syev_init_kernel gave G (norm null: 1)
 template <typename T>
-__global__ void syev_diag_kernel(const T* __restrict__ G, int np, double* __restrict__ d) {
+__global__ void syev_diag_kernel(const T* __restrict__ G, int np, const unsigned long long* __restrict__ norm,
+                                 double* __restrict__ d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < np) d[i] = (double)G[(long long)i * np + i];
+  if (i >= np) return;
+  const double v = (double)G[(long long)i * np + i];
+  d[i] = norm ? v / unit_scale(*norm) : v;
 }
 
 // out[r * ldo + c] = V[r * np + perm[c]] for r < n, c < ncols (transposed:
@@ -810,12 +814,12 @@ int syev_gemm(SyevWs& ws, int tA, int m, int n, int k, const double* A, long lon
 }
 
 // Sorted eigenvalues to the host and the permutation to the workspace.
-// (G null: the eigenvalues are in ws.diag)
+// (G null: the eigenvalues are in ws.diag; norm: of G's scale, or null)
 template <typename T>
-int syev_finish(int n, SyevWs& ws, const T* G, double* w, cudaStream_t s) {
+int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, double* w, cudaStream_t s) {
   const int np = ws.np;
   if (G) {
-    syev_diag_kernel<T><<<(np + 255) / 256, 256, 0, s>>>(G, np, ws.diag);
+    syev_diag_kernel<T><<<(np + 255) / 256, 256, 0, s>>>(G, np, norm, ws.diag);
     DMRG_CHECK_LAUNCH();
   }
   std::vector<double> d(n);
@@ -953,7 +957,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     if (mx <= PASS_DONE && (p >= 2 || polish)) {
       // eigenvalues; then what is left of the off-diagonals (up to PASS_DONE
       // of the threshold, where a converged sweep leaves their square) out of V
-      syev_diag_kernel<double><<<(np + 255) / 256, 256, 0, s>>>(ws.G, np, ws.diag);
+      syev_diag_kernel<double><<<(np + 255) / 256, 256, 0, s>>>(ws.G, np, nullptr, ws.diag);
       DMRG_CHECK_LAUNCH();
       syev_first_order_kernel<<<grid_for(nn), 256, 0, s>>>(ws.G, np, ws.T);
       DMRG_CHECK_LAUNCH();
@@ -999,9 +1003,15 @@ int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, 
     started = !overflow;   // else the FP64 sweeps begin with A itself
     passed = conv != 0;
   }
+  // FP32 squares what it rotates: of order 1, whatever A's scale
+  unsigned long long* norm = sizeof(T) == 4 ? ws.scale + 2 : nullptr;
   if (!conv && !started) {
-    DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, sizeof(unsigned long long), s));
-    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale, nullptr, ws.dd);
+    DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 3 * sizeof(unsigned long long), s));
+    if (norm) {
+      syev_norm_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(A, lda, n, norm);
+      DMRG_CHECK_LAUNCH();
+    }
+    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale, norm, ws.dd);
     DMRG_CHECK_LAUNCH();
   }
   if (!conv) {
@@ -1013,7 +1023,7 @@ int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, 
     if (f32 && conv) DMRG_TRY(syev_sweeps<T>(ws, G, V, 1, JacTol<T>::rel, JacTol<T>::abs, true, &done, &last, s));
   }
   if (sweeps) *sweeps = done;
-  DMRG_TRY(syev_finish<T>(n, ws, passed ? nullptr : G, w, s));
+  DMRG_TRY(syev_finish<T>(n, ws, passed ? nullptr : G, norm, w, s));
   return conv ? DMRG_OK : DMRG_ERR_NOCONV;
 }
 
