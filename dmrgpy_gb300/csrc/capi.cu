@@ -60,14 +60,21 @@ size_t heff_lean_ws(const dmrg_heff_t* o) {
   return align_up(P * esize(o->dtype)) + align_up(Q * esize(o->dtype));
 }
 
-size_t heff_min_ws(const dmrg_heff_t* o) { return std::min(heff_ws(o), heff_lean_ws(o)); }
+// Whether an operator takes its preparation and digits in this workspace
+bool heff_full(const dmrg_heff_t* o, const void* work, size_t bytes) {
+  return o->precision == DMRG_PREC_TF32X3 || (holds_digits(work) && bytes >= heff_ws(o));
+}
+
+bool heff_holds(const dmrg_heff_t* o, const void* work, size_t bytes) {
+  return work && (heff_full(o, work, bytes) ? bytes >= heff_ws(o) : bytes >= heff_lean_ws(o));
+}
 
 // One-off preparation of an operator (split-TF32: operand splitting of L, R
 // and the two-site MPO; FP64: digits of L and R, the MPO's row lists), then
 // heff_run per Krylov iteration.  bytes: what the workspace holds.
 template <typename T>
 int heff_prepare(const dmrg_heff_t* o, void* work, size_t bytes, cudaStream_t s) {
-  if (o->precision != DMRG_PREC_TF32X3) return bytes < heff_ws(o) ? DMRG_OK : heff64_prepare<T>(*o, work, s);
+  if (o->precision != DMRG_PREC_TF32X3) return heff_full(o, work, bytes) ? heff64_prepare<T>(*o, work, s) : DMRG_OK;
   if (o->dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
   return tf32x3_heff_prepare(*o, work, s);
 }
@@ -84,7 +91,7 @@ int heff_run(const dmrg_heff_t* o, const T* x, T* y, void* work, size_t bytes, c
     if (o->dtype != DMRG_REAL64) return DMRG_ERR_UNSUPPORTED;
     return tf32x3_heff_apply_prepared(*o, reinterpret_cast<const double*>(x), reinterpret_cast<double*>(y), work, s);
   }
-  if (bytes >= heff_ws(o)) return heff64_run<T>(*o, x, y, work, s);
+  if (heff_full(o, work, bytes)) return heff64_run<T>(*o, x, y, work, s);
   size_t P, Q;
   heff_fp64_elems<T>(*o, &P, &Q);
   T* Pp = static_cast<T*>(work);
@@ -289,7 +296,8 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
   const int m = (int)std::min<long long>(niter, n);
   if (m < 1) return DMRG_ERR_ARG;
   KrylovWs ws;
-  if (krylov_ws(o, m, false, &ws, work) > work_bytes && krylov_ws(o, m, true, &ws, work) > work_bytes)
+  if ((!holds_digits(work) || krylov_ws(o, m, false, &ws, work) > work_bytes) &&
+      krylov_ws(o, m, true, &ws, work) > work_bytes)
     return DMRG_ERR_WORKSPACE;
   T* Q = static_cast<T*>(ws.Q);
   T* w = static_cast<T*>(ws.w);
@@ -384,7 +392,8 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
   if (m < 1) return DMRG_ERR_ARG;
   if (sizeof(T) == 8 && coeff.imag() != 0.0) return DMRG_ERR_UNSUPPORTED;
   KrylovWs ws;
-  if (krylov_ws(o, m, false, &ws, work) > work_bytes && krylov_ws(o, m, true, &ws, work) > work_bytes)
+  if ((!holds_digits(work) || krylov_ws(o, m, false, &ws, work) > work_bytes) &&
+      krylov_ws(o, m, true, &ws, work) > work_bytes)
     return DMRG_ERR_WORKSPACE;
   T* Q = static_cast<T*>(ws.Q);
   T* w = static_cast<T*>(ws.w);
@@ -587,7 +596,7 @@ size_t dmrg_heff_workspace_bytes(const dmrg_heff_t* op) {
 
 int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (op->dtype == DMRG_COMPLEX128) {
     DMRG_TRY(heff_prepare<cplx>(op, work, work_bytes, s));
@@ -600,7 +609,7 @@ int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y, void* work, s
 
 int dmrg_heff_prepare(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (op->dtype == DMRG_COMPLEX128) return heff_prepare<cplx>(op, work, work_bytes, s);
   return heff_prepare<double>(op, work, work_bytes, s);
@@ -609,7 +618,7 @@ int dmrg_heff_prepare(const dmrg_heff_t* op, void* work, size_t work_bytes, void
 int dmrg_heff_apply_prepared(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes,
                              void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (heff_min_ws(op) > work_bytes || (!work && heff_min_ws(op) > 0)) return DMRG_ERR_WORKSPACE;
+  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (op->dtype == DMRG_COMPLEX128)
     return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, work_bytes, s);
@@ -618,7 +627,7 @@ int dmrg_heff_apply_prepared(const dmrg_heff_t* op, const void* x, void* y, void
 
 int dmrg_heff_status(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (heff_min_ws(op) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   return heff_finish<double>(op, work, s);
@@ -741,7 +750,7 @@ int dmrg_gemm(int dtype, int precision, int m, int k, int n, const void* A, cons
   g.c_m = st(n); g.c_n = st(1);
   // digit products where they pay and the caller's workspace holds them; the
   // FP64 pipe needs no workspace
-  if (need > 0 && work && need <= work_bytes) {
+  if (need > 0 && work && need <= work_bytes && holds_digits(work)) {
     if (dtype == DMRG_COMPLEX128)
       return dg_product<cplx>(g, static_cast<const cplx*>(A), static_cast<const cplx*>(B), 1.0, 0,
                               static_cast<cplx*>(C), work, s);

@@ -134,6 +134,11 @@ int launch_after(void (*fn)(P...), dim3 grid, int threads, cudaStream_t s, A... 
 
 inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
+// Whether a caller's workspace can hold digit blocks, which are stored as 16
+// bytes and copied in bulk; one that starts in between runs the FP64 pipe,
+// whose loads are of single elements.
+inline bool holds_digits(const void* work) { return (reinterpret_cast<uintptr_t>(work) & 15) == 0; }
+
 // Bump allocator over a caller-provided workspace.
 struct Arena {
   char* base;

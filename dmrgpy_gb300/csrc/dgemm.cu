@@ -1044,7 +1044,7 @@ int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumul
 int fgemm(const TGemm& g, double alpha, const double* A, const double* B, int accumulate, double* C, void* ws,
           size_t ws_bytes, cudaStream_t s) {
   const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
-  if (ws_bytes > 0 && ws && (long long)g.B.n1 * g.B.n2 == 1 && M > 0 && N > 0 && K > 0 &&
+  if (ws_bytes > 0 && ws && holds_digits(ws) && (long long)g.B.n1 * g.B.n2 == 1 && M > 0 && N > 0 && K > 0 &&
       dg_pays(false, M, N, K, false) && dg_product_bytes<double>(g) <= ws_bytes)
     return dg_product<double>(g, A, B, alpha, accumulate, C, ws, s);
   return tgemm<double>(g, alpha, A, B, accumulate ? 1.0 : 0.0, C, s);

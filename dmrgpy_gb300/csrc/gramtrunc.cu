@@ -173,8 +173,10 @@ __global__ void gt_half_dev_kernel(const double* __restrict__ G, int k, double* 
 
 // Operands of digit products (bytes may be 0: products on the FP64 pipe).
 struct Scratch {
-  void* p;
-  size_t bytes;
+  void* p = nullptr;
+  size_t bytes = 0;
+  Scratch() = default;
+  Scratch(void* at, size_t n) : p(at), bytes(holds_digits(at) ? n : 0) {}
 };
 
 // C (m x n) = op(A) op(B) in FP64 (tgemm with strides); A is m x k (ld lda)
@@ -258,7 +260,7 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
   double* fdev = reinterpret_cast<double*>(p); p += align_up(d * (size_t)c);
   void* sw = p;
   const size_t sw_bytes = work_bytes - (size_t)(p - static_cast<char*>(work));
-  const Scratch x{static_cast<char*>(sw) + syev_lean_bytes(c), sw_bytes - syev_lean_bytes(c)};
+  const Scratch x(static_cast<char*>(sw) + syev_lean_bytes(c), sw_bytes - syev_lean_bytes(c));
   // G = X^T X with X = M^T (rows route) or M
   if (rows && dig_need(c, c, r) > 0 && dig_need(c, c, r) <= x.bytes) {
     DMRG_TRY(gemm64(0, 1, c, c, r, M, n, M, n, G, c, x, s));
@@ -381,7 +383,7 @@ size_t rr_layout(int m, int n, int k, bool lean, size_t bytes, RRWs* w, void* ba
     dig = std::max(dig, std::max(dig_need(k, n, m), dig_need(k, m, n)));
     take(dig);
   }
-  r.x = Scratch{p ? p + head : nullptr, bytes > head ? bytes - head : 0};
+  r.x = Scratch(p ? p + head : nullptr, bytes > head ? bytes - head : 0);
   r.sw_bytes = syev_lean_bytes(k) + r.x.bytes;
   if (w) *w = r;
   return off;

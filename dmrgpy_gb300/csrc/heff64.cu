@@ -221,7 +221,8 @@ template <typename T>
 int env64(int side, long long clb, long long crb, long long clk, long long crk, long long d, long long wl,
           long long wr, const T* E, const T* W, const T* B, const T* A, T* Enew, void* work, size_t work_bytes,
           cudaStream_t s) {
-  const bool lean = env_plan(side, sizeof(T) == 16, clb, crb, clk, crk, d, wl, wr, false, nullptr).total > work_bytes;
+  const bool lean = !holds_digits(work) ||
+                    env_plan(side, sizeof(T) == 16, clb, crb, clk, crk, d, wl, wr, false, nullptr).total > work_bytes;
   const E64 h = env_plan(side, sizeof(T) == 16, clb, crb, clk, crk, d, wl, wr, lean, work);
   if (h.total > work_bytes) return DMRG_ERR_WORKSPACE;
   T* y1 = static_cast<T*>(h.y1);

@@ -14,8 +14,8 @@ template <typename T> int heff64_run(const dmrg_heff_t& o, const T* x, T* y, voi
 
 // Environment extension with bra B and ket A (equal for an expectation
 // value), sides and shapes as dmrg_env_extend_mixed.  A workspace below
-// env64_workspace_bytes that holds the two intermediates runs on the FP64
-// pipe with a dense MPO step.
+// env64_workspace_bytes that holds the two intermediates, or one off a
+// 16-byte boundary, runs on the FP64 pipe with a dense MPO step.
 size_t env64_workspace_bytes(int side, int dtype, long long clb, long long crb, long long clk, long long crk,
                              long long d, long long wl, long long wr);
 template <typename T>

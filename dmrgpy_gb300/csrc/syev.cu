@@ -987,7 +987,7 @@ template <typename T>
 int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, int* sweeps, void* work,
               size_t work_bytes, cudaStream_t s) {
   SyevWs ws;
-  const bool lean = syev_layout(n, nullptr, nullptr, false) > work_bytes;
+  const bool lean = !holds_digits(work) || syev_layout(n, nullptr, nullptr, false) > work_bytes;
   syev_layout(n, &ws, work, lean);
   const int np = ws.np, nb = ws.nb;
   std::vector<int> tab;

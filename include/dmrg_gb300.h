@@ -5,7 +5,9 @@
  * (passed as void*), allocates nothing itself (scratch comes from a
  * caller-provided workspace whose size the matching *_workspace_bytes()
  * reports), and returns an int status (DMRG_OK = 0).  No entry point
- * traps, aborts or waits without a bound.
+ * traps, aborts or waits without a bound.  A workspace starts on a multiple
+ * of its element size; FP64 calls keep to the FP64 pipe in one that is off a
+ * 16-byte boundary (digit products store and copy 16 bytes at a time).
  *
  * Array layouts (row-major, element type double or interleaved complex
  * double as selected by `dtype`):
