@@ -65,8 +65,9 @@ bool heff_full(const dmrg_heff_t* o, const void* work, size_t bytes) {
   return o->precision == DMRG_PREC_TF32X3 || (holds_digits(work) && bytes >= heff_ws(o));
 }
 
-bool heff_holds(const dmrg_heff_t* o, const void* work, size_t bytes) {
-  return work && (heff_full(o, work, bytes) ? bytes >= heff_ws(o) : bytes >= heff_lean_ws(o));
+// the least an operator runs in, in that workspace
+size_t heff_need(const dmrg_heff_t* o, const void* work) {
+  return holds_digits(work) ? std::min(heff_ws(o), heff_lean_ws(o)) : heff_lean_ws(o);
 }
 
 // One-off preparation of an operator (split-TF32: operand splitting of L, R
@@ -596,7 +597,7 @@ size_t dmrg_heff_workspace_bytes(const dmrg_heff_t* op) {
 
 int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
+  if (!work || heff_need(op, work) > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (op->dtype == DMRG_COMPLEX128) {
     DMRG_TRY(heff_prepare<cplx>(op, work, work_bytes, s));
@@ -609,25 +610,24 @@ int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y, void* work, s
 
 int dmrg_heff_prepare(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (op->dtype == DMRG_COMPLEX128) return heff_prepare<cplx>(op, work, work_bytes, s);
-  return heff_prepare<double>(op, work, work_bytes, s);
+  if (!work || heff_need(op, work) > work_bytes) return DMRG_ERR_WORKSPACE;
+  if (op->precision != DMRG_PREC_TF32X3) return DMRG_OK;   // nothing of it is kept: apply_prepared does it
+  return heff_prepare<double>(op, work, work_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int dmrg_heff_apply_prepared(const dmrg_heff_t* op, const void* x, void* y, void* work, size_t work_bytes,
                              void* stream) {
   if (!heff_valid(op) || !x || !y || x == y) return DMRG_ERR_ARG;
-  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
+  if (!work || heff_need(op, work) > work_bytes) return DMRG_ERR_WORKSPACE;
+  // FP64: the workspace is scratch between calls, and L, R and W may have changed
+  if (op->precision != DMRG_PREC_TF32X3) return dmrg_heff_apply(op, x, y, work, work_bytes, stream);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (op->dtype == DMRG_COMPLEX128)
-    return heff_run<cplx>(op, static_cast<const cplx*>(x), static_cast<cplx*>(y), work, work_bytes, s);
   return heff_run<double>(op, static_cast<const double*>(x), static_cast<double*>(y), work, work_bytes, s);
 }
 
 int dmrg_heff_status(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream) {
   if (!heff_valid(op)) return DMRG_ERR_ARG;
-  if (!heff_holds(op, work, work_bytes)) return DMRG_ERR_WORKSPACE;
+  if (heff_need(op, work) > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   return heff_finish<double>(op, work, s);

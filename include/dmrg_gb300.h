@@ -95,8 +95,8 @@ int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y,
 
 /* The same matvec split in two, for callers that drive their own Krylov
  * loop: dmrg_heff_prepare() does the per-operator work once (split-TF32:
- * splitting L, R and the two-site MPO into the workspace; FP64: the digits
- * of L and R and the MPO's row lists),
+ * splitting L, R and the two-site MPO into the workspace; FP64: nothing, and
+ * the workspace is free for other use between calls),
  * dmrg_heff_apply_prepared() applies H_eff for each new vector with the same
  * op and workspace (the plan-once / replay-per-iteration structure of
  * pyitensor/kernels.py:353-410).  dmrg_heff_status() synchronises the stream
