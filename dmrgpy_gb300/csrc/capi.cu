@@ -86,6 +86,19 @@ int heff_finish(const dmrg_heff_t* o, void* work, cudaStream_t s) {
   return tf32x3_heff_status(*o, work, s);
 }
 
+// a wait of the tensor-core kernels that gave up since the prepare (either
+// precision; synchronises)
+int heff_gave_up(const dmrg_heff_t* o, void* work, size_t bytes, cudaStream_t s) {
+  if (o->precision == DMRG_PREC_TF32X3) return tf32x3_heff_status(*o, work, s);
+  return heff_full(o, work, bytes) ? heff64_status(*o, work, s) : DMRG_OK;
+}
+
+// status of a Krylov loop that met a nan: the wait behind it, if one gave up
+int heff_nan(const dmrg_heff_t* o, void* work, size_t bytes, cudaStream_t s) {
+  const int st = heff_gave_up(o, work, bytes, s);
+  return st != DMRG_OK ? st : DMRG_ERR_NAN;
+}
+
 template <typename T>
 int heff_run(const dmrg_heff_t* o, const T* x, T* y, void* work, size_t bytes, cudaStream_t s) {
   if (o->precision == DMRG_PREC_TF32X3) {
@@ -337,7 +350,7 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
   std::vector<double> al{hbuf[0]}, be;
   double beta = hbuf[2];
   if (hbuf[3] != 0.0) return (int)hbuf[3];
-  if (!(hbuf[0] == hbuf[0]) || !(beta == beta)) return DMRG_ERR_NAN;
+  if (!(hbuf[0] == hbuf[0]) || !(beta == beta)) return heff_nan(o, ws.hw, ws.hbytes, s);
   double prev = al[0];
   int k = 1;
   for (int j = 1; j < m; ++j) {
@@ -363,7 +376,7 @@ int lanczos_impl(const dmrg_heff_t* o, T* x, int niter, double tol, double* ener
     DMRG_CUDA_TRY(cudaMemcpyAsync(hbuf, ws.sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
     if (hbuf[3] != 0.0) return (int)hbuf[3];
-    if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return DMRG_ERR_NAN;
+    if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return heff_nan(o, ws.hw, ws.hbytes, s);
     al.push_back(hbuf[0]);
     beta = hbuf[2];
     k = j + 1;
@@ -437,7 +450,7 @@ int expm_impl(const dmrg_heff_t* o, T* x, std::complex<double> coeff, int niter,
     DMRG_CUDA_TRY(cudaMemcpyAsync(hbuf, ws.sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
     if (hbuf[3] != 0.0) return (int)hbuf[3];
-    if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return DMRG_ERR_NAN;
+    if (!(hbuf[0] == hbuf[0]) || !(hbuf[2] == hbuf[2])) return heff_nan(o, ws.hw, ws.hbytes, s);
     al.push_back(hbuf[0]);
     const double beta = hbuf[2];
     const int k = it + 1;
@@ -630,7 +643,7 @@ int dmrg_heff_status(const dmrg_heff_t* op, void* work, size_t work_bytes, void*
   if (heff_need(op, work) > work_bytes) return DMRG_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
-  return heff_finish<double>(op, work, s);
+  return work ? heff_gave_up(op, work, work_bytes, s) : DMRG_OK;
 }
 
 // whether an operator runs in `bytes` of scratch (dmrg_heff_apply_noalloc)
@@ -728,7 +741,7 @@ size_t dmrg_gemm_workspace_bytes(int dtype, int precision, int m, int k, int n) 
   if (precision == DMRG_PREC_TF32X3) return tf32x3_gemm_workspace_bytes(m, k, n);
   const bool c = dtype == DMRG_COMPLEX128;
   if (m <= 0 || k <= 0 || n <= 0 || !dg_pays(c, m, n, k, false)) return 0;
-  return dg_bytes(0, c, m, k) + dg_bytes(1, c, n, k);
+  return dg_product_bytes(c, m, n, k);
 }
 
 int dmrg_gemm(int dtype, int precision, int m, int k, int n, const void* A, const void* B, void* C, void* work,
@@ -753,9 +766,9 @@ int dmrg_gemm(int dtype, int precision, int m, int k, int n, const void* A, cons
   if (need > 0 && work && need <= work_bytes && holds_digits(work)) {
     if (dtype == DMRG_COMPLEX128)
       return dg_product<cplx>(g, static_cast<const cplx*>(A), static_cast<const cplx*>(B), 1.0, 0,
-                              static_cast<cplx*>(C), work, s);
+                              static_cast<cplx*>(C), work, nullptr, s);
     return dg_product<double>(g, static_cast<const double*>(A), static_cast<const double*>(B), 1.0, 0,
-                              static_cast<double*>(C), work, s);
+                              static_cast<double*>(C), work, nullptr, s);
   }
   if (dtype == DMRG_COMPLEX128)
     return tgemm<cplx>(g, Sc<cplx>::one(), static_cast<const cplx*>(A), static_cast<const cplx*>(B), Sc<cplx>::zero(),

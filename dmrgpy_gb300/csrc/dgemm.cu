@@ -46,7 +46,8 @@
 //   warps 2-9 epilogue: after every run the eight accumulators are read,
 //             converted to integers and added to the running sums (registers),
 //             two warps per TMEM lane quarter, 32 columns each.
-// All mbarrier waits are bounded; a wait that gives up makes the CTA write NaN.
+// All mbarrier waits are bounded; a wait that gives up makes the CTA write NaN
+// and records it in the product's status word.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -73,9 +74,6 @@ constexpr int DG_THREADS = 320;
 // the 64-bit sums grow by up to 3 2^46 per k: at most 20480 k per launch
 constexpr int MAX_STEPS = 1280;
 constexpr int EXP_BAD = INT_MAX;            // row with a non-finite element
-
-// set by a wait that gave up; the kernel then writes NaN to its tiles
-__device__ int g_dg_timeout;
 
 __host__ __device__ constexpr int tile_rows(int side) { return side == 0 ? TM : TN; }
 
@@ -278,11 +276,19 @@ struct SplitJob {
   int* exps;
   int* sq;
   uint4* dig;
+  DgStatus* clear;
   unsigned grid;
 };
 
+__device__ __forceinline__ void clear_status(DgStatus* st, unsigned block) {
+  if (!st || block != 0 || threadIdx.x != 0) return;
+  st->err = 0;
+  st->mark = DG_CLEARED;
+}
+
 template <int CPLX, int R>
 __global__ void __launch_bounds__(256) dg_split_kernel(const SplitJob j) {
+  clear_status(j.clear, blockIdx.x);
   split8<CPLX, R>(j.a, j.exps, j.sq, j.dig, blockIdx.x);
 }
 
@@ -290,6 +296,7 @@ __global__ void __launch_bounds__(256) dg_split_kernel(const SplitJob j) {
 // fill and tail (3.6 us each at 256 x 256)
 template <bool C>
 __global__ void __launch_bounds__(256) dg_split2_kernel(const SplitJob A, const SplitJob B) {
+  clear_status(A.clear, blockIdx.x);
   if (blockIdx.x < A.grid) split8<C ? 1 : 0, TM>(A.a, A.exps, A.sq, A.dig, blockIdx.x);
   else split8<C ? 2 : 0, TN>(B.a, B.exps, B.sq, B.dig, blockIdx.x - A.grid);
 }
@@ -316,6 +323,7 @@ struct GArgs {
   int nflat;            // columns at one stride cn1
   int cplx_;
   int negate, accumulate;
+  int* err;             // status word
 };
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -544,7 +552,7 @@ __device__ __forceinline__ void store4(const GArgs& a, const RowOut& o, int gn, 
 }
 
 __global__ void __launch_bounds__(DG_THREADS, 1) dg_gemm_kernel(const GArgs a) {
-  int* err = &g_dg_timeout;
+  int* const err = a.err;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -718,7 +726,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(SK, 1, 1) dg_s
   // exchange area: sums of [source][column][row], 8 then 4 bytes each, then a flag per source
   constexpr int XM = SK * CN * TM * 8, XH = SK * CN * TM * 4;
   static_assert(XM + XH + 64 <= STAGES * ST_BYTES, "exchange area");
-  int* err = &g_dg_timeout;
+  int* const err = a.err;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -934,14 +942,16 @@ static int split_job(int side, const DgOperand& o, void* buf, SplitJob* job) {
   job->sq = reinterpret_cast<int*>(static_cast<char*>(buf) + exps_bytes(side, a.R));
   job->dig = reinterpret_cast<uint4*>(static_cast<char*>(buf) + head_bytes(side, a.R));
   job->grid = (unsigned)(Rp / 8);
+  job->clear = nullptr;
   return DMRG_OK;
 }
 
 template <typename T>
-int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
+int dg_split(int side, const DgOperand& o, void* buf, DgStatus* clear, cudaStream_t s) {
   constexpr bool C = sizeof(T) == 16;
   SplitJob j;
   DMRG_TRY(split_job<T>(side, o, buf, &j));
+  j.clear = clear;
   if (side == 0) dg_split_kernel<C ? 1 : 0, TM><<<j.grid, 256, 0, s>>>(j);
   else dg_split_kernel<C ? 2 : 0, TN><<<j.grid, 256, 0, s>>>(j);
   DMRG_CHECK_LAUNCH();
@@ -949,14 +959,15 @@ int dg_split(int side, const DgOperand& o, void* buf, cudaStream_t s) {
 }
 
 template <typename T>
-int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, cudaStream_t s) {
+int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, DgStatus* clear, cudaStream_t s) {
   SplitJob a, b;
   DMRG_TRY(split_job<T>(0, A, bufa, &a));
   DMRG_TRY(split_job<T>(1, B, bufb, &b));
   if ((unsigned long long)a.grid + b.grid > 0x7fffffffull) {
-    DMRG_TRY(dg_split<T>(0, A, bufa, s));
-    return dg_split<T>(1, B, bufb, s);
+    DMRG_TRY(dg_split<T>(0, A, bufa, clear, s));
+    return dg_split<T>(1, B, bufb, nullptr, s);
   }
+  a.clear = clear;
   dg_split2_kernel<sizeof(T) == 16><<<a.grid + b.grid, 256, 0, s>>>(a, b);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
@@ -964,9 +975,9 @@ int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, cu
 
 template <typename T>
 int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long long K, const DgOut& out,
-            cudaStream_t s) {
+            DgStatus* st, cudaStream_t s) {
   constexpr bool C = sizeof(T) == 16;
-  if (M < 1 || N < 1 || K < 1 || !Adig || !Bdig || !out.C) return DMRG_ERR_ARG;
+  if (M < 1 || N < 1 || K < 1 || !Adig || !Bdig || !out.C || !st) return DMRG_ERR_ARG;
   const long long Mr = C ? 2 * M : M, Kr = C ? 2 * K : K;
   const long long tm = up(Mr, TM), tn = up(N, TN);
   if (Mr > 0x7fffffffLL || N > 0x7fffffffLL || tm * tn > 0x7fffffffLL) return DMRG_ERR_ARG;
@@ -989,6 +1000,7 @@ int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long l
   else if (out.N.n1 == 1 || a.cn1 == a.cn2 * a.N2) { a.nflat = 1; a.cn1 = a.cn2; }
   a.cplx_ = C ? 1 : 0;
   a.negate = out.alpha < 0.0;
+  a.err = &st->err;
   const int sk = split_of(tm * tn, a.steps);
   static std::atomic<unsigned long long> attr[4];
   const void* fn = sk == 8   ? reinterpret_cast<const void*>(dg_splitk_kernel<8>)
@@ -1023,45 +1035,57 @@ int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long l
   return DMRG_OK;
 }
 
+size_t dg_product_bytes(bool cplx_, long long M, long long N, long long K) {
+  return DG_STATUS_BYTES + dg_bytes(0, cplx_, M, K) + dg_bytes(1, cplx_, N, K);
+}
+
 template <typename T>
 size_t dg_product_bytes(const TGemm& g) {
-  constexpr bool C = sizeof(T) == 16;
-  const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
-  return dg_bytes(0, C, M, K) + dg_bytes(1, C, N, K);
+  return dg_product_bytes(sizeof(T) == 16, (long long)g.M.n1 * g.M.n2, (long long)g.N.n1 * g.N.n2,
+                          (long long)g.K.n1 * g.K.n2);
+}
+
+int dg_gave_up(const DgStatus* st, bool marked, cudaStream_t s) {
+  DgStatus h = {0, 0};
+  DMRG_CUDA_TRY(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
+  DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+  return h.err == DMRG_ERR_TIMEOUT && (!marked || h.mark == DG_CLEARED) ? DMRG_ERR_TIMEOUT : DMRG_OK;
 }
 
 template <typename T>
 int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumulate, T* C, void* work,
-               cudaStream_t s) {
+               DgStatus* st, cudaStream_t s) {
   const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
-  void* da = work;
-  void* db = static_cast<char*>(work) + dg_bytes(0, sizeof(T) == 16, M, K);
+  DgStatus* own = static_cast<DgStatus*>(work);
+  void* da = static_cast<char*>(work) + DG_STATUS_BYTES;
+  void* db = static_cast<char*>(da) + dg_bytes(0, sizeof(T) == 16, M, K);
   DMRG_TRY(dg_split2<T>(DgOperand{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, da,
-                        DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, s));
-  return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, s);
+                        DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, st ? nullptr : own, s));
+  return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, st ? st : own, s);
 }
 
 int fgemm(const TGemm& g, double alpha, const double* A, const double* B, int accumulate, double* C, void* ws,
-          size_t ws_bytes, cudaStream_t s) {
+          size_t ws_bytes, DgStatus* st, cudaStream_t s) {
   const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
   if (ws_bytes > 0 && ws && holds_digits(ws) && (long long)g.B.n1 * g.B.n2 == 1 && M > 0 && N > 0 && K > 0 &&
       dg_pays(false, M, N, K, false) && dg_product_bytes<double>(g) <= ws_bytes)
-    return dg_product<double>(g, A, B, alpha, accumulate, C, ws, s);
+    return dg_product<double>(g, A, B, alpha, accumulate, C, ws, st, s);
   return tgemm<double>(g, alpha, A, B, accumulate ? 1.0 : 0.0, C, s);
 }
 
 template size_t dg_product_bytes<double>(const TGemm&);
 template size_t dg_product_bytes<cplx>(const TGemm&);
-template int dg_product<double>(const TGemm&, const double*, const double*, double, int, double*, void*,
+template int dg_product<double>(const TGemm&, const double*, const double*, double, int, double*, void*, DgStatus*,
                                 cudaStream_t);
-template int dg_product<cplx>(const TGemm&, const cplx*, const cplx*, double, int, cplx*, void*, cudaStream_t);
-template int dg_split<double>(int, const DgOperand&, void*, cudaStream_t);
-template int dg_split<cplx>(int, const DgOperand&, void*, cudaStream_t);
-template int dg_split2<double>(const DgOperand&, void*, const DgOperand&, void*, cudaStream_t);
-template int dg_split2<cplx>(const DgOperand&, void*, const DgOperand&, void*, cudaStream_t);
-template int dg_gemm<double>(const void*, const void*, long long, long long, long long, const DgOut&,
+template int dg_product<cplx>(const TGemm&, const cplx*, const cplx*, double, int, cplx*, void*, DgStatus*,
+                              cudaStream_t);
+template int dg_split<double>(int, const DgOperand&, void*, DgStatus*, cudaStream_t);
+template int dg_split<cplx>(int, const DgOperand&, void*, DgStatus*, cudaStream_t);
+template int dg_split2<double>(const DgOperand&, void*, const DgOperand&, void*, DgStatus*, cudaStream_t);
+template int dg_split2<cplx>(const DgOperand&, void*, const DgOperand&, void*, DgStatus*, cudaStream_t);
+template int dg_gemm<double>(const void*, const void*, long long, long long, long long, const DgOut&, DgStatus*,
                              cudaStream_t);
-template int dg_gemm<cplx>(const void*, const void*, long long, long long, long long, const DgOut&,
+template int dg_gemm<cplx>(const void*, const void*, long long, long long, long long, const DgOut&, DgStatus*,
                            cudaStream_t);
 
 }  // namespace dmrg

@@ -171,13 +171,23 @@ __global__ void gt_half_dev_kernel(const double* __restrict__ G, int k, double* 
   if ((threadIdx.x & 31) == 0 && mx) atomicMax(dev, mx);
 }
 
-// Operands of digit products (bytes may be 0: products on the FP64 pipe).
+// Operands of digit products (bytes may be 0: products on the FP64 pipe), and
+// the word, cleared at the call's start, in which their waits record.
 struct Scratch {
   void* p = nullptr;
   size_t bytes = 0;
+  DgStatus* st = nullptr;
   Scratch() = default;
-  Scratch(void* at, size_t n) : p(at), bytes(holds_digits(at) ? n : 0) {}
+  Scratch(void* at, size_t n, DgStatus* status) : p(at), bytes(holds_digits(at) ? n : 0), st(status) {}
 };
+
+// What a call that met a nan, or did not converge, returns: the wait behind
+// it, if one gave up.
+int gave_up_or(int status, const Scratch& x, cudaStream_t s) {
+  if ((status != DMRG_ERR_NAN && status != DMRG_ERR_NOCONV) || x.bytes == 0) return status;
+  const int st = dg_gave_up(x.st, false, s);
+  return st != DMRG_OK ? st : status;
+}
 
 // C (m x n) = op(A) op(B) in FP64 (tgemm with strides); A is m x k (ld lda)
 // or, transposed, k x m; B is k x n (ldb) or, transposed, n x k
@@ -188,13 +198,13 @@ int gemm64(int tA, int tB, int m, int n, int k, const double* A, long long lda, 
   if (!tA) { g.a_m = st(lda); g.a_k = st(1); } else { g.a_m = st(1); g.a_k = st(lda); }
   if (!tB) { g.b_k = st(ldb); g.b_n = st(1); } else { g.b_k = st(1); g.b_n = st(ldb); }
   g.c_m = st(ldc); g.c_n = st(1);
-  return fgemm(g, 1.0, A, B, 0, C, x.p, x.bytes, s);
+  return fgemm(g, 1.0, A, B, 0, C, x.p, x.bytes, x.st, s);
 }
 
 // scratch that lets gemm64 of this shape run as a digit product (0 where the
 // FP64 pipe is as fast)
 size_t dig_need(long long m, long long n, long long k) {
-  return dg_pays(false, m, n, k, false) ? dg_bytes(0, false, m, k) + dg_bytes(1, false, n, k) : 0;
+  return dg_pays(false, m, n, k, false) ? dg_product_bytes(false, m, n, k) : 0;
 }
 
 // G (k x k) = X^T X, X m x k (ld)
@@ -212,7 +222,7 @@ int gemm64_sub(int rows, int cols, int k, const double* A, long long lda, const 
   g.a_m = st(lda); g.a_k = st(1);
   g.b_k = st(ldb); g.b_n = st(1);
   g.c_m = st(ldc); g.c_n = st(1);
-  return fgemm(g, -1.0, A, B, 1, C, x.p, x.bytes, s);
+  return fgemm(g, -1.0, A, B, 1, C, x.p, x.bytes, x.st, s);
 }
 
 }  // namespace
@@ -260,7 +270,10 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
   double* fdev = reinterpret_cast<double*>(p); p += align_up(d * (size_t)c);
   void* sw = p;
   const size_t sw_bytes = work_bytes - (size_t)(p - static_cast<char*>(work));
-  const Scratch x(static_cast<char*>(sw) + syev_lean_bytes(c), sw_bytes - syev_lean_bytes(c));
+  // (the status word is fdev's first: the factors come after the last product)
+  const Scratch x(static_cast<char*>(sw) + syev_lean_bytes(c), sw_bytes - syev_lean_bytes(c),
+                  reinterpret_cast<DgStatus*>(fdev));
+  if (x.bytes > 0) DMRG_CUDA_TRY(cudaMemsetAsync(x.st, 0, sizeof(DgStatus), s));
   // G = X^T X with X = M^T (rows route) or M
   if (rows && dig_need(c, c, r) > 0 && dig_need(c, c, r) <= x.bytes) {
     DMRG_TRY(gemm64(0, 1, c, c, r, M, n, M, n, G, c, x, s));
@@ -271,7 +284,7 @@ int gram_truncate(int m, int n, const double* M, double cutoff, int maxdim, int 
     DMRG_TRY(gram64(M, n, r, c, G, x, s));
   }
   std::vector<double> w(c);
-  DMRG_TRY(syev_jacobi(c, G, c, w.data(), 40, sweeps, sw, sw_bytes, s));
+  DMRG_TRY(gave_up_or(syev_jacobi(c, G, c, w.data(), 40, sweeps, sw, sw_bytes, s), x, s));
   std::vector<double> sv(cmin);
   for (int i = 0; i < cmin; ++i) sv[i] = std::sqrt(std::max(w[i], 0.0));
   int kp;
@@ -383,7 +396,7 @@ size_t rr_layout(int m, int n, int k, bool lean, size_t bytes, RRWs* w, void* ba
     dig = std::max(dig, std::max(dig_need(k, n, m), dig_need(k, m, n)));
     take(dig);
   }
-  r.x = Scratch(p ? p + head : nullptr, bytes > head ? bytes - head : 0);
+  r.x = Scratch(p ? p + head : nullptr, bytes > head ? bytes - head : 0, reinterpret_cast<DgStatus*>(r.acc + 6));
   r.sw_bytes = syev_lean_bytes(k) + r.x.bytes;
   if (w) *w = r;
   return off;
@@ -499,12 +512,20 @@ size_t rr_truncate_workspace_bytes(int m, int n, int k) {
 
 size_t rr_truncate_lean_bytes(int m, int n, int k) { return rr_layout(m, n, k, true, 0, nullptr, nullptr); }
 
+namespace {
+
 // theta (m x n).  absorb 0 keeps an orthonormal LEFT basis, X = the right
 // tensor across the bond (kx x n, orthonormal rows); absorb 1 keeps a RIGHT
 // basis, X = the left tensor (m x kx, ld kx, orthonormal columns).  Start
 // vectors beyond kx are random.  Keeps at most k vectors by the rule of
 // pyitensor/svd.py:32-68; svals (host, >= k) receives the singular-value
 // estimates of the kept space (nvals of them).
+int rr_run(int m, int n, int k, const double* theta, const double* X, int kx, int absorb, int iters, double cutoff,
+           int mindim, double* lo, double* ro, double* svals, int* nvals, int* keep, double* disc, RRWs& w,
+           cudaStream_t s);
+
+}  // namespace
+
 int rr_truncate(int m, int n, int k, const double* theta, const double* X, int kx, int absorb, int iters,
                 double cutoff, int mindim, double* lo, double* ro, double* svals, int* nvals, int* keep, double* disc,
                 void* work, size_t work_bytes, cudaStream_t s) {
@@ -514,6 +535,15 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
   if (!work || rr_truncate_lean_bytes(m, n, k) > work_bytes) return DMRG_ERR_WORKSPACE;
   RRWs w;
   rr_layout(m, n, k, true, work_bytes, &w, work);
+  return gave_up_or(
+      rr_run(m, n, k, theta, X, kx, absorb, iters, cutoff, mindim, lo, ro, svals, nvals, keep, disc, w, s), w.x, s);
+}
+
+namespace {
+
+int rr_run(int m, int n, int k, const double* theta, const double* X, int kx, int absorb, int iters, double cutoff,
+           int mindim, double* lo, double* ro, double* svals, int* nvals, int* keep, double* disc, RRWs& w,
+           cudaStream_t s) {
   const double nul = null_fraction(cutoff);
   const double* Th = theta;
   int M = m, N = n;
@@ -585,6 +615,8 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
     wt.assign(kw, 0.0);
     DMRG_CUDA_TRY(cudaMemcpyAsync(wt.data(), w.f, sizeof(double) * kw, cudaMemcpyDeviceToHost, s));
     DMRG_CUDA_TRY(cudaStreamSynchronize(s));
+    for (int j = 0; j < kw; ++j)
+      if (!(wt[j] == wt[j])) return DMRG_ERR_NAN;
     double dc;
     keep_rule_partial(wt.data(), kw, std::min(m, n), hacc, cutoff, k, std::max(1, mindim), -1.0, &kp, &dc);
     double kept_all = 0.0;
@@ -637,6 +669,8 @@ int rr_truncate(int m, int n, int k, const double* theta, const double* X, int k
   if (disc) *disc = hacc > 0.0 ? std::max(0.0, 1.0 - kept / hacc) : 0.0;
   return DMRG_OK;
 }
+
+}  // namespace
 
 // ---------------------------------------------------------------- Ritz values after the split-TF32 subspace
 size_t subspace_ritz_workspace_bytes(int m, int n, int k) {

@@ -43,6 +43,7 @@ struct H64 {
   bool dig1, dig2;
   MpoShape mpo;
   void *x1, *x3, *list, *ldig, *rdig, *vdig;
+  DgStatus* status;          // where dig1 or dig2
   size_t total;
 };
 
@@ -70,6 +71,7 @@ H64 plan(const dmrg_heff_t& o, void* work) {
   // the vector's digits and X3's are never alive together
   const size_t v1 = h.dig1 ? dg_bytes(1, h.c, h.n1, h.cl) : 0, v2 = h.dig2 ? dg_bytes(0, h.c, h.cl * h.dd, h.k2) : 0;
   h.vdig = b.take(std::max(v1, v2));
+  h.status = h.dig1 || h.dig2 ? static_cast<DgStatus*>(b.take(DG_STATUS_BYTES)) : nullptr;
   h.total = b.off;
   return h;
 }
@@ -108,9 +110,9 @@ int heff64_prepare(const dmrg_heff_t& o, void* work, cudaStream_t s) {
     DMRG_TRY(mpo_list_build<T>(h.mpo, static_cast<const T*>(o.W1), static_cast<const T*>(o.W2), h.list, s));
   const TGemm gl = gemm_l<T>(o, h), gr = gemm_r<T>(h);
   const DgOperand l{o.L, gl.M, gl.K, gl.a_m, gl.a_k, 0}, r{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0};
-  if (h.dig1 && h.dig2) return dg_split2<T>(l, h.ldig, r, h.rdig, s);
-  if (h.dig1) return dg_split<T>(0, l, h.ldig, s);
-  if (h.dig2) return dg_split<T>(1, r, h.rdig, s);
+  if (h.dig1 && h.dig2) return dg_split2<T>(l, h.ldig, r, h.rdig, h.status, s);
+  if (h.dig1) return dg_split<T>(0, l, h.ldig, h.status, s);
+  if (h.dig2) return dg_split<T>(1, r, h.rdig, h.status, s);
   return DMRG_OK;
 }
 
@@ -121,17 +123,24 @@ int heff64_run(const dmrg_heff_t& o, const T* x, T* y, void* work, cudaStream_t 
   T* x3 = static_cast<T*>(h.x3);
   const TGemm gl = gemm_l<T>(o, h), gr = gemm_r<T>(h);
   if (h.dig1) {
-    DMRG_TRY(dg_split<T>(1, DgOperand{x, gl.N, gl.K, gl.b_n, gl.b_k, 0}, h.vdig, s));
-    DMRG_TRY(dg_gemm<T>(h.ldig, h.vdig, h.cl * o.wl, h.n1, h.cl, DgOut{x1, gl.M, gl.N, gl.c_m, gl.c_n, 1.0, 0}, s));
+    DMRG_TRY(dg_split<T>(1, DgOperand{x, gl.N, gl.K, gl.b_n, gl.b_k, 0}, h.vdig, nullptr, s));
+    DMRG_TRY(dg_gemm<T>(h.ldig, h.vdig, h.cl * o.wl, h.n1, h.cl, DgOut{x1, gl.M, gl.N, gl.c_m, gl.c_n, 1.0, 0},
+                        h.status, s));
   } else {
     DMRG_TRY(plain<T>(gl, static_cast<const T*>(o.L), x, x1, s));
   }
   if (o.kind != 0) DMRG_TRY(mpo_apply<T>(h.mpo, h.list, x1, x3, h.cl, h.cr, s));
   if (h.dig2) {
-    DMRG_TRY(dg_split<T>(0, DgOperand{x3, gr.M, gr.K, gr.a_m, gr.a_k, 0}, h.vdig, s));
-    return dg_gemm<T>(h.vdig, h.rdig, h.cl * h.dd, h.cr, h.k2, DgOut{y, gr.M, gr.N, gr.c_m, gr.c_n, 1.0, 0}, s);
+    DMRG_TRY(dg_split<T>(0, DgOperand{x3, gr.M, gr.K, gr.a_m, gr.a_k, 0}, h.vdig, nullptr, s));
+    return dg_gemm<T>(h.vdig, h.rdig, h.cl * h.dd, h.cr, h.k2, DgOut{y, gr.M, gr.N, gr.c_m, gr.c_n, 1.0, 0},
+                      h.status, s);
   }
   return plain<T>(gr, x3, static_cast<const T*>(o.R), y, s);
+}
+
+int heff64_status(const dmrg_heff_t& o, void* work, cudaStream_t s) {
+  const H64 h = plan(o, work);
+  return h.status ? dg_gave_up(h.status, true, s) : DMRG_OK;
 }
 
 // ---------------------------------------------------------------- environments
@@ -233,10 +242,10 @@ int env64(int side, long long clb, long long crb, long long clk, long long crk, 
     return plain<T>(h.g2, B, y2, Enew, s);
   }
   DMRG_TRY(mpo_list_build<T>(h.mpo, W, nullptr, h.list, s));
-  if (h.dig1) DMRG_TRY(dg_product<T>(h.g1, E, A, 1.0, 0, y1, h.dig, s));
+  if (h.dig1) DMRG_TRY(dg_product<T>(h.g1, E, A, 1.0, 0, y1, h.dig, nullptr, s));
   else DMRG_TRY(plain<T>(h.g1, E, A, y1, s));
   DMRG_TRY(mpo_apply<T>(h.mpo, h.list, y1, y2, h.outer, h.inner, s));
-  if (h.dig2) return dg_product<T>(h.g2, B, y2, 1.0, 0, Enew, h.dig, s);
+  if (h.dig2) return dg_product<T>(h.g2, B, y2, 1.0, 0, Enew, h.dig, nullptr, s);
   return plain<T>(h.g2, B, y2, Enew, s);
 }
 

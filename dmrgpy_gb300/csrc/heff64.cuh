@@ -11,6 +11,9 @@ size_t heff64_workspace_bytes(const dmrg_heff_t& o);
 template <typename T> int heff64_prepare(const dmrg_heff_t& o, void* work, cudaStream_t s);
 // y = H_eff x after heff64_prepare on the same workspace.
 template <typename T> int heff64_run(const dmrg_heff_t& o, const T* x, T* y, void* work, cudaStream_t s);
+// DMRG_ERR_TIMEOUT where a wait of the digit products gave up since the
+// prepare (synchronises)
+int heff64_status(const dmrg_heff_t& o, void* work, cudaStream_t s);
 
 // Environment extension with bra B and ket A (equal for an expectation
 // value), sides and shapes as dmrg_env_extend_mixed.  A workspace below

@@ -74,7 +74,8 @@ struct SyevWs {
   int* ident;                // npair
   int* pairs;                // (nb-1) x npair x 2
   int* flag;                 // [0] rotating subproblems in the sweep, [1] those with a large rotation
-  unsigned long long* scale; // max |a_ii| as ordered bits; then two words of the passes
+  unsigned long long* scale; // 16 words: max |a_ii| as ordered bits; words of the passes
+  DgStatus* status;          // of the digit products (word 3 of those)
   double* diag;              // np
   float2* dd;                // np: diagonal of an FP32 run as hi + lo
   int* perm;                 // np
@@ -102,10 +103,11 @@ size_t syev_layout(int n, SyevWs* w, void* base, bool lean) {
   s.pairs = static_cast<int*>(take(sizeof(int) * 2 * (size_t)(nb - 1 > 0 ? nb - 1 : 1) * npair));
   s.flag = static_cast<int*>(take(sizeof(int) * 4));
   s.scale = static_cast<unsigned long long*>(take(16 * sizeof(unsigned long long)));
+  s.status = reinterpret_cast<DgStatus*>(s.scale + 3);
   s.diag = static_cast<double*>(take(sizeof(double) * np));
   s.dd = static_cast<float2*>(take(sizeof(float2) * np));
   s.perm = static_cast<int*>(take(sizeof(int) * np));
-  s.dig_bytes = lean || !dg_pays(false, np, np, np, false) ? 0 : dg_bytes(0, false, np, np) + dg_bytes(1, false, np, np);
+  s.dig_bytes = lean || !dg_pays(false, np, np, np, false) ? 0 : dg_product_bytes(false, np, np, np);
   s.dig = take(s.dig_bytes);
   if (w) *w = s;
   return off;
@@ -810,7 +812,7 @@ int syev_gemm(SyevWs& ws, int tA, int m, int n, int k, const double* A, long lon
   if (!tA) { g.a_m = st(lda); g.a_k = st(1); } else { g.a_m = st(1); g.a_k = st(lda); }
   g.b_k = st(n); g.b_n = st(1);
   g.c_m = st(n); g.c_n = st(1);
-  return fgemm(g, 1.0, A, B, 0, C, ws.dig, ws.dig_bytes, s);
+  return fgemm(g, 1.0, A, B, 0, C, ws.dig, ws.dig_bytes, ws.status, s);
 }
 
 // Sorted eigenvalues to the host and the permutation to the workspace.
@@ -824,6 +826,7 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
   }
   std::vector<double> d(n);
   DMRG_CUDA_TRY(cudaMemcpyAsync(d.data(), ws.diag, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+  if (sizeof(T) == 8 && n > 1 && ws.dig_bytes > 0) DMRG_TRY(dg_gave_up(ws.status, false, s));
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   for (int i = 0; i < n; ++i)
     if (!(d[i] == d[i])) return DMRG_ERR_NAN;
@@ -868,7 +871,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
   unsigned long long* offs = ws.scale + 4;
   int* counts = reinterpret_cast<int*>(ws.scale + 8);
   DMRG_CUDA_TRY(cudaMemsetAsync(offs, 0, 4 * sizeof(unsigned long long), s));
-  DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, sizeof(unsigned long long), s));
+  DMRG_CUDA_TRY(cudaMemsetAsync(norm, 0, 2 * sizeof(unsigned long long), s));   // and the status word
   syev_norm_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(A, lda, n, norm);
   DMRG_CHECK_LAUNCH();
   bool polish = false;   // V diagonalises A but is orthonormal to 1e-12 only

@@ -101,7 +101,10 @@ int dmrg_heff_apply(const dmrg_heff_t* op, const void* x, void* y,
  * op and workspace (the plan-once / replay-per-iteration structure of
  * pyitensor/kernels.py:353-410).  dmrg_heff_status() synchronises the stream
  * and reports a bounded-wait timeout recorded by the tensor-core kernels
- * since the last prepare. */
+ * since the last prepare (FP64: in the last matvec on the workspace).  Krylov
+ * loops and truncations report it themselves.  The other FP64 calls do not
+ * synchronise: a wait that gave up leaves nan in their output, which the next
+ * such loop or truncation reports as a non-finite value. */
 int dmrg_heff_prepare(const dmrg_heff_t* op, void* work, size_t work_bytes, void* stream);
 int dmrg_heff_apply_prepared(const dmrg_heff_t* op, const void* x, void* y,
                              void* work, size_t work_bytes, void* stream);
