@@ -73,7 +73,8 @@ constexpr int DG_SMEM = STAGES * ST_BYTES + 1024 + 256;
 constexpr int DG_THREADS = 320;
 // the 64-bit sums grow by up to 3 2^46 per k: at most 20480 k per launch
 constexpr int MAX_STEPS = 1280;
-constexpr int EXP_BAD = INT_MAX;            // row with a non-finite element
+// in place of the exponent of a row with a nan, or with infinities only
+constexpr int EXP_NAN = INT_MAX, EXP_INF = INT_MAX - 1;
 
 __host__ __device__ constexpr int tile_rows(int side) { return side == 0 ? TM : TN; }
 
@@ -89,8 +90,10 @@ struct SplitArgs {
   long long steps;      // K steps
 };
 
-// |x| exponent field of a double's high word
-__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// high word of |x|: the exponent field in its upper bits; above that of an
+// infinity for a nan (one whose high word is an infinity's is found with those)
+__device__ __forceinline__ int magnitude(double x) { return __double2hiint(x) & 0x7fffffff; }
+constexpr int HI_INF = 0x7ff00000;
 
 // Q = rint(x 2^(63 - e)) for a row whose largest exponent field is E
 // (E >= 1, e = E - 1022), |Q| < 2^63
@@ -179,23 +182,23 @@ __device__ __forceinline__ void split8(const SplitArgs& a, int* __restrict__ exp
   const long long row = (long long)block * 8 + rl;
   const long long cols = a.steps * 2;            // 8-wide k columns (padded)
   const bool live = row < a.R;
-  int E = 0;
+  int most_hi = 0;
   if (live)
     for (long long c = kt; c * 8 < a.K; c += 32) {
       double v[8];
       load8<CPLX>(a, row, c * 8, v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) E = max(E, expo(v[j]));
+      for (int j = 0; j < 8; ++j) most_hi = max(most_hi, magnitude(v[j]));
     }
-  E = max(E, __shfl_xor_sync(0xffffffffu, E, 8));
-  E = max(E, __shfl_xor_sync(0xffffffffu, E, 16));
-  if ((tid & 31) < 8) sh[tid >> 5][rl] = E;
+  most_hi = max(most_hi, __shfl_xor_sync(0xffffffffu, most_hi, 8));
+  most_hi = max(most_hi, __shfl_xor_sync(0xffffffffu, most_hi, 16));
+  if ((tid & 31) < 8) sh[tid >> 5][rl] = most_hi;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 8; ++w) E = max(E, sh[w][rl]);
-  const bool bad = E == 0x7ff;
-  if (E < 1) E = 1;
-  if (kt == 0) exps[row] = bad ? EXP_BAD : E - 1022;
+  for (int w = 0; w < 8; ++w) most_hi = max(most_hi, sh[w][rl]);
+  const bool bad = most_hi >= HI_INF;
+  const int E = max(most_hi >> 20, 1);
+  if (kt == 0) exps[row] = most_hi > HI_INF ? EXP_NAN : bad ? EXP_INF : E - 1022;
   // block (row tile, K step): [kc][digit][row][16 bytes]
   const long long tile = row / R;
   const int rt = (int)(row - tile * R);
@@ -324,6 +327,7 @@ struct GArgs {
   int cplx_;
   int negate, accumulate;
   int* err;             // status word
+  SplitArgs opA, opB;   // the operands themselves, for rows with infinities
 };
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -494,16 +498,55 @@ __device__ __forceinline__ void drain_run(uint32_t lane_addr, int* h0, long long
   }
 }
 
+// element k of an operand's (real) row
+__device__ __forceinline__ double operand_at(const SplitArgs& a, bool cplx_, int side, long long row, long long k) {
+  if (!cplx_) return a.p[(row / a.R2) * a.r1 + (row % a.R2) * a.r2 + (k / a.K2) * a.k1 + (k % a.K2) * a.k2];
+  const long long el = side == 0 ? row >> 1 : row, kc = k >> 1;
+  const double* q = a.p + 2 * ((el / a.R2) * a.r1 + (el % a.R2) * a.r2 + (kc / a.K2) * a.k1 + (kc % a.K2) * a.k2);
+  const double re = q[0], im = a.conj ? -q[1] : q[1];
+  // N side: (re, im); M side: (re, -im) in the real part's row, (im, re) in the other
+  if (side == 1) return k & 1 ? im : re;
+  if (row & 1) return k & 1 ? re : im;
+  return k & 1 ? -im : re;
+}
+
+// Row gm of A against columns gn .. gn + n - 1 of B, of which the row or some
+// columns hold infinities: the sum of the products those take part in, which
+// decides the result (an infinity, or nan where they cancel or meet a zero),
+// as the plain sum does.  Reads the operands, the row once per four columns;
+// finite input never comes here.
+__device__ __noinline__ void infinite_row(const GArgs& a, int gm, int gn, int n, bool row_inf, double* s) {
+  const long long K = a.opA.K;
+  for (int j = 0; j < n; ++j) s[j] = 0.0;
+  if (row_inf) {
+#pragma unroll 4
+    for (long long k = 0; k < K; ++k) {
+      const double v = operand_at(a.opA, a.cplx_, 0, gm, k);
+      if (magnitude(v) < HI_INF) continue;
+      for (int j = 0; j < n; ++j) s[j] += v * operand_at(a.opB, a.cplx_, 1, gn + j, k);
+    }
+  }
+  for (int j = 0; j < n; ++j) {
+    if (a.eB[gn + j] != EXP_INF) continue;
+#pragma unroll 4
+    for (long long k = 0; k < K; ++k) {
+      const double u = operand_at(a.opB, a.cplx_, 1, gn + j, k);
+      if (magnitude(u) >= HI_INF) s[j] += operand_at(a.opA, a.cplx_, 0, gm, k) * u;
+    }
+  }
+}
+
 // where a row of C goes
 struct RowOut {
   bool live, vec;
-  int ea, es;
+  int gm, ea, es;
   double* pc;
 };
 
 __device__ __forceinline__ RowOut row_out(const GArgs& a, int gm, int n0, int width) {
   RowOut o;
   o.live = gm < a.M;
+  o.gm = gm;
   o.ea = o.live ? a.eA[gm] : 0;
   const int el = a.cplx_ ? gm >> 1 : gm;
   o.es = a.cplx_ ? 2 : 1;
@@ -524,14 +567,23 @@ __device__ __forceinline__ void store4(const GArgs& a, const RowOut& o, int gn, 
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int eb = __shfl_sync(0xffffffffu, ebl, c + j);
-    odd = odd || o.ea == EXP_BAD || eb == EXP_BAD;
+    odd = odd || o.ea >= EXP_INF || eb >= EXP_INF;
     r[j] = assemble(h[j], m[j], o.ea + eb + 2, a.negate, &odd);
   }
   if (__any_sync(0xffffffffu, odd)) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    bool inf = o.ea == EXP_INF;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int eb = __shfl_sync(0xffffffffu, ebl, c + j);
-      if (!ok || o.ea == EXP_BAD || eb == EXP_BAD) r[j] = __longlong_as_double(0x7ff8000000000000ll);
+      inf = inf || eb == EXP_INF;
+    }
+    if (inf && ok && o.live && o.ea != EXP_NAN) infinite_row(a, o.gm, gn, min(4, a.N - gn), o.ea == EXP_INF, s);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int eb = __shfl_sync(0xffffffffu, ebl, c + j);
+      if (!ok || o.ea == EXP_NAN || eb == EXP_NAN) r[j] = __longlong_as_double(0x7ff8000000000000ll);
+      else if (o.ea == EXP_INF || eb == EXP_INF) r[j] = a.negate ? -s[j] : s[j];
       else r[j] = assemble_edge(h[j], m[j], o.ea + eb + 2, a.negate);
     }
   }
@@ -551,7 +603,7 @@ __device__ __forceinline__ void store4(const GArgs& a, const RowOut& o, int gn, 
   }
 }
 
-__global__ void __launch_bounds__(DG_THREADS, 1) dg_gemm_kernel(const GArgs a) {
+__global__ void __launch_bounds__(DG_THREADS, 1) dg_gemm_kernel(const __grid_constant__ GArgs a) {
   int* const err = a.err;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
@@ -721,7 +773,7 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank) {
 }
 
 template <int SK>
-__global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(SK, 1, 1) dg_splitk_kernel(const GArgs a) {
+__global__ void __launch_bounds__(DG_THREADS, 1) __cluster_dims__(SK, 1, 1) dg_splitk_kernel(const __grid_constant__ GArgs a) {
   constexpr int CN = TN / SK;            // columns a CTA finishes
   // exchange area: sums of [source][column][row], 8 then 4 bytes each, then a flag per source
   constexpr int XM = SK * CN * TM * 8, XH = SK * CN * TM * 4;
@@ -920,11 +972,11 @@ size_t dg_bytes(int side, bool cplx_, long long rows, long long K) {
 }
 
 template <typename T>
-static int split_job(int side, const DgOperand& o, void* buf, SplitJob* job) {
+static int operand_args(int side, const DgOperand& o, SplitArgs* out) {
   constexpr bool C = sizeof(T) == 16;
-  SplitArgs& a = job->a;
+  SplitArgs& a = *out;
   const long long rows = (long long)o.rows.n1 * o.rows.n2, K = (long long)o.K.n1 * o.K.n2;
-  if (rows < 1 || K < 1 || !o.p || !buf) return DMRG_ERR_ARG;
+  if (rows < 1 || K < 1 || !o.p) return DMRG_ERR_ARG;
   a.p = static_cast<const double*>(o.p);
   a.R = real_rows(side, C, rows);
   a.K = C ? 2 * K : K;
@@ -935,6 +987,14 @@ static int split_job(int side, const DgOperand& o, void* buf, SplitJob* job) {
   const long long kin = a.K2 == 1 ? a.k1 : (a.k1 == a.k2 * a.K2 ? a.k2 : 0);
   a.kvec = !C && kin == 1 && (reinterpret_cast<uintptr_t>(o.p) & 15) == 0 && a.r1 % 2 == 0 &&
            (a.R2 == 1 || a.r2 % 2 == 0);
+  return DMRG_OK;
+}
+
+template <typename T>
+static int split_job(int side, const DgOperand& o, void* buf, SplitJob* job) {
+  const SplitArgs& a = job->a;
+  if (!buf) return DMRG_ERR_ARG;
+  DMRG_TRY(operand_args<T>(side, o, &job->a));
   const int tr = tile_rows(side);
   const long long Rp = up(a.R, tr) * tr;
   if (Rp / 8 > 0x7fffffffLL) return DMRG_ERR_ARG;
@@ -974,14 +1034,18 @@ int dg_split2(const DgOperand& A, void* bufa, const DgOperand& B, void* bufb, Dg
 }
 
 template <typename T>
-int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long long K, const DgOut& out,
+int dg_gemm(const DgOperand& A, const void* Adig, const DgOperand& B, const void* Bdig, const DgOut& out,
             DgStatus* st, cudaStream_t s) {
   constexpr bool C = sizeof(T) == 16;
+  const long long M = (long long)A.rows.n1 * A.rows.n2, N = (long long)B.rows.n1 * B.rows.n2;
+  const long long K = (long long)A.K.n1 * A.K.n2;
   if (M < 1 || N < 1 || K < 1 || !Adig || !Bdig || !out.C || !st) return DMRG_ERR_ARG;
   const long long Mr = C ? 2 * M : M, Kr = C ? 2 * K : K;
   const long long tm = up(Mr, TM), tn = up(N, TN);
   if (Mr > 0x7fffffffLL || N > 0x7fffffffLL || tm * tn > 0x7fffffffLL) return DMRG_ERR_ARG;
   GArgs a;
+  DMRG_TRY(operand_args<T>(0, A, &a.opA));
+  DMRG_TRY(operand_args<T>(1, B, &a.opB));
   a.eA = static_cast<const int*>(Adig);
   a.eB = static_cast<const int*>(Bdig);
   a.sqA = reinterpret_cast<const int*>(static_cast<const char*>(Adig) + exps_bytes(0, Mr));
@@ -1055,13 +1119,13 @@ int dg_gave_up(const DgStatus* st, bool marked, cudaStream_t s) {
 template <typename T>
 int dg_product(const TGemm& g, const T* A, const T* B, double alpha, int accumulate, T* C, void* work,
                DgStatus* st, cudaStream_t s) {
-  const long long M = (long long)g.M.n1 * g.M.n2, N = (long long)g.N.n1 * g.N.n2, K = (long long)g.K.n1 * g.K.n2;
+  const long long M = (long long)g.M.n1 * g.M.n2, K = (long long)g.K.n1 * g.K.n2;
   DgStatus* own = static_cast<DgStatus*>(work);
   void* da = static_cast<char*>(work) + DG_STATUS_BYTES;
   void* db = static_cast<char*>(da) + dg_bytes(0, sizeof(T) == 16, M, K);
-  DMRG_TRY(dg_split2<T>(DgOperand{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, da,
-                        DgOperand{B, g.N, g.K, g.b_n, g.b_k, g.conjB}, db, st ? nullptr : own, s));
-  return dg_gemm<T>(da, db, M, N, K, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, st ? st : own, s);
+  const DgOperand a{A, g.M, g.K, g.a_m, g.a_k, g.conjA}, b{B, g.N, g.K, g.b_n, g.b_k, g.conjB};
+  DMRG_TRY(dg_split2<T>(a, da, b, db, st ? nullptr : own, s));
+  return dg_gemm<T>(a, da, b, db, DgOut{C, g.M, g.N, g.c_m, g.c_n, alpha, accumulate}, st ? st : own, s);
 }
 
 int fgemm(const TGemm& g, double alpha, const double* A, const double* B, int accumulate, double* C, void* ws,
@@ -1083,9 +1147,9 @@ template int dg_split<double>(int, const DgOperand&, void*, DgStatus*, cudaStrea
 template int dg_split<cplx>(int, const DgOperand&, void*, DgStatus*, cudaStream_t);
 template int dg_split2<double>(const DgOperand&, void*, const DgOperand&, void*, DgStatus*, cudaStream_t);
 template int dg_split2<cplx>(const DgOperand&, void*, const DgOperand&, void*, DgStatus*, cudaStream_t);
-template int dg_gemm<double>(const void*, const void*, long long, long long, long long, const DgOut&, DgStatus*,
+template int dg_gemm<double>(const DgOperand&, const void*, const DgOperand&, const void*, const DgOut&, DgStatus*,
                              cudaStream_t);
-template int dg_gemm<cplx>(const void*, const void*, long long, long long, long long, const DgOut&, DgStatus*,
+template int dg_gemm<cplx>(const DgOperand&, const void*, const DgOperand&, const void*, const DgOut&, DgStatus*,
                            cudaStream_t);
 
 }  // namespace dmrg

@@ -43,8 +43,9 @@ struct DgOut {
   double alpha;
   int accumulate;
 };
+// (the operands themselves are read only for rows and columns with infinities)
 template <typename T>
-int dg_gemm(const void* Adig, const void* Bdig, long long M, long long N, long long K, const DgOut& out,
+int dg_gemm(const DgOperand& A, const void* Adig, const DgOperand& B, const void* Bdig, const DgOut& out,
             DgStatus* st, cudaStream_t s);
 // whether the digit product of this shape is faster than the FP64 pipe
 // (one_split: the other operand's digits are kept from an earlier call)

@@ -123,17 +123,17 @@ int heff64_run(const dmrg_heff_t& o, const T* x, T* y, void* work, cudaStream_t 
   T* x3 = static_cast<T*>(h.x3);
   const TGemm gl = gemm_l<T>(o, h), gr = gemm_r<T>(h);
   if (h.dig1) {
-    DMRG_TRY(dg_split<T>(1, DgOperand{x, gl.N, gl.K, gl.b_n, gl.b_k, 0}, h.vdig, nullptr, s));
-    DMRG_TRY(dg_gemm<T>(h.ldig, h.vdig, h.cl * o.wl, h.n1, h.cl, DgOut{x1, gl.M, gl.N, gl.c_m, gl.c_n, 1.0, 0},
-                        h.status, s));
+    const DgOperand l{o.L, gl.M, gl.K, gl.a_m, gl.a_k, 0}, v{x, gl.N, gl.K, gl.b_n, gl.b_k, 0};
+    DMRG_TRY(dg_split<T>(1, v, h.vdig, nullptr, s));
+    DMRG_TRY(dg_gemm<T>(l, h.ldig, v, h.vdig, DgOut{x1, gl.M, gl.N, gl.c_m, gl.c_n, 1.0, 0}, h.status, s));
   } else {
     DMRG_TRY(plain<T>(gl, static_cast<const T*>(o.L), x, x1, s));
   }
   if (o.kind != 0) DMRG_TRY(mpo_apply<T>(h.mpo, h.list, x1, x3, h.cl, h.cr, s));
   if (h.dig2) {
-    DMRG_TRY(dg_split<T>(0, DgOperand{x3, gr.M, gr.K, gr.a_m, gr.a_k, 0}, h.vdig, nullptr, s));
-    return dg_gemm<T>(h.vdig, h.rdig, h.cl * h.dd, h.cr, h.k2, DgOut{y, gr.M, gr.N, gr.c_m, gr.c_n, 1.0, 0},
-                      h.status, s);
+    const DgOperand v{x3, gr.M, gr.K, gr.a_m, gr.a_k, 0}, r{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0};
+    DMRG_TRY(dg_split<T>(0, v, h.vdig, nullptr, s));
+    return dg_gemm<T>(v, h.vdig, r, h.rdig, DgOut{y, gr.M, gr.N, gr.c_m, gr.c_n, 1.0, 0}, h.status, s);
   }
   return plain<T>(gr, x3, static_cast<const T*>(o.R), y, s);
 }
