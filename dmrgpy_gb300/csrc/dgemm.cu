@@ -16,11 +16,17 @@
 // rounding of Q (2^-64 of the row's largest element), the digit pairs left
 // out (i + j > 7: together about 2^-64 of both rows' largest elements per
 // product), the run's last place (2^-63 of both rows' largest elements) and
-// that final rounding.  Rows of a sweep mix magnitudes (Schmidt-weighted
-// tensors; an environment's energy channel beside its small entries), which
-// a fixed point pays for and FP64 does not: with seven digits a chi = 1024
-// matvec erred by 4e-15 (28 pairs: 4e-14) where the FP64 sum errs by 2e-15,
-// with eight by less than the FP64 sum (tests/test_gpu_dgemm.py).
+// that final rounding.  The bound is one by norms: of max|row of A| max|row of
+// B|, not of the products themselves.  Rows of a sweep mix magnitudes
+// (Schmidt-weighted tensors; an environment's energy channel beside its small
+// entries), which a fixed point pays for and FP64 does not: with seven digits
+// a chi = 1024 matvec erred by 4e-15 (28 pairs: 4e-14) and with eight by
+// 1.8e-15, where the FP64 pipe's sums err by 2.0e-15 (against a contraction in
+// 64 bits, relative to the largest output).  Where large elements of a row
+// meet zeros or far smaller ones, though, an element below 2^-11 of its row's
+// largest is held to fewer than 53 bits and one below 2^-64 not at all; the
+// FP64 pipe, which a caller gets by passing less workspace, keeps
+// K 2^-53 sum |a||b| there (tests/test_gpu_digit_bounds.py has both).
 //
 // Why: GB300's FP64 pipe does 2 FMA per clock per SM (1.06 TFLOP/s measured),
 // the FP16 tensor cores 4096; 36 digit products still leave a factor ~55.

@@ -84,8 +84,17 @@ unsigned long long dmrg_kernel_launches(void);
 /* ---- effective-Hamiltonian matvec ------------------------------------- */
 /* Workspace for dmrg_heff_apply (also covers the operand preparation).  An
  * FP64 operator also runs in the two intermediates of its contraction chain
- * alone, without the operands of the tensor-core digit products: slower,
- * same accuracy class; below that DMRG_ERR_WORKSPACE. */
+ * alone, without the operands of the tensor-core digit products: slower, and
+ * with the error bound of plain FP64 sums; below that DMRG_ERR_WORKSPACE.
+ *
+ * Error of an FP64 contraction of K products: on the FP64 pipe K 2^-53
+ * sum |a||b|.  As a digit product (dmrg_gemm, matvecs, environments and
+ * truncations of large bonds, given the workspace they ask for)
+ * 2^-53 |c| + (K + 128) 2^-58 max|row of A| max|column of B|, which is the smaller
+ * one for rows and columns of like magnitudes, but not where large elements
+ * meet zeros or far smaller ones.  Data of that kind gets the other bound
+ * with less workspace: none for dmrg_gemm, the two intermediates for matvecs,
+ * environments and Krylov loops. */
 size_t dmrg_heff_workspace_bytes(const dmrg_heff_t* op);
 /* y = H_eff x.  Replaces the matvec closure of pyitensor/kernels.py:353-410
  * (_make_matvec_planned) built by pyitensor/dmrg.py:224-299.  x and y must
@@ -393,7 +402,8 @@ int dmrg_wait_timeout_probe(void* work, size_t work_bytes, void* stream);
 /* ---- dense contraction ---------------------------------------------------- */
 size_t dmrg_gemm_workspace_bytes(int dtype, int precision, int m, int k, int n);
 /* (FP64 products need none: with the workspace they run as digit products on
- * the tensor cores where that is faster, without it on the FP64 pipe.) */
+ * the tensor cores where that is faster, without it on the FP64 pipe; the
+ * error bounds of both stand at dmrg_heff_workspace_bytes.) */
 /* C (m x n) = A (m x k) . B (k x n), all row-major.  Used for the two-site
  * merge theta = A_i . A_{i+1} (pyitensor/dmrg.py:233, Ti * Tj) and for the
  * bond-matrix absorption of one-site TDVP (pyitensor/tdvp.py:300-313). */
