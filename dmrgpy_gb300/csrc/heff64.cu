@@ -8,6 +8,8 @@
 //
 //   kind 2  X1[(a',k)][(s,t,b)] = L[(a',k)][a] x[a][(s,t,b)]
 //           X3[(a',s',t')][(n,b)] = sum_{k,s,t} W12 X1
+//             or (wide MPOs, combined_pays) X2[a'][(s',m)][(t,b)] = W1 X1,
+//             X3[(a',s')][(t',n)][b] = W2 X2
 //           y[(a',s',t')][b'] = X3[(a',s',t')][(n,b)] R[b'][(n,b)]
 //   kind 1  the same with one site; kind 0 without the MPO step
 //   left    Y1[(a',k)][(s,b)] = L A;  Y2[a'][(s',m)][b] = W Y1;
@@ -41,11 +43,32 @@ struct H64 {
   long long cl, cr, dd;      // dd: physical legs of x (d1 d2, d1 or 1)
   long long n1, k2;          // columns of X1 per row, contracted length with R
   bool dig1, dig2;
-  MpoShape mpo;
-  void *x1, *x3, *list, *ldig, *rdig, *vdig;
+  bool two;                  // one MPO step per site instead of one per bond
+  MpoShape mpo, mpo2;
+  void *x1, *x2, *x3, *list, *list2, *ldig, *rdig, *vdig;
   DgStatus* status;          // where dig1 or dig2
   size_t total;
 };
+
+// Whether a bond's MPO step goes over the product of its two site tensors, in
+// one pass, rather than over one after the other.  The product of sparse
+// tensors is the quicker (S=1 Heisenberg: 90 non-zeros against 156 products in
+// the two steps, and a pass less), but a dense one has (d1 d2)^2 wl wr elements
+// where the two steps take d1^2 wl wm d2 + d2^2 wm wr d1 products, and forming
+// it takes wm products an element for each operator.  The tensors are known to
+// the device alone, so sizes decide: one pass where even a dense product is no
+// more work, or of at most COMBINED_MOST elements.  Measured, one pass and two,
+// us: dense, chi = 64: d = 4, w = 8 (16k elements) 222 and, with the strided plan
+// that a small workspace gets, 255; w = 11 (31k) 396 and 209; d = 8, w = 4 752
+// and 194; d = 4, w = 32 4220 and 1276; chi = 8, d = 4, w = 32 3850 and 119.
+// Sums of exponentials (three channels each), chi = 250: d = 4, w = 11 525 and
+// 575, d = 3, w = 17 516 and 538.
+constexpr long long COMBINED_MOST = 1 << 14;
+bool combined_pays(const dmrg_heff_t& o) {
+  const long long d1 = o.d1, d2 = o.d2, wl = o.wl, wm = o.wm, wr = o.wr;
+  const long long one = d1 * d2 * d1 * d2 * wl * wr, two = d1 * wm * d2 * (d1 * wl + d2 * wr);
+  return one <= two || one <= COMBINED_MOST;
+}
 
 H64 plan(const dmrg_heff_t& o, void* work) {
   H64 h{};
@@ -56,21 +79,28 @@ H64 plan(const dmrg_heff_t& o, void* work) {
   h.k2 = (long long)o.wr * h.cr;
   h.dig1 = dg_pays(h.c, h.cl * o.wl, h.n1, h.cl, true);
   h.dig2 = dg_pays(h.c, h.cl * h.dd, h.cr, h.k2, true);
-  h.mpo = MpoShape{o.kind == 2 ? MPO_TWO : MPO_LEFT, o.d1, o.kind == 2 ? o.d2 : 1, o.wl, o.kind == 2 ? o.wm : 1, o.wr};
+  h.two = o.kind == 2 && !combined_pays(o);
+  h.mpo = h.two           ? MpoShape{MPO_LEFT, o.d1, 1, o.wl, 1, o.wm}
+          : o.kind == 2   ? MpoShape{MPO_TWO, o.d1, o.d2, o.wl, o.wm, o.wr}
+                          : MpoShape{MPO_LEFT, o.d1, 1, o.wl, 1, o.wr};
+  h.mpo2 = MpoShape{MPO_LEFT, o.d2, 1, o.wm, 1, o.wr};
   Bump b{static_cast<char*>(work), 0};
   const size_t e = esz(h.c);
   h.x1 = b.take(e * (size_t)(h.cl * o.wl * h.n1));
   if (o.kind != 0) {
     h.x3 = b.take(e * (size_t)(h.cl * h.dd * h.k2));
     h.list = b.take(mpo_list_bytes(h.mpo, e));
+    if (h.two) h.list2 = b.take(mpo_list_bytes(h.mpo2, e));
   } else {
     h.x3 = h.x1;
   }
   if (h.dig1) h.ldig = b.take(dg_bytes(0, h.c, h.cl * o.wl, h.cl));
   if (h.dig2) h.rdig = b.take(dg_bytes(1, h.c, h.cr, h.k2));
-  // the vector's digits and X3's are never alive together
+  // of the vector's digits, X2 and X3's digits no two are alive together
   const size_t v1 = h.dig1 ? dg_bytes(1, h.c, h.n1, h.cl) : 0, v2 = h.dig2 ? dg_bytes(0, h.c, h.cl * h.dd, h.k2) : 0;
-  h.vdig = b.take(std::max(v1, v2));
+  const size_t m = h.two ? e * (size_t)(h.cl * o.wm * h.n1) : 0;
+  h.vdig = b.take(std::max(std::max(v1, v2), m));
+  h.x2 = h.vdig;
   h.status = h.dig1 || h.dig2 ? static_cast<DgStatus*>(b.take(DG_STATUS_BYTES)) : nullptr;
   h.total = b.off;
   return h;
@@ -108,6 +138,7 @@ int heff64_prepare(const dmrg_heff_t& o, void* work, cudaStream_t s) {
   const H64 h = plan(o, work);
   if (o.kind != 0)
     DMRG_TRY(mpo_list_build<T>(h.mpo, static_cast<const T*>(o.W1), static_cast<const T*>(o.W2), h.list, s));
+  if (h.two) DMRG_TRY(mpo_list_build<T>(h.mpo2, static_cast<const T*>(o.W2), nullptr, h.list2, s));
   const TGemm gl = gemm_l<T>(o, h), gr = gemm_r<T>(h);
   const DgOperand l{o.L, gl.M, gl.K, gl.a_m, gl.a_k, 0}, r{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0};
   if (h.dig1 && h.dig2) return dg_split2<T>(l, h.ldig, r, h.rdig, h.status, s);
@@ -129,7 +160,12 @@ int heff64_run(const dmrg_heff_t& o, const T* x, T* y, void* work, cudaStream_t 
   } else {
     DMRG_TRY(plain<T>(gl, static_cast<const T*>(o.L), x, x1, s));
   }
-  if (o.kind != 0) DMRG_TRY(mpo_apply<T>(h.mpo, h.list, x1, x3, h.cl, h.cr, s));
+  if (h.two) {
+    DMRG_TRY(mpo_apply<T>(h.mpo, h.list, x1, static_cast<T*>(h.x2), h.cl, o.d2 * h.cr, s));
+    DMRG_TRY(mpo_apply<T>(h.mpo2, h.list2, static_cast<const T*>(h.x2), x3, h.cl * o.d1, h.cr, s));
+  } else if (o.kind != 0) {
+    DMRG_TRY(mpo_apply<T>(h.mpo, h.list, x1, x3, h.cl, h.cr, s));
+  }
   if (h.dig2) {
     const DgOperand v{x3, gr.M, gr.K, gr.a_m, gr.a_k, 0}, r{o.R, gr.N, gr.K, gr.b_n, gr.b_k, 0};
     DMRG_TRY(dg_split<T>(0, v, h.vdig, nullptr, s));

@@ -1,13 +1,13 @@
-// MPO steps of the FP64 contractions: the site tensors (for a bond, their
-// product over the shared link) applied to the physical and MPO legs of an
-// intermediate.
+// MPO steps of the FP64 contractions: a site tensor (for a bond of a narrow MPO
+// the product of both over the shared link, heff64.cu) applied to the physical
+// and MPO legs of an intermediate.
 //
 // A Hamiltonian's MPO tensors are mostly zeros (the two-site operator of the
-// S=1 Heisenberg chain has about 110 non-zeros in 45 x 45), and GB300's FP64
+// S=1 Heisenberg chain has 90 non-zeros in 45 x 45), and GB300's FP64
 // pipe (2 FMA per clock per SM) is what a dense step is bound by, so the
 // non-zeros are listed per output row once per operator and only they are
-// multiplied.  A dense tensor (a compressed long-range MPO) gives full
-// lists and the same work as a dense step.
+// multiplied.  A dense tensor (a compressed long-range MPO) gives full lists:
+// for one site the same products as a dense step.
 //
 // Apply: a warp owns 32 consecutive inner indices (one bond leg) of one outer
 // index and every eighth output row; the lists are read as warp
