@@ -302,7 +302,10 @@ int batch_lanczos(int nprob, const dmrg_heff_t* ops, void* const* x, int kmax, d
     pl.gtab[k] = base + L.gemm_tab[k];
     key += ":" + std::to_string(pl.gn[k]) + "/" + std::to_string(pl.gtiles[k]) + "x" + std::to_string(pl.gtile[k]);
   }
-  key += ":" + std::to_string(nmax);
+  // the steps carry the tolerance (their breakdown test) as an argument
+  unsigned long long tol_bits;
+  std::memcpy(&tol_bits, &tol, sizeof(tol_bits));
+  key += ":" + std::to_string(nmax) + ":" + std::to_string(tol_bits);
   DMRG_CUDA_TRY(cudaMemcpyAsync(base + L.seg_tab, seg.data(), sizeof(LSeg<T>) * nprob, cudaMemcpyHostToDevice, s));
   lz_init_kernel<T><<<nprob, kVecThreads, 0, s>>>(pl.seg);
   DMRG_CHECK_LAUNCH();
