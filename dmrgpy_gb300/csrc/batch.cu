@@ -8,7 +8,8 @@
 //     tile table), built from the same step plans as the single-chain path;
 //   * Lanczos: the recurrence runs for all chains in lock step; the vector
 //     work of a step (dot, axpy, reorthogonalisation, norm, next vector) is
-//     one launch, a cluster of eight CTAs per chain; blocks of kBlock steps are captured once as a CUDA graph
+//     one launch, a cluster of eight CTAs per chain (four launches for a few
+//     long vectors); blocks of kBlock steps are captured once as a CUDA graph
 //     and replayed (the graph is cached per shape signature, so the same bond
 //     of the next sweep replays it); only alpha/beta of all chains cross to
 //     the host after each block, where each chain's tridiagonal problem and
@@ -17,6 +18,7 @@
 //     reference's truncation rule per chain on the host.
 // FP64 / complex FP64 throughout (the bond dimensions of such batches are
 // small enough that the FP64 pipe is not the limit).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -111,6 +113,89 @@ lz_step_kernel(const LSeg<T>* __restrict__ tab, int j, int ldh, double tol) {
   }
 }
 
+// The same step in four launches, the reorthogonalisation over all SMs, where
+// a few long problems leave most of them idle (lz_wide): alpha and the three-term
+// update by a cluster per problem,
+template <typename T>
+__global__ void __launch_bounds__(LZ_THREADS) __cluster_dims__(LZ_CTAS, 1, 1)
+lz_alpha_kernel(const LSeg<T>* __restrict__ tab, int j) {
+  __shared__ LzShared sh;
+  const LSeg<T> a = tab[blockIdx.x / LZ_CTAS];
+  const double bp = j > 0 ? *((volatile double*)a.beta + j - 1) : 0.0;
+  double are, aim;
+  lz_cluster_alpha<T>(LzSlice(a.n), sh, a.Q, a.w, a.n, j, bp, are, aim);
+  if (blockIdx.x % LZ_CTAS == 0 && threadIdx.x == 0) a.alpha[j] = are;
+  lz_cluster_sync();   // the others have read this CTA's sums
+}
+
+// h_i = <q_i, w> for i < j, a part of the vector per CTA: row `part` of h;
+// grid (parts, j, nprob),
+template <typename T>
+__global__ void __launch_bounds__(256) lz_dots_kernel(const LSeg<T>* __restrict__ tab, int ldh) {
+  __shared__ double red[32];
+  const LSeg<T> a = tab[blockIdx.z];
+  const int i = blockIdx.y;
+  const T* q = a.Q + (long long)i * a.n;
+  const long long len = (a.n + gridDim.x - 1) / gridDim.x, lo = blockIdx.x * len, hi = lo + len < a.n ? lo + len : a.n;
+  double re = 0.0, im = 0.0;
+#pragma unroll 4
+  for (long long e = lo + threadIdx.x; e < hi; e += 256) {
+    const T c = Sc<T>::mul(Sc<T>::conj(q[e]), a.w[e]);
+    re += Sc<T>::re(c);
+    if (sizeof(T) == 16) im += Sc<T>::im(c);
+  }
+  re = block_sum<T>(re, red);
+  if (sizeof(T) == 16) im = block_sum<T>(im, red);
+  if (threadIdx.x == 0) a.h[(long long)blockIdx.x * ldh + i] = Sc<T>::make(re, im);
+}
+
+// w -= sum_{i<j} h_i q_i; grid (blocks, nprob), h in shared memory,
+template <typename T>
+__global__ void __launch_bounds__(256) lz_update_kernel(const LSeg<T>* __restrict__ tab, int j, int parts, int ldh) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* hs = reinterpret_cast<T*>(smem_raw);
+  const LSeg<T> a = tab[blockIdx.y];
+  for (int i = threadIdx.x; i < j; i += 256) {
+    T s = Sc<T>::zero();
+    for (int r = 0; r < parts; ++r) s = Sc<T>::add(s, a.h[(long long)r * ldh + i]);
+    hs[i] = s;
+  }
+  __syncthreads();
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < a.n; e += (long long)gridDim.x * 256) {
+    T acc = Sc<T>::zero();
+#pragma unroll 4
+    for (int i = 0; i < j; ++i) acc = Sc<T>::fma(a.Q[(long long)i * a.n + e], hs[i], acc);
+    a.w[e] = Sc<T>::sub(a.w[e], acc);
+  }
+}
+
+// beta and the next vector by a cluster per problem.
+template <typename T>
+__global__ void __launch_bounds__(LZ_THREADS) __cluster_dims__(LZ_CTAS, 1, 1)
+lz_next_kernel(const LSeg<T>* __restrict__ tab, int j, double tol) {
+  __shared__ LzShared sh;
+  const LSeg<T> a = tab[blockIdx.x / LZ_CTAS];
+  const LzSlice p(a.n);
+  bool dead = *((volatile int*)a.dead) != 0;
+  double s = 0.0, beta;
+  for (long long e = p.lo + threadIdx.x; e < p.hi; e += LZ_THREADS) s += Sc<T>::abs2(a.w[e]);
+  lz_cluster_next<T>(p, sh, a.Q, a.w, a.v, a.n, j, true, s, tol, dead, beta);
+  if (blockIdx.x % LZ_CTAS == 0 && threadIdx.x == 0) {
+    a.beta[j] = beta;
+    if (dead) *a.dead = 1;
+  }
+}
+
+// Whether step j of a batch takes the four launches: clusters on at most half of
+// the SMs and 2 n j sums a problem that are worth three launches more.  200
+// steps of one problem, one launch a step and four: n = 4096 22.2 -> 19.0 ms,
+// 262144 949 -> 337, 640000 2602 -> 1036; 40 steps, n = 16384, 1, 4 and 8 problems
+// 4.26 -> 3.68, 7.40 -> 7.05, 13.6 -> 13.3; eight of 4096 (below the line), 200
+// steps, 97.9 -> 99.5.
+inline bool lz_wide(int nprob, long long nmax, int j) {
+  return nprob * LZ_CTAS <= 152 / 2 && j <= 2048 && nmax * j >= (1ll << 18) * nprob;
+}
+
 // x = sum_{i<kused} y_i q_i over the kused rows every problem has computed
 // (the host pads y with zeros past each problem's own dimension); grid
 // (blocks, nprob)
@@ -188,6 +273,7 @@ struct LzPlan {
   int gtile[4];
   int nprob;
   int kmax;
+  long long nmax;
   double tol;
 };
 
@@ -198,6 +284,20 @@ int lz_steps(const LzPlan<T>& pl, int j0, int j1, unsigned long long* kernels, c
   for (int j = j0; j < j1; ++j) {
     for (int k = 0; k < 4; ++k)
       DMRG_TRY(tgemm_grouped_launch<T>(pl.gtab[k], pl.gn[k], pl.gtiles[k], pl.gtile[k], Sc<T>::one(), Sc<T>::zero(), s));
+    if (lz_wide(pl.nprob, pl.nmax, j)) {
+      const int ldh = pl.kmax + 1;
+      const int parts = std::min(2 * LZ_CTAS, std::max(1, 2 * 152 / (j * pl.nprob)));   // rows of h
+      lz_alpha_kernel<T><<<pl.nprob * LZ_CTAS, LZ_THREADS, 0, s>>>(pl.seg, j);
+      DMRG_CHECK_LAUNCH();
+      lz_dots_kernel<T><<<dim3((unsigned)parts, (unsigned)j, (unsigned)pl.nprob), 256, 0, s>>>(pl.seg, ldh);
+      DMRG_CHECK_LAUNCH();
+      lz_update_kernel<T><<<dim3((unsigned)(4 * 152 / pl.nprob), (unsigned)pl.nprob), 256, j * sizeof(T), s>>>(
+          pl.seg, j, parts, ldh);
+      DMRG_CHECK_LAUNCH();
+      lz_next_kernel<T><<<pl.nprob * LZ_CTAS, LZ_THREADS, 0, s>>>(pl.seg, j, pl.tol);
+      DMRG_CHECK_LAUNCH();
+      continue;
+    }
     lz_step_kernel<T><<<pl.nprob * LZ_CTAS, LZ_THREADS, 0, s>>>(pl.seg, j, pl.kmax + 1, pl.tol);
     DMRG_CHECK_LAUNCH();
   }
@@ -280,6 +380,7 @@ int batch_lanczos(int nprob, const dmrg_heff_t* ops, void* const* x, int kmax, d
   pl.seg = reinterpret_cast<const LSeg<T>*>(base + L.seg_tab);
   pl.nprob = nprob;
   pl.kmax = kmax;
+  pl.nmax = nmax;
   pl.tol = tol;
   std::vector<char> hdesc(tgemm_grouped_desc_bytes(nprob));
   std::vector<TGemm> g(nprob);

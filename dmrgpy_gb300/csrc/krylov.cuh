@@ -96,36 +96,80 @@ __device__ __forceinline__ void lz_cluster_sum(double& re, double& im, int act, 
   im = all[1];
 }
 
-// alpha = q_j^H w, w -= Re(alpha) q_j + bprev q_(j-1), w -= Q_nq Q_nq^H w,
-// beta = |w|, q_(j+1) = w / beta (next; also into v where given; zero after a
-// breakdown: dead, or beta below tol).  CTA `rank` of the cluster handles an
-// eighth of the vectors.  h: 2 LZ_CTAS rows of ldh elements.  On return dead
-// is set after a breakdown; every CTA has the same scalars, bit for bit.
-// The caller returns right after it.
+// A CTA's part of a vector (an eighth), and the warps that have elements of it.
+struct LzSlice {
+  int rank, act;
+  long long lo, hi;
+  __device__ __forceinline__ explicit LzSlice(long long n) {
+    rank = (int)(blockIdx.x % LZ_CTAS);
+    const long long slice = (n + LZ_CTAS - 1) / LZ_CTAS;
+    lo = rank * slice;
+    hi = lo + slice < n ? lo + slice : n;
+    act = hi - lo >= LZ_THREADS ? LZ_THREADS / 32 : hi > lo ? (int)(hi - lo + 31) / 32 : 1;
+  }
+};
+
+struct LzShared {
+  double red[LZ_THREADS / 32][2];
+  double sums[4][2];
+};
+
+// alpha = q_j^H w, w -= Re(alpha) q_j + bprev q_(j-1)
 template <typename T>
-__device__ __forceinline__ void lz_cluster_step(T* Q, T* w, T* v, long long n, int j, int nq, bool next, double bprev,
-                                                T* h, int ldh, double tol, bool& dead, double& are, double& aim,
-                                                double& beta) {
-  __shared__ double red[LZ_THREADS / 32][2];
-  __shared__ double sums[4][2];
+__device__ __forceinline__ void lz_cluster_alpha(const LzSlice& p, LzShared& sh, const T* Q, T* w, long long n, int j,
+                                                 double bprev, double& are, double& aim) {
   constexpr bool C = sizeof(T) == 16;
-  const int rank = (int)(blockIdx.x % LZ_CTAS), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long slice = (n + LZ_CTAS - 1) / LZ_CTAS;
-  const long long lo = rank * slice, hi = lo + slice < n ? lo + slice : n;
-  const int act = hi - lo >= LZ_THREADS ? LZ_THREADS / 32 : hi > lo ? (int)(hi - lo + 31) / 32 : 1;
   const T* qj = Q + (long long)j * n;
   are = aim = 0.0;
-  for (long long e = lo + threadIdx.x; e < hi; e += LZ_THREADS) {
+  for (long long e = p.lo + threadIdx.x; e < p.hi; e += LZ_THREADS) {
     const T c = Sc<T>::mul(Sc<T>::conj(qj[e]), w[e]);
     are += Sc<T>::re(c);
     if (C) aim += Sc<T>::im(c);
   }
-  lz_cluster_sum<C, false>(are, aim, act, red, sums[0], sums[1]);
-  for (long long e = lo + threadIdx.x; e < hi; e += LZ_THREADS) {
+  lz_cluster_sum<C, false>(are, aim, p.act, sh.red, sh.sums[0], sh.sums[1]);
+  for (long long e = p.lo + threadIdx.x; e < p.hi; e += LZ_THREADS) {
     T x = Sc<T>::sub(w[e], Sc<T>::scale(qj[e], are));
     if (j > 0) x = Sc<T>::sub(x, Sc<T>::scale(qj[e - n], bprev));
     w[e] = x;
   }
+}
+
+// beta = |w| from this thread's share s of |w|^2, q_(j+1) = w / beta (next; also
+// into v where given; zero after a breakdown: dead, or beta below tol).  On
+// return dead is set after a breakdown.  The caller returns right after it.
+template <typename T>
+__device__ __forceinline__ void lz_cluster_next(const LzSlice& p, LzShared& sh, T* Q, const T* w, T* v, long long n,
+                                                int j, bool next, double s, double tol, bool& dead, double& beta) {
+  double inv = 0.0;
+  __syncthreads();
+  lz_cluster_sum<false, true>(s, inv, p.act, sh.red, sh.sums[2], sh.sums[3]);
+  beta = s;
+  dead = dead || !(beta >= tol);
+  if (next) {
+    if (dead) inv = 0.0;
+    T* qn = Q + (long long)(j + 1) * n;
+    for (long long e = p.lo + threadIdx.x; e < p.hi; e += LZ_THREADS) {
+      const T q = Sc<T>::scale(w[e], inv);
+      qn[e] = q;
+      if (v) v[e] = q;
+    }
+  }
+  lz_cluster_sync();   // the others have read this CTA's sums
+}
+
+// A whole step: alpha and the three-term update, w -= Q_nq Q_nq^H w, beta and
+// the next vector.  h: 2 LZ_CTAS rows of ldh elements.  Every CTA has the same
+// scalars, bit for bit.  The caller returns right after it.
+template <typename T>
+__device__ __forceinline__ void lz_cluster_step(T* Q, T* w, T* v, long long n, int j, int nq, bool next, double bprev,
+                                                T* h, int ldh, double tol, bool& dead, double& are, double& aim,
+                                                double& beta) {
+  __shared__ LzShared sh;
+  constexpr bool C = sizeof(T) == 16;
+  const LzSlice p(n);
+  const int rank = p.rank, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long lo = p.lo, hi = p.hi;
+  lz_cluster_alpha<T>(p, sh, Q, w, n, j, bprev, are, aim);
   T* hs = h + (long long)(LZ_CTAS + rank) * ldh;
   if (nq > 0) {
     __syncthreads();
@@ -151,7 +195,7 @@ __device__ __forceinline__ void lz_cluster_step(T* Q, T* w, T* v, long long n, i
     }
     __syncthreads();
   }
-  double s = 0.0, inv = 0.0;
+  double s = 0.0;
   for (long long e = lo + threadIdx.x; e < hi; e += LZ_THREADS) {
     T x = w[e];
     if (nq > 0) {
@@ -163,20 +207,7 @@ __device__ __forceinline__ void lz_cluster_step(T* Q, T* w, T* v, long long n, i
     }
     s += Sc<T>::abs2(x);
   }
-  __syncthreads();
-  lz_cluster_sum<false, true>(s, inv, act, red, sums[2], sums[3]);
-  beta = s;
-  dead = dead || !(beta >= tol);
-  if (next) {
-    if (dead) inv = 0.0;
-    T* qn = Q + (long long)(j + 1) * n;
-    for (long long e = lo + threadIdx.x; e < hi; e += LZ_THREADS) {
-      const T q = Sc<T>::scale(w[e], inv);
-      qn[e] = q;
-      if (v) v[e] = q;
-    }
-  }
-  lz_cluster_sync();   // the others have read this CTA's sums
+  lz_cluster_next<T>(p, sh, Q, w, v, n, j, next, s, tol, dead, beta);
 }
 
 }  // namespace dmrg
