@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
         const int p = tour(tid, ir), q = tour(JP - 1 - tid, ir);
         const T apq = a[p][q], app = a[p][p], aqq = a[q][q];
         T c = (T)1, s = (T)0, cm1 = (T)0;
-        if (fabs(apq) > fmax(rtol * sqrt(fabs(app * aqq)), floor_)) {
+        if (fabs(apq) > fmax(rtol * (sqrt(fabs(app)) * sqrt(fabs(aqq))), floor_)) {
           // symmetric Schur rotation (Golub & Van Loan, Alg. 8.4.1)
           const T tau = (aqq - app) / ((T)2 * apq);
           const T at = fabs(tau);
@@ -717,14 +717,20 @@ __global__ void syev_scale_kernel(const double* __restrict__ G, int np, long lon
   if (mx) atomicMax(scale, mx);
 }
 
-// d = diagonal of G, over the scale that syev_init_kernel gave G (norm null: 1)
+// d = diagonal of G; with the norm of A: nan where that holds one, and over the
+// scale that syev_init_kernel gave an FP32 matrix
 template <typename T>
 __global__ void syev_diag_kernel(const T* __restrict__ G, int np, const unsigned long long* __restrict__ norm,
                                  double* __restrict__ d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
-  const double v = (double)G[(long long)i * np + i];
-  d[i] = norm ? v / unit_scale(*norm) : v;
+  double v = (double)G[(long long)i * np + i];
+  if (norm) {
+    const unsigned long long b = *norm;
+    if (b > 0x7ff0000000000000ull) v = __longlong_as_double(0x7ff8000000000000ll);
+    else if (sizeof(T) == 4) v /= unit_scale(b);
+  }
+  d[i] = v;
 }
 
 // out[r * ldo + c] = V[r * np + perm[c]] for r < n, c < ncols (transposed:
@@ -816,7 +822,7 @@ int syev_gemm(SyevWs& ws, int tA, int m, int n, int k, const double* A, long lon
 }
 
 // Sorted eigenvalues to the host and the permutation to the workspace.
-// (G null: the eigenvalues are in ws.diag; norm: of G's scale, or null)
+// (G null: the eigenvalues are in ws.diag; norm: of A, or null)
 template <typename T>
 int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, double* w, cudaStream_t s) {
   const int np = ws.np;
@@ -826,7 +832,7 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
   }
   std::vector<double> d(n);
   DMRG_CUDA_TRY(cudaMemcpyAsync(d.data(), ws.diag, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-  if (sizeof(T) == 8 && n > 1 && ws.dig_bytes > 0) DMRG_TRY(dg_gave_up(ws.status, false, s));
+  if (sizeof(T) == 8 && ws.dig_bytes > 0) DMRG_TRY(dg_gave_up(ws.status, false, s));
   DMRG_CUDA_TRY(cudaStreamSynchronize(s));
   for (int i = 0; i < n; ++i)
     if (!(d[i] == d[i])) return DMRG_ERR_NAN;
@@ -1000,21 +1006,22 @@ int syev_impl(int n, const double* A, long long lda, double* w, int max_sweeps, 
   T* G = reinterpret_cast<T*>(ws.G);
   T* V = reinterpret_cast<T*>(ws.V);
   bool started = false, passed = false;
-  if (sizeof(T) == 8 && n > 1) {
+  // (a 2 x 2 matrix takes two FP64 sweeps, 216 us, where three passes take 250;
+  // from n = 3 on the passes are the faster, 260 us against 390)
+  if (sizeof(T) == 8 && n > 2) {
     int overflow = 0;
     DMRG_TRY(syev_passes(n, A, lda, ws, &done, &conv, &overflow, s));
     started = !overflow;   // else the FP64 sweeps begin with A itself
     passed = conv != 0;
   }
-  // FP32 squares what it rotates: of order 1, whatever A's scale
-  unsigned long long* norm = sizeof(T) == 4 ? ws.scale + 2 : nullptr;
+  unsigned long long* norm = ws.scale + 2;
   if (!conv && !started) {
     DMRG_CUDA_TRY(cudaMemsetAsync(ws.scale, 0, 3 * sizeof(unsigned long long), s));
-    if (norm) {
-      syev_norm_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(A, lda, n, norm);
-      DMRG_CHECK_LAUNCH();
-    }
-    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale, norm, ws.dd);
+    syev_norm_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(A, lda, n, norm);
+    DMRG_CHECK_LAUNCH();
+    // FP32 squares what it rotates: of order 1, whatever A's scale
+    syev_init_kernel<T><<<grid_for((long long)np * np), 256, 0, s>>>(A, lda, n, np, G, V, ws.scale,
+                                                                     sizeof(T) == 4 ? norm : nullptr, ws.dd);
     DMRG_CHECK_LAUNCH();
   }
   if (!conv) {
