@@ -162,14 +162,13 @@ __global__ void syev_init_kernel(const double* __restrict__ A, long long lda, in
 // index at tournament position pos (0..31) in inner round ir
 __device__ __forceinline__ int tour(int pos, int ir) { return pos == 0 ? 0 : 1 + (pos - 1 + ir) % (JP - 1); }
 
-template <typename T>
-__global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G, int np,
-                                                         const int* __restrict__ pr, T* __restrict__ R,
+__global__ void __launch_bounds__(256) syev_solve_kernel(const double* __restrict__ G, int np,
+                                                         const int* __restrict__ pr, double* __restrict__ R,
                                                          int* __restrict__ ident, int* __restrict__ flag,
                                                          const unsigned long long* __restrict__ scale) {
-  __shared__ T a[JP][JLD];
-  __shared__ T r[JP][JLD];
-  __shared__ T cs[JB], sn[JB], cm[JB];
+  __shared__ double a[JP][JLD];
+  __shared__ double r[JP][JLD];
+  __shared__ double cs[JB], sn[JB], cm[JB];
   __shared__ int pp[JB], qq[JB];
   const int pair = blockIdx.x;
   const int bi = pr[2 * pair], bj = pr[2 * pair + 1];
@@ -179,14 +178,14 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
     const unsigned long long b = *scale;
     memcpy(&sc, &b, sizeof(sc));
   }
-  const T floor_ = (T)(JacTol<T>::abs * sc);
-  const T rtol = (T)JacTol<T>::rel;
+  const double floor_ = JacTol<double>::abs * sc;
+  const double rtol = JacTol<double>::rel;
   for (int e = tid; e < JP * JP; e += blockDim.x) {
     const int i = e / JP, j = e - (e / JP) * JP;
     const int gi = i < JB ? bi * JB + i : bj * JB + i - JB;
     const int gj = j < JB ? bi * JB + j : bj * JB + j - JB;
     a[i][j] = G[(long long)gi * np + gj];
-    r[i][j] = (T)0;
+    r[i][j] = 0.0;
   }
   __syncthreads();
   int any = 0;
@@ -195,20 +194,20 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
     for (int ir = 0; ir < JP - 1; ++ir) {
       if (tid < JB) {
         const int p = tour(tid, ir), q = tour(JP - 1 - tid, ir);
-        const T apq = a[p][q], app = a[p][p], aqq = a[q][q];
-        T c = (T)1, s = (T)0, cm1 = (T)0;
+        const double apq = a[p][q], app = a[p][p], aqq = a[q][q];
+        double c = 1.0, s = 0.0, cm1 = 0.0;
         if (fabs(apq) > fmax(rtol * (sqrt(fabs(app)) * sqrt(fabs(aqq))), floor_)) {
           // symmetric Schur rotation (Golub & Van Loan, Alg. 8.4.1)
-          const T tau = (aqq - app) / ((T)2 * apq);
-          const T at = fabs(tau);
-          const T big = sizeof(T) == 8 ? (T)1e150 : (T)1e18;
-          T t = at < big ? (T)1 / (at + sqrt((T)1 + at * at)) : (T)0.5 / at;
+          const double tau = (aqq - app) / (2.0 * apq);
+          const double at = fabs(tau);
+          const double big = 1e150;
+          double t = at < big ? 1.0 / (at + sqrt(1.0 + at * at)) : 0.5 / at;
           t = copysign(t, tau);
-          const T u = sqrt((T)1 + t * t);
-          c = (T)1 / u;
-          cm1 = -t * t / (u * ((T)1 + u));   // c - 1 without cancellation
+          const double u = sqrt(1.0 + t * t);
+          c = 1.0 / u;
+          cm1 = -t * t / (u * (1.0 + u));   // c - 1 without cancellation
           s = t * c;
-          if (s != (T)0) rotated = 1;
+          if (s != 0.0) rotated = 1;
         }
         pp[tid] = p; qq[tid] = q; cs[tid] = c; sn[tid] = s; cm[tid] = cm1;
       }
@@ -217,22 +216,22 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
         const int ti = tid >> 4, tj = tid & 15;
         if (ti <= tj) {
           const int pi = pp[ti], qi = qq[ti], pj = pp[tj], qj = qq[tj];
-          const T ci = cs[ti], si = sn[ti], cj = cs[tj], sj = sn[tj];
+          const double ci = cs[ti], si = sn[ti], cj = cs[tj], sj = sn[tj];
           if (ti == tj) {
-            if (si != (T)0) {
-              const T t = si / ci;
-              const T apq = a[pi][qi];
+            if (si != 0.0) {
+              const double t = si / ci;
+              const double apq = a[pi][qi];
               a[pi][pi] -= t * apq;
               a[qi][qi] += t * apq;
-              a[pi][qi] = (T)0;
-              a[qi][pi] = (T)0;
+              a[pi][qi] = 0.0;
+              a[qi][pi] = 0.0;
             }
-          } else if (si != (T)0 || sj != (T)0) {
-            const T x00 = a[pi][pj], x01 = a[pi][qj], x10 = a[qi][pj], x11 = a[qi][qj];
-            const T y00 = ci * x00 - si * x10, y01 = ci * x01 - si * x11;
-            const T y10 = si * x00 + ci * x10, y11 = si * x01 + ci * x11;
-            const T z00 = cj * y00 - sj * y01, z01 = sj * y00 + cj * y01;
-            const T z10 = cj * y10 - sj * y11, z11 = sj * y10 + cj * y11;
+          } else if (si != 0.0 || sj != 0.0) {
+            const double x00 = a[pi][pj], x01 = a[pi][qj], x10 = a[qi][pj], x11 = a[qi][qj];
+            const double y00 = ci * x00 - si * x10, y01 = ci * x01 - si * x11;
+            const double y10 = si * x00 + ci * x10, y11 = si * x01 + ci * x11;
+            const double z00 = cj * y00 - sj * y01, z01 = sj * y00 + cj * y01;
+            const double z10 = cj * y10 - sj * y11, z11 = sj * y10 + cj * y11;
             a[pi][pj] = z00; a[pi][qj] = z01; a[qi][pj] = z10; a[qi][qj] = z11;
             a[pj][pi] = z00; a[qj][pi] = z01; a[pj][qi] = z10; a[qj][qi] = z11;
           }
@@ -240,15 +239,15 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
         // D <- (D + I) J - I = D J + (J - I) on columns p, q of pair
         // (tid & 15), rows tid >> 4 and +16
         const int pj = tid & 15;
-        const T s = sn[pj], cm1 = cm[pj];
-        if (s != (T)0) {
+        const double s = sn[pj], cm1 = cm[pj];
+        if (s != 0.0) {
           const int p = pp[pj], q = qq[pj];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int rr = (tid >> 4) + 16 * h;
-            const T u = r[rr][p], v = r[rr][q];
-            T np_ = fma(cm1, u, u) - s * v;
-            T nq_ = fma(s, u, fma(cm1, v, v));
+            const double u = r[rr][p], v = r[rr][q];
+            double np_ = fma(cm1, u, u) - s * v;
+            double nq_ = fma(s, u, fma(cm1, v, v));
             if (rr == p) { np_ += cm1; nq_ += s; }
             if (rr == q) { np_ -= s; nq_ += cm1; }
             r[rr][p] = np_;
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(256) syev_solve_kernel(const T* __restrict__ G
     if (!__syncthreads_or(rotated)) break;
     any = 1;
   }
-  T* Rp = R + (size_t)pair * JP * JP;
+  double* Rp = R + (size_t)pair * JP * JP;
   for (int e = tid; e < JP * JP; e += blockDim.x) Rp[e] = r[e / JP][e % JP];
   if (tid == 0) {
     ident[pair] = any ? 0 : 1;
@@ -775,7 +774,7 @@ void tournament(int nb, std::vector<int>& out) {
 // apply's places).  Pointers of both kernels are not __restrict__, which would
 // let the compiler move loads up past the wait.
 inline int solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, double, double, cudaStream_t s) {
-  syev_solve_kernel<double><<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
+  syev_solve_kernel<<<ws.npair, 256, 0, s>>>(G, ws.np, pr, R, ws.ident, ws.flag, ws.scale);
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
