@@ -328,7 +328,7 @@ __device__ __forceinline__ float2 add_hl(float2 a, float x) {
 // with a thread for each of the 256 blocks and all of D in one CTA 13.2, with
 // four CTAs of 128 threads 16.6 (a warp then has two blocks in turn).
 __global__ void __launch_bounds__(256) __cluster_dims__(2, 1, 1)
-syev_solve32_kernel(const float* G, int np, const int* pr, float* R,
+syev_solve32_kernel(float* G, int np, const int* pr, float* R,
                     int* ident, int* flag, const unsigned long long* scale,
                     float2* dd, float rel, float abs_) {
   constexpr int LD = JP + 2, H = JP / 2;   // LD even: strides LD + 1 and LD - 1 across lanes
@@ -409,6 +409,19 @@ syev_solve32_kernel(const float* G, int np, const int* pr, float* R,
   float* Rp = R + (size_t)pair * JP * JP + sub * H * JP;
   for (int e = tid; e < H * JP; e += 256) Rp[e] = r[e / JP][e % JP];
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (any) {
+    // the pair's own block: the apply would form its off-diagonals from the
+    // diagonal's FP32 values, which loses them where those agree to six digits
+    // and more (eigenvalues 1 + 1e-6 x, n = 100: 17.7 ms, ended by FP64 sweeps;
+    // 1.6 with this)
+    const float* x = a[(JP - 1) & 1];
+    for (int e = sub * (JP * JP / 2) + tid; e < (sub + 1) * (JP * JP / 2); e += 256) {
+      const int i = e / JP, j = e % JP;
+      const int gi = i < JB ? bi * JB + i : bj * JB + i - JB;
+      const int gj = j < JB ? bi * JB + j : bj * JB + j - JB;
+      G[(long long)gi * np + gj] = i == j ? dg[(JP - 1) & 1][i].x : x[i * LD + j];
+    }
+  }
   if (sub == 0) {
     if (tid < JP) dd[tid < JB ? bi * JB + tid : bj * JB + tid - JB] = dg[(JP - 1) & 1][tid];
     if (tid == 0) {
@@ -524,8 +537,9 @@ __global__ void __launch_bounds__(256) syev_small32_kernel(const double* __restr
 
 __device__ __forceinline__ int pair_index(int b0, int b1, int l) { return l < JB ? b0 * JB + l : b1 * JB + l - JB; }
 
-// G <- P^T G P on blocks (X, Y), X <= Y (grid part 1, npair^2 CTAs, the
-// lower triangle exits) and V <- V P on 32-row panels (grid part 2)
+// G <- P^T G P on blocks (X, Y), X <= Y (FP32: X < Y, the solve writes the
+// pair's own block; grid part 1, npair^2 CTAs, the lower triangle exits) and
+// V <- V P on 32-row panels (grid part 2)
 template <typename T>
 __global__ void __launch_bounds__(256) syev_apply_kernel(T* G, T* V, int np,
                                                          const int* pr, const T* R,
@@ -541,7 +555,7 @@ __global__ void __launch_bounds__(256) syev_apply_kernel(T* G, T* V, int np,
   const int nG = npair * npair;
   if (b < nG) {
     const int X = b / npair, Y = b - (b / npair) * npair;
-    if (X > Y) return;
+    if (X > Y || (sizeof(T) == 4 && X == Y)) return;
     const int idX = ident[X], idY = ident[Y];
     if (idX && idY) return;
     const int xb0 = pr[2 * X], xb1 = pr[2 * X + 1], yb0 = pr[2 * Y], yb1 = pr[2 * Y + 1];
@@ -778,7 +792,7 @@ inline int solve_launch(SyevWs& ws, const double* G, const int* pr, double* R, d
   DMRG_CHECK_LAUNCH();
   return DMRG_OK;
 }
-inline int solve_launch(SyevWs& ws, const float* G, const int* pr, float* R, double rel, double abs_, cudaStream_t s) {
+inline int solve_launch(SyevWs& ws, float* G, const int* pr, float* R, double rel, double abs_, cudaStream_t s) {
   return launch_after(syev_solve32_kernel, dim3(2u * (unsigned)ws.npair), 256, s, G, ws.np, pr, R, ws.ident, ws.flag, ws.scale, ws.dd,
                       (float)rel, (float)abs_);
 }
