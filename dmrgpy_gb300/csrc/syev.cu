@@ -864,13 +864,18 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
 // Newton-Schulz steps, G = V^T A V in FP64.  The first pass leaves what FP32
 // cannot see, about 1e-7 of the largest eigenvalue, so it stops there
 // (PASS0_ABS); the later ones work on that remainder, which FP32 holds
-// elementwise (1e-15 floor, one sweep where all rotations are small).  Up to
+// elementwise (one sweep where all rotations are small), down to PASS_ABS of
+// the largest element: what is left between the many eigenvalues of a steep
+// spectrum that are below the FP64 sweeps' own floor of 1e-15 adds up (n = 200,
+// eigenvalues from 1 to 1e-26: errors up to 6.2e-15, together 5.9e-14, with that
+// floor, 1.1e-15 and 6.8e-15 with this one, 1.2e-15 and 8.8e-15 by FP64 sweeps;
+// 6.5 -> 7.0 ms).  Up to
 // np = 64 a pass's sweeps are one launch.  Done
 // when every off-diagonal is within PASS_DONE of the FP64 sweeps' threshold:
 // three or four passes, about twenty FP32 sweeps, against ten to twenty FP64
 // sweeps of a cold start (n = 200: 41 ms).  *done_: sweeps run.
 constexpr int MAX_PASSES = 8;
-constexpr double PASS0_ABS = 1e-6;
+constexpr double PASS0_ABS = 1e-6, PASS_ABS = 1e-17;
 constexpr float PASS_DONE = 3.f;
 
 // *overflow: a pass was not finite, where A holds an infinity or elements so
@@ -901,7 +906,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     // the pass's rotation Q (FP64) into ws.G; into ws.T where the kernel's
     // CTAs read ws.G as they please
     double* Q = np <= 64 && p > 0 ? ws.T : ws.G;
-    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : JacTol<double>::abs;
+    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : PASS_ABS;
     const int most = p == 0 ? 12 : 8;
     const double* src0 = p == 0 ? A : ws.G;
     const long long ld0 = p == 0 ? lda : np;
