@@ -869,8 +869,10 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
 // spectrum that are below the FP64 sweeps' own floor of 1e-15 adds up (n = 200,
 // eigenvalues from 1 to 1e-26: errors up to 6.2e-15, together 5.9e-14, with that
 // floor, 1.1e-15 and 6.8e-15 with this one, 1.2e-15 and 8.8e-15 by FP64 sweeps;
-// 6.5 -> 7.0 ms).  Up to
-// np = 64 a pass's sweeps are one launch.  Done
+// 6.5 -> 7.0 ms).  Up to np = 64 a pass's sweeps are one launch, and of the
+// three passes that run there the last alone goes that far: where eigenvalues
+// are rounding (a rank of 16 at n = 64) the second would rotate what its own
+// products replace (780 us, 640 without).  Done
 // when every off-diagonal is within PASS_DONE of the FP64 sweeps' threshold:
 // three or four passes, about twenty FP32 sweeps, against ten to twenty FP64
 // sweeps of a cold start (n = 200: 41 ms).  *done_: sweeps run.
@@ -906,7 +908,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     // the pass's rotation Q (FP64) into ws.G; into ws.T where the kernel's
     // CTAs read ws.G as they please
     double* Q = np <= 64 && p > 0 ? ws.T : ws.G;
-    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : PASS_ABS;
+    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : p == 1 && np <= 64 ? JacTol<double>::abs : PASS_ABS;
     const int most = p == 0 ? 12 : 8;
     const double* src0 = p == 0 ? A : ws.G;
     const long long ld0 = p == 0 ? lda : np;
