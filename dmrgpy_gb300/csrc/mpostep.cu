@@ -12,8 +12,9 @@
 // Apply: a warp owns 32 consecutive inner indices (one bond leg) of one outer
 // index and every eighth output row; the lists are read as warp
 // broadcasts, the inputs as 256-byte segments which the CTA's eight warps
-// share through L1.  Where that makes fewer than two CTAs per SM the rows are
-// spread over several (grid.z): a CTA's chain of rows x list entries is what a
+// share through L1.  Where that makes fewer than two CTAs per SM and the lists
+// may be long (rows x columns 2048 and more) the rows are spread over several
+// CTAs (grid.z): a CTA's chain of rows x list entries is what a
 // narrow bond waits for (environment of chi = 4, d = 3, w = 100, dense: 1427 us
 // with all 300 rows in one CTA, 105 spread).  Bound: FP64 FMAs (non-zeros per
 // output column) and the HBM traffic of one read and one write of the
@@ -167,9 +168,11 @@ int mpo_apply(const MpoShape& sh, const void* list, const T* in, T* out, long lo
   const int* cnt = static_cast<const int*>(list);
   const Entry<T>* ent = reinterpret_cast<const Entry<T>*>(static_cast<const char*>(list) + cnt_bytes(sh));
   if ((inner + 31) / 32 > 0x7fffffffLL) return DMRG_ERR_ARG;
-  // few CTAs: the rows over several, up to two CTAs per SM
+  // few CTAs with long lists: the rows over several, up to two CTAs per SM
   const long long gx = (inner + 31) / 32, gy = outer < 65535 ? outer : 65535, most = 2 * 152;
-  const long long gz = gx * gy >= most ? 1 : std::min<long long>((d.rows + 7) / 8, (most + gx * gy - 1) / (gx * gy));
+  const long long gz = gx * gy >= most || (long long)d.rows * d.cols < 2048
+                           ? 1
+                           : std::min<long long>((d.rows + 7) / 8, (most + gx * gy - 1) / (gx * gy));
   const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)gz);
   return launch_after(mpo_apply_kernel<T>, grid, 256, s, d.rows, d.cols, cnt, ent, in, out, outer, inner);
 }
