@@ -93,6 +93,7 @@ class Engine:
                                   device=self.device) for w in W]
         self.n = len(W)
         self.ws = Workspace(self.device)
+        self.ws_limit = float("inf")     # bytes that the device refused
         self.edge = torch.ones((1, 1, 1), dtype=self.tdtype, device=self.device)
         self.krylov_budget = krylov_budget_bytes
         self.stats = SweepStats()
@@ -163,12 +164,42 @@ class Engine:
         w = L.shape[1]
         return self._heff(0, L, None, None, R, cl, 1, 1, cr, w, w, w)
 
+    def _scratch(self, need, least, *args):
+        """Workspace of `need` bytes or, where the device has no room for
+        the operands of digit products beside what is resident, of
+        least(*args): the call then runs on the FP64 pipe."""
+        if need < self.ws_limit:
+            try:
+                return self.ws.get(need)
+            except _torch().cuda.OutOfMemoryError:
+                if least(*args) >= need:
+                    raise
+                self.ws_limit = need
+        return self.ws.get(min(need, least(*args)))
+
+    def _heff_least(self, h, need):
+        """Bytes of the two intermediates that an FP64 operator runs in."""
+        if h.precision != _lib.PREC_FP64:
+            return need
+        cl, cr, d1, d2, wl, wm, wr = h.chil, h.chir, h.d1, h.d2, h.wl, h.wm, h.wr
+        if h.kind == 2:
+            p, q = cl * d1 * d2 * max(wl, wr) * cr, cl * d1 * wm * d2 * cr
+        elif h.kind == 1:
+            p, q = cl * wl * d1 * cr, cl * d1 * wr * cr
+        else:
+            p, q = cl * wl * cr, 0
+        return sum((n * self.esize + 255) // 256 * 256 for n in (p, q))
+
+    def _krylov_least(self, h, need):
+        heff = self.lib.dmrg_heff_workspace_bytes(ctypes.byref(h))
+        return need - heff + self._heff_least(h, heff)
+
     def apply(self, h, x):
         """y = H_eff x (one matvec; used by tests and the benchmark)."""
         torch = _torch()
         y = torch.empty_like(x)
         need = self.lib.dmrg_heff_workspace_bytes(ctypes.byref(h))
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, self._heff_least, h, need)
         _lib.check("dmrg_heff_apply", self.lib.dmrg_heff_apply(ctypes.byref(h), x.data_ptr(), y.data_ptr(),
                                                                  ptr, size, self.stream))
         return y
@@ -182,7 +213,7 @@ class Engine:
         normalised eigenvector."""
         k = self._kcap(x.numel(), max(niter, LANCZOS_NITER_FLOOR))
         need = self.lib.dmrg_lanczos_workspace_bytes(ctypes.byref(h), k)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, self._krylov_least, h, need)
         e = ctypes.c_double(0.0)
         it = ctypes.c_int(0)
         tol = self.lanczos_tol_tf32 if h.precision == _lib.PREC_TF32X3 else LANCZOS_TOL
@@ -193,7 +224,7 @@ class Engine:
     def expm(self, h, x, coeff, niter):
         k = self._kcap(x.numel(), niter)
         need = self.lib.dmrg_expm_workspace_bytes(ctypes.byref(h), k)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, self._krylov_least, h, need)
         it = ctypes.c_int(0)
         coeff = complex(coeff)
         _lib.check("dmrg_krylov_expm", self.lib.dmrg_krylov_expm(
@@ -210,7 +241,7 @@ class Engine:
         C = torch.empty((m, n), dtype=self.tdtype, device=self.device)
         prec = self.prec_for(min(m, n), k)
         need = self.lib.dmrg_gemm_workspace_bytes(self.cdtype, prec, m, k, n)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, lambda: 0 if prec == _lib.PREC_FP64 else need)
         _lib.check("dmrg_gemm", self.lib.dmrg_gemm(self.cdtype, prec, m, k, n, A2.data_ptr(), B2.data_ptr(),
                                                    C.data_ptr(), ptr, size, self.stream))
         return C
@@ -307,7 +338,7 @@ class Engine:
         out = torch.empty((cr, wr, cr), dtype=self.tdtype, device=self.device)
         prec = self.prec_for(cl, cr) if fp64 is False else _lib.PREC_FP64
         need = self.lib.dmrg_env_workspace_bytes(self.cdtype, prec, cl, d, cr, wl, wr)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, lambda: self.esize * cl * d * cr * (wl + wr) if prec == _lib.PREC_FP64 else need)
         _lib.check("dmrg_env_extend_left", self.lib.dmrg_env_extend_left(
             self.cdtype, prec, cl, d, cr, wl, wr, L.data_ptr(), W.data_ptr(), A.data_ptr(), out.data_ptr(),
             ptr, size, self.stream))
@@ -320,7 +351,7 @@ class Engine:
         out = torch.empty((cl, wl, cl), dtype=self.tdtype, device=self.device)
         prec = self.prec_for(cl, cr) if fp64 is False else _lib.PREC_FP64
         need = self.lib.dmrg_env_workspace_bytes(self.cdtype, prec, cl, d, cr, wl, wr)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, lambda: self.esize * cl * d * cr * (wl + wr) if prec == _lib.PREC_FP64 else need)
         _lib.check("dmrg_env_extend_right", self.lib.dmrg_env_extend_right(
             self.cdtype, prec, cl, d, cr, wl, wr, R.data_ptr(), W.data_ptr(), B.data_ptr(), out.data_ptr(),
             ptr, size, self.stream))
@@ -348,7 +379,7 @@ class Engine:
         shape = (crb, wr, crk) if side == 0 else (clb, wl, clk)
         out = torch.empty(shape, dtype=self.tdtype, device=self.device)
         need = self.lib.dmrg_env_mixed_workspace_bytes(side, self.cdtype, clb, crb, clk, crk, d, wl, wr)
-        ptr, size = self.ws.get(need)
+        ptr, size = self._scratch(need, lambda: self.esize * d * (wl + wr) * (clb * crk if side == 0 else crb * clk))
         _lib.check("dmrg_env_extend_mixed", self.lib.dmrg_env_extend_mixed(
             side, self.cdtype, clb, crb, clk, crk, d, wl, wr, E.data_ptr(), W.data_ptr(), B.data_ptr(),
             A.data_ptr(), out.data_ptr(), ptr, size, self.stream))
