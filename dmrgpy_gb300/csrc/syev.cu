@@ -864,12 +864,15 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
 // Newton-Schulz steps, G = V^T A V in FP64.  The first pass leaves what FP32
 // cannot see, about 1e-7 of the largest eigenvalue, so it stops there
 // (PASS0_ABS); the later ones work on that remainder, which FP32 holds
-// elementwise (one sweep where all rotations are small), down to PASS_ABS of
+// elementwise (one sweep where all rotations are small), down to pass_abs of
 // the largest element: what is left between the many eigenvalues of a steep
 // spectrum that are below the FP64 sweeps' own floor of 1e-15 adds up (n = 200,
 // eigenvalues from 1 to 1e-26: errors up to 6.2e-15, together 5.9e-14, with that
-// floor, 1.1e-15 and 6.8e-15 with this one, 1.2e-15 and 8.8e-15 by FP64 sweeps;
-// 6.5 -> 7.0 ms).  Up to np = 64 a pass's sweeps are one launch, and of the
+// floor, 1.1e-15 and 6.8e-15 with 1e-17, 1.2e-15 and 8.8e-15 by FP64 sweeps;
+// 6.5 -> 7.0 ms).  From 256 on, where sweeps are long (n = 512: 19.9 ms, with 1e-17
+// 22.6; every Ritz problem of a chi = 1024 sweep 20% more), it is 1e-15: errors
+// up to 1.3e-14, together 2.6e-13 there, as FP64 sweeps after an FP32 start
+// leave.  Up to np = 64 a pass's sweeps are one launch, and of the
 // three passes that run there the last alone goes that far: where eigenvalues
 // are rounding (a rank of 16 at n = 64) the second would rotate what its own
 // products replace (780 us, 640 without).  Done
@@ -877,7 +880,8 @@ int syev_finish(int n, SyevWs& ws, const T* G, const unsigned long long* norm, d
 // three or four passes, about twenty FP32 sweeps, against ten to twenty FP64
 // sweeps of a cold start (n = 200: 41 ms).  *done_: sweeps run.
 constexpr int MAX_PASSES = 8;
-constexpr double PASS0_ABS = 1e-6, PASS_ABS = 1e-17;
+constexpr double PASS0_ABS = 1e-6;
+inline double pass_abs(int n) { return n < 256 ? 1e-17 : JacTol<double>::abs; }
 constexpr float PASS_DONE = 3.f;
 
 // *overflow: a pass was not finite, where A holds an infinity or elements so
@@ -908,7 +912,7 @@ int syev_passes(int n, const double* A, long long lda, SyevWs& ws, int* done_, i
     // the pass's rotation Q (FP64) into ws.G; into ws.T where the kernel's
     // CTAs read ws.G as they please
     double* Q = np <= 64 && p > 0 ? ws.T : ws.G;
-    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : p == 1 && np <= 64 ? JacTol<double>::abs : PASS_ABS;
+    const double rel = p == 0 ? 0.0 : JacTol<double>::rel, abs_ = p == 0 ? PASS0_ABS : p == 1 && np <= 64 ? JacTol<double>::abs : pass_abs(n);
     const int most = p == 0 ? 12 : 8;
     const double* src0 = p == 0 ? A : ws.G;
     const long long ld0 = p == 0 ? lda : np;
